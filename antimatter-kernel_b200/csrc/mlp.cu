@@ -12,9 +12,12 @@
 // layer is tracked by tcgen05.commit on an mbarrier whose waits are
 // bounded (a timeout sets an error flag and the kernel returns).
 //
-// Training (forward with stored activations, backward, Adam) runs in FP32
-// on the CUDA cores with the same BF16-rounded weights: it is small next to
-// inference and is checked against an FP64 CPU implementation.
+// Training runs in FP32 on the CUDA cores with the same BF16-rounded
+// weights, two kernels per step: mlp_backprop_kernel (forward, loss, backward
+// and weight gradients of a tile of samples, everything in shared memory)
+// and mlp_update_kernel (the tiles' gradients summed in a fixed order, Adam).
+// It is checked against an FP64 CPU implementation.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -47,9 +50,10 @@ constexpr int kMlpParams = kOffB4 + kMlpOut;
 struct Mlp {
   DevBuf master, grad, adam_m, adam_v;  // FP32, kMlpParams each
   DevBuf packed;                         // BF16 weights in the tensor-core smem image + FP32 biases
+  DevBuf train;                          // BF16 weights in the training kernels' layouts (TrainImg)
   DevBuf status;                         // int error flag
   long adam_step = 0;
-  bool packed_valid = false;
+  bool packed_valid = false, train_valid = false;
   bool initialized = false;
 };
 
@@ -233,87 +237,319 @@ __global__ void mlp_pack_kernel(const float* __restrict__ p, unsigned char* __re
 }
 
 // ---------------------------------------------------------------- training (FP32)
-__device__ __forceinline__ float bf16r(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
+// BF16 weights for training, [contraction index][output]: W1..W3 transposed
+// for the forward pass, W4 as it is (its rows are its three outputs), then W3
+// and W2 as they are for the backward pass.
+constexpr int kTrW1 = 0;                                     // [35][128]
+constexpr int kTrW2 = kTrW1 + kMlpIn * kMlpHidden;           // [128][128]
+constexpr int kTrW3 = kTrW2 + kMlpHidden * kMlpHidden;
+constexpr int kTrW4 = kTrW3 + kMlpHidden * kMlpHidden;       // [3][128]
+constexpr int kTrFwd = kTrW4 + kMlpOut * kMlpHidden;         // elements the forward pass stages
+constexpr int kTrBack = kTrFwd;                              // W3, W2 [out][in]
+constexpr int kTrElems = kTrBack + 2 * kMlpHidden * kMlpHidden;
+static_assert(kTrW2 % 8 == 0 && kTrFwd % 8 == 0 && kTrElems % 8 == 0, "16-byte staging copies");
 
-// Z = W_bf16 X + b for a batch: one thread per (sample, output unit).
-__global__ void mlp_dense_kernel(const float* __restrict__ p, int w_off, int b_off, int in, int out,
-                                 const float* __restrict__ xin, long batch, float* __restrict__ z,
-                                 float* __restrict__ h, bool act) {
-  const long t = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
-  if (t >= batch * out) return;
-  const long s = t / out;
-  const int o = static_cast<int>(t - s * out);
-  const float* w = p + w_off + o * in;
-  const float* xi = xin + s * in;
-  float acc = 0.f;
-  for (int k = 0; k < in; ++k) acc = fmaf(bf16r(w[k]), xi[k], acc);
-  acc += p[b_off + o];
-  z[t] = acc;
-  if (h) h[t] = act ? gelu(acc) : acc;
-}
-
-// dX[s][k] = sum_o dZ[s][o] W[o][k]
-__global__ void mlp_back_input_kernel(const float* __restrict__ p, int w_off, int in, int out,
-                                      const float* __restrict__ dz, long batch, const float* __restrict__ zprev,
-                                      float* __restrict__ dzprev) {
-  const long t = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
-  if (t >= batch * in) return;
-  const long s = t / in;
-  const int k = static_cast<int>(t - s * in);
-  float acc = 0.f;
-  for (int o = 0; o < out; ++o) acc = fmaf(dz[s * out + o], bf16r(p[w_off + o * in + k]), acc);
-  dzprev[t] = acc * gelu_grad(zprev[t]);
-}
-
-// dW[o][k] = sum_s dZ[s][o] X[s][k], db[o] = sum_s dZ[s][o] (fixed summation order)
-__global__ void mlp_back_weight_kernel(int w_off, int b_off, int in, int out, const float* __restrict__ dz,
-                                       const float* __restrict__ xin, long batch, float* __restrict__ g) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < out * in) {
-    const int o = t / in, k = t % in;
-    float acc = 0.f;
-    for (long s = 0; s < batch; ++s) acc = fmaf(dz[s * out + o], xin[s * in + k], acc);
-    g[w_off + t] = acc;
-  }
-  if (t < out) {
-    float acc = 0.f;
-    for (long s = 0; s < batch; ++s) acc += dz[s * out + t];
-    g[b_off + t] = acc;
+// Parameter i of the flat master vector into the training image (biases are
+// read from the masters).
+__device__ __forceinline__ void train_image_put(int i, float v, __nv_bfloat16* __restrict__ img) {
+  const __nv_bfloat16 b = __float2bfloat16_rn(v);
+  if (i < kOffB1) {
+    img[kTrW1 + (i % kMlpIn) * kMlpHidden + i / kMlpIn] = b;
+  } else if (i >= kOffW2 && i < kOffB2) {
+    const int e = i - kOffW2, o = e / kMlpHidden, k = e % kMlpHidden;
+    img[kTrW2 + k * kMlpHidden + o] = b;
+    img[kTrBack + kMlpHidden * kMlpHidden + e] = b;
+  } else if (i >= kOffW3 && i < kOffB3) {
+    const int e = i - kOffW3, o = e / kMlpHidden, k = e % kMlpHidden;
+    img[kTrW3 + k * kMlpHidden + o] = b;
+    img[kTrBack + e] = b;
+  } else if (i >= kOffW4 && i < kOffB4) {
+    img[kTrW4 + i - kOffW4] = b;
   }
 }
 
-// loss = mean over batch and outputs of (y - target)^2; dY = 2 (y - target) / (batch * 3)
-__global__ void mlp_loss_kernel(const float* __restrict__ yhat, const float* __restrict__ target, long batch,
-                                float* __restrict__ dy, float* __restrict__ loss_part) {
-  __shared__ float sh[256];
-  float acc = 0.f;
-  const long total = batch * kMlpOut;
-  for (long t = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; t < total;
-       t += static_cast<long>(gridDim.x) * blockDim.x) {
-    const float d = yhat[t] - target[t];
-    dy[t] = 2.f * d / static_cast<float>(total);
-    acc += d * d;
-  }
-  sh[threadIdx.x] = acc;
-  __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
-    if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) loss_part[blockIdx.x] = sh[0];
-}
-
-__global__ void mlp_adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
-                                float* __restrict__ v, int n, float lr, float b1, float b2, float eps, float c1,
-                                float c2) {
+__global__ void mlp_train_pack_kernel(const float* __restrict__ p, __nv_bfloat16* __restrict__ img) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float gi = g[i];
-  const float mi = b1 * m[i] + (1.f - b1) * gi;
-  const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+  if (i < kMlpParams) train_image_put(i, p[i], img);
+}
+
+// Forward, loss, backward and weight gradients of tiles of T samples, one
+// tile per CTA (more tiles than SMs: a CTA walks them and adds to its own
+// partial gradient). Everything of a tile lives in shared memory: activations
+// h1-h3, the GELU derivatives (turned into the layer gradients dz in place)
+// and the inputs, stored [unit][sample] with a row pitch of T + 4 floats, so
+// that 16-byte reads of eight different rows or of eight sample groups touch
+// 32 distinct banks; the weights as BF16 (exact: they are used rounded to
+// BF16), re-staged in the other orientation for the backward pass.
+//   layer products   a thread computes 4 samples x T/8 outputs, the
+//                    contraction in ascending order as one FMA chain
+//   weight gradients a thread owns 8 x 8 of the 128 x 128 (rows 16 apart),
+//                    summed over the tile's samples in order
+// A CTA writes its gradient to part[blockIdx.x]; mlp_update_kernel adds the
+// CTAs' parts in order, so a step is deterministic.
+// The previous form ran one thread per gradient element over the whole batch
+// (64 CTAs of a 4,096-long serial chain per layer: 5.2 ms of the 5.8 ms that
+// the step's kernels took one by one, 3.4 ms a step overlapped). A
+// 4,096-sample step is 2 x 3 x 37,632 x 4,096 flop (0.92 GFLOP, 13 us at the
+// FP32 rate); it takes 54 us with the update, bound by the latency of the
+// layers' chains at 8 warps per SM.
+constexpr int kBpThreads = 256;
+template <int T>
+struct BpSmem {
+  static constexpr int kPitch = T + 4;
+  static constexpr int kRow = kMlpHidden * kPitch;  // one [128][pitch] array
+  static constexpr int kX = 6 * kRow;               // inputs [35][pitch]
+  static constexpr int kDy = kX + kMlpIn * kPitch;  // dY [3][pitch]
+  static constexpr int kRed = kDy + kMlpOut * kPitch;  // reduction words
+  static constexpr int kFloats = kRed + 8;
+  static constexpr size_t kBytes = kFloats * sizeof(float) + kTrFwd * sizeof(__nv_bfloat16);
+  static_assert(kFloats % 4 == 0 && kBytes <= 227 * 1024, "training tile shared memory");
+};
+
+// acc[j][c] = sum_r in[r][4 sg + c] * w[r][out0 + j] over the rows r in order
+template <int T, int kOutPer>
+__device__ __forceinline__ void bp_product(const float* __restrict__ in, const __nv_bfloat16* __restrict__ w, int rows,
+                                           int sg, int out0, float (&acc)[kOutPer][4]) {
+  constexpr int kPitch = T + 4;
+#pragma unroll
+  for (int j = 0; j < kOutPer; ++j)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) acc[j][c] = 0.f;
+#pragma unroll 4
+  for (int r = 0; r < rows; ++r) {
+    const float4 x = *reinterpret_cast<const float4*>(in + r * kPitch + 4 * sg);
+    float wv[kOutPer];
+    if constexpr (kOutPer == 4) {
+      const uint2 u = *reinterpret_cast<const uint2*>(w + r * kMlpHidden + out0);
+      wv[0] = __uint_as_float(u.x << 16);
+      wv[1] = __uint_as_float(u.x & 0xffff0000u);
+      wv[2] = __uint_as_float(u.y << 16);
+      wv[3] = __uint_as_float(u.y & 0xffff0000u);
+    } else if constexpr (kOutPer == 2) {
+      const uint32_t u = *reinterpret_cast<const uint32_t*>(w + r * kMlpHidden + out0);
+      wv[0] = __uint_as_float(u << 16);
+      wv[1] = __uint_as_float(u & 0xffff0000u);
+    } else {
+#pragma unroll
+      for (int j = 0; j < kOutPer; ++j) wv[j] = __bfloat162float(w[r * kMlpHidden + out0 + j]);
+    }
+#pragma unroll
+    for (int j = 0; j < kOutPer; ++j) {
+      acc[j][0] = fmaf(wv[j], x.x, acc[j][0]);
+      acc[j][1] = fmaf(wv[j], x.y, acc[j][1]);
+      acc[j][2] = fmaf(wv[j], x.z, acc[j][2]);
+      acc[j][3] = fmaf(wv[j], x.w, acc[j][3]);
+    }
+  }
+}
+
+// g[w_off + o * in + k] (+)= sum_s dz[o][s] h[k][s] for the 128 x kIn matrix,
+// g[b_off + o] (+)= sum_s dz[o][s]
+template <int T, int kIn>
+__device__ __forceinline__ void bp_weight_grad(const float* __restrict__ dz, const float* __restrict__ h, int w_off,
+                                               int b_off, bool add, float* __restrict__ g) {
+  constexpr int kPitch = T + 4, kJ = (kIn + 15) / 16;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  float acc[8][kJ];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < kJ; ++j) acc[i][j] = 0.f;
+#pragma unroll 1
+  for (int s = 0; s < T; s += 4) {
+    float4 a[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const float4*>(dz + (ty + 16 * i) * kPitch + s);
+#pragma unroll
+    for (int j = 0; j < kJ; ++j) {
+      const int k = tx + 16 * j;
+      const float4 b = k < kIn ? *reinterpret_cast<const float4*>(h + k * kPitch + s) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        acc[i][j] = fmaf(a[i].x, b.x, acc[i][j]);
+        acc[i][j] = fmaf(a[i].y, b.y, acc[i][j]);
+        acc[i][j] = fmaf(a[i].z, b.z, acc[i][j]);
+        acc[i][j] = fmaf(a[i].w, b.w, acc[i][j]);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < kJ; ++j) {
+      const int k = tx + 16 * j;
+      if (k >= kIn) continue;
+      float* dst = g + w_off + (ty + 16 * i) * kIn + k;
+      *dst = add ? *dst + acc[i][j] : acc[i][j];
+    }
+  if (threadIdx.x < kMlpHidden) {
+    float b = 0.f;
+    for (int s = 0; s < T; s += 4) {
+      const float4 v = *reinterpret_cast<const float4*>(dz + threadIdx.x * kPitch + s);
+      b += v.x;
+      b += v.y;
+      b += v.z;
+      b += v.w;
+    }
+    float* dst = g + b_off + threadIdx.x;
+    *dst = add ? *dst + b : b;
+  }
+}
+
+// loss_part[block] = sum over its samples and outputs of (y - target)^2;
+// dY = 2 (y - target) / (3 batch); yhat (may be null) receives y.
+template <int T>
+__global__ void __launch_bounds__(kBpThreads, 1)
+mlp_backprop_kernel(const float* __restrict__ p, const __nv_bfloat16* __restrict__ img, const float* __restrict__ xin,
+                    const float* __restrict__ target, long batch, float* __restrict__ part,
+                    float* __restrict__ loss_part, float* __restrict__ yhat) {
+  using S = BpSmem<T>;
+  constexpr int kPitch = S::kPitch, kSg = T / 4, kOutPer = kSg / 2;
+  extern __shared__ __align__(16) float bp_smem[];
+  float* h[3] = {bp_smem, bp_smem + S::kRow, bp_smem + 2 * S::kRow};
+  float* dz[3] = {bp_smem + 3 * S::kRow, bp_smem + 4 * S::kRow, bp_smem + 5 * S::kRow};
+  float* xs = bp_smem + S::kX;
+  float* dy = bp_smem + S::kDy;
+  __nv_bfloat16* w = reinterpret_cast<__nv_bfloat16*>(bp_smem + S::kFloats);
+  const int tid = threadIdx.x, sg = tid % kSg, out0 = (tid / kSg) * kOutPer;
+  float* g = part + static_cast<size_t>(blockIdx.x) * kMlpParams;
+  const float dscale = static_cast<float>(batch * kMlpOut);
+  const long tiles = (batch + T - 1) / T;
+  float loss = 0.f;
+  bool add = false;
+  for (long tile = blockIdx.x; tile < tiles; tile += gridDim.x, add = true) {
+    const long s0 = tile * T;
+    const int ns = static_cast<int>(min(static_cast<long>(T), batch - s0));
+    if (add) __syncthreads();  // the previous tile's gradients have read the arrays
+    for (int e = tid; e < kTrFwd / 8; e += kBpThreads)
+      reinterpret_cast<uint4*>(w)[e] = reinterpret_cast<const uint4*>(img)[e];
+    for (int e = tid; e < T * kMlpIn; e += kBpThreads) {
+      const int s = e / kMlpIn, k = e - s * kMlpIn;
+      xs[k * kPitch + s] = s < ns ? xin[s0 * kMlpIn + e] : 0.f;
+    }
+    __syncthreads();
+    // ---- forward: z = W in + b, h = gelu(z), dz = gelu'(z)
+    const int w_off[3] = {kTrW1, kTrW2, kTrW3}, b_off[3] = {kOffB1, kOffB2, kOffB3};
+#pragma unroll
+    for (int l = 0; l < 3; ++l) {
+      float acc[kOutPer][4];
+      bp_product<T, kOutPer>(l == 0 ? xs : h[l - 1], w + w_off[l], l == 0 ? kMlpIn : kMlpHidden, sg, out0, acc);
+#pragma unroll
+      for (int j = 0; j < kOutPer; ++j) {
+        const float b = p[b_off[l] + out0 + j];
+        float hv[4], gv[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const float z = acc[j][c] + b;
+          hv[c] = gelu(z);
+          gv[c] = gelu_grad(z);
+        }
+        const int at = (out0 + j) * kPitch + 4 * sg;
+        *reinterpret_cast<float4*>(h[l] + at) = make_float4(hv[0], hv[1], hv[2], hv[3]);
+        *reinterpret_cast<float4*>(dz[l] + at) = make_float4(gv[0], gv[1], gv[2], gv[3]);
+      }
+      __syncthreads();
+    }
+    // ---- outputs, loss and dY (a thread per sample and output); the other
+    // threads stage W3 and W2 for the backward pass over the forward copies
+    if (tid < T * kMlpOut) {
+      const int s = tid % T, o = tid / T;
+      const __nv_bfloat16* w4 = w + kTrW4 + o * kMlpHidden;
+      float acc = 0.f;
+#pragma unroll 8
+      for (int k = 0; k < kMlpHidden; ++k) acc = fmaf(__bfloat162float(w4[k]), h[2][k * kPitch + s], acc);
+      acc += p[kOffB4 + o];
+      float d = 0.f;
+      if (s < ns) {
+        const long at = (s0 + s) * kMlpOut + o;
+        if (yhat) yhat[at] = acc;
+        d = acc - target[at];
+      }
+      loss += d * d;
+      dy[o * kPitch + s] = 2.f * d / dscale;
+    } else {
+      for (int e = tid - T * kMlpOut; e < 2 * kMlpHidden * kMlpHidden / 8; e += kBpThreads - T * kMlpOut)
+        reinterpret_cast<uint4*>(w + kTrW2)[e] = reinterpret_cast<const uint4*>(img + kTrBack)[e];
+    }
+    __syncthreads();
+    // ---- layer 4: dW4, db4, dz3 = (W4^T dY) gelu'(z3)
+    for (int e = tid; e < kMlpOut * kMlpHidden + kMlpOut; e += kBpThreads) {
+      const bool bias = e >= kMlpOut * kMlpHidden;
+      const int o = bias ? e - kMlpOut * kMlpHidden : e / kMlpHidden, k = e % kMlpHidden;
+      float acc = 0.f;
+      for (int s = 0; s < T; ++s) acc = bias ? acc + dy[o * kPitch + s] : fmaf(dy[o * kPitch + s], h[2][k * kPitch + s], acc);
+      float* dst = g + (bias ? kOffB4 + o : kOffW4 + e);
+      *dst = add ? *dst + acc : acc;
+    }
+    for (int e = tid; e < kMlpHidden * kSg; e += kBpThreads) {
+      const int k = e / kSg, c = 4 * (e % kSg);
+      float4 v = *reinterpret_cast<float4*>(dz[2] + k * kPitch + c);
+      float a[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int o = 0; o < kMlpOut; ++o) {
+        const float wv = __bfloat162float(w[kTrW4 + o * kMlpHidden + k]);
+        const float4 d = *reinterpret_cast<const float4*>(dy + o * kPitch + c);
+        a[0] = fmaf(d.x, wv, a[0]);
+        a[1] = fmaf(d.y, wv, a[1]);
+        a[2] = fmaf(d.z, wv, a[2]);
+        a[3] = fmaf(d.w, wv, a[3]);
+      }
+      *reinterpret_cast<float4*>(dz[2] + k * kPitch + c) = make_float4(a[0] * v.x, a[1] * v.y, a[2] * v.z, a[3] * v.w);
+    }
+    __syncthreads();
+    // ---- layers 3 and 2: dz_(l-1) = (W_l^T dz_l) gelu'(z_(l-1)), dW_l, db_l
+#pragma unroll
+    for (int l = 2; l >= 1; --l) {
+      float acc[kOutPer][4];
+      bp_product<T, kOutPer>(dz[l], w + kTrW2 + (l == 2 ? 0 : kMlpHidden * kMlpHidden), kMlpHidden, sg, out0, acc);
+#pragma unroll
+      for (int j = 0; j < kOutPer; ++j) {
+        float4* at = reinterpret_cast<float4*>(dz[l - 1] + (out0 + j) * kPitch + 4 * sg);
+        const float4 v = *at;
+        *at = make_float4(acc[j][0] * v.x, acc[j][1] * v.y, acc[j][2] * v.z, acc[j][3] * v.w);
+      }
+      bp_weight_grad<T, kMlpHidden>(dz[l], h[l - 1], l == 2 ? kOffW3 : kOffW2, l == 2 ? kOffB3 : kOffB2, add, g);
+      __syncthreads();
+    }
+    bp_weight_grad<T, kMlpIn>(dz[0], xs, kOffW1, kOffB1, add, g);
+  }
+  // the block's loss: warp sums, then the warps in order
+  for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+  float* red = bp_smem + S::kRed;
+  if ((tid & 31) == 0) red[tid >> 5] = loss;
+  __syncthreads();
+  if (tid == 0) {
+    float l = 0.f;
+    for (int k = 0; k < kBpThreads / 32; ++k) l += red[k];
+    loss_part[blockIdx.x] = l;
+  }
+}
+
+// The CTAs' gradients summed in order; with adam_m the Adam update of the
+// masters and of their BF16 training image, else the gradient into grad.
+__global__ void mlp_update_kernel(const float* __restrict__ part, int n_part, float* __restrict__ grad,
+                                  float* __restrict__ p, float* __restrict__ adam_m, float* __restrict__ adam_v,
+                                  __nv_bfloat16* __restrict__ img, float lr, float b1, float b2, float eps, float c1,
+                                  float c2) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= kMlpParams) return;
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  int k = 0;
+#pragma unroll 2
+  for (; k + 4 <= n_part; k += 4)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) acc[u] += part[static_cast<size_t>(k + u) * kMlpParams + i];
+  for (; k < n_part; ++k) acc[0] += part[static_cast<size_t>(k) * kMlpParams + i];
+  const float gi = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+  grad[i] = gi;
+  if (adam_m == nullptr) return;
+  const float mi = b1 * adam_m[i] + (1.f - b1) * gi;
+  const float vi = b2 * adam_v[i] + (1.f - b2) * gi * gi;
+  adam_m[i] = mi;
+  adam_v[i] = vi;
+  const float v = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+  p[i] = v;
+  train_image_put(i, v, img);
 }
 
 __global__ void mlp_init_kernel(float* __restrict__ p, uint32_t seed) {
@@ -351,6 +587,7 @@ static int mlp_get(amk_ctx* c, Mlp** out) {
     AMK_TRY(m->adam_m.reserve(pb));
     AMK_TRY(m->adam_v.reserve(pb));
     AMK_TRY(m->packed.reserve(kImgBytes));
+    AMK_TRY(m->train.reserve(kTrElems * sizeof(__nv_bfloat16)));
     AMK_TRY(m->status.reserve(16));
     AMK_CUDA_TRY(cudaMemsetAsync(m->adam_m.ptr, 0, pb, c->stream));
     AMK_CUDA_TRY(cudaMemsetAsync(m->adam_v.ptr, 0, pb, c->stream));
@@ -358,7 +595,7 @@ static int mlp_get(amk_ctx* c, Mlp** out) {
     mlp_init_kernel<<<(kMlpParams + 255) / 256, 256, 0, c->stream>>>(m->master.as<float>(), 12345u);
     AMK_TRY(check_launch(c, "mlp_init_kernel"));
     m->initialized = true;
-    m->packed_valid = false;
+    m->packed_valid = m->train_valid = false;
   }
   *out = m;
   return AMK_OK;
@@ -407,69 +644,69 @@ int mlp_check_status(amk_ctx* c) {
   return AMK_OK;
 }
 
-// FP32 forward + backward on a device batch; fills m->grad, returns the loss.
-int mlp_gradients_device(amk_ctx* c, const float* x, const float* target, long batch, float* loss_host,
-                         float* yhat_out) {
-  Mlp* m = nullptr;
-  AMK_TRY(mlp_get(c, &m));
-  int rc = AMK_OK;
-  const long H = kMlpHidden;
-  // activations: z1 h1 z2 h2 z3 h3 (batch x 128), z4 (batch x 3), dz buffers
-  float* buf = slot<float>(c, kSlotMlp0, static_cast<size_t>(batch) * (6 * H + 2 * kMlpOut + 2 * H) + 1024, &rc);
-  AMK_TRY(rc);
-  float *z1 = buf, *h1 = z1 + batch * H, *z2 = h1 + batch * H, *h2 = z2 + batch * H, *z3 = h2 + batch * H,
-        *h3 = z3 + batch * H, *y = h3 + batch * H, *dy = y + batch * kMlpOut, *da = dy + batch * kMlpOut,
-        *db = da + batch * H;
-  float* lp = slot<float>(c, kSlotMlp1, 256, &rc);
-  AMK_TRY(rc);
-  const float* p = m->master.as<float>();
-  float* g = m->grad.as<float>();
-  auto grid = [](long work) { return static_cast<unsigned>((work + 255) / 256); };
-  mlp_dense_kernel<<<grid(batch * H), 256, 0, c->stream>>>(p, kOffW1, kOffB1, kMlpIn, H, x, batch, z1, h1, true);
-  mlp_dense_kernel<<<grid(batch * H), 256, 0, c->stream>>>(p, kOffW2, kOffB2, H, H, h1, batch, z2, h2, true);
-  mlp_dense_kernel<<<grid(batch * H), 256, 0, c->stream>>>(p, kOffW3, kOffB3, H, H, h2, batch, z3, h3, true);
-  mlp_dense_kernel<<<grid(batch * kMlpOut), 256, 0, c->stream>>>(p, kOffW4, kOffB4, H, kMlpOut, h3, batch, y,
-                                                                 nullptr, false);
-  AMK_TRY(check_launch(c, "mlp_dense_kernel"));
-  const int lblocks = 128;
-  mlp_loss_kernel<<<lblocks, 256, 0, c->stream>>>(y, target, batch, dy, lp);
-  AMK_TRY(check_launch(c, "mlp_loss_kernel"));
-  // layer 4
-  mlp_back_weight_kernel<<<grid(kMlpOut * H), 256, 0, c->stream>>>(kOffW4, kOffB4, H, kMlpOut, dy, h3, batch, g);
-  mlp_back_input_kernel<<<grid(batch * H), 256, 0, c->stream>>>(p, kOffW4, H, kMlpOut, dy, batch, z3, da);
-  // layer 3
-  mlp_back_weight_kernel<<<grid(H * H), 256, 0, c->stream>>>(kOffW3, kOffB3, H, H, da, h2, batch, g);
-  mlp_back_input_kernel<<<grid(batch * H), 256, 0, c->stream>>>(p, kOffW3, H, H, da, batch, z2, db);
-  // layer 2
-  mlp_back_weight_kernel<<<grid(H * H), 256, 0, c->stream>>>(kOffW2, kOffB2, H, H, db, h1, batch, g);
-  mlp_back_input_kernel<<<grid(batch * H), 256, 0, c->stream>>>(p, kOffW2, H, H, db, batch, z1, da);
-  // layer 1
-  mlp_back_weight_kernel<<<grid(H * kMlpIn), 256, 0, c->stream>>>(kOffW1, kOffB1, kMlpIn, H, da, x, batch, g);
-  AMK_TRY(check_launch(c, "mlp_backward"));
-  if (yhat_out) AMK_CUDA_TRY(cudaMemcpyAsync(yhat_out, y, batch * kMlpOut * sizeof(float), cudaMemcpyDeviceToDevice, c->stream));
-  if (loss_host) {
-    float h[lblocks];
-    AMK_CUDA_TRY(cudaMemcpyAsync(h, lp, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
-    AMK_CUDA_TRY(cudaStreamSynchronize(c->stream));
-    double s = 0.0;
-    for (int b = 0; b < lblocks; ++b) s += h[b];
-    *loss_host = static_cast<float>(s / static_cast<double>(batch * kMlpOut));
-  }
-  return AMK_OK;
+// Samples per tile of mlp_backprop_kernel: a tile's time falls more slowly
+// than its samples, so the tiles are made smaller only while all of them run
+// at once. us per training step with tiles of 8 / 16 / 32 samples (148 SMs):
+// batch 256 33.7 / 39.6 / 48.4, 1,184 38.8 / 43.9 / 50.0, 1,500 61.7 / 46.0 /
+// 52.1, 2,368 62.7 / 47.1 / 52.2, 3,000 85.2 / 76.4 / 54.3, 4,096 108 / 77.4 /
+// 54.3.
+static int mlp_tile_rows(long batch, int sms) {
+  if (batch > 16L * sms) return 32;
+  return batch > 8L * sms ? 16 : 8;
 }
 
-int mlp_adam_step(amk_ctx* c, float lr) {
+// Forward, backward and (lr given) one Adam step on a device batch; the
+// summed gradient is left in m->grad. loss_host and yhat_out may be null.
+static int mlp_step_device(amk_ctx* c, const float* x, const float* target, long batch, const float* lr,
+                           float* loss_host, float* yhat_out) {
   Mlp* m = nullptr;
   AMK_TRY(mlp_get(c, &m));
-  m->adam_step++;
+  if (!m->train_valid) {
+    mlp_train_pack_kernel<<<(kMlpParams + 255) / 256, 256, 0, c->stream>>>(m->master.as<float>(),
+                                                                           m->train.as<__nv_bfloat16>());
+    AMK_TRY(check_launch(c, "mlp_train_pack_kernel"));
+    m->train_valid = true;
+  }
+  int rc = AMK_OK, sms = 0;
+  AMK_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
+  const int rows = mlp_tile_rows(batch, sms);
+  const int grid = static_cast<int>(std::min<long>((batch + rows - 1) / rows, sms));
+  float* part = slot<float>(c, kSlotMlp0, static_cast<size_t>(grid) * kMlpParams, &rc);
+  AMK_TRY(rc);
+  float* lp = slot<float>(c, kSlotMlp1, std::max(256, grid), &rc);
+  AMK_TRY(rc);
+  auto launch = [&](auto kernel, size_t smem) -> int {
+    AMK_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    kernel<<<grid, kBpThreads, smem, c->stream>>>(m->master.as<float>(), m->train.as<__nv_bfloat16>(), x, target,
+                                                  batch, part, lp, yhat_out);
+    return check_launch(c, "mlp_backprop_kernel");
+  };
+  if (rows == 32)
+    AMK_TRY(launch(mlp_backprop_kernel<32>, BpSmem<32>::kBytes));
+  else if (rows == 16)
+    AMK_TRY(launch(mlp_backprop_kernel<16>, BpSmem<16>::kBytes));
+  else
+    AMK_TRY(launch(mlp_backprop_kernel<8>, BpSmem<8>::kBytes));
   const float b1 = 0.9f, b2 = 0.999f;
-  const float c1 = 1.f - std::pow(b1, static_cast<float>(m->adam_step));
-  const float c2 = 1.f - std::pow(b2, static_cast<float>(m->adam_step));
-  mlp_adam_kernel<<<(kMlpParams + 255) / 256, 256, 0, c->stream>>>(m->master.as<float>(), m->grad.as<float>(),
-                                                                   m->adam_m.as<float>(), m->adam_v.as<float>(),
-                                                                   kMlpParams, lr, b1, b2, 1e-8f, c1, c2);
-  AMK_TRY(check_launch(c, "mlp_adam_kernel"));
-  m->packed_valid = false;
+  float c1 = 1.f, c2 = 1.f;
+  if (lr) {
+    m->adam_step++;
+    c1 = 1.f - std::pow(b1, static_cast<float>(m->adam_step));
+    c2 = 1.f - std::pow(b2, static_cast<float>(m->adam_step));
+    m->packed_valid = false;
+  }
+  mlp_update_kernel<<<(kMlpParams + 127) / 128, 128, 0, c->stream>>>(
+      part, grid, m->grad.as<float>(), m->master.as<float>(), lr ? m->adam_m.as<float>() : nullptr,
+      lr ? m->adam_v.as<float>() : nullptr, m->train.as<__nv_bfloat16>(), lr ? *lr : 0.f, b1, b2, 1e-8f, c1, c2);
+  AMK_TRY(check_launch(c, "mlp_update_kernel"));
+  if (loss_host) {
+    std::vector<float> h(grid);
+    AMK_CUDA_TRY(cudaMemcpyAsync(h.data(), lp, grid * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
+    AMK_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    double s = 0.0;
+    for (float v : h) s += v;
+    *loss_host = static_cast<float>(s / static_cast<double>(batch * kMlpOut));
+  }
   return AMK_OK;
 }
 
@@ -482,9 +719,8 @@ int mlp_train_device(amk_ctx* c, const float* x, const float* target, long n, in
   for (int s = 0; s < steps; ++s) {
     const long start = (static_cast<long>(s) * batch) % std::max(1L, n - batch + 1);
     const bool last = s + 1 == steps;
-    AMK_TRY(mlp_gradients_device(c, x + start * kMlpIn, target + start * kMlpOut, batch, last ? &loss : nullptr,
-                                 nullptr));
-    AMK_TRY(mlp_adam_step(c, lr));
+    AMK_TRY(mlp_step_device(c, x + start * kMlpIn, target + start * kMlpOut, batch, &lr, last ? &loss : nullptr,
+                            nullptr));
   }
   if (final_loss) *final_loss = loss;
   return AMK_OK;
@@ -509,7 +745,7 @@ extern "C" int amk_mlp_set_params(amk_ctx* c, const float* params, long n) {
   AMK_CUDA_TRY(cudaMemsetAsync(m->adam_m.ptr, 0, kMlpParams * sizeof(float), c->stream));
   AMK_CUDA_TRY(cudaMemsetAsync(m->adam_v.ptr, 0, kMlpParams * sizeof(float), c->stream));
   m->adam_step = 0;
-  m->packed_valid = false;
+  m->packed_valid = m->train_valid = false;
   AMK_CUDA_TRY(cudaStreamSynchronize(c->stream));
   return AMK_OK;
 }
@@ -552,7 +788,7 @@ extern "C" int amk_mlp_gradients(amk_ctx* c, const float* x, const float* target
   AMK_CUDA_TRY(cudaMemcpyAsync(dx, x, n * kMlpIn * sizeof(float), cudaMemcpyHostToDevice, c->stream));
   AMK_CUDA_TRY(cudaMemcpyAsync(dt, target, n * kMlpOut * sizeof(float), cudaMemcpyHostToDevice, c->stream));
   float l = 0.f;
-  AMK_TRY(mlp_gradients_device(c, dx, dt, n, &l, dyh));
+  AMK_TRY(mlp_step_device(c, dx, dt, n, nullptr, &l, dyh));
   if (loss) *loss = l;
   if (grad)
     AMK_CUDA_TRY(cudaMemcpyAsync(grad, c->mlp->grad.ptr, kMlpParams * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
