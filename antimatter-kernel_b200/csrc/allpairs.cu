@@ -39,6 +39,7 @@
 #include <algorithm>
 
 #include "amk_internal.cuh"
+#include "bbox.cuh"
 #include "morton.cuh"
 
 namespace amk {
@@ -65,29 +66,8 @@ __device__ __forceinline__ bool usable(const View& v, long i) {
 }
 
 // ------------------------------------------------------------ ordering
-__global__ void ap_bbox_kernel(View v, unsigned long long* bb) {
-  double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-  for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < v.n;
-       i += static_cast<long>(gridDim.x) * blockDim.x) {
-    if (!usable(v, i)) continue;
-    const double p[3] = {v.x[i], v.y[i], v.z[i]};
-    for (int d = 0; d < 3; ++d) {
-      lo[d] = fmin(lo[d], p[d]);
-      hi[d] = fmax(hi[d], p[d]);
-    }
-  }
-  for (int d = 0; d < 3; ++d) {
-    for (int o = 16; o > 0; o >>= 1) {
-      lo[d] = fmin(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
-      hi[d] = fmax(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
-    }
-  }
-  if ((threadIdx.x & 31) == 0) {
-    for (int d = 0; d < 3; ++d) {
-      atomicMin(&bb[d], double_order_bits(lo[d]));
-      atomicMin(&bb[3 + d], double_order_bits(-hi[d]));
-    }
-  }
+__global__ void __launch_bounds__(kBboxThreads) ap_bbox_kernel(View v, unsigned long long* bb) {
+  bbox_block(v, [&](long i) { return usable(v, i); }, bb);
 }
 
 // 30-bit Morton key (10 bits per axis) inside the live bounding box; unusable
@@ -467,7 +447,7 @@ int allpairs_forces(amk_ctx* c, const View& v) {
     uint64_t* skeys = slot<uint64_t>(c, kSlotTreeKeys, n, &rc);
     AMK_TRY(rc);
     AMK_CUDA_TRY(cudaMemsetAsync(bb, 0xFF, 6 * sizeof(unsigned long long), c->stream));
-    ap_bbox_kernel<<<148, 256, 0, c->stream>>>(v, bb);
+    ap_bbox_kernel<<<bbox_grid(n), kBboxThreads, 0, c->stream>>>(v, bb);
     AMK_TRY(check_launch(c, "ap_bbox_kernel"));
     ap_key_kernel<<<(n + 255) / 256, 256, 0, c->stream>>>(v, bb, keys, vals);
     AMK_TRY(check_launch(c, "ap_key_kernel"));

@@ -86,10 +86,7 @@ struct DevBuf {
 
 // ---------------------------------------------------------------- particle views
 // Structure-of-arrays particle set on the device. Positions are FP64 and
-// trap-centred. `q_e` is the charge in units of e (float, exact for +-e) and
-// `hq`/`lo` are the double-float split of the scaled position used by the
-// FP32 pair kernels: x / L = hq.x + lo.x (|lo| <= ulp(hq)/2), hq.w = q_e
-// (0 for dead or neutral particles so that they drop out of every sum).
+// trap-centred. The FP32 pair kernels stage their own double-float copies.
 struct View {
   long n = 0;
   double* x = nullptr;
@@ -97,8 +94,6 @@ struct View {
   double* z = nullptr;
   double* q = nullptr;      // charge [C]
   uint8_t* alive = nullptr; // may be null = all alive
-  float4* hq = nullptr;
-  float4* lo = nullptr;
   double* fx = nullptr;     // force outputs [N]
   double* fy = nullptr;
   double* fz = nullptr;
@@ -236,17 +231,17 @@ struct amk_ctx {
   long n = 0;
   long capacity = 0;
   // particle state (device)
-  amk::DevBuf x, y, z, vx, vy, vz, fx, fy, fz, q, m, hq, lo, species, alive, ids;
+  amk::DevBuf x, y, z, vx, vy, vz, fx, fy, fz, q, m, species, alive, ids;
+  amk::DevBuf hq, lo;  // staged positions of the batched all-pairs kernel
   double length_scale = 1.0;
   bool staggered = false;     // first push done (lorentz.h:34)
   long step = 0;              // completed steps
-  bool stage_dirty = true;    // hq/lo must be rebuilt from x,y,z
   // Morton order of the all-pairs kernel, reused for a few calls
   amk::DevBuf ap_perm;
   long ap_perm_n = -1;
   int ap_perm_age = 0;
   // aux particle set for the stateless solver mirrors
-  amk::DevBuf ax, ay, az, aq, ahq, alo, afx, afy, afz, aphi;
+  amk::DevBuf ax, ay, az, aq, afx, afy, afz, aphi;
   long aux_capacity = 0;
 
   amk::Scratch scratch;
@@ -255,6 +250,10 @@ struct amk_ctx {
   // energy time-centring (EnergyHistory, energy_analysis.h:23-28)
   bool energy_has_previous = false;
   double prev_trap = 0.0, prev_coulomb = 0.0;
+
+  // small-set annihilation: a matching whose outcome has not been read yet,
+  // and whether the words it counts in start cleared (cellist.cu)
+  bool ann_pending = false, ann_words_clear = false;
 
   bool profiling = false;
   amk::PhaseClock clock;
@@ -303,9 +302,6 @@ bool is_antiparticle_pair(int a, int b);
 
 // View over the context's main particle state.
 View main_view(amk_ctx* c);
-
-// Rebuilds hq/lo (double-float staging) of a view on the context stream.
-int stage_view(amk_ctx* c, const View& v);
 
 // Solvers on a view; outputs into v.fx/fy/fz (and v.phi when non-null).
 int allpairs_forces(amk_ctx* c, const View& v);
@@ -378,7 +374,10 @@ int reduce_sum(amk_ctx* c, const double* in, long n, double* out_dev);
 // Per-step behaviours (push.cu, cellist.cu).
 int push_step(amk_ctx* c, uint64_t step_index);
 int annihilate_step(amk_ctx* c, uint64_t step_index, long* marked);
-// Annihilation on a view (indices, species and ids relative to the view).
+// Annihilation on a view (indices, species and ids relative to the view). A
+// small set's outcome is left on the device when `marked` is null;
+// annihilate_check reads it (an error if a matching did not converge).
+int annihilate_check(amk_ctx* c, long* marked);
 int annihilate_view(amk_ctx* c, const View& v, const uint8_t* species, const uint32_t* ids, double radius,
                     double probability, uint32_t seed, uint64_t step_index, long* marked);
 // Batched instances (batch.cu).

@@ -607,8 +607,6 @@ View instance_view(amk_ctx* c, const Batch& B, int i) {
   v.z += off;
   v.q += off;
   v.alive += off;
-  v.hq += off;
-  v.lo += off;
   v.fx += off;
   v.fy += off;
   v.fz += off;
@@ -740,7 +738,7 @@ int serial_step_once(amk_ctx* c, Batch& B, bool stagger) {
                               p.annihilation_probability, static_cast<uint32_t>(p.seed), st, nullptr));
     }
   }
-  return AMK_OK;
+  return annihilate_check(c, nullptr);
 }
 
 }  // namespace
@@ -917,7 +915,6 @@ extern "C" int amk_batch_step(amk_ctx* c, int nsteps, int graph_chunk, int seria
     c->step += graph_chunk;
     done += graph_chunk;
   }
-  c->stage_dirty = true;
   if (graphed) {
     unsigned long long ov = 0;
     AMK_CUDA_TRY(cudaMemcpyAsync(&ov, B.call_overflow(), sizeof(ov), cudaMemcpyDeviceToHost, c->stream));

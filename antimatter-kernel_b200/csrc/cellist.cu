@@ -1,6 +1,4 @@
-// Uniform-grid cell list (cell edge >= the interaction radius) built by
-// Morton-keying the live particles and radix-sorting the keys, and the two
-// kernels that walk it:
+// Pairs closer than a radius, and the two behaviours that walk them:
 //   * the cutoff direct sum of ComputeStandardCoulombForces
 //     (interaction/coulomb_interaction.cc:23-80) with the shifted-cutoff pair
 //     energy of ComputeStandardEnergy (analysis/energy_analysis.cc:16-43);
@@ -13,9 +11,20 @@
 //     that has the smallest priority at both of its endpoints.
 // Pair geometry is FP64 with contraction-free arithmetic so that contact
 // decisions are bit-identical to a scalar FP64 evaluation.
+//
+// Up to kBruteMax particles every pair is tested (one launch, no list). Above
+// it the particles are binned into a dense grid over their bounding box:
+// cells no smaller than the radius and at most 4 per particle, x fastest, so
+// that the 27 neighbour cells of a particle are nine contiguous runs of the
+// sorted records. A counting sort builds it (count, scan, scatter; the
+// members of a cell ordered by particle index, so sums have a fixed order).
+// The allocation-free solver keeps its Morton-sorted keys: its static scratch
+// has no room for the grid's counters.
 #include <algorithm>
 
 #include "amk_internal.cuh"
+#include "bbox.cuh"
+#include "contacts.cuh"
 #include "philox.cuh"
 
 namespace amk {
@@ -25,57 +34,12 @@ constexpr uint64_t kDeadKey = ~0ull;
 constexpr int kCellBits = 21;
 constexpr double kCellMax = 2097150.0;  // 2^21 - 2
 
-__device__ __forceinline__ uint64_t spread3(uint64_t v) {
-  v &= 0x1fffffull;
-  v = (v | (v << 32)) & 0x1f00000000ffffull;
-  v = (v | (v << 16)) & 0x1f0000ff0000ffull;
-  v = (v | (v << 8)) & 0x100f00f00f00f00full;
-  v = (v | (v << 4)) & 0x10c30c30c30c30c3ull;
-  v = (v | (v << 2)) & 0x1249249249249249ull;
-  return v;
-}
-
-__device__ __forceinline__ uint64_t morton3(uint32_t x, uint32_t y, uint32_t z) {
-  return spread3(x) | (spread3(y) << 1) | (spread3(z) << 2);
-}
-
-__device__ __forceinline__ unsigned long long order_bits(double v) {
-  const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(v));
-  return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
-}
-__device__ __forceinline__ double from_order_bits(unsigned long long b) {
-  const unsigned long long r = (b >> 63) ? (b & 0x7fffffffffffffffull) : ~b;
-  return __longlong_as_double(static_cast<long long>(r));
-}
-
 __device__ __forceinline__ bool usable(const View& v, long i) {
   return (v.alive == nullptr || v.alive[i]) && isfinite(v.x[i]) && isfinite(v.y[i]) && isfinite(v.z[i]);
 }
 
-// bb[0..2] = ordered-bits min, bb[3..5] = ordered-bits of -max.
-__global__ void bbox_kernel(View v, unsigned long long* bb) {
-  double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-  for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < v.n;
-       i += static_cast<long>(gridDim.x) * blockDim.x) {
-    if (!usable(v, i)) continue;
-    const double p[3] = {v.x[i], v.y[i], v.z[i]};
-    for (int d = 0; d < 3; ++d) {
-      lo[d] = fmin(lo[d], p[d]);
-      hi[d] = fmax(hi[d], p[d]);
-    }
-  }
-  for (int d = 0; d < 3; ++d) {
-    for (int o = 16; o > 0; o >>= 1) {
-      lo[d] = fmin(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
-      hi[d] = fmax(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
-    }
-  }
-  if ((threadIdx.x & 31) == 0) {
-    for (int d = 0; d < 3; ++d) {
-      atomicMin(&bb[d], order_bits(lo[d]));
-      atomicMin(&bb[3 + d], order_bits(-hi[d]));
-    }
-  }
+__global__ void __launch_bounds__(kBboxThreads) bbox_kernel(View v, unsigned long long* bb) {
+  bbox_block(v, [&](long i) { return usable(v, i); }, bb);
 }
 
 struct Grid {
@@ -85,8 +49,8 @@ struct Grid {
 
 __device__ __forceinline__ Grid grid_from(const unsigned long long* bb, double radius) {
   Grid g;
-  const double lo0 = from_order_bits(bb[0]), lo1 = from_order_bits(bb[1]), lo2 = from_order_bits(bb[2]);
-  const double hi0 = -from_order_bits(bb[3]), hi1 = -from_order_bits(bb[4]), hi2 = -from_order_bits(bb[5]);
+  const double lo0 = double_from_order_bits(bb[0]), lo1 = double_from_order_bits(bb[1]), lo2 = double_from_order_bits(bb[2]);
+  const double hi0 = -double_from_order_bits(bb[3]), hi1 = -double_from_order_bits(bb[4]), hi2 = -double_from_order_bits(bb[5]);
   double ext = fmax(hi0 - lo0, fmax(hi1 - lo1, hi2 - lo2));
   if (!(ext >= 0.0)) ext = 0.0;  // no live particle
   double cs = radius * (1.0 + 1e-9);
@@ -121,7 +85,7 @@ __global__ void cell_key_kernel(View v, const unsigned long long* bb, double rad
   const Grid g = grid_from(bb, radius);
   int c[3];
   cell_of(g, v.x[i], v.y[i], v.z[i], c);
-  keys[i] = morton3(c[0], c[1], c[2]);
+  keys[i] = morton3_21(c[0], c[1], c[2]);
 }
 
 __device__ __forceinline__ long lower_bound(const uint64_t* keys, long n, uint64_t k) {
@@ -140,15 +104,14 @@ __device__ __forceinline__ double dist2_exact(double rx, double ry, double rz) {
   return __dadd_rn(__dadd_rn(__dmul_rn(rx, rx), __dmul_rn(ry, ry)), __dmul_rn(rz, rz));
 }
 
-// One thread per sorted particle. Forces in SI (N), potential sums in
-// e_i = sum_j q_j (1/r - 1/rc) for the energy.
+// Allocation-free solver: one thread per particle of the Morton-sorted keys.
 __global__ void __launch_bounds__(128)
 cutoff_kernel(View v, const unsigned long long* bb, double rc, const uint64_t* __restrict__ skeys,
-              const uint32_t* __restrict__ sidx, double* __restrict__ epart) {
+              const uint32_t* __restrict__ sidx) {
   const long s = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
   if (s >= v.n) return;
   const long i = sidx[s];
-  double fx = 0.0, fy = 0.0, fz = 0.0, ei = 0.0;
+  double fx = 0.0, fy = 0.0, fz = 0.0;
   const double qi = v.q[i];
   if (skeys[s] != kDeadKey && qi != 0.0) {
     const Grid g = grid_from(bb, rc);
@@ -156,7 +119,6 @@ cutoff_kernel(View v, const unsigned long long* bb, double rc, const uint64_t* _
     int c[3];
     cell_of(g, xi, yi, zi, c);
     const double rc2 = rc * rc;
-    const double inv_rc = 1.0 / rc;
     for (int dz = -1; dz <= 1; ++dz) {
       const int cz = c[2] + dz;
       if (cz < 0 || cz > static_cast<int>(g.nmax)) continue;
@@ -166,7 +128,7 @@ cutoff_kernel(View v, const unsigned long long* bb, double rc, const uint64_t* _
         for (int dx = -1; dx <= 1; ++dx) {
           const int cx = c[0] + dx;
           if (cx < 0 || cx > static_cast<int>(g.nmax)) continue;
-          const uint64_t key = morton3(cx, cy, cz);
+          const uint64_t key = morton3_21(cx, cy, cz);
           for (long k = lower_bound(skeys, v.n, key); k < v.n && skeys[k] == key; ++k) {
             const long j = sidx[k];
             if (j == i) continue;
@@ -183,7 +145,6 @@ cutoff_kernel(View v, const unsigned long long* bb, double rc, const uint64_t* _
               fy += ry * w;
               fz += rz * w;
             }
-            if (epart && d2 <= rc2) ei += qj * (1.0 / sqrt(d2) - inv_rc);  // energy_analysis.cc:30-40
           }
         }
       }
@@ -192,7 +153,6 @@ cutoff_kernel(View v, const unsigned long long* bb, double rc, const uint64_t* _
   v.fx[i] = fx;
   v.fy[i] = fy;
   v.fz[i] = fz;
-  if (epart) epart[i] = qi * ei;
 }
 
 __global__ void zero_forces_kernel(View v) {
@@ -203,94 +163,411 @@ __global__ void zero_forces_kernel(View v) {
   v.fz[i] = 0.0;
 }
 
-}  // namespace
-}  // namespace amk
-#include "contacts.cuh"
-namespace amk {
-namespace {
-__global__ void __launch_bounds__(128)
-contact_kernel(View v, const uint8_t* __restrict__ species, const uint32_t* __restrict__ ids,
-               const unsigned long long* bb, double rc, double prob, uint32_t seed, uint64_t step,
-               const uint64_t* __restrict__ skeys, const uint32_t* __restrict__ sidx, Contact* out,
-               unsigned long long* count, long cap) {
-  const long s = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
-  if (s >= v.n) return;
-  if (skeys[s] == kDeadKey) return;
-  const long i = sidx[s];
-  const int si = species[i];
-  const bool has_partner = si == AMK_POSITRON || si == AMK_ELECTRON || si == AMK_PROTON || si == AMK_ANTIPROTON;
-  if (!has_partner) return;
-  const Grid g = grid_from(bb, rc);
-  const double xi = v.x[i], yi = v.y[i], zi = v.z[i];
-  int c[3];
-  cell_of(g, xi, yi, zi, c);
-  const double rc2 = rc * rc;
-  for (int dz = -1; dz <= 1; ++dz) {
-    const int cz = c[2] + dz;
-    if (cz < 0 || cz > static_cast<int>(g.nmax)) continue;
-    for (int dy = -1; dy <= 1; ++dy) {
-      const int cy = c[1] + dy;
-      if (cy < 0 || cy > static_cast<int>(g.nmax)) continue;
-      for (int dx = -1; dx <= 1; ++dx) {
-        const int cx = c[0] + dx;
-        if (cx < 0 || cx > static_cast<int>(g.nmax)) continue;
-        const uint64_t key = morton3(cx, cy, cz);
-        for (long k = lower_bound(skeys, v.n, key); k < v.n && skeys[k] == key; ++k) {
-          const long j = sidx[k];
-          if (j == i) continue;
-          const int sj = species[j];
-          const bool pair = (si == AMK_ANTIPROTON && sj == AMK_PROTON) || (si == AMK_PROTON && sj == AMK_ANTIPROTON) ||
-                            (si == AMK_POSITRON && sj == AMK_ELECTRON) || (si == AMK_ELECTRON && sj == AMK_POSITRON);
-          if (!pair) continue;
-          const double d2 = dist2_exact(xi - v.x[j], yi - v.y[j], zi - v.z[j]);
-          if (!(d2 < rc2)) continue;
-          const Philox4 w = philox4x32(seed, kTagAnnihilation, ids[i], ids[j], static_cast<uint32_t>(step),
-                                       static_cast<uint32_t>(step >> 32));
-          if (!(u01(w.w[0]) < prob)) continue;
-          const unsigned long long slot_i = atomicAdd(count, 1ull);
-          if (static_cast<long>(slot_i) < cap) {
-            Contact e;
-            e.a = static_cast<uint32_t>(i);
-            e.b = static_cast<uint32_t>(j);
-            e.prio = (static_cast<uint64_t>(ids[i]) << 32) | ids[j];
-            out[slot_i] = e;
-          }
-        }
-      }
-    }
+// ---------------------------------------------------------------- all pairs
+// Small sets: every pair, kBruteLanes lanes per target over the sources
+// staged in shared memory 256 at a time; the lanes' sums are added by a
+// shuffle tree (a fixed order).
+constexpr int kBruteLanes = 32;
+constexpr int kBruteThreads = 256;
+constexpr int kBruteTile = 256;
+// Pairs are tested all against all up to this many particles. us per step of
+// a mixed cloud (cutoff + push + cooling + annihilation), all pairs / grid,
+// with 1, 20 and 200 neighbours inside the cutoff: 200 particles 24/24/25 and
+// 72/83/80, 1,024 39/42/42 and 86/108/143, 2,048 87/94/95 and 166/190/234,
+// 4,096 159/154/136 and 183/204/254, 6,000 362/327/220 and 187/210/267. (With
+// radix-sorted Morton cells and a binary search per neighbour cell: 340 us at
+// 200 particles, 880 us at 100,000, of which the two 8-pass sorts were 600;
+// the grid takes 220 us there.)
+constexpr long kBruteMax = 4096;
+
+inline unsigned brute_grid(long n, int threads) {
+  const long per = threads / kBruteLanes;
+  return static_cast<unsigned>((n + per - 1) / per);
+}
+
+// One pair of the cutoff sum: field and (kEnergy) shifted potential of a
+// charge qj at distance^2 d2 (coulomb_interaction.cc:60-73,
+// energy_analysis.cc:30-40), without k q_i.
+template <bool kEnergy>
+__device__ __forceinline__ void cutoff_pair(double rx, double ry, double rz, double qj, double rc2, double inv_rc,
+                                            double f[3], double& e) {
+  const double d2 = dist2_exact(rx, ry, rz);
+  if (d2 > rc2 || d2 < kMinSquaredDistance) return;
+  const double inv = rsqrt(d2);
+  if (kEnergy) e += qj * (inv - inv_rc);
+  if (d2 < rc2) {
+    const double w = qj * (inv * inv * inv);
+    f[0] += rx * w;
+    f[1] += ry * w;
+    f[2] += rz * w;
   }
 }
 
-struct CellList {
-  unsigned long long* bb;
-  uint64_t* skeys;
-  uint32_t* sidx;
+template <bool kEnergy>
+__device__ __forceinline__ void cutoff_store(const View& v, long i, double qi, const double f[3], double e,
+                                             double* __restrict__ epart) {
+  const double c = kCoulombConstant * qi;
+  v.fx[i] = c * f[0];
+  v.fy[i] = c * f[1];
+  v.fz[i] = c * f[2];
+  if (kEnergy) epart[i] = qi * e;
+}
+
+template <bool kEnergy>
+__global__ void __launch_bounds__(kBruteThreads)
+cutoff_brute_kernel(View v, double rc, double* __restrict__ epart) {
+  __shared__ double4 tile[kBruteTile];
+  const int sub = threadIdx.x % kBruteLanes;
+  const long i = (blockIdx.x * static_cast<long>(kBruteThreads) + threadIdx.x) / kBruteLanes;
+  const bool live = i < v.n && usable(v, i) && v.q[i] != 0.0;
+  const double xi = live ? v.x[i] : 0.0, yi = live ? v.y[i] : 0.0, zi = live ? v.z[i] : 0.0;
+  const double rc2 = rc * rc, inv_rc = 1.0 / rc;
+  double f[3] = {0.0, 0.0, 0.0}, e = 0.0;
+  for (long j0 = 0; j0 < v.n; j0 += kBruteTile) {
+    __syncthreads();
+    const long j = j0 + threadIdx.x;
+    tile[threadIdx.x] = j < v.n && usable(v, j) ? make_double4(v.x[j], v.y[j], v.z[j], v.q[j])
+                                                : make_double4(0.0, 0.0, 0.0, 0.0);
+    __syncthreads();
+    const int cnt = static_cast<int>(min(static_cast<long>(kBruteTile), v.n - j0));
+    if (live)
+      for (int k = sub; k < cnt; k += kBruteLanes) {
+        const double4 s = tile[k];
+        if (j0 + k == i || s.w == 0.0) continue;
+        cutoff_pair<kEnergy>(xi - s.x, yi - s.y, zi - s.z, s.w, rc2, inv_rc, f, e);
+      }
+  }
+#pragma unroll
+  for (int o = kBruteLanes / 2; o > 0; o >>= 1) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) f[d] += __shfl_xor_sync(0xffffffffu, f[d], o);
+    if (kEnergy) e += __shfl_xor_sync(0xffffffffu, e, o);
+  }
+  if (sub == 0 && i < v.n) cutoff_store<kEnergy>(v, i, live ? v.q[i] : 0.0, f, e, epart);
+}
+
+// ---------------------------------------------------------------- contacts
+__device__ __forceinline__ bool has_partner(int s) {
+  return s == AMK_POSITRON || s == AMK_ELECTRON || s == AMK_PROTON || s == AMK_ANTIPROTON;
+}
+__device__ __forceinline__ int partner_of(int s) {
+  return s == AMK_POSITRON ? AMK_ELECTRON : s == AMK_ELECTRON ? AMK_POSITRON : s == AMK_PROTON ? AMK_ANTIPROTON : AMK_PROTON;
+}
+
+struct ContactRule {
+  double rc2, prob;
+  uint32_t seed;
+  uint64_t step;
 };
 
-int build_cell_list(amk_ctx* c, const View& v, double radius, CellList* out) {
+// The directed contact i -> j of two partners at distance^2 d2: kept when it
+// is inside the radius and its Philox draw is below the probability.
+__device__ __forceinline__ void contact_pair(const ContactRule& R, double d2, uint32_t i, uint32_t j, uint32_t id_i,
+                                             uint32_t id_j, Contact* __restrict__ out, unsigned long long* count,
+                                             long cap) {
+  if (!(d2 < R.rc2)) return;
+  const Philox4 w = philox4x32(R.seed, kTagAnnihilation, id_i, id_j, static_cast<uint32_t>(R.step),
+                               static_cast<uint32_t>(R.step >> 32));
+  if (!(u01(w.w[0]) < R.prob)) return;
+  const unsigned long long at = atomicAdd(count, 1ull);
+  if (static_cast<long>(at) < cap) {
+    Contact e;
+    e.a = i;
+    e.b = j;
+    e.prio = (static_cast<uint64_t>(id_i) << 32) | id_j;
+    out[at] = e;
+  }
+}
+
+// Words of kSlotAnnAux: [0] contacts found, [1] finished blocks of the fused
+// kernel, [2] particles marked, [3] sticky "did not converge".
+constexpr int kFusedThreads = 1024;
+// Up to this many particles the contact search and the matching are one
+// launch whose last block matches, with room for every possible contact
+// (n^2 / 2 of 16 bytes), so that nothing is read back between steps.
+constexpr long kFusedMax = 1024;
+
+template <int kThreads, bool kFused>
+__global__ void __launch_bounds__(kThreads)
+contact_brute_kernel(View v, const uint8_t* __restrict__ species, const uint32_t* __restrict__ ids, ContactRule R,
+                     Contact* __restrict__ out, unsigned long long* words, long cap, unsigned long long* best,
+                     uint8_t* matched, uint8_t* live_e) {
+  __shared__ double tx[kBruteTile], ty[kBruteTile], tz[kBruteTile];
+  __shared__ int ts[kBruteTile];
+  __shared__ uint32_t tid_s[kBruteTile];
+  __shared__ bool s_last;
+  const int sub = threadIdx.x % kBruteLanes;
+  const long i = (blockIdx.x * static_cast<long>(kThreads) + threadIdx.x) / kBruteLanes;
+  const bool live = i < v.n && usable(v, i) && has_partner(species[i]);
+  const int want = live ? partner_of(species[i]) : -2;
+  const double xi = live ? v.x[i] : 0.0, yi = live ? v.y[i] : 0.0, zi = live ? v.z[i] : 0.0;
+  const uint32_t id_i = live ? ids[i] : 0u;
+  for (long j0 = 0; j0 < v.n; j0 += kBruteTile) {
+    __syncthreads();
+    if (threadIdx.x < kBruteTile) {
+      const long j = j0 + threadIdx.x;
+      const bool ok = j < v.n && usable(v, j);
+      tx[threadIdx.x] = ok ? v.x[j] : 0.0;
+      ty[threadIdx.x] = ok ? v.y[j] : 0.0;
+      tz[threadIdx.x] = ok ? v.z[j] : 0.0;
+      ts[threadIdx.x] = ok ? species[j] : -1;
+      tid_s[threadIdx.x] = ok ? ids[j] : 0u;
+    }
+    __syncthreads();
+    const int cnt = static_cast<int>(min(static_cast<long>(kBruteTile), v.n - j0));
+    if (live)
+      for (int k = sub; k < cnt; k += kBruteLanes)
+        if (ts[k] == want)
+          contact_pair(R, dist2_exact(xi - tx[k], yi - ty[k], zi - tz[k]), static_cast<uint32_t>(i),
+                       static_cast<uint32_t>(j0 + k), id_i, tid_s[k], out, words, cap);
+  }
+  if (!kFused) return;
+  // the last block to finish matches; the words are ready for the next call
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(words + 1, 1ull) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  const long m = static_cast<long>(*static_cast<volatile unsigned long long*>(words));
+  unsigned long long marked = 0;
+  bool open = false;
+  if (m > 0) {
+    for (long k = threadIdx.x; k < m; k += kThreads) {
+      live_e[k] = 1;
+      matched[out[k].a] = 0;
+      matched[out[k].b] = 0;
+    }
+    open = match_rounds(out, m, best, matched, live_e, v.alive, &marked);
+  }
+  if (threadIdx.x == 0) {
+    words[2] = marked;
+    if (open) words[3] = 1;
+    words[0] = words[1] = 0;
+  }
+}
+
+// ---------------------------------------------------------------- dense grid
+struct CellGrid {
+  double o[3], inv_cs;
+  int dim[3];
+  int species;  // bit s: a live particle of species s
+};
+
+constexpr long kGridCellsPer = 4;          // cells per particle at most
+constexpr long kGridCellsMax = 1L << 25;
+inline long grid_cell_cap(long n) { return std::min(kGridCellsMax, std::max(4096L, kGridCellsPer * n)); }
+
+// Box of the particles that take part; the last block turns it into the grid.
+// bb: six box words, the species mask (~0 preset: complemented bits are
+// cleared) and the count of finished blocks (preset ~0).
+__global__ void __launch_bounds__(kBboxThreads)
+grid_setup_kernel(View v, const uint8_t* __restrict__ species, double radius, long cell_cap, unsigned long long* bb,
+                  CellGrid* __restrict__ grid) {
+  unsigned mask = 0;
+  bbox_block(
+      v,
+      [&](long i) {
+        const bool ok = usable(v, i);
+        if (ok && species) mask |= 1u << species[i];
+        return ok;
+      },
+      bb);
+  mask = __reduce_or_sync(0xffffffffu, mask);
+  if ((threadIdx.x & 31) == 0 && mask) atomicAnd(&bb[6], ~static_cast<unsigned long long>(mask));
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x != 0 || atomicAdd(&bb[7], 1ull) + 2 != gridDim.x) return;
+  __threadfence();
+  volatile unsigned long long* vb = bb;
+  CellGrid g;
+  double ext[3];
+  bool fin = true;
+  for (int d = 0; d < 3; ++d) {
+    const double lo = double_from_order_bits(vb[d]), hi = -double_from_order_bits(vb[3 + d]);
+    ext[d] = hi - lo;
+    g.o[d] = isfinite(lo) ? lo : 0.0;
+    fin = fin && ext[d] >= 0.0 && isfinite(ext[d]);
+  }
+  double cs = radius * (1.0 + 1e-9);
+  double cells = INFINITY, dim[3] = {1.0, 1.0, 1.0};
+  for (int it = 0; fin && it < 256; ++it) {  // cells no smaller than the radius, at most cell_cap of them
+    for (int d = 0; d < 3; ++d) dim[d] = floor(ext[d] / cs) + 1.0;
+    cells = dim[0] * dim[1] * dim[2];
+    if (cells <= static_cast<double>(cell_cap)) break;
+    cs *= fmax(1.05, fmin(cbrt(cells / static_cast<double>(cell_cap)), 1e6));
+  }
+  const bool ok = fin && cells <= static_cast<double>(cell_cap);
+  g.inv_cs = ok ? 1.0 / cs : 0.0;
+  for (int d = 0; d < 3; ++d) g.dim[d] = ok ? static_cast<int>(dim[d]) : 1;
+  g.species = static_cast<int>(~vb[6] & 0xffull);
+  *grid = g;
+}
+
+__device__ __forceinline__ void grid_cell(const CellGrid& g, double x, double y, double z, int c[3]) {
+  const double p[3] = {x, y, z};
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+    c[d] = max(0, static_cast<int>(fmin(floor((p[d] - g.o[d]) * g.inv_cs), static_cast<double>(g.dim[d] - 1))));
+}
+
+// cell[i] = cell of particle i, -1 when it takes no part; rank[i] = a place
+// among the cell's members. Cutoff (species null): live charged particles;
+// the others get their zero force here. Contacts: live particles whose
+// partner species is alive.
+template <bool kEnergy>
+__global__ void grid_count_kernel(View v, const uint8_t* __restrict__ species, const CellGrid* __restrict__ grid,
+                                  int* __restrict__ cell, int* __restrict__ rank, int* __restrict__ count,
+                                  double* __restrict__ epart) {
+  const long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
+  if (i >= v.n) return;
+  const CellGrid g = *grid;
+  bool part = usable(v, i);
+  if (species)
+    part = part && has_partner(species[i]) && ((g.species >> partner_of(species[i])) & 1);
+  else
+    part = part && v.q[i] != 0.0;
+  if (!part) {
+    cell[i] = -1;
+    if (!species) {
+      const double f[3] = {0.0, 0.0, 0.0};
+      cutoff_store<kEnergy>(v, i, 0.0, f, 0.0, epart);
+    }
+    return;
+  }
+  int c[3];
+  grid_cell(g, v.x[i], v.y[i], v.z[i], c);
+  const int id = (c[2] * g.dim[1] + c[1]) * g.dim[0] + c[0];
+  cell[i] = id;
+  rank[i] = atomicAdd(&count[id], 1);
+}
+
+__global__ void grid_scatter_kernel(long n, const int* __restrict__ cell, const int* __restrict__ rank,
+                                    const int* __restrict__ start, int* __restrict__ member) {
+  const long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
+  if (i < n && cell[i] >= 0) member[start[cell[i]] + rank[i]] = static_cast<int>(i);
+}
+
+// The records in cell order, a cell's members in ascending particle index:
+// position and charge (cutoff) or position and {id, species} (contacts).
+__global__ void grid_record_kernel(View v, const uint8_t* __restrict__ species, const uint32_t* __restrict__ ids,
+                                   const int* __restrict__ cell, const int* __restrict__ start, const int* __restrict__ m,
+                                   const int* __restrict__ member, double4* __restrict__ rec, int* __restrict__ index) {
+  const long p = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
+  if (p >= *m) return;
+  const int i = member[p], b = start[cell[i]], e = start[cell[i] + 1];
+  int r = 0;
+  for (int k = b; k < e; ++k) r += member[k] < i ? 1 : 0;
+  const double w = species ? __longlong_as_double(static_cast<long long>(
+                                 (static_cast<unsigned long long>(ids[i]) << 8) | species[i]))
+                           : v.q[i];
+  rec[b + r] = make_double4(v.x[i], v.y[i], v.z[i], w);
+  index[b + r] = i;
+}
+
+// Calls f(first, last) for the nine runs of records of the neighbour cells.
+template <typename F>
+__device__ __forceinline__ void neighbour_runs(const CellGrid& g, const int* __restrict__ start, double x, double y,
+                                               double z, F f) {
+  int c[3];
+  grid_cell(g, x, y, z, c);
+  const int x0 = max(c[0] - 1, 0), x1 = min(c[0] + 1, g.dim[0] - 1);
+  for (int cz = max(c[2] - 1, 0); cz <= min(c[2] + 1, g.dim[2] - 1); ++cz)
+    for (int cy = max(c[1] - 1, 0); cy <= min(c[1] + 1, g.dim[1] - 1); ++cy) {
+      const int row = (cz * g.dim[1] + cy) * g.dim[0];
+      f(start[row + x0], start[row + x1 + 1]);
+    }
+}
+
+template <bool kEnergy>
+__global__ void __launch_bounds__(128)
+cutoff_grid_kernel(View v, const CellGrid* __restrict__ grid, double rc, const int* __restrict__ start,
+                   const int* __restrict__ m, const double4* __restrict__ rec, const int* __restrict__ index,
+                   double* __restrict__ epart) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= *m) return;
+  const double4 me = rec[p];
+  const double rc2 = rc * rc, inv_rc = 1.0 / rc;
+  double f[3] = {0.0, 0.0, 0.0}, e = 0.0;
+  neighbour_runs(*grid, start, me.x, me.y, me.z, [&](int b, int end) {
+    for (int k = b; k < end; ++k) {
+      const double4 s = rec[k];
+      if (k != p) cutoff_pair<kEnergy>(me.x - s.x, me.y - s.y, me.z - s.z, s.w, rc2, inv_rc, f, e);
+    }
+  });
+  cutoff_store<kEnergy>(v, index[p], me.w, f, e, epart);
+}
+
+__global__ void __launch_bounds__(128)
+contact_grid_kernel(const CellGrid* __restrict__ grid, ContactRule R, const int* __restrict__ start,
+                    const int* __restrict__ m, const double4* __restrict__ rec, const int* __restrict__ index,
+                    Contact* __restrict__ out, unsigned long long* count, long cap) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= *m) return;
+  const double4 me = rec[p];
+  const unsigned long long tag = static_cast<unsigned long long>(__double_as_longlong(me.w));
+  const unsigned want = static_cast<unsigned>(partner_of(static_cast<int>(tag & 0xff)));
+  neighbour_runs(*grid, start, me.x, me.y, me.z, [&](int b, int end) {
+    for (int k = b; k < end; ++k) {
+      const double4 s = rec[k];
+      const unsigned long long st = static_cast<unsigned long long>(__double_as_longlong(s.w));
+      if ((st & 0xff) != want) continue;
+      contact_pair(R, dist2_exact(me.x - s.x, me.y - s.y, me.z - s.z), static_cast<uint32_t>(index[p]),
+                   static_cast<uint32_t>(index[k]), static_cast<uint32_t>(tag >> 8), static_cast<uint32_t>(st >> 8),
+                   out, count, cap);
+    }
+  });
+}
+
+struct CellList {
+  CellGrid* grid;
+  int* start;      // per cell, and the member count after the last one
+  int* m;          // = start + cells
+  double4* rec;
+  int* index;
+};
+
+// species null: the cutoff's list (zero forces written for the others).
+int build_cell_list(amk_ctx* c, const View& v, double radius, const uint8_t* species, const uint32_t* ids,
+                    double* epart, CellList* out) {
   int rc = AMK_OK;
-  const long n = v.n;
-  unsigned long long* bb = slot<unsigned long long>(c, kSlotCellStart, 8, &rc);
+  const long n = v.n, cells = grid_cell_cap(n);
+  unsigned long long* bb = slot<unsigned long long>(c, kSlotCellStart, 8 + (sizeof(CellGrid) + 7) / 8, &rc);
   AMK_TRY(rc);
-  uint64_t* keys = slot<uint64_t>(c, kSlotKeysA, n, &rc);
+  CellGrid* grid = reinterpret_cast<CellGrid*>(bb + 8);
+  int* cell = slot<int>(c, kSlotKeysA, 2 * static_cast<size_t>(n), &rc);
   AMK_TRY(rc);
-  uint32_t* vals = slot<uint32_t>(c, kSlotValsA, n, &rc);
+  int* rank = cell + n;
+  int* start = slot<int>(c, kSlotKeysB, static_cast<size_t>(cells) + 1, &rc);
   AMK_TRY(rc);
-  uint64_t* skeys = slot<uint64_t>(c, kSlotTreeKeys, n, &rc);
+  int* member = slot<int>(c, kSlotValsA, static_cast<size_t>(n), &rc);
   AMK_TRY(rc);
-  uint32_t* sidx = slot<uint32_t>(c, kSlotSorted0, n, &rc);
+  int* index = slot<int>(c, kSlotValsB, static_cast<size_t>(n), &rc);
   AMK_TRY(rc);
-  AMK_CUDA_TRY(cudaMemsetAsync(bb, 0xFF, 6 * sizeof(unsigned long long), c->stream));
-  bbox_kernel<<<148, 256, 0, c->stream>>>(v, bb);
-  AMK_TRY(check_launch(c, "bbox_kernel"));
-  cell_key_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, c->stream>>>(v, bb, radius, keys, vals);
-  AMK_TRY(check_launch(c, "cell_key_kernel"));
+  double4* rec = slot<double4>(c, kSlotSorted1, static_cast<size_t>(n), &rc);
+  AMK_TRY(rc);
+  const unsigned gn = static_cast<unsigned>((n + 255) / 256);
   AMK_TRY(phase_begin(c, AMK_PHASE_SORT));
-  AMK_TRY(radix_sort_pairs(c, keys, vals, skeys, sidx, n, 64));
+  AMK_CUDA_TRY(cudaMemsetAsync(bb, 0xFF, 8 * sizeof(unsigned long long), c->stream));
+  AMK_CUDA_TRY(cudaMemsetAsync(start, 0, static_cast<size_t>(cells) * sizeof(int), c->stream));
+  grid_setup_kernel<<<bbox_grid(n), kBboxThreads, 0, c->stream>>>(v, species, radius, cells, bb, grid);
+  AMK_TRY(check_launch(c, "grid_setup_kernel"));
+  if (epart)
+    grid_count_kernel<true><<<gn, 256, 0, c->stream>>>(v, species, grid, cell, rank, start, epart);
+  else
+    grid_count_kernel<false><<<gn, 256, 0, c->stream>>>(v, species, grid, cell, rank, start, nullptr);
+  AMK_TRY(check_launch(c, "grid_count_kernel"));
+  AMK_TRY(exclusive_scan_int(c, start, cells, start, start + cells));
+  grid_scatter_kernel<<<gn, 256, 0, c->stream>>>(n, cell, rank, start, member);
+  AMK_TRY(check_launch(c, "grid_scatter_kernel"));
+  grid_record_kernel<<<gn, 256, 0, c->stream>>>(v, species, ids, cell, start, start + cells, member, rec, index);
+  AMK_TRY(check_launch(c, "grid_record_kernel"));
   AMK_TRY(phase_end(c, AMK_PHASE_SORT));
-  out->bb = bb;
-  out->skeys = skeys;
-  out->sidx = sidx;
+  out->grid = grid;
+  out->start = start;
+  out->m = start + cells;
+  out->rec = rec;
+  out->index = index;
   return AMK_OK;
 }
 
@@ -304,19 +581,35 @@ int cutoff_forces(amk_ctx* c, const View& v, double cutoff, double* energy_out) 
     zero_forces_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, c->stream>>>(v);
     return check_launch(c, "zero_forces_kernel");
   }
-  CellList cl;
-  AMK_TRY(build_cell_list(c, v, cutoff, &cl));
   int rc = AMK_OK;
   double* epart = nullptr;
   if (energy_out) {
     epart = slot<double>(c, kSlotAuxState2, static_cast<size_t>(n) + 8, &rc);
     AMK_TRY(rc);
   }
-  AMK_TRY(phase_begin(c, AMK_PHASE_CUTOFF));
-  cutoff_kernel<<<static_cast<unsigned>((n + 127) / 128), 128, 0, c->stream>>>(v, cl.bb, cutoff, cl.skeys, cl.sidx,
-                                                                               epart);
-  AMK_TRY(check_launch(c, "cutoff_kernel"));
-  AMK_TRY(phase_end(c, AMK_PHASE_CUTOFF));
+  if (n <= kBruteMax) {
+    AMK_TRY(phase_begin(c, AMK_PHASE_CUTOFF));
+    const unsigned grid = brute_grid(n, kBruteThreads);
+    if (epart)
+      cutoff_brute_kernel<true><<<grid, kBruteThreads, 0, c->stream>>>(v, cutoff, epart);
+    else
+      cutoff_brute_kernel<false><<<grid, kBruteThreads, 0, c->stream>>>(v, cutoff, nullptr);
+    AMK_TRY(check_launch(c, "cutoff_brute_kernel"));
+    AMK_TRY(phase_end(c, AMK_PHASE_CUTOFF));
+  } else {
+    CellList cl;
+    AMK_TRY(build_cell_list(c, v, cutoff, nullptr, nullptr, epart, &cl));
+    AMK_TRY(phase_begin(c, AMK_PHASE_CUTOFF));
+    const unsigned grid = static_cast<unsigned>((n + 127) / 128);
+    if (epart)
+      cutoff_grid_kernel<true><<<grid, 128, 0, c->stream>>>(v, cl.grid, cutoff, cl.start, cl.m, cl.rec, cl.index,
+                                                            epart);
+    else
+      cutoff_grid_kernel<false><<<grid, 128, 0, c->stream>>>(v, cl.grid, cutoff, cl.start, cl.m, cl.rec, cl.index,
+                                                             nullptr);
+    AMK_TRY(check_launch(c, "cutoff_grid_kernel"));
+    AMK_TRY(phase_end(c, AMK_PHASE_CUTOFF));
+  }
   if (energy_out) {
     double* res = slot<double>(c, kSlotAuxState4, 8, &rc);
     AMK_TRY(rc);
@@ -329,41 +622,87 @@ int cutoff_forces(amk_ctx* c, const View& v, double cutoff, double* energy_out) 
   return AMK_OK;
 }
 
+// Buffers of a matching over the contacts of n particles.
+static int match_buffers(amk_ctx* c, long n, long m, unsigned long long** best, uint8_t** flags) {
+  int rc = AMK_OK;
+  // two per-particle priority arrays, then the matching state
+  *best = slot<unsigned long long>(c, kSlotAnnBest, 2 * static_cast<size_t>(n) + sizeof(MatchState) / 8 + 1, &rc);
+  AMK_TRY(rc);
+  *flags = slot<uint8_t>(c, kSlotAuxState1, static_cast<size_t>(n) + static_cast<size_t>(m) + 16, &rc);
+  return rc;
+}
+
+int annihilate_check(amk_ctx* c, long* marked) {
+  if (!c->ann_pending) return AMK_OK;
+  c->ann_pending = false;
+  int rc = AMK_OK;
+  unsigned long long* words = slot<unsigned long long>(c, kSlotAnnAux, 8, &rc);
+  AMK_TRY(rc);
+  unsigned long long res[2] = {0, 0};
+  AMK_CUDA_TRY(cudaMemcpyAsync(res, words + 2, sizeof(res), cudaMemcpyDeviceToHost, c->stream));
+  AMK_CUDA_TRY(cudaStreamSynchronize(c->stream));
+  if (res[1]) {
+    c->ann_words_clear = false;
+    return fail(AMK_ERR_TIMEOUT, "annihilation matching did not converge");
+  }
+  if (marked) *marked = static_cast<long>(res[0]);
+  return AMK_OK;
+}
+
 int annihilate_view(amk_ctx* c, const View& v, const uint8_t* species, const uint32_t* ids, double radius,
                     double probability, uint32_t seed, uint64_t step_index, long* marked) {
   if (marked) *marked = 0;
   if (!(radius > 0.0) || v.n == 0) return AMK_OK;  // annihilation.cc:34-35
-  CellList cl;
-  AMK_TRY(build_cell_list(c, v, radius, &cl));
+  const ContactRule R{radius * radius, probability, seed, step_index};
   int rc = AMK_OK;
-  unsigned long long* counters = slot<unsigned long long>(c, kSlotAnnAux, 8, &rc);
+  unsigned long long* words = slot<unsigned long long>(c, kSlotAnnAux, 8, &rc);
   AMK_TRY(rc);
+  unsigned long long* best = nullptr;
+  uint8_t* flags = nullptr;
+  if (v.n <= kFusedMax && match_grid_min() >= kMatchGridMin) {
+    const long cap = v.n * v.n / 2 + 1;  // directed contacts of a two-species set: at most 2 (n/2)^2
+    Contact* edges = slot<Contact>(c, kSlotAnnEdges, static_cast<size_t>(cap), &rc);
+    AMK_TRY(rc);
+    AMK_TRY(match_buffers(c, v.n, cap, &best, &flags));
+    if (!c->ann_words_clear) {
+      AMK_CUDA_TRY(cudaMemsetAsync(words, 0, 4 * sizeof(unsigned long long), c->stream));
+      c->ann_words_clear = true;
+    }
+    contact_brute_kernel<kFusedThreads, true><<<brute_grid(v.n, kFusedThreads), kFusedThreads, 0, c->stream>>>(
+        v, species, ids, R, edges, words, cap, best, flags, flags + v.n);
+    AMK_TRY(check_launch(c, "contact_brute_kernel"));
+    c->ann_pending = true;
+    return marked ? annihilate_check(c, marked) : AMK_OK;
+  }
+  AMK_TRY(annihilate_check(c, nullptr));  // the words are about to be reused
+  c->ann_words_clear = false;
+  CellList cl{};
+  if (v.n > kBruteMax) AMK_TRY(build_cell_list(c, v, radius, species, ids, nullptr, &cl));
   long cap = std::max<long>(1024, v.n / 16);
   for (int attempt = 0; attempt < 3; ++attempt) {
     Contact* edges = slot<Contact>(c, kSlotAnnEdges, static_cast<size_t>(cap), &rc);
     AMK_TRY(rc);
-    AMK_CUDA_TRY(cudaMemsetAsync(counters, 0, 4 * sizeof(unsigned long long), c->stream));
-    contact_kernel<<<static_cast<unsigned>((v.n + 127) / 128), 128, 0, c->stream>>>(
-        v, species, ids, cl.bb, radius, probability, seed, step_index, cl.skeys, cl.sidx, edges, counters, cap);
-    AMK_TRY(check_launch(c, "contact_kernel"));
+    AMK_CUDA_TRY(cudaMemsetAsync(words, 0, 4 * sizeof(unsigned long long), c->stream));
+    if (v.n <= kBruteMax)
+      contact_brute_kernel<kBruteThreads, false><<<brute_grid(v.n, kBruteThreads), kBruteThreads, 0, c->stream>>>(
+          v, species, ids, R, edges, words, cap, nullptr, nullptr, nullptr);
+    else
+      contact_grid_kernel<<<static_cast<unsigned>((v.n + 127) / 128), 128, 0, c->stream>>>(
+          cl.grid, R, cl.start, cl.m, cl.rec, cl.index, edges, words, cap);
+    AMK_TRY(check_launch(c, "contact kernel"));
     unsigned long long m = 0;
-    AMK_CUDA_TRY(cudaMemcpyAsync(&m, counters, sizeof(m), cudaMemcpyDeviceToHost, c->stream));
+    AMK_CUDA_TRY(cudaMemcpyAsync(&m, words, sizeof(m), cudaMemcpyDeviceToHost, c->stream));
     AMK_CUDA_TRY(cudaStreamSynchronize(c->stream));
     if (static_cast<long>(m) > cap) {
       cap = static_cast<long>(m) + 1024;
       continue;
     }
     if (m == 0) break;
-    // two per-particle priority arrays, then the matching state
-    unsigned long long* best = slot<unsigned long long>(
-        c, kSlotAnnBest, 2 * static_cast<size_t>(v.n) + sizeof(MatchState) / 8 + 1, &rc);
-    AMK_TRY(rc);
-    uint8_t* flags = slot<uint8_t>(c, kSlotAuxState1, static_cast<size_t>(v.n) + static_cast<size_t>(m) + 16, &rc);
-    AMK_TRY(rc);
+    AMK_TRY(match_buffers(c, v.n, static_cast<long>(m), &best, &flags));
     AMK_TRY(queue_matching(c, c->stream, edges, static_cast<long>(m), nullptr, best, best + v.n, flags, flags + v.n,
-                           v.alive, reinterpret_cast<MatchState*>(best + 2 * v.n), counters + 2));
+                           v.alive, reinterpret_cast<MatchState*>(best + 2 * v.n), words + 2));
     unsigned long long res[2] = {0, 0};
-    AMK_CUDA_TRY(cudaMemcpyAsync(res, counters + 2, sizeof(res), cudaMemcpyDeviceToHost, c->stream));
+    AMK_CUDA_TRY(cudaMemcpyAsync(res, words + 2, sizeof(res), cudaMemcpyDeviceToHost, c->stream));
     AMK_CUDA_TRY(cudaStreamSynchronize(c->stream));
     if (res[1]) return fail(AMK_ERR_TIMEOUT, "annihilation matching did not converge");
     if (marked) *marked = static_cast<long>(res[0]);
@@ -488,6 +827,11 @@ extern "C" int amk_coulomb_standard_noalloc(const double* x, const double* y, co
     AMK_CUDA_TRY(cudaGetLastError());
     return AMK_OK;
   }
+  if (n <= kBruteMax) {  // needs no scratch
+    cutoff_brute_kernel<false><<<brute_grid(n, kBruteThreads), kBruteThreads, 0, s>>>(v, cutoff_radius, nullptr);
+    AMK_CUDA_TRY(cudaGetLastError());
+    return AMK_OK;
+  }
   unsigned long long* bb = reinterpret_cast<unsigned long long*>(base + kNaBbox);
   uint64_t* keys = reinterpret_cast<uint64_t*>(base + kNaKeys);
   uint32_t* vals = reinterpret_cast<uint32_t*>(base + kNaVals);
@@ -497,11 +841,11 @@ extern "C" int amk_coulomb_standard_noalloc(const double* x, const double* y, co
   uint32_t* vtmp = reinterpret_cast<uint32_t*>(base + kNaTVals);
   uint32_t* hist = reinterpret_cast<uint32_t*>(base + kNaHist);
   AMK_CUDA_TRY(cudaMemsetAsync(bb, 0xFF, 6 * sizeof(unsigned long long), s));
-  bbox_kernel<<<148, 256, 0, s>>>(v, bb);
+  bbox_kernel<<<bbox_grid(n), kBboxThreads, 0, s>>>(v, bb);
   cell_key_kernel<<<blocks, 256, 0, s>>>(v, bb, cutoff_radius, keys, vals);
   AMK_CUDA_TRY(cudaGetLastError());
   AMK_CUDA_TRY(radix_sort_pairs_buffers(s, keys, vals, skeys, sidx, ktmp, vtmp, hist, n, 64));
-  cutoff_kernel<<<static_cast<unsigned>((n + 127) / 128), 128, 0, s>>>(v, bb, cutoff_radius, skeys, sidx, nullptr);
+  cutoff_kernel<<<static_cast<unsigned>((n + 127) / 128), 128, 0, s>>>(v, bb, cutoff_radius, skeys, sidx);
   AMK_CUDA_TRY(cudaGetLastError());
   return AMK_OK;
 }

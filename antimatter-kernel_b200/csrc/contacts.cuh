@@ -101,25 +101,16 @@ __global__ void match_select_kernel(const Contact* __restrict__ e, long m_cap, c
   if ((threadIdx.x & 31) == 0 && marked) atomicAdd(&result[0], marked);
 }
 
-// One CTA: the whole matching (resume = 0), or the continuation of the
-// grid-wide rounds from their live / matched flags and marked count
-// (resume = 1; nothing left to do when the last grid round saw no live
-// contact).
-__global__ void __launch_bounds__(1024)
-match_kernel(const Contact* __restrict__ e, long m_cap, const unsigned long long* __restrict__ m_count, unsigned long long* best, uint8_t* matched, uint8_t* live_e,
-             uint8_t* alive, unsigned long long* result, int resume, const MatchState* st) {
+// The rounds of the matching by one block, from the live / matched flags of
+// the contacts e[0, m): adds the particles marked to *marked_out (thread 0's
+// value counts) and returns whether contacts were left (it did not converge:
+// cannot happen, a round selects at least one contact).
+__device__ __forceinline__ bool match_rounds(const Contact* __restrict__ e, long m, unsigned long long* best,
+                                             uint8_t* matched, uint8_t* live_e, uint8_t* alive,
+                                             unsigned long long* marked_out) {
   __shared__ int s_remaining;
   __shared__ unsigned long long s_marked;
-  const long m = match_count(m_cap, m_count);
-  if (resume && st->live[kMatchRounds - 1] == 0) return;  // converged in the grid rounds (result kept)
-  if (!resume) {
-    for (long k = threadIdx.x; k < m; k += blockDim.x) {
-      live_e[k] = 1;
-      matched[e[k].a] = 0;
-      matched[e[k].b] = 0;
-    }
-  }
-  if (threadIdx.x == 0) s_marked = resume ? result[0] : 0;
+  if (threadIdx.x == 0) s_marked = *marked_out;
   __syncthreads();
   long rounds = 0;
   for (;;) {
@@ -163,18 +154,41 @@ match_kernel(const Contact* __restrict__ e, long m_cap, const unsigned long long
     if (s_remaining == 0 || rounds > m + 1) break;
     __syncthreads();
   }
+  *marked_out = s_marked;
+  return s_remaining != 0;
+}
+
+// One CTA: the whole matching (resume = 0), or the continuation of the
+// grid-wide rounds from their live / matched flags and marked count
+// (resume = 1; nothing left to do when the last grid round saw no live
+// contact).
+__global__ void __launch_bounds__(1024)
+match_kernel(const Contact* __restrict__ e, long m_cap, const unsigned long long* __restrict__ m_count, unsigned long long* best, uint8_t* matched, uint8_t* live_e,
+             uint8_t* alive, unsigned long long* result, int resume, const MatchState* st) {
+  const long m = match_count(m_cap, m_count);
+  if (resume && st->live[kMatchRounds - 1] == 0) return;  // converged in the grid rounds (result kept)
+  if (!resume) {
+    for (long k = threadIdx.x; k < m; k += blockDim.x) {
+      live_e[k] = 1;
+      matched[e[k].a] = 0;
+      matched[e[k].b] = 0;
+    }
+  }
+  unsigned long long marked = resume ? result[0] : 0;
+  const bool open = match_rounds(e, m, best, matched, live_e, alive, &marked);
   if (threadIdx.x == 0) {
-    result[0] = s_marked;
-    result[1] = s_remaining ? 1ull : 0ull;  // 1 = did not converge (cannot happen)
+    result[0] = marked;
+    result[1] = open ? 1ull : 0ull;
   }
 }
 
 // Contacts from which the grid-wide rounds are used (AMK_MATCH_GRID_MIN
 // overrides it: tests of that path on small sets).
+constexpr long kMatchGridMin = 8192;
 inline long match_grid_min() {
   const char* s = getenv("AMK_MATCH_GRID_MIN");
   if (s && *s) return atol(s);
-  return 8192;
+  return kMatchGridMin;
 }
 
 // Queues the matching of the contacts e[0, m) (m = min(m_cap, *m_count) when

@@ -73,52 +73,11 @@ View main_view(amk_ctx* c) {
   v.z = c->z.as<double>();
   v.q = c->q.as<double>();
   v.alive = c->alive.as<uint8_t>();
-  v.hq = c->hq.as<float4>();
-  v.lo = c->lo.as<float4>();
   v.fx = c->fx.as<double>();
   v.fy = c->fy.as<double>();
   v.fz = c->fz.as<double>();
   v.length_scale = c->length_scale;
   return v;
-}
-
-// x / L split into a float pair: hi = fl(x/L), lo = fl(x/L - hi). Dead,
-// neutral and non-finite particles get q_e = 0 and a zero position so that
-// they drop out of every pair sum (coulomb_interaction.cc:52-56,64-66).
-__global__ void stage_kernel(long n, const double* __restrict__ x, const double* __restrict__ y,
-                             const double* __restrict__ z, const double* __restrict__ q,
-                             const uint8_t* __restrict__ alive, double inv_l, float4* __restrict__ hq,
-                             float4* __restrict__ lo) {
-  const long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
-  if (i >= n) return;
-  const double xs = x[i] * inv_l, ys = y[i] * inv_l, zs = z[i] * inv_l;
-  const bool ok = (alive == nullptr || alive[i]) && q[i] != 0.0 && isfinite(xs) && isfinite(ys) &&
-                  isfinite(zs);
-  float4 h, l;
-  if (ok) {
-    h.x = __double2float_rn(xs);
-    h.y = __double2float_rn(ys);
-    h.z = __double2float_rn(zs);
-    h.w = __double2float_rn(q[i] / kElementaryCharge);
-    l.x = __double2float_rn(xs - static_cast<double>(h.x));
-    l.y = __double2float_rn(ys - static_cast<double>(h.y));
-    l.z = __double2float_rn(zs - static_cast<double>(h.z));
-    l.w = 0.0f;
-  } else {
-    h = make_float4(0.f, 0.f, 0.f, 0.f);
-    l = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-  hq[i] = h;
-  lo[i] = l;
-}
-
-int stage_view(amk_ctx* c, const View& v) {
-  if (v.n == 0) return AMK_OK;
-  const int threads = 256;
-  const long blocks = (v.n + threads - 1) / threads;
-  stage_kernel<<<static_cast<unsigned>(blocks), threads, 0, c->stream>>>(
-      v.n, v.x, v.y, v.z, v.q, v.alive, 1.0 / v.length_scale, v.hq, v.lo);
-  return check_launch(c, "stage_kernel");
 }
 
 int phase_begin(amk_ctx* c, int phase) { return phase_begin_on(c, phase, c->stream); }
@@ -455,7 +414,6 @@ static int finish_load(amk_ctx* c, long n) {
   double mabs;
   std::memcpy(&mabs, &bits, sizeof(mabs));
   c->length_scale = length_scale_for(mabs);
-  c->stage_dirty = true;
   return AMK_OK;
 }
 
@@ -515,7 +473,6 @@ extern "C" int amk_update_state(amk_ctx* c, const double* x, const double* y, co
   AMK_CUDA_TRY(cudaMemcpyAsync(c->vx.ptr, vx, nd, cudaMemcpyHostToDevice, c->stream));
   AMK_CUDA_TRY(cudaMemcpyAsync(c->vy.ptr, vy, nd, cudaMemcpyHostToDevice, c->stream));
   AMK_CUDA_TRY(cudaMemcpyAsync(c->vz.ptr, vz, nd, cudaMemcpyHostToDevice, c->stream));
-  c->stage_dirty = true;
   return AMK_OK;
 }
 
@@ -525,7 +482,6 @@ extern "C" int amk_set_charge_mass(amk_ctx* c, const double* charge, const doubl
   if (c->n == 0) return AMK_OK;
   if (charge) AMK_CUDA_TRY(cudaMemcpyAsync(c->q.ptr, charge, nd, cudaMemcpyHostToDevice, c->stream));
   if (mass) AMK_CUDA_TRY(cudaMemcpyAsync(c->m.ptr, mass, nd, cudaMemcpyHostToDevice, c->stream));
-  c->stage_dirty = true;
   return AMK_OK;
 }
 
@@ -556,7 +512,6 @@ extern "C" int amk_set_alive(amk_ctx* c, const uint8_t* alive) {
   if (c->n == 0) return AMK_OK;
   if (!alive) return fail(AMK_ERR_INVALID, "amk_set_alive: null array");
   AMK_CUDA_TRY(cudaMemcpyAsync(c->alive.ptr, alive, static_cast<size_t>(c->n), cudaMemcpyHostToDevice, c->stream));
-  c->stage_dirty = true;
   return AMK_OK;
 }
 
@@ -817,7 +772,6 @@ extern "C" int amk_push(amk_ctx* c) {
   if (c->batch) return fail(AMK_ERR_STATE, "the context holds a batch: step it with amk_batch_step");
   if (c->n > 0) {
     AMK_TRY(push_step(c, static_cast<uint64_t>(c->step + 1)));
-    c->stage_dirty = true;
   }
   c->step++;
   return AMK_OK;
@@ -829,8 +783,7 @@ extern "C" int amk_annihilate(amk_ctx* c, long* marked) {
   if (marked) *marked = 0;
   if (c->n == 0 || !c->p.annihilation_enabled) return AMK_OK;
   AMK_TRY(annihilate_step(c, static_cast<uint64_t>(c->step > 0 ? c->step : 1), marked));
-  c->stage_dirty = true;
-  return AMK_OK;
+  return annihilate_check(c, nullptr);
 }
 
 extern "C" int amk_step(amk_ctx* c, int nsteps) {
@@ -852,9 +805,9 @@ extern "C" int amk_step(amk_ctx* c, int nsteps) {
     }
     if (c->n > 0) AMK_TRY(amk_coulomb(c));
     AMK_TRY(amk_push(c));
-    if (c->n > 0 && c->p.annihilation_enabled) AMK_TRY(amk_annihilate(c, nullptr));
+    if (c->n > 0 && c->p.annihilation_enabled) AMK_TRY(annihilate_step(c, static_cast<uint64_t>(c->step), nullptr));
   }
-  return AMK_OK;
+  return annihilate_check(c, nullptr);  // small sets match without a read-back per step
 }
 
 extern "C" long amk_step_count(const amk_ctx* c) { return c ? c->step : -1; }

@@ -164,6 +164,9 @@ extern "C" int amk_energy(amk_ctx* c, int time_centre, amk_energy_out* out) {
       c->n, c->x.as<double>(), c->y.as<double>(), c->z.as<double>(), c->vx.as<double>(), c->vy.as<double>(),
       c->vz.as<double>(), c->q.as<double>(), c->m.as<double>(), c->alive.as<uint8_t>(), trap_coef, part);
   AMK_TRY(check_launch(c, "ke_trap_kernel"));
+  double coul = 0.0;
+  if (c->p.coulomb_forces_enabled)
+    AMK_TRY(coulomb_energy_view(c, main_view(c), c->p, c->p.energy_method, &coul));
   std::vector<double> h(3 * kRedBlocks);
   AMK_CUDA_TRY(cudaMemcpyAsync(h.data(), part, h.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   AMK_CUDA_TRY(cudaStreamSynchronize(c->stream));
@@ -172,14 +175,6 @@ extern "C" int amk_energy(amk_ctx* c, int time_centre, amk_energy_out* out) {
     ke += h[3 * b];
     pe += h[3 * b + 1];
     cnt += h[3 * b + 2];
-  }
-  double coul = 0.0;
-  if (c->p.coulomb_forces_enabled) {
-    if (c->stage_dirty) {
-      AMK_TRY(stage_view(c, main_view(c)));
-      c->stage_dirty = false;
-    }
-    AMK_TRY(coulomb_energy_view(c, main_view(c), c->p, c->p.energy_method, &coul));
   }
   AMK_TRY(phase_end(c, AMK_PHASE_ENERGY));
   out->kinetic = ke;

@@ -302,7 +302,6 @@ extern "C" int amk_checkpoint_load(amk_ctx* c, const char* path) {
   c->learned_fallback = h.learned_fallback != 0;
   c->learned_last_error = h.learned_last_error;
   c->length_scale = h.length_scale;
-  c->stage_dirty = true;
   return AMK_OK;
 }
 

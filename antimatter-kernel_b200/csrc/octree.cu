@@ -26,6 +26,7 @@
 #include <algorithm>
 
 #include "amk_internal.cuh"
+#include "bbox.cuh"
 
 namespace amk {
 namespace {
@@ -38,29 +39,8 @@ __device__ __forceinline__ bool is_source(const View& v, long i, int mode) {
   return isfinite(v.x[i]) && isfinite(v.y[i]) && isfinite(v.z[i]);
 }
 
-__global__ void tree_bbox_kernel(View v, int mode, unsigned long long* bb) {
-  double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-  for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < v.n;
-       i += static_cast<long>(gridDim.x) * blockDim.x) {
-    if (!is_source(v, i, mode)) continue;
-    const double p[3] = {v.x[i], v.y[i], v.z[i]};
-    for (int d = 0; d < 3; ++d) {
-      lo[d] = fmin(lo[d], p[d]);
-      hi[d] = fmax(hi[d], p[d]);
-    }
-  }
-  for (int d = 0; d < 3; ++d) {
-    for (int o = 16; o > 0; o >>= 1) {
-      lo[d] = fmin(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
-      hi[d] = fmax(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
-    }
-  }
-  if ((threadIdx.x & 31) == 0) {
-    for (int d = 0; d < 3; ++d) {
-      atomicMin(&bb[d], double_order_bits(lo[d]));
-      atomicMin(&bb[3 + d], double_order_bits(-hi[d]));
-    }
-  }
+__global__ void __launch_bounds__(kBboxThreads) tree_bbox_kernel(View v, int mode, unsigned long long* bb) {
+  bbox_block(v, [&](long i) { return is_source(v, i, mode); }, bb);
 }
 
 // Root cube: barnes-hut.cc:46-61 (Barnes-Hut) / fast-multipole.cc:355-397.
@@ -296,7 +276,7 @@ int build_octree(amk_ctx* c, const View& v, int leaf_cap, int mode, Octree* t) {
   AMK_TRY(rc);
 
   AMK_CUDA_TRY(cudaMemsetAsync(bb, 0xFF, 6 * sizeof(unsigned long long), c->stream));
-  tree_bbox_kernel<<<148, 256, 0, c->stream>>>(v, mode, bb);
+  tree_bbox_kernel<<<bbox_grid(n), kBboxThreads, 0, c->stream>>>(v, mode, bb);
   AMK_TRY(check_launch(c, "tree_bbox_kernel"));
   tree_root_kernel<<<1, 1, 0, c->stream>>>(bb, mode, frame);
   AMK_TRY(check_launch(c, "tree_root_kernel"));

@@ -16,8 +16,6 @@ int load_aux_view(amk_ctx* c, long n, const double* x, const double* y, const do
   if (n > c->aux_capacity) {
     const size_t nd = static_cast<size_t>(n) * sizeof(double);
     for (DevBuf* b : {&c->ax, &c->ay, &c->az, &c->aq, &c->afx, &c->afy, &c->afz, &c->aphi}) AMK_TRY(b->reserve(nd));
-    AMK_TRY(c->ahq.reserve(static_cast<size_t>(n) * sizeof(float4)));
-    AMK_TRY(c->alo.reserve(static_cast<size_t>(n) * sizeof(float4)));
     c->aux_capacity = n;
   }
   const size_t nd = static_cast<size_t>(n) * sizeof(double);
@@ -39,14 +37,11 @@ int load_aux_view(amk_ctx* c, long n, const double* x, const double* y, const do
   v.z = c->az.as<double>();
   v.q = c->aq.as<double>();
   v.alive = nullptr;
-  v.hq = c->ahq.as<float4>();
-  v.lo = c->alo.as<float4>();
   v.fx = c->afx.as<double>();
   v.fy = c->afy.as<double>();
   v.fz = c->afz.as<double>();
   v.phi = nullptr;
   v.length_scale = length_scale_for(mx);
-  AMK_TRY(stage_view(c, v));
   *out = v;
   return AMK_OK;
 }
