@@ -64,11 +64,20 @@ struct FmmHostTables {
   std::vector<int> deg_start;                // n_d entries grouped by degree
   std::vector<int> rec_axis;                 // per k
   std::vector<int> rec_delta, rec_m1, rec_m2;  // 3 per k
-  std::vector<int> m2l_index;                // [g * n_m + a]
   std::vector<short> m2l_index_t;            // [a * n_m + g]
   std::vector<int> m2m_off, m2m_b, m2m_c;    // CSR by a
   std::vector<int> l2l_off, l2l_b, l2l_c;    // CSR by a
   std::vector<int> grad;                     // 3 per g, -1 none
+  // Harmonic basis of the FP64 M2L products (see m2l_class_mma_kernel): the
+  // n_r = (p+1)^2 coefficients with z exponent 0 or 1, the derivatives with
+  // z exponent at most 2 (n_d2 of them, with their own recurrence), the map
+  // of the source coefficients onto the basis and of its sums back.
+  int n_r = 0, n_d2 = 0;
+  std::vector<int> red_deg;                  // degree per basis coefficient
+  std::vector<int> rd_off, rd_a, ex_off, ex_r;
+  std::vector<double> rd_c, ex_c;
+  std::vector<int> deg_start2, rec_axis2, rec_delta2, rec_m12, rec_m22;
+  std::vector<short> red_index_t;            // [a * n_r + g]
 
   explicit FmmHostTables(int order) : p(order) {
     const int dmax = 2 * p;
@@ -112,13 +121,11 @@ struct FmmHostTables {
         if (m[j] >= 2) rec_m2[3 * k + j] = pos(t);
       }
     }
-    // M2L: D_{g+a}; transposed copy for the class products
-    m2l_index.resize(static_cast<size_t>(n_m) * n_m);
+    // M2L: D_{g+a}, the source index a first
     m2l_index_t.resize(static_cast<size_t>(n_m) * n_m);
     for (int g = 0; g < n_m; ++g)
       for (int a = 0; a < n_m; ++a) {
         const int s3[3] = {multi[g].x + multi[a].x, multi[g].y + multi[a].y, multi[g].z + multi[a].z};
-        m2l_index[static_cast<size_t>(g) * n_m + a] = pos(s3);
         m2l_index_t[static_cast<size_t>(a) * n_m + g] = static_cast<short>(pos(s3));
       }
     // M2M (child -> parent): M_a += M_b * d^(a-b) / (a-b)! over b <= a;
@@ -154,23 +161,98 @@ struct FmmHostTables {
           grad[3 * g + k] = pos(t);
         }
     }
+    // 1/r is harmonic: d_z^2 = -(d_x^2 + d_y^2), so for z = 2 k + r
+    //   D_(x,y,z) = (-1)^k sum_j C(k,j) D_(x+2j, y+2(k-j), r).
+    // The source side collects M_a into the basis with those weights, the
+    // target side builds the other coefficients from the basis.
+    std::vector<int> red(n_m, -1);
+    std::vector<int> full;
+    for (int a = 0; a < n_m; ++a)
+      if (multi[a].z <= 1) {
+        red[a] = n_r++;
+        full.push_back(a);
+        red_deg.push_back(multi[a].w);
+      }
+    auto choose = [](int n, int k) {
+      double c = 1.0;
+      for (int i = 1; i <= k; ++i) c = c * (n - k + i) / i;
+      return c;
+    };
+    std::vector<std::vector<std::pair<int, double>>> collect(n_r);
+    ex_off.push_back(0);
+    for (int a = 0; a < n_m; ++a) {
+      const int4 m = multi[a];
+      const int k = m.z / 2;
+      for (int j = 0; j <= k; ++j) {
+        const double w = (k % 2 ? -1.0 : 1.0) * choose(k, j);
+        const int r = red[graded_index(m.x + 2 * j, m.y + 2 * (k - j), m.z % 2)];
+        collect[r].push_back({a, w});
+        ex_r.push_back(r);
+        ex_c.push_back(w);
+      }
+      ex_off.push_back(static_cast<int>(ex_r.size()));
+    }
+    rd_off.push_back(0);
+    for (const auto& l : collect) {
+      for (const auto& e : l) {
+        rd_a.push_back(e.first);
+        rd_c.push_back(e.second);
+      }
+      rd_off.push_back(static_cast<int>(rd_a.size()));
+    }
+    std::vector<int> pos2(n_d, -1);
+    for (int k = 0; k < n_d; ++k) {
+      if (k == deg_start[deg_start2.size()]) deg_start2.push_back(n_d2);
+      if (multi[k].z <= 2) pos2[k] = n_d2++;
+    }
+    deg_start2.push_back(n_d2);
+    for (int k = 0; k < n_d; ++k) {
+      if (pos2[k] < 0) continue;
+      rec_axis2.push_back(rec_axis[k]);
+      for (int j = 0; j < 3; ++j) {
+        rec_delta2.push_back(rec_delta[3 * k + j]);
+        rec_m12.push_back(rec_m1[3 * k + j] < 0 ? -1 : pos2[rec_m1[3 * k + j]]);
+        rec_m22.push_back(rec_m2[3 * k + j] < 0 ? -1 : pos2[rec_m2[3 * k + j]]);
+      }
+    }
+    for (int a = 0; a < n_r; ++a)
+      for (int g = 0; g < n_r; ++g) {
+        const int4 u = multi[full[a]], v = multi[full[g]];
+        red_index_t.push_back(static_cast<short>(pos2[graded_index(u.x + v.x, u.y + v.y, u.z + v.z)]));
+      }
   }
 };
 
 // Device copy of one order's tables.
+// Recurrence of the derivatives of 1/r over one index set.
+struct DerivTables {
+  int p, n;  // degrees up to 2 p, n indices
+  const int* deg_start;
+  const int* axis;
+  const int* delta;
+  const int* m1;
+  const int* m2;
+};
+
 struct FmmDevTables {
   int p, n_m, n_d;
   const int4* multi;
   const double* fact;
   const double* inv_fact;
   const double* sign;
-  const int* deg_start;
-  const int* rec_axis;
-  const int* rec_delta;
-  const int* rec_m1;
-  const int* rec_m2;
-  const int* m2l_index;
+  DerivTables d_all;  // every index up to degree 2 p
   const short* m2l_index_t;
+  // harmonic basis (FP64 products)
+  int n_r, n_rp;      // coefficients; row pitch of the per-cell and per-pair rows (a multiple of 4)
+  DerivTables d_red;  // the indices with z exponent at most 2
+  const short* red_index_t;
+  const int* red_deg;
+  const int* rd_off;
+  const int* rd_a;
+  const double* rd_c;
+  const int* ex_off;
+  const int* ex_r;
+  const double* ex_c;
   const int* m2m_off;
   const int* m2m_b;
   const int* m2m_c;
@@ -247,9 +329,13 @@ int get_tables(amk_ctx* c, int order, FmmDevTables* out) {
   const size_t o_multi = append(blob, h.multi), o_fact = append(blob, h.fact), o_if = append(blob, h.inv_fact),
                o_sign = append(blob, h.sign), o_ds = append(blob, h.deg_start), o_ax = append(blob, h.rec_axis),
                o_de = append(blob, h.rec_delta), o_m1 = append(blob, h.rec_m1), o_m2 = append(blob, h.rec_m2),
-               o_idx = append(blob, h.m2l_index), o_idt = append(blob, h.m2l_index_t), o_mo = append(blob, h.m2m_off), o_mb = append(blob, h.m2m_b),
+               o_idt = append(blob, h.m2l_index_t), o_mo = append(blob, h.m2m_off), o_mb = append(blob, h.m2m_b),
                o_mc = append(blob, h.m2m_c), o_lo = append(blob, h.l2l_off), o_lb = append(blob, h.l2l_b),
-               o_lc = append(blob, h.l2l_c), o_g = append(blob, h.grad);
+               o_lc = append(blob, h.l2l_c), o_g = append(blob, h.grad), o_ds2 = append(blob, h.deg_start2),
+               o_ax2 = append(blob, h.rec_axis2), o_de2 = append(blob, h.rec_delta2), o_m12 = append(blob, h.rec_m12),
+               o_m22 = append(blob, h.rec_m22), o_rit = append(blob, h.red_index_t), o_rdeg = append(blob, h.red_deg),
+               o_rdo = append(blob, h.rd_off), o_rda = append(blob, h.rd_a), o_rdc = append(blob, h.rd_c),
+               o_exo = append(blob, h.ex_off), o_exr = append(blob, h.ex_r), o_exc = append(blob, h.ex_c);
   DevBuf* buf = new DevBuf();
   int rc = buf->reserve(blob.size());
   if (rc != AMK_OK) {
@@ -266,12 +352,19 @@ int get_tables(amk_ctx* c, int order, FmmDevTables* out) {
   t.fact = reinterpret_cast<const double*>(b + o_fact);
   t.inv_fact = reinterpret_cast<const double*>(b + o_if);
   t.sign = reinterpret_cast<const double*>(b + o_sign);
-  t.deg_start = reinterpret_cast<const int*>(b + o_ds);
-  t.rec_axis = reinterpret_cast<const int*>(b + o_ax);
-  t.rec_delta = reinterpret_cast<const int*>(b + o_de);
-  t.rec_m1 = reinterpret_cast<const int*>(b + o_m1);
-  t.rec_m2 = reinterpret_cast<const int*>(b + o_m2);
-  t.m2l_index = reinterpret_cast<const int*>(b + o_idx);
+  auto ints = [&](size_t o) { return reinterpret_cast<const int*>(b + o); };
+  t.d_all = DerivTables{h.p, h.n_d, ints(o_ds), ints(o_ax), ints(o_de), ints(o_m1), ints(o_m2)};
+  t.n_r = h.n_r;
+  t.n_rp = 4 * ((h.n_r + 3) / 4);
+  t.d_red = DerivTables{h.p, h.n_d2, ints(o_ds2), ints(o_ax2), ints(o_de2), ints(o_m12), ints(o_m22)};
+  t.red_index_t = reinterpret_cast<const short*>(b + o_rit);
+  t.red_deg = ints(o_rdeg);
+  t.rd_off = ints(o_rdo);
+  t.rd_a = ints(o_rda);
+  t.rd_c = reinterpret_cast<const double*>(b + o_rdc);
+  t.ex_off = ints(o_exo);
+  t.ex_r = ints(o_exr);
+  t.ex_c = reinterpret_cast<const double*>(b + o_exc);
   t.m2l_index_t = reinterpret_cast<const short*>(b + o_idt);
   t.m2m_off = reinterpret_cast<const int*>(b + o_mo);
   t.m2m_b = reinterpret_cast<const int*>(b + o_mb);
@@ -690,6 +783,26 @@ __global__ void m2l_rescale_kernel(const Octree t, FmmDevTables T, const double*
   Mh[e] = M[e] * f;
 }
 
+// The same on the harmonic basis (FP64 products): row s of n_rp doubles,
+// Mr[s][r] = sum over the a collected by r of w (-1)^|a| M[s][a] h_s^{-|a|},
+// zero past n_r.
+__global__ void m2l_rescale_red_kernel(const Octree t, FmmDevTables T, const double* __restrict__ M,
+                                       double* __restrict__ Mr) {
+  const long e = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
+  if (e >= t.n_nodes * T.n_rp) return;
+  const int s = static_cast<int>(e / T.n_rp), r = static_cast<int>(e - static_cast<long>(s) * T.n_rp);
+  double v = 0.0;
+  if (r < T.n_r) {
+    const double* m = M + static_cast<size_t>(s) * T.n_m;
+    for (int k = T.rd_off[r]; k < T.rd_off[r + 1]; ++k) v += T.rd_c[k] * m[T.rd_a[k]];
+    const double ih = 1.0 / t.center[s].w;
+    double f = T.red_deg[r] & 1 ? -1.0 : 1.0;
+    for (int d = 0; d < T.red_deg[r]; ++d) f *= ih;
+    v *= f;
+  }
+  Mr[e] = v;
+}
+
 // Class slot (-1: per-pair path) and target of every pair (a warp per target);
 // refl (tensor-core mode) is cleared: every pair starts unreflected.
 __global__ void m2l_classify_kernel(const Octree t, const int* __restrict__ off, const int* __restrict__ count,
@@ -809,22 +922,22 @@ __global__ void m2l_scatter_kernel(const int* __restrict__ codes, long e0, long 
   }
 }
 
-// D recurrence (fast-multipole.cc:207-232) for displacement xs into D[0, n_d), one warp.
-__device__ __forceinline__ void m2l_derivatives(const FmmDevTables& T, int lane, const double xs[3], double* D) {
+// D recurrence (fast-multipole.cc:207-232) for displacement xs into D[0, T.n), one warp.
+__device__ __forceinline__ void m2l_derivatives(const DerivTables& T, int lane, const double xs[3], double* D) {
   const double inv_r2 = 1.0 / (xs[0] * xs[0] + xs[1] * xs[1] + xs[2] * xs[2]);
   if (lane == 0) D[0] = sqrt(inv_r2);
   __syncwarp();
   for (int deg = 1; deg <= 2 * T.p; ++deg) {
     for (int k = T.deg_start[deg] + lane; k < T.deg_start[deg + 1]; k += 32) {
-      const int i = T.rec_axis[k];
-      const int di = T.rec_delta[3 * k + i];
-      double sum = (2 * di - 1) * xs[i] * D[T.rec_m1[3 * k + i]];
-      if (T.rec_m2[3 * k + i] >= 0) sum += (di - 1) * (di - 1) * D[T.rec_m2[3 * k + i]];
+      const int i = T.axis[k];
+      const int di = T.delta[3 * k + i];
+      double sum = (2 * di - 1) * xs[i] * D[T.m1[3 * k + i]];
+      if (T.m2[3 * k + i] >= 0) sum += (di - 1) * (di - 1) * D[T.m2[3 * k + i]];
       for (int j = 0; j < 3; ++j) {
-        const int dj = T.rec_delta[3 * k + j];
+        const int dj = T.delta[3 * k + j];
         if (j == i || dj == 0) continue;
-        sum += 2.0 * dj * xs[j] * D[T.rec_m1[3 * k + j]];
-        if (T.rec_m2[3 * k + j] >= 0) sum += dj * (dj - 1) * D[T.rec_m2[3 * k + j]];
+        sum += 2.0 * dj * xs[j] * D[T.m1[3 * k + j]];
+        if (T.m2[3 * k + j] >= 0) sum += dj * (dj - 1) * D[T.m2[3 * k + j]];
       }
       D[k] = -sum * inv_r2;
     }
@@ -834,16 +947,16 @@ __device__ __forceinline__ void m2l_derivatives(const FmmDevTables& T, int lane,
 
 __device__ __forceinline__ void split3_bf16(double v, __nv_bfloat16* t);
 
-// D(v) of every class: a warp per class, into table[class * n_d + k], or
+// D(v) of every class: a warp per class, into table[class * n + k], or
 // (tensor-core mode, table3 given) split into three BF16 terms packed as
-// {t0 | t1 << 16, t2} into table3[class * nd3 + k], zero for k >= n_d.
+// {t0 | t1 << 16, t2} into table3[class * nd3 + k], zero for k >= n.
 __global__ void __launch_bounds__(32 * kFmmWarps)
-m2l_table_kernel(FmmDevTables T, const int* __restrict__ cls_code, int n_classes,
+m2l_table_kernel(DerivTables T, const int* __restrict__ cls_code, int n_classes,
                  const unsigned long long* __restrict__ keys, double* __restrict__ table,
                  uint2* __restrict__ table3, int nd3) {
   extern __shared__ __align__(16) unsigned char tab_smem[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  double* D = reinterpret_cast<double*>(tab_smem) + static_cast<size_t>(w) * T.n_d;
+  double* D = reinterpret_cast<double*>(tab_smem) + static_cast<size_t>(w) * T.n;
   const int cls = blockIdx.x * kFmmWarps + w;
   if (cls >= n_classes) return;
   const unsigned long long key = keys[cls_code[cls]];
@@ -851,12 +964,12 @@ m2l_table_kernel(FmmDevTables T, const int* __restrict__ cls_code, int n_classes
                         static_cast<double>(m2l_key_v(key, 2))};
   m2l_derivatives(T, lane, xs, D);
   if (table3 == nullptr) {
-    for (int k = lane; k < T.n_d; k += 32) table[static_cast<size_t>(cls) * T.n_d + k] = D[k];
+    for (int k = lane; k < T.n; k += 32) table[static_cast<size_t>(cls) * T.n + k] = D[k];
     return;
   }
   for (int k = lane; k < nd3; k += 32) {
     __nv_bfloat16 t3[3];
-    split3_bf16(k < T.n_d ? D[k] : 0.0, t3);
+    split3_bf16(k < T.n ? D[k] : 0.0, t3);
     table3[static_cast<size_t>(cls) * nd3 + k] =
         make_uint2(static_cast<uint32_t>(__bfloat16_as_ushort(t3[0])) |
                        (static_cast<uint32_t>(__bfloat16_as_ushort(t3[1])) << 16),
@@ -864,54 +977,63 @@ m2l_table_kernel(FmmDevTables T, const int* __restrict__ cls_code, int n_classes
   }
 }
 
-constexpr int kM2lBs = kM2lTileP + 2;   // B row stride (doubles): 16-byte rows, 2-way store conflicts
-constexpr int kM2lStages = 3;           // B pipeline depth (k chunks)
+constexpr int kM2lStages = 2;  // B tiles in flight
 
-__device__ __forceinline__ void cp_async8(double* dst, const double* src, bool valid) {
-  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-  const int n = valid ? 8 : 0;  // 0: zero fill, nothing read
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(n) : "memory");
-}
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool valid);
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// Tensor-core form of the class product: mma.m8n8k4 with FP64 operands
-// (256 FMAs per warp instruction, the same FP64 rate as FMA instructions but
-// an eighth of the issue slots). A block covers 8 * kGb >= n_m rows and 64
-// pairs; warp (wr, wc) owns kWr x kWc 8 x 8 output tiles. A fragments are
-// gathered from the class's D(v) through the transposed index map (both in
-// shared memory) and scaled by the source factor; B fragments come from the
-// cp.async pipeline ([k][pair] rows, k padded to a multiple of 4 with zeros,
-// so padded A entries only need to be finite).
+// FP64 class product on the tensor cores: mma.m8n8k4 with FP64 operands (256
+// FMAs per warp instruction, the same FP64 rate as FMA instructions but an
+// eighth of the issue slots), on the harmonic basis.
+//
+// D is harmonic, d_z^2 = -(d_x^2 + d_y^2), so of the n_m = (p+1)(p+2)(p+3)/6
+// rows and columns of A[g][a] = D_{g+a} only the n_r = (p+1)^2 with z exponent
+// 0 or 1 are independent: m2l_rescale_red_kernel collects the source
+// coefficients onto them, m2l_reduce_red_kernel builds the other target
+// coefficients from the summed rows, both exactly the linear relation above.
+// n_r^2 against n_m^2 products per pair: 625 against 1,225 at p = 4, 2,401
+// against 7,056 at p = 6, 6,561 against 27,225 at p = 8; and n_r instead of
+// n_m doubles per pair written and read back.
+//
+// A block covers 8 * kGb >= n_r rows and 64 pairs; warp (wr, wc) owns
+// kWr x kWc 8 x 8 output tiles. A fragments are gathered from the class's
+// D(v) through the transposed index map (both in shared memory) and scaled by
+// the source factor where the source is the larger cell; B is a tile of 64
+// source rows [pair][k], copied whole by cp.async (16-byte copies, two tiles
+// in flight) with a row pitch that is 4 or 12 doubles past a multiple of 16,
+// so that the fragments' eight rows fall into distinct banks. Rows are
+// zero-padded to kNk, so padded A entries only need to be finite.
 template <int P>
 struct M2lMma;
-#define AMK_M2L_MMA(P, WR, WC, KC)                                                               \
-  template <>                                                                                    \
-  struct M2lMma<P> {                                                                             \
-    static constexpr int kNm = (P + 1) * (P + 2) * (P + 3) / 6;                                  \
-    static constexpr int kNd = (2 * P + 1) * (2 * P + 2) * (2 * P + 3) / 6;                      \
-    static constexpr int kGb = (kNm + 7) / 8, kNg = 8 * kGb, kNk = 4 * ((kNm + 3) / 4);           \
-    static constexpr int kWr = WR, kWc = WC, kKc = KC;                                           \
-    static constexpr int kWarpsR = kGb / WR, kWarps = kWarpsR * (8 / WC), kThreads = 32 * kWarps; \
-    static_assert(kGb % WR == 0 && 8 % WC == 0 && kNk % KC == 0 && KC % 4 == 0, "M2L mma shape"); \
+#define AMK_M2L_MMA(P, WR, WC)                                                                    \
+  template <>                                                                                     \
+  struct M2lMma<P> {                                                                              \
+    static constexpr int kNr = (P + 1) * (P + 1);                                                 \
+    static constexpr int kNd = (2 * P + 1) * (P + 1) + (2 * P) * (2 * P + 1) / 2 + (2 * P - 1) * P; \
+    static constexpr int kGb = (kNr + 7) / 8, kNg = 8 * kGb, kNk = 4 * ((kNr + 3) / 4);           \
+    static constexpr int kPitch = kNk + ((kNk & 7) == 0 ? 4 : 0);                                 \
+    static constexpr int kWr = WR, kWc = WC;                                                      \
+    static constexpr int kWarpsR = kGb / WR, kWarps = kWarpsR * (8 / WC), kThreads = 32 * kWarps;  \
+    static_assert(kGb % WR == 0 && 8 % WC == 0, "M2L mma shape");                                 \
   };
-AMK_M2L_MMA(1, 1, 8, 4)
-AMK_M2L_MMA(2, 2, 4, 12)
-AMK_M2L_MMA(3, 3, 4, 20)
-AMK_M2L_MMA(4, 5, 4, 12)
-AMK_M2L_MMA(5, 7, 4, 8)
-AMK_M2L_MMA(6, 11, 2, 12)
-AMK_M2L_MMA(7, 5, 4, 24)
-AMK_M2L_MMA(8, 7, 4, 24)
+AMK_M2L_MMA(1, 1, 4)
+AMK_M2L_MMA(2, 2, 4)
+AMK_M2L_MMA(3, 2, 4)
+AMK_M2L_MMA(4, 4, 4)
+AMK_M2L_MMA(5, 5, 4)
+AMK_M2L_MMA(6, 7, 4)
+AMK_M2L_MMA(7, 8, 2)
+AMK_M2L_MMA(8, 11, 2)
 #undef AMK_M2L_MMA
 
 template <int P>
 size_t m2l_mma_smem() {
   using S = M2lMma<P>;
-  return sizeof(double) * (static_cast<size_t>(kM2lStages) * S::kKc * kM2lBs + S::kNd + S::kNg + S::kNk) +
+  return sizeof(double) * (static_cast<size_t>(kM2lStages) * kM2lTileP * S::kPitch + S::kNd + S::kNg + S::kNk) +
          sizeof(short) * static_cast<size_t>(S::kNk) * S::kNg + 2 * kM2lUnitPairs * sizeof(int) + 16;
 }
 
@@ -927,18 +1049,14 @@ __device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
 // tile.
 template <int P>
 __global__ void __launch_bounds__(M2lMma<P>::kThreads)
-m2l_class_mma_kernel(FmmDevTables T, int n_units, int* __restrict__ unit_counter,
-                     const int* __restrict__ unit_cls, const int* __restrict__ unit_pos,
-                     const int* __restrict__ cls_code, const int* __restrict__ cls_end,
-                     const int* __restrict__ perm, const int* __restrict__ src, const double* __restrict__ Mh,
-                     const double* __restrict__ table, const unsigned long long* __restrict__ keys, long e0,
-                     double* __restrict__ out) {
+m2l_class_mma_kernel(FmmDevTables T, int n_units, int* __restrict__ unit_counter, const int4* __restrict__ ud,
+                     const int* __restrict__ perm, const int* __restrict__ psrc, const double* __restrict__ Mr,
+                     const double* __restrict__ table, long e0, double* __restrict__ out) {
   using S = M2lMma<P>;
-  constexpr int kNm = S::kNm, kNg = S::kNg, kNk = S::kNk, kKc = S::kKc, kTh = S::kThreads;
-  constexpr int kChunks = kNk / kKc;
+  constexpr int kNr = S::kNr, kNg = S::kNg, kNk = S::kNk, kTh = S::kThreads, kPitch = S::kPitch;
   extern __shared__ __align__(16) unsigned char mma_smem[];
-  double* Bs = reinterpret_cast<double*>(mma_smem);  // [kM2lStages][kKc][kM2lBs]
-  double* Ds = Bs + kM2lStages * kKc * kM2lBs;        // [kNd]
+  double* Bs = reinterpret_cast<double*>(mma_smem);   // [kM2lStages][kM2lTileP][kPitch]
+  double* Ds = Bs + kM2lStages * kM2lTileP * kPitch;  // [kNd]
   double* rowf = Ds + S::kNd;                         // [kNg]
   double* colf = rowf + kNg;                          // [kNk]
   int* pe = reinterpret_cast<int*>(colf + kNk);       // [kM2lUnitPairs]
@@ -951,63 +1069,59 @@ m2l_class_mma_kernel(FmmDevTables T, int n_units, int* __restrict__ unit_counter
   const int g_base = 8 * S::kWr * wr + lr, p_base = 8 * S::kWc * wc + lr;
   for (int x = tid; x < kNk * kNg; x += kTh) {
     const int a = x / kNg, g = x - a * kNg;
-    idx[x] = (a < kNm && g < kNm) ? T.m2l_index_t[a * kNm + g] : 0;
+    idx[x] = (a < kNr && g < kNr) ? T.red_index_t[a * kNr + g] : 0;
   }
+  int next = 0;  // thread 0: the unit after the current one
+  if (tid == 0) next = atomicAdd(unit_counter, 1);
   for (;;) {
-    if (tid == 0) s_unit = atomicAdd(unit_counter, 1);
+    if (tid == 0) s_unit = next;
     __syncthreads();  // also: the previous unit is done with the shared arrays
     const int unit = s_unit;
     if (unit >= n_units) break;
-    const int cls = unit_cls[unit], pos0 = unit_pos[unit];
-    const int np = min(kM2lUnitPairs, cls_end[cls] - pos0);
-    const int n_tiles = (np + kM2lTileP - 1) / kM2lTileP, n_steps = n_tiles * kChunks;
-    const int dd = m2l_key_dd(keys[cls_code[cls]]);
-    const int et = dd < 0 ? -dd : 0, es = dd > 0 ? dd : 0;  // log2(h_t / u), log2(h_s / u)
+    if (tid == 0) next = atomicAdd(unit_counter, 1);
+    const int4 u = ud[unit];
+    const int cls = u.x, pos0 = u.y, np = u.z;
+    const int n_tiles = (np + kM2lTileP - 1) / kM2lTileP;
+    const int et = u.w < 0 ? -u.w : 0, es = u.w > 0 ? u.w : 0;  // log2(h_t / u), log2(h_s / u)
     for (int k = tid; k < S::kNd; k += kTh) Ds[k] = table[static_cast<size_t>(cls) * S::kNd + k];
-    for (int g = tid; g < kNg; g += kTh) rowf[g] = g < kNm ? ldexp(T.inv_fact[g], (T.multi[g].w + 1) * et) : 0.0;
-    for (int a = tid; a < kNk; a += kTh) colf[a] = a < kNm ? ldexp(1.0, T.multi[a].w * es) : 0.0;
+    for (int g = tid; g < kNg; g += kTh) rowf[g] = g < kNr ? ldexp(1.0, (T.red_deg[g] + 1) * et) : 0.0;
+    for (int a = tid; a < kNk; a += kTh) colf[a] = a < kNr ? ldexp(1.0, T.red_deg[a] * es) : 0.0;
     for (int p = tid; p < n_tiles * kM2lTileP; p += kTh) {
-      const int e = p < np ? perm[pos0 + p] : -1;
-      pe[p] = e;
-      ps[p] = e >= 0 ? src[e] : -1;
+      pe[p] = p < np ? perm[pos0 + p] : -1;
+      ps[p] = p < np ? psrc[pos0 + p] : -1;
     }
     __syncthreads();
-    auto issue = [&](int step) {
-      if (step < n_steps) {
-        const int tile = step / kChunks, chunk = step - tile * kChunks;
-        const int live = min(kM2lTileP, np - tile * kM2lTileP);
-        double* B = Bs + (step % kM2lStages) * kKc * kM2lBs;
-        for (int x = tid; x < kKc * kM2lTileP; x += kTh) {
-          const int p = x / kKc, kk = x - p * kKc, a = chunk * kKc + kk;
-          if (p >= ((live + 7) & ~7)) continue;  // column blocks no warp reads
+    auto issue = [&](int tile) {
+      if (tile < n_tiles) {
+        const int rows = (min(kM2lTileP, np - tile * kM2lTileP) + 7) & ~7;  // column blocks past them are not read
+        double* B = Bs + (tile % kM2lStages) * kM2lTileP * kPitch;
+        for (int x = tid; x < rows * (kNk / 2); x += kTh) {
+          const int p = x / (kNk / 2), v = x - p * (kNk / 2);
           const int sp = ps[tile * kM2lTileP + p];
-          const bool ok = sp >= 0 && a < kNm;
-          cp_async8(B + kk * kM2lBs + p, ok ? Mh + static_cast<size_t>(sp) * kNm + a : Mh, ok);
+          cp_async16(B + p * kPitch + 2 * v, Mr + static_cast<size_t>(max(sp, 0)) * kNk + 2 * v, sp >= 0);
         }
       }
       cp_async_commit();
     };
-    for (int st = 0; st < kM2lStages - 1; ++st) issue(st);
-    double acc[S::kWr][S::kWc][2];
-#pragma unroll
-    for (int i = 0; i < S::kWr; ++i)
-#pragma unroll
-      for (int j = 0; j < S::kWc; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    issue(0);
 #pragma unroll 1
-    for (int step = 0; step < n_steps; ++step) {
-      const int tile = step / kChunks, chunk = step - tile * kChunks;
+    for (int tile = 0; tile < n_tiles; ++tile) {
+      cp_async_wait<0>();
+      __syncthreads();  // the tile is complete, and the one before it has been read
+      issue(tile + 1);
       const int live = min(kM2lTileP, np - tile * kM2lTileP);  // pairs in this tile
       const int jn = min(S::kWc, max(0, (live - 8 * S::kWc * wc + 7) / 8));  // this warp's live column blocks
-      cp_async_wait<kM2lStages - 2>();
-      __syncthreads();
-      issue(step + kM2lStages - 1);
-      // k chunk: A fragments from D(v) (scaled by the source factor when the
-      // source is the larger cell), B fragments from the staged rows
-      auto chunk_products = [&](auto scaled) {
-        const double* B = Bs + (step % kM2lStages) * kKc * kM2lBs;
+      if (jn == 0) continue;
+      const double* B = Bs + (tile % kM2lStages) * kM2lTileP * kPitch + p_base * kPitch + lc;
+      double acc[S::kWr][S::kWc][2];
 #pragma unroll
-        for (int ks = 0; ks < kKc / 4; ++ks) {
-          const int a = chunk * kKc + 4 * ks + lc;
+      for (int i = 0; i < S::kWr; ++i)
+#pragma unroll
+        for (int j = 0; j < S::kWc; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+      auto products = [&](auto scaled) {
+#pragma unroll 2
+        for (int ks = 0; ks < kNk / 4; ++ks) {
+          const int a = 4 * ks + lc;
           const short* irow = idx + a * kNg + g_base;
           double af[S::kWr], bf[S::kWc];
 #pragma unroll
@@ -1019,7 +1133,7 @@ m2l_class_mma_kernel(FmmDevTables T, int n_units, int* __restrict__ unit_counter
           }
 #pragma unroll
           for (int j = 0; j < S::kWc; ++j)
-            if (j < jn) bf[j] = B[(4 * ks + lc) * kM2lBs + p_base + 8 * j];
+            if (j < jn) bf[j] = B[8 * j * kPitch + 4 * ks];
 #pragma unroll
           for (int j = 0; j < S::kWc; ++j)
             if (j < jn)
@@ -1027,26 +1141,23 @@ m2l_class_mma_kernel(FmmDevTables T, int n_units, int* __restrict__ unit_counter
               for (int i = 0; i < S::kWr; ++i) mma_f64(acc[i][j], af[i], bf[j]);
         }
       };
-      if (jn > 0) {
-        if (es > 0)
-          chunk_products(std::true_type());
-        else
-          chunk_products(std::false_type());
-      }
-      if (chunk == kChunks - 1) {
+      if (es > 0)
+        products(std::true_type());
+      else
+        products(std::false_type());
 #pragma unroll
-        for (int j = 0; j < S::kWc; ++j)
+      for (int j = 0; j < S::kWc; ++j)
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int e = pe[tile * kM2lTileP + 8 * S::kWc * wc + 8 * j + 2 * lc + h];
+        for (int h = 0; h < 2; ++h) {
+          const int e = pe[tile * kM2lTileP + 8 * S::kWc * wc + 8 * j + 2 * lc + h];
+          if (e < 0) continue;
+          double* o = out + static_cast<size_t>(e - e0) * kNk;
 #pragma unroll
-            for (int i = 0; i < S::kWr; ++i) {
-              const int g = 8 * S::kWr * wr + 8 * i + lr;
-              if (e >= 0 && g < kNm) out[static_cast<size_t>(e - e0) * kNm + g] = acc[i][j][h] * rowf[g];
-              acc[i][j][h] = 0.0;
-            }
+          for (int i = 0; i < S::kWr; ++i) {
+            const int g = 8 * S::kWr * wr + 8 * i + lr;
+            if (g < kNr) o[g] = acc[i][j][h] * rowf[g];
           }
-      }
+        }
     }
     cp_async_wait<0>();
   }
@@ -1067,7 +1178,7 @@ m2l_class_mma_kernel(FmmDevTables T, int n_units, int* __restrict__ unit_counter
 // are split into BF16 rows of kKp elements (m2l_split_kernel), each class's
 // D(v) into packed BF16 terms (m2l_table_kernel), and every unit gets a
 // descriptor {class, first pair, pairs, depth difference} and every pair its
-// source cell (m2l_tc_prep_kernel), so each role reads one value where it
+// source cell (m2l_unit_prep_kernel), so each role reads one value where it
 // would otherwise follow a chain of dependent loads.
 //
 // Roles (one CTA per SM, units of one class taken in a fixed stride; every
@@ -1165,8 +1276,8 @@ __global__ void m2l_split_kernel(long n_cells, int nm, int kp, const int4* __res
 }
 
 // Unit descriptors {class, first pair, pairs, depth difference} and the
-// source cell of every class pair.
-__global__ void m2l_tc_prep_kernel(int n_units, const int* __restrict__ unit_cls, const int* __restrict__ unit_pos,
+// source row of every class pair.
+__global__ void m2l_unit_prep_kernel(int n_units, const int* __restrict__ unit_cls, const int* __restrict__ unit_pos,
                                    const int* __restrict__ cls_code, const int* __restrict__ cls_end,
                                    const unsigned long long* __restrict__ keys, int n_pairs,
                                    const int* __restrict__ perm, const int* __restrict__ src,
@@ -1513,14 +1624,13 @@ m2l_class_tc_kernel(FmmDevTables T, int n_units, const int4* __restrict__ ud, co
   if (tid == 0 && *abort_flag) atomicExch(status, 1);
 }
 
-// Pairs outside the classes: a warp per pair (persistent blocks), the
-// derivative tensor by the recurrence, the product through the transposed
-// index map staged once per block, written in the rescaled form
+// Pairs outside the classes (tensor-core mode): a warp per pair (persistent
+// blocks), the derivative tensor by the recurrence, the product through the
+// transposed index map staged once per block, written in the rescaled form
 // Lh = h_t^{|g|+1} L.
-template <typename OutT>
 __global__ void __launch_bounds__(32 * kFmmWarps)
 m2l_pair_kernel(const Octree t, FmmDevTables T, const int* __restrict__ list, int n, const int* __restrict__ tgt,
-                const int* __restrict__ src, const double* __restrict__ M, long e0, OutT* __restrict__ out) {
+                const int* __restrict__ src, const double* __restrict__ M, long e0, float* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char pair_smem[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nm = T.n_m;
   double* D = reinterpret_cast<double*>(pair_smem) + static_cast<size_t>(w) * (T.n_d + nm);
@@ -1534,73 +1644,109 @@ m2l_pair_kernel(const Octree t, FmmDevTables T, const int* __restrict__ list, in
     const double4 tc = t.center[ti], sc = t.center[si];
     for (int a = lane; a < nm; a += 32) Ms[a] = T.sign[a] * M[static_cast<size_t>(si) * nm + a];
     const double xs[3] = {tc.x - sc.x, tc.y - sc.y, tc.z - sc.z};
-    m2l_derivatives(T, lane, xs, D);  // ends with __syncwarp
+    m2l_derivatives(T.d_all, lane, xs, D);  // ends with __syncwarp
     for (int g = lane; g < nm; g += 32) {
       double s = 0.0;
       for (int a = 0; a < nm; ++a) s += Ms[a] * D[idx[a * nm + g]];
       double f = T.inv_fact[g];
       for (int d = 0; d <= T.multi[g].w; ++d) f *= tc.w;
-      out[static_cast<size_t>(e - e0) * nm + g] = static_cast<OutT>(s * f);
+      out[static_cast<size_t>(e - e0) * nm + g] = static_cast<float>(s * f);
     }
     __syncwarp();
   }
 }
 
-// L(t) += h_t^{-|g|-1} sum over the target's pairs in [e0, e1) in pair order;
-// a warp per target, lanes over coefficients (R rows of 32), four pairs'
-// rows in flight.
-template <int R, typename InT>
-__global__ void __launch_bounds__(256)
-m2l_reduce_kernel(const Octree t, FmmDevTables T, const int* __restrict__ off, const int* __restrict__ count,
-                  int t_first, int n_targets, long e0, long e1, const InT* __restrict__ out,
-                  double* __restrict__ L) {
-  constexpr int kU = 4;
-  const int lane = threadIdx.x & 31;
-  const int k = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (k >= n_targets) return;
-  const int ti = t_first + k, nm = T.n_m;
-  const long b = max(static_cast<long>(off[ti]), e0), end = min(static_cast<long>(off[ti]) + count[ti], e1);
-  if (b >= end) return;
-  double s[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) s[r] = 0.0;
-  const InT* o = out + static_cast<size_t>(b - e0) * nm;
-  long e = b;
-  for (; e + kU <= end; e += kU, o += kU * nm) {
-    double v[kU][R];
-#pragma unroll
-    for (int u = 0; u < kU; ++u)
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int g = lane + 32 * r;
-        v[u][r] = g < nm ? o[u * nm + g] : 0.0;
-      }
-#pragma unroll
-    for (int u = 0; u < kU; ++u)
-#pragma unroll
-      for (int r = 0; r < R; ++r) s[r] += v[u][r];
-  }
-  for (; e < end; ++e, o += nm)
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int g = lane + 32 * r;
-      if (g < nm) s[r] += o[g];
+// The same on the harmonic basis (FP64 mode): rows Q_g = h_t^{|g|+1} sum_a
+// (-1)^|a| M_a D_{g+a} over g in the basis, from the rescaled source rows.
+__global__ void __launch_bounds__(32 * kFmmWarps)
+m2l_pair_red_kernel(const Octree t, FmmDevTables T, const int* __restrict__ list, int n, const int* __restrict__ tgt,
+                    const int* __restrict__ src, const double* __restrict__ Mr, long e0, double* __restrict__ out) {
+  extern __shared__ __align__(16) unsigned char pair_smem[];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nr = T.n_r, nd = T.d_red.n;
+  double* D = reinterpret_cast<double*>(pair_smem) + static_cast<size_t>(w) * (nd + nr);
+  double* Ms = D + nd;
+  short* idx = reinterpret_cast<short*>(reinterpret_cast<double*>(pair_smem) +
+                                        static_cast<size_t>(kFmmWarps) * (nd + nr));  // [a][g]
+  for (int x = threadIdx.x; x < nr * nr; x += blockDim.x) idx[x] = T.red_index_t[x];
+  __syncthreads();
+  for (int k = blockIdx.x * kFmmWarps + w; k < n; k += gridDim.x * kFmmWarps) {
+    const int e = list[k], ti = tgt[e], si = src[e];
+    const double4 tc = t.center[ti], sc = t.center[si];
+    for (int a = lane; a < nr; a += 32) {
+      double f = 1.0;  // a power of two
+      for (int d = 0; d < T.red_deg[a]; ++d) f *= sc.w;
+      Ms[a] = Mr[static_cast<size_t>(si) * T.n_rp + a] * f;
     }
-  const double ih = 1.0 / t.center[ti].w;
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int g = lane + 32 * r;
-    if (g >= nm) continue;
-    double f = s[r];
-    for (int d = 0; d <= T.multi[g].w; ++d) f *= ih;
-    L[static_cast<size_t>(ti) * nm + g] += f;
+    const double xs[3] = {tc.x - sc.x, tc.y - sc.y, tc.z - sc.z};
+    m2l_derivatives(T.d_red, lane, xs, D);  // ends with __syncwarp
+    for (int g = lane; g < nr; g += 32) {
+      double s = 0.0;
+      for (int a = 0; a < nr; ++a) s += Ms[a] * D[idx[a * nr + g]];
+      double f = 1.0;
+      for (int d = 0; d <= T.red_deg[g]; ++d) f *= tc.w;
+      out[static_cast<size_t>(e - e0) * T.n_rp + g] = s * f;
+    }
+    __syncwarp();
   }
 }
 
-// The same sum over FP32 per-pair products (tensor-core mode, n_m a multiple
-// of 4): lane l holds coefficients 4l..4l+3 and reads them as one 16-byte
-// vector, eight pairs' rows in flight per warp. The sum per coefficient is
-// the FP64 sum in pair order, as in m2l_reduce_kernel.
+// L_g(t) += 1/g! h_t^{-|g|-1} Q_g, Q the sum of the target's rows in [e0, e1)
+// in pair order on the harmonic basis, its other coefficients built from it.
+// A warp per target; a lane holds V 16-byte vectors of a row (n_rp a multiple
+// of 4), eight (V = 1) or four rows in flight.
+template <int V>
+__global__ void __launch_bounds__(256)
+m2l_reduce_red_kernel(const Octree t, FmmDevTables T, const int* __restrict__ off, const int* __restrict__ count,
+                      int t_first, int n_targets, long e0, long e1, const double* __restrict__ out,
+                      double* __restrict__ L) {
+  constexpr int kU = V == 1 ? 8 : 4;
+  __shared__ double2 qs[8][32 * V];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int k = blockIdx.x * 8 + w;
+  if (k >= n_targets) return;
+  const int ti = t_first + k, nv = T.n_rp >> 1;
+  const long b = max(static_cast<long>(off[ti]), e0), end = min(static_cast<long>(off[ti]) + count[ti], e1);
+  if (b >= end) return;
+  double2 s[V];
+#pragma unroll
+  for (int r = 0; r < V; ++r) s[r] = make_double2(0.0, 0.0);
+  const double2* o = reinterpret_cast<const double2*>(out + static_cast<size_t>(b - e0) * T.n_rp) + lane;
+  long e = b;
+  for (; e + kU <= end; e += kU, o += kU * nv) {
+    double2 v[kU][V];
+#pragma unroll
+    for (int u = 0; u < kU; ++u)
+#pragma unroll
+      for (int r = 0; r < V; ++r) v[u][r] = lane + 32 * r < nv ? o[u * nv + 32 * r] : make_double2(0.0, 0.0);
+#pragma unroll
+    for (int u = 0; u < kU; ++u)
+#pragma unroll
+      for (int r = 0; r < V; ++r) {
+        s[r].x += v[u][r].x;
+        s[r].y += v[u][r].y;
+      }
+  }
+  for (; e < end; ++e, o += nv)
+#pragma unroll
+    for (int r = 0; r < V; ++r)
+      if (lane + 32 * r < nv) {
+        s[r].x += o[32 * r].x;
+        s[r].y += o[32 * r].y;
+      }
+#pragma unroll
+  for (int r = 0; r < V; ++r) qs[w][lane + 32 * r] = s[r];
+  __syncwarp();
+  const double* q = reinterpret_cast<const double*>(qs[w]);
+  const double ih = 1.0 / t.center[ti].w;
+  for (int g = lane; g < T.n_m; g += 32) {
+    double f = 0.0;
+    for (int x = T.ex_off[g]; x < T.ex_off[g + 1]; ++x) f += T.ex_c[x] * q[T.ex_r[x]];
+    f *= T.inv_fact[g];
+    for (int d = 0; d <= T.multi[g].w; ++d) f *= ih;
+    L[static_cast<size_t>(ti) * T.n_m + g] += f;
+  }
+}
+
 // Reflection-folded class pairs (tensor-core mode): the product row of a
 // pair with reflection R gets s^g on coefficient g, in place (refl = 0 for
 // every other pair, the per-pair path's included). A warp takes 32 pairs and
@@ -1638,6 +1784,10 @@ m2l_refl_sign_kernel(FmmDevTables T, long e0, long e1, const unsigned char* __re
   }
 }
 
+// The sum over FP32 per-pair products (tensor-core mode, n_m a multiple of
+// 4, at most 128): lane l holds coefficients 4l..4l+3 and reads them as one
+// 16-byte vector, eight pairs' rows in flight per warp. The sum per
+// coefficient is the FP64 sum in pair order.
 __global__ void __launch_bounds__(256)
 m2l_reduce_f4_kernel(const Octree t, FmmDevTables T, const int* __restrict__ off, const int* __restrict__ count,
                      int t_first, int n_targets, long e0, long e1, const float* __restrict__ out,
@@ -1682,41 +1832,10 @@ m2l_reduce_f4_kernel(const Octree t, FmmDevTables T, const int* __restrict__ off
   }
 }
 
-template <typename InT>
-int m2l_reduce(amk_ctx* c, cudaStream_t stream, const Octree& t, const FmmDevTables& T, const int* off,
-               const int* count, int t_first, int n_targets, long e0, long e1, const InT* out, double* L) {
-  const unsigned grid = static_cast<unsigned>((n_targets + 7) / 8);
-  if constexpr (std::is_same<InT, float>::value) {
-    if (T.n_m % 4 == 0 && T.n_m <= 128) {
-      m2l_reduce_f4_kernel<<<grid, 256, 0, stream>>>(t, T, off, count, t_first, n_targets, e0, e1, out, L);
-      return check_launch(c, "m2l_reduce_f4_kernel");
-    }
-  }
-  switch ((T.n_m + 31) / 32) {
-    case 1:
-      m2l_reduce_kernel<1, InT><<<grid, 256, 0, stream>>>(t, T, off, count, t_first, n_targets, e0, e1, out, L);
-      break;
-    case 2:
-      m2l_reduce_kernel<2, InT><<<grid, 256, 0, stream>>>(t, T, off, count, t_first, n_targets, e0, e1, out, L);
-      break;
-    case 3:
-      m2l_reduce_kernel<3, InT><<<grid, 256, 0, stream>>>(t, T, off, count, t_first, n_targets, e0, e1, out, L);
-      break;
-    case 4:
-      m2l_reduce_kernel<4, InT><<<grid, 256, 0, stream>>>(t, T, off, count, t_first, n_targets, e0, e1, out, L);
-      break;
-    default:
-      static_assert((kMaxNm + 31) / 32 == 6, "rows per lane");
-      m2l_reduce_kernel<6, InT><<<grid, 256, 0, stream>>>(t, T, off, count, t_first, n_targets, e0, e1, out, L);
-      break;
-  }
-  return check_launch(c, "m2l_reduce_kernel");
-}
-
 template <int P>
-int launch_class_product(amk_ctx* c, const FmmDevTables& T, int n_units, int* unit_counter, const int* unit_cls, const int* unit_pos,
-                         const int* cls_code, const int* cls_end, const int* perm, const int* src, const double* Mh,
-                         const double* table, const unsigned long long* keys, long e0, double* out) {
+int launch_class_product(amk_ctx* c, const FmmDevTables& T, int n_units, int* unit_counter, const int4* ud,
+                         const int* perm, const int* psrc, const double* Mr, const double* table, long e0,
+                         double* out) {
   const size_t smem = m2l_mma_smem<P>();
   AMK_CUDA_TRY(cudaFuncSetAttribute(m2l_class_mma_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     static_cast<int>(smem)));
@@ -1727,18 +1846,15 @@ int launch_class_product(amk_ctx* c, const FmmDevTables& T, int n_units, int* un
   AMK_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
   const int grid = std::max(1, std::min(n_units, std::max(1, per_sm) * sms));
   AMK_CUDA_TRY(cudaMemsetAsync(unit_counter, 0, sizeof(int), c->stream));
-  m2l_class_mma_kernel<P><<<grid, M2lMma<P>::kThreads, smem, c->stream>>>(
-      T, n_units, unit_counter, unit_cls, unit_pos, cls_code, cls_end, perm, src, Mh, table, keys, e0, out);
+  m2l_class_mma_kernel<P><<<grid, M2lMma<P>::kThreads, smem, c->stream>>>(T, n_units, unit_counter, ud, perm, psrc,
+                                                                          Mr, table, e0, out);
   return check_launch(c, "m2l_class_mma_kernel");
 }
 
-int class_product(amk_ctx* c, int order, const FmmDevTables& T, int n_units, int* unit_counter, const int* unit_cls,
-                  const int* unit_pos, const int* cls_code, const int* cls_end, const int* perm, const int* src,
-                  const double* Mh, const double* table, const unsigned long long* keys, long e0, double* out) {
-#define AMK_M2L_CASE(P)                                                                                         \
-  case P:                                                                                                     \
-    return launch_class_product<P>(c, T, n_units, unit_counter, unit_cls, unit_pos, cls_code, cls_end, perm, src, Mh, table, \
-                                   keys, e0, out);
+int class_product(amk_ctx* c, int order, const FmmDevTables& T, int n_units, int* unit_counter, const int4* ud,
+                  const int* perm, const int* psrc, const double* Mr, const double* table, long e0, double* out) {
+#define AMK_M2L_CASE(P) \
+  case P: return launch_class_product<P>(c, T, n_units, unit_counter, ud, perm, psrc, Mr, table, e0, out);
   switch (order) {
     AMK_M2L_CASE(1)
     AMK_M2L_CASE(2)
@@ -1806,7 +1922,12 @@ int m2l_products(amk_ctx* c, int order, const Octree& t, const FmmDevTables& T, 
   const long n_codes = kM2lHashSlots;
   unsigned long long* keys = slot<unsigned long long>(c, kSlotM2lHash, kM2lHashSlots, &rc);
   AMK_TRY(rc);
-  double* Mh = slot<double>(c, kSlotFmmWork5, static_cast<size_t>(nn) * T.n_m, &rc);
+  // the tensor-core products (split BF16) write FP32 per-pair products and
+  // take classes folded over the 8 reflections; the FP64 products run on the
+  // harmonic basis
+  const bool tc = c->fmm_precision == AMK_FMM_TENSOR && tc_order(order);
+  const int row = tc ? T.n_m : T.n_rp;  // coefficients of a cell's and of a pair's row
+  double* Mh = slot<double>(c, kSlotFmmWork5, static_cast<size_t>(nn) * row, &rc);
   AMK_TRY(rc);
   int* codes = slot<int>(c, kSlotM2lCodes, n_m2l, &rc);
   AMK_TRY(rc);
@@ -1826,12 +1947,12 @@ int m2l_products(amk_ctx* c, int order, const Octree& t, const FmmDevTables& T, 
   AMK_TRY(rc);
   int* counters = slot<int>(c, kSlotM2lCounters, 8, &rc);  // pairs, classes, units, fallback pairs
   AMK_TRY(rc);
-  const long total = nn * T.n_m;
-  m2l_rescale_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, c->stream>>>(t, T, M, Mh);
+  const unsigned gr = static_cast<unsigned>((nn * row + 255) / 256);
+  if (tc)
+    m2l_rescale_kernel<<<gr, 256, 0, c->stream>>>(t, T, M, Mh);
+  else
+    m2l_rescale_red_kernel<<<gr, 256, 0, c->stream>>>(t, T, M, Mh);
   AMK_TRY(check_launch(c, "m2l_rescale_kernel"));
-  // the tensor-core products (split BF16) write FP32 per-pair products and
-  // take classes folded over the 8 reflections
-  const bool tc = c->fmm_precision == AMK_FMM_TENSOR && tc_order(order);
   unsigned char* refl = nullptr;
   if (tc) {
     refl = slot<unsigned char>(c, kSlotM2lRefl, n_m2l, &rc);
@@ -1850,7 +1971,7 @@ int m2l_products(amk_ctx* c, int order, const Octree& t, const FmmDevTables& T, 
     AMK_TRY(check_launch(c, "m2l_refold_kernel"));
   }
   const size_t esz = tc ? sizeof(float) : sizeof(double);
-  long cap = std::max<long>(1L << 20, static_cast<long>((tc ? kM2lTcChunkBytes : kM2lChunkBytes) / (esz * T.n_m)));
+  long cap = std::max<long>(1L << 20, static_cast<long>((tc ? kM2lTcChunkBytes : kM2lChunkBytes) / (esz * row)));
   if (const char* env = getenv("AMK_FMM_M2L_CHUNK_PAIRS")) {  // smaller chunks (tests of the chunk seams)
     const long v = atol(env);
     if (v > 0) cap = std::min(cap, v);
@@ -1889,7 +2010,7 @@ int m2l_products(amk_ctx* c, int order, const Octree& t, const FmmDevTables& T, 
   }
   const int n_buf = n_m2l > cap ? 2 : 1;
   for (int i = 0; i < n_buf; ++i)
-    AMK_TRY(f->m2l_out[i].reserve(static_cast<size_t>(std::min(cap, n_m2l)) * T.n_m * esz));
+    AMK_TRY(f->m2l_out[i].reserve(static_cast<size_t>(std::min(cap, n_m2l)) * row * esz));
   int chunk = 0;
   for (long e0 = 0; e0 < n_m2l; e0 += cap, ++chunk) {
     const long e1 = std::min(n_m2l, e0 + cap), ne = e1 - e0;
@@ -1928,41 +2049,39 @@ int m2l_products(amk_ctx* c, int order, const Octree& t, const FmmDevTables& T, 
     if (n_cls > 0) {
       // D(v) per class: FP64 rows for the FP64 product, split BF16 rows for
       // the tensor-core product
+      const DerivTables& dt = tc ? T.d_all : T.d_red;
       const int nd3 = tc_nd3(T.n_d);
       double* table = nullptr;
       uint2* table3 = nullptr;
       if (tc)
         table3 = slot<uint2>(c, kSlotM2lTable3, static_cast<size_t>(n_cls) * nd3, &rc);
       else
-        table = slot<double>(c, kSlotM2lTable, static_cast<size_t>(n_cls) * T.n_d, &rc);
+        table = slot<double>(c, kSlotM2lTable, static_cast<size_t>(n_cls) * dt.n, &rc);
       AMK_TRY(rc);
-      const size_t tsm = static_cast<size_t>(kFmmWarps) * T.n_d * sizeof(double);
+      const size_t tsm = static_cast<size_t>(kFmmWarps) * dt.n * sizeof(double);
       AMK_CUDA_TRY(cudaFuncSetAttribute(m2l_table_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         static_cast<int>(tsm)));
       m2l_table_kernel<<<(n_cls + kFmmWarps - 1) / kFmmWarps, 32 * kFmmWarps, tsm, c->stream>>>(
-          T, cls_code, n_cls, keys, table, table3, nd3);
+          dt, cls_code, n_cls, keys, table, table3, nd3);
       AMK_TRY(check_launch(c, "m2l_table_kernel"));
-      int4* ud = nullptr;
-      int* psrc = nullptr;
-      if (tc) {  // the tensor-core product's other inputs: unit descriptors, pair sources
-        const long n_cp = ne - n_fb;  // pairs in classes: perm[0, n_cp)
-        ud = slot<int4>(c, kSlotM2lUnitDesc, static_cast<size_t>(n_units), &rc);
-        AMK_TRY(rc);
-        psrc = slot<int>(c, kSlotM2lPairSrc, static_cast<size_t>(std::max<long>(1, n_cp)), &rc);
-        AMK_TRY(rc);
-        const long np_ = std::max<long>(n_units, n_cp);
-        m2l_tc_prep_kernel<<<static_cast<unsigned>((np_ + 255) / 256), 256, 0, c->stream>>>(
-            n_units, unit_cls, unit_pos, cls_code, cls_end, keys, static_cast<int>(n_cp), perm, gm.src, refl,
-            static_cast<int>(nn), ud, psrc);
-        AMK_TRY(check_launch(c, "m2l_tc_prep_kernel"));
-      }
+      // unit descriptors, pair sources
+      const long n_cp = ne - n_fb;  // pairs in classes: perm[0, n_cp)
+      int4* ud = slot<int4>(c, kSlotM2lUnitDesc, static_cast<size_t>(n_units), &rc);
+      AMK_TRY(rc);
+      int* psrc = slot<int>(c, kSlotM2lPairSrc, static_cast<size_t>(std::max<long>(1, n_cp)), &rc);
+      AMK_TRY(rc);
+      const long np_ = std::max<long>(n_units, n_cp);
+      m2l_unit_prep_kernel<<<static_cast<unsigned>((np_ + 255) / 256), 256, 0, c->stream>>>(
+          n_units, unit_cls, unit_pos, cls_code, cls_end, keys, static_cast<int>(n_cp), perm, gm.src, refl,
+          static_cast<int>(nn), ud, psrc);
+      AMK_TRY(check_launch(c, "m2l_unit_prep_kernel"));
       AMK_TRY(phase_begin(c, AMK_PHASE_FMM_M2L_PRODUCTS));
       if (tc)
         AMK_TRY(class_tc(c, order, T, n_units, ud, perm, psrc, Mh3, table3, e0, static_cast<float*>(out),
                          tc_status));
       else
-        AMK_TRY(class_product(c, order, T, n_units, counters + 4, unit_cls, unit_pos, cls_code, cls_end, perm,
-                              gm.src, Mh, table, keys, e0, static_cast<double*>(out)));
+        AMK_TRY(class_product(c, order, T, n_units, counters + 4, ud, perm, psrc, Mh, table, e0,
+                              static_cast<double*>(out)));
       AMK_TRY(phase_end(c, AMK_PHASE_FMM_M2L_PRODUCTS));
       if (tc) {  // the signs s^g of the reflection-folded pairs
         m2l_refl_sign_kernel<<<static_cast<unsigned>((ne + 255) / 256), 256, 0, c->stream>>>(
@@ -1971,21 +2090,22 @@ int m2l_products(amk_ctx* c, int order, const Octree& t, const FmmDevTables& T, 
       }
     }
     if (n_fb > 0) {
-      const size_t psm = static_cast<size_t>(kFmmWarps) * (T.n_d + T.n_m) * sizeof(double) +
-                         static_cast<size_t>(T.n_m) * T.n_m * sizeof(short);
-      auto launch_pairs = [&](auto kernel, auto* dst) -> int {
+      const int pd = tc ? T.n_d : T.d_red.n, pm = tc ? T.n_m : T.n_r;
+      const size_t psm = static_cast<size_t>(kFmmWarps) * (pd + pm) * sizeof(double) +
+                         static_cast<size_t>(pm) * pm * sizeof(short);
+      auto launch_pairs = [&](auto kernel, const double* m, auto* dst) -> int {
         AMK_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(psm)));
         int per_sm = 0, sms = 0;
         AMK_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * kFmmWarps, psm));
         AMK_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
         const int grid = std::max(1, std::min((n_fb + kFmmWarps - 1) / kFmmWarps, std::max(1, per_sm) * sms));
-        kernel<<<grid, 32 * kFmmWarps, psm, c->stream>>>(t, T, fallback, n_fb, tgt, gm.src, M, e0, dst);
+        kernel<<<grid, 32 * kFmmWarps, psm, c->stream>>>(t, T, fallback, n_fb, tgt, gm.src, m, e0, dst);
         return check_launch(c, "m2l_pair_kernel");
       };
       if (tc)
-        AMK_TRY(launch_pairs(m2l_pair_kernel<float>, static_cast<float*>(out)));
+        AMK_TRY(launch_pairs(m2l_pair_kernel, M, static_cast<float*>(out)));
       else
-        AMK_TRY(launch_pairs(m2l_pair_kernel<double>, static_cast<double*>(out)));
+        AMK_TRY(launch_pairs(m2l_pair_red_kernel, static_cast<const double*>(Mh), static_cast<double*>(out)));
     }
     // after the per-pair products (run concurrently with them, the near
     // field took longer than both in sequence)
@@ -1993,12 +2113,18 @@ int m2l_products(amk_ctx* c, int order, const Octree& t, const FmmDevTables& T, 
     // per-target sums on the side stream, in chunk order
     AMK_CUDA_TRY(cudaEventRecord(f->products_done[buf], c->stream));
     AMK_CUDA_TRY(cudaStreamWaitEvent(f->side, f->products_done[buf], 0));
+    const int n_tgt = tr[1] - tr[0] + 1;
+    const unsigned gt = static_cast<unsigned>((n_tgt + 7) / 8);
     if (tc)
-      AMK_TRY(m2l_reduce(c, f->side, t, T, gm.off, gm.count, tr[0], tr[1] - tr[0] + 1, e0, e1,
-                         static_cast<const float*>(out), L));
+      m2l_reduce_f4_kernel<<<gt, 256, 0, f->side>>>(t, T, gm.off, gm.count, tr[0], n_tgt, e0, e1,
+                                                    static_cast<const float*>(out), L);
+    else if (T.n_rp <= 64)
+      m2l_reduce_red_kernel<1><<<gt, 256, 0, f->side>>>(t, T, gm.off, gm.count, tr[0], n_tgt, e0, e1,
+                                                        static_cast<const double*>(out), L);
     else
-      AMK_TRY(m2l_reduce(c, f->side, t, T, gm.off, gm.count, tr[0], tr[1] - tr[0] + 1, e0, e1,
-                         static_cast<const double*>(out), L));
+      m2l_reduce_red_kernel<2><<<gt, 256, 0, f->side>>>(t, T, gm.off, gm.count, tr[0], n_tgt, e0, e1,
+                                                        static_cast<const double*>(out), L);
+    AMK_TRY(check_launch(c, "m2l_reduce_kernel"));
     AMK_CUDA_TRY(cudaEventRecord(f->sums_done[buf], f->side));
   }
   // the context stream resumes after the last sums
