@@ -133,7 +133,6 @@ enum ScratchSlot {
   kSlotFmmLists0,
   kSlotFmmLists1,
   kSlotFmmLists2,
-  kSlotFmmLists3,
   kSlotFmmAux0,
   kSlotFmmAux1,
   kSlotFmmAux2,

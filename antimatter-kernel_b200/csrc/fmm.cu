@@ -11,9 +11,9 @@
 //   radii, P2M      leaves in parallel (a thread per leaf / a warp per leaf)
 //   M2M, L2L        level-synchronous, a warp per node, lanes over coefficients
 //   lists           the reference's dual-tree recursion run breadth-first over
-//                   (target, source) pairs; M2L and P2P pairs are radix-sorted
-//                   by (target, source), so every sum has a fixed order
-//                   (run-to-run deterministic)
+//                   (target, source) pairs; each target's M2L and P2P sources
+//                   are sorted, so every sum has a fixed order (run-to-run
+//                   deterministic)
 //   M2L             a warp per target cell; per source the derivative tensor
 //                   is built degree by degree in shared memory (lanes over the
 //                   multi-indices of one degree) and contracted with the
@@ -264,6 +264,7 @@ struct FmmDevTables {
 
 struct FmmLists {
   DevBuf cur, next, m2l, p2p;
+  DevBuf m2l_rank, p2p_rank;  // a pair's place among its target's pairs
   // list lengths the last traversal needed (the next one reserves them)
   long need_front = 0, need_m2l = 0, need_p2p = 0;
 };
@@ -525,15 +526,17 @@ fmm_m2m_kernel(const Octree t, FmmDevTables T, int depth, double* __restrict__ M
 
 // ------------------------------------------------------------ dual traversal
 // One level of the dual-tree recursion (fast-multipole.cc:484-526): each
-// pair is accepted for M2L, kept for P2P, or split into its children. The
-// emissions of a warp are reserved with one atomic per list (ballot / warp
-// prefix sums); the order of the lists is irrelevant, they are sorted after.
+// pair is accepted for M2L, kept for P2P, or split into its children. A block
+// takes 2 x 256 pairs at a time and reserves its emissions with one atomic per
+// list (warp prefix sums, then a sum over the warps; a reservation per warp
+// queued up at the three counters); the order of the lists is irrelevant,
+// every target's sources are sorted after.
 // The level's pair count is read on the device (lv[0]), the children are
 // counted into lv[1]; a slot past a list's capacity is not written and
 // raises cnt[2], so the host can grow the lists and run the traversal again
 // (counts keep growing past the capacity, and every slot below it is
 // written). A pair that is not a pair of nodes raises cnt[3] and is
-// skipped. Warps stride over the level's pairs, so one grid size serves
+// skipped. Blocks stride over the level's pairs, so one grid size serves
 // every level.
 // Per node, what the traversal reads of it in one 32-byte record: the
 // centre and the radius, negated for a leaf (a leaf of radius 0 stores -0.0;
@@ -557,114 +560,279 @@ __global__ void fmm_traverse_root_kernel(int2* __restrict__ cur, int* __restrict
 struct TraverseLists {
   int2* m2l;
   int2* p2p;
+  int* m2l_rank;
+  int* p2p_rank;
+  int* m2l_count;  // per target
+  int* p2p_count;
   long cap_m2l, cap_p2p, cap_front;
 };
 
-__global__ void fmm_traverse_kernel(const Octree t, const double4* __restrict__ rec, double theta2,
-                                    const int2* __restrict__ cur, int2* __restrict__ next, TraverseLists out,
-                                    int* __restrict__ lv, int* __restrict__ cnt) {
-  const int lane = threadIdx.x & 31;
+constexpr int kTravThreads = 256;
+constexpr int kTravPer = 2;  // pairs per thread and pass
+
+__global__ void __launch_bounds__(kTravThreads)
+fmm_traverse_kernel(const Octree t, const double4* __restrict__ rec, double theta2, const int2* __restrict__ cur,
+                    int2* __restrict__ next, TraverseLists out, int* __restrict__ lv, int* __restrict__ cnt) {
+  constexpr int kW = kTravThreads / 32;
+  __shared__ int w_count[3][kW];   // per warp: M2L, P2P, children
+  __shared__ int w_first[3][kW];   // the warps' first slots
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned below = (1u << lane) - 1u;
   const long n_cur = min(static_cast<long>(lv[0]), out.cap_front);
-  const long warp0 = (blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x) >> 5;
-  const long n_warps = (static_cast<long>(gridDim.x) * blockDim.x) >> 5;
-  for (long base = warp0 * 32; base < n_cur; base += n_warps * 32) {
-    const long i = base + lane;
-    int2 pr = make_int2(0, 0);
-    int kind = -1;  // 0 M2L, 1 P2P, 2 split
-    int kids[8], nk = 0;
-    bool split_target = false;
-    if (i < n_cur) pr = cur[i];
-    if (i < n_cur && (static_cast<unsigned>(pr.x) >= static_cast<unsigned>(t.n_nodes) ||
-                      static_cast<unsigned>(pr.y) >= static_cast<unsigned>(t.n_nodes))) {
-      cnt[3] = 1;  // not a node pair: recorded and skipped
-    } else if (i < n_cur) {
-      const int ti = pr.x, si = pr.y;
-      const double4 tc = rec[ti], sc = rec[si];
+  for (long base = static_cast<long>(blockIdx.x) * (kTravThreads * kTravPer); base < n_cur;
+       base += static_cast<long>(gridDim.x) * (kTravThreads * kTravPer)) {
+    int2 pr[kTravPer];
+    int kind[kTravPer];  // 0 M2L, 1 P2P, 2 split the source, 3 split the target, -1 none
+    int4 kid[kTravPer][2];
+    int nk[kTravPer];
+#pragma unroll
+    for (int u = 0; u < kTravPer; ++u) {
+      const long i = base + u * kTravThreads + threadIdx.x;
+      kind[u] = -1;
+      pr[u] = make_int2(0, 0);
+      if (i < n_cur) {
+        pr[u] = cur[i];
+        kind[u] = 0;
+        if (static_cast<unsigned>(pr[u].x) >= static_cast<unsigned>(t.n_nodes) ||
+            static_cast<unsigned>(pr[u].y) >= static_cast<unsigned>(t.n_nodes)) {
+          cnt[3] = 1;  // not a node pair: recorded and skipped
+          kind[u] = -1;
+          pr[u] = make_int2(0, 0);
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kTravPer; ++u) {
+      const double4 tc = rec[pr[u].x], sc = rec[pr[u].y];
       const double dx = tc.x - sc.x, dy = tc.y - sc.y, dz = tc.z - sc.z;
       const double dist2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
       const double rt = fabs(tc.w), rs = fabs(sc.w);
       const double rsum = rt + rs;
-      if (__dmul_rn(rsum, rsum) < __dmul_rn(theta2, dist2)) {
-        kind = 0;
-      } else {
+      if (kind[u] == 0 && !(__dmul_rn(rsum, rsum) < __dmul_rn(theta2, dist2))) {
         const bool tleaf = signbit(tc.w), sleaf = signbit(sc.w);
-        if (tleaf && sleaf) {
-          kind = 1;
+        kind[u] = tleaf && sleaf ? 1 : (sleaf || (!tleaf && rt >= rs)) ? 3 : 2;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kTravPer; ++u) {
+      nk[u] = 0;
+      if (kind[u] >= 2) {
+        const int4* c = reinterpret_cast<const int4*>(t.child + 8 * static_cast<size_t>(kind[u] == 3 ? pr[u].x : pr[u].y));
+        kid[u][0] = c[0];
+        kid[u][1] = c[1];
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          nk[u] += (kid[u][h].x >= 0) + (kid[u][h].y >= 0) + (kid[u][h].z >= 0) + (kid[u][h].w >= 0);
+      }
+    }
+    // slots: within the warp, then the warps' shares of the block's reservation
+    int at[kTravPer] = {}, tot[3] = {0, 0, 0};
+#pragma unroll
+    for (int u = 0; u < kTravPer; ++u) {
+      const unsigned m0 = __ballot_sync(0xffffffffu, kind[u] == 0), m1 = __ballot_sync(0xffffffffu, kind[u] == 1);
+      if (kind[u] == 0) at[u] = tot[0] + __popc(m0 & below);
+      if (kind[u] == 1) at[u] = tot[1] + __popc(m1 & below);
+      tot[0] += __popc(m0);
+      tot[1] += __popc(m1);
+      int incl = nk[u];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      if (kind[u] >= 2) at[u] = tot[2] + incl - nk[u];
+      tot[2] += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane < 3) w_count[lane][warp] = lane == 0 ? tot[0] : lane == 1 ? tot[1] : tot[2];
+    __syncthreads();
+    if (threadIdx.x < 3) {
+      const int l = threadIdx.x;
+      int sum = 0;
+      for (int w = 0; w < kW; ++w) sum += w_count[l][w];
+      int first = sum ? atomicAdd(l == 2 ? &lv[1] : &cnt[l], sum) : 0;
+      for (int w = 0; w < kW; ++w) {
+        w_first[l][w] = first;
+        first += w_count[l][w];
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kTravPer; ++u) {
+      if (kind[u] < 0) continue;
+      const long slot = static_cast<long>(w_first[min(kind[u], 2)][warp]) + at[u];
+      if (kind[u] < 2) {
+        const bool m2l = kind[u] == 0;
+        const int rank = atomicAdd((m2l ? out.m2l_count : out.p2p_count) + pr[u].x, 1);
+        if (slot < (m2l ? out.cap_m2l : out.cap_p2p)) {
+          (m2l ? out.m2l : out.p2p)[slot] = pr[u];
+          (m2l ? out.m2l_rank : out.p2p_rank)[slot] = rank;
         } else {
-          kind = 2;
-          split_target = sleaf || (!tleaf && rt >= rs);
-          const int node = split_target ? ti : si;
-          for (int o = 0; o < 8; ++o) {
-            const int ch = t.child[8 * node + o];
-            if (ch >= 0) kids[nk++] = ch;
+          cnt[2] = 1;
+        }
+      } else {
+        // every slot below the capacity is written (the reservations are
+        // contiguous), so the next level reads only pairs of this one
+        if (slot + nk[u] > out.cap_front) cnt[2] = 1;
+        long k = slot;
+        const int ch[8] = {kid[u][0].x, kid[u][0].y, kid[u][0].z, kid[u][0].w,
+                           kid[u][1].x, kid[u][1].y, kid[u][1].z, kid[u][1].w};
+#pragma unroll
+        for (int o = 0; o < 8; ++o)
+          if (ch[o] >= 0) {
+            if (k < out.cap_front) next[k] = kind[u] == 3 ? make_int2(ch[o], pr[u].y) : make_int2(pr[u].x, ch[o]);
+            ++k;
           }
+      }
+    }
+  }
+}
+
+// Pairs grouped by target: the traversal counts every target's pairs and
+// notes each pair's place among them, a scan of the counts gives the groups,
+// a scatter writes the sources, and each group is then sorted by source index
+// (a fixed summation order, independent of the emission order). (A radix sort
+// of (target, source) keys over all pairs took 0.95 of the 2.06 ms that the
+// lists took at 262,144 particles, p = 4, and 4.2 of 7.7 ms at 1,048,576,
+// p = 6.)
+__global__ void pair_scatter_kernel(const int2* __restrict__ pairs, const int* __restrict__ rank,
+                                    const int* __restrict__ n_pairs, long cap, const int* __restrict__ off,
+                                    int* __restrict__ src) {
+  const long n = min(static_cast<long>(*n_pairs), cap);
+  for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < n;
+       i += static_cast<long>(gridDim.x) * blockDim.x) {
+    const int2 p = pairs[i];
+    const long at = static_cast<long>(off[p.x]) + rank[i];
+    if (at < cap) src[at] = p.y;  // (past it only when the lists overflowed: the traversal runs again)
+  }
+}
+
+// Ascending sort of 32 K values, element r * 32 + lane in v[r]: bitonic merges
+// in the form whose comparisons all point the same way (each merge starts
+// with the mirrored partner).
+template <int K>
+__device__ __forceinline__ void warp_sort(unsigned (&v)[K], int lane) {
+#pragma unroll
+  for (int size = 2; size <= 32 * K; size *= 2) {
+    if (size <= 32) {
+#pragma unroll
+      for (int r = 0; r < K; ++r) {
+        const unsigned o = __shfl_xor_sync(0xffffffffu, v[r], size - 1);
+        v[r] = (lane & (size / 2)) ? max(v[r], o) : min(v[r], o);
+      }
+    } else {
+      const int m = size / 32 - 1;
+#pragma unroll
+      for (int r = 0; r < K; ++r)
+        if (r < (r ^ m)) {
+          const unsigned a = v[r], b = v[r ^ m];
+          const unsigned ob = __shfl_xor_sync(0xffffffffu, b, 31), oa = __shfl_xor_sync(0xffffffffu, a, 31);
+          v[r] = min(a, ob);
+          v[r ^ m] = max(b, oa);
+        }
+    }
+#pragma unroll
+    for (int st = size / 4; st >= 1; st /= 2) {
+      if (st >= 32) {
+        const int q = st / 32;
+#pragma unroll
+        for (int r = 0; r < K; ++r)
+          if (!(r & q)) {
+            const unsigned a = v[r], b = v[r + q];
+            v[r] = min(a, b);
+            v[r + q] = max(a, b);
+          }
+      } else {
+#pragma unroll
+        for (int r = 0; r < K; ++r) {
+          const unsigned o = __shfl_xor_sync(0xffffffffu, v[r], st);
+          v[r] = (lane & st) ? max(v[r], o) : min(v[r], o);
         }
       }
     }
-    // M2L and P2P: one slot per lane
-    for (int list = 0; list < 2; ++list) {
-      const unsigned m = __ballot_sync(0xffffffffu, kind == list);
-      if (m == 0) continue;
-      int b = 0;
-      if (lane == __ffs(m) - 1) b = atomicAdd(&cnt[list], __popc(m));
-      b = __shfl_sync(0xffffffffu, b, __ffs(m) - 1);
-      const long slot = static_cast<long>(b) + __popc(m & below);
-      if (kind == list) {
-        if (slot < (list == 0 ? out.cap_m2l : out.cap_p2p))
-          (list == 0 ? out.m2l : out.p2p)[slot] = pr;
-        else
-          cnt[2] = 1;
-      }
-    }
-    // children: a warp prefix sum of the counts
-    int incl = nk;
+  }
+}
+
+template <int K>
+__device__ __forceinline__ void warp_sort_group(const int* __restrict__ in, int* __restrict__ src, int n, int lane) {
+  unsigned v[K];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += v;
-    }
-    const int total = __shfl_sync(0xffffffffu, incl, 31);
-    if (total == 0) continue;
-    int b = 0;
-    if (lane == 31) b = atomicAdd(&lv[1], total);
-    const long first = static_cast<long>(__shfl_sync(0xffffffffu, b, 31)) + incl - nk;
-    // every slot below the capacity is written (the reservations are
-    // contiguous), so the next level reads only pairs of this one
-    for (int k = 0; k < nk; ++k) {
-      if (first + k < out.cap_front)
-        next[first + k] = split_target ? make_int2(kids[k], pr.y) : make_int2(pr.x, kids[k]);
-      else
-        cnt[2] = 1;
-    }
-  }
+  for (int r = 0; r < K; ++r) v[r] = r * 32 + lane < n ? static_cast<unsigned>(in[r * 32 + lane]) : 0xffffffffu;
+  warp_sort<K>(v, lane);
+#pragma unroll
+  for (int r = 0; r < K; ++r)
+    if (r * 32 + lane < n) src[r * 32 + lane] = static_cast<int>(v[r]);
 }
 
-// Group pairs by target: pack (target, source) into one key and radix-sort
-// it, so each target's sources are contiguous and in ascending source order
-// (a fixed summation order, independent of the emission order).
-__global__ void pair_pack_kernel(const int2* __restrict__ pairs, int n, int bits, uint64_t* __restrict__ keys,
-                                 uint32_t* __restrict__ vals) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int2 p = pairs[i];
-  keys[i] = (static_cast<uint64_t>(p.x) << bits) | static_cast<uint64_t>(p.y);
-  vals[i] = static_cast<uint32_t>(i);
-}
+constexpr int kSortWarpMax = 512;      // sources a warp sorts in registers
+constexpr int kSortThreads = 256;
+constexpr int kSortBits = 1 << 19;     // sources per bitmap pass (64 KB of shared memory)
 
-// Sorted keys: a warp's lanes with the same target add their count once.
-__global__ void pair_unpack_kernel(const uint64_t* __restrict__ keys, int n, int bits, int* __restrict__ src,
-                                   int* __restrict__ count) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int lane = threadIdx.x & 31;
-  int target = -1;
-  if (i < n) {
-    const uint64_t k = keys[i];
-    src[i] = static_cast<int>(k & ((1ull << bits) - 1ull));
-    target = static_cast<int>(k >> bits);
+// Eight targets per block. Groups of up to 512 sources: a warp each, bitonic
+// merges in registers. Larger ones: the block marks the group's sources in a
+// bitmap over the nodes (a target's sources are distinct) and writes the set
+// bits out in order, so the work is n + n_nodes / 32 whatever the group's
+// size (groups of several thousand sources are common: a large leaf next to a
+// dense region).
+__global__ void __launch_bounds__(kSortThreads)
+group_sort_kernel(int n_nodes, const int* __restrict__ off, const int* __restrict__ count, long cap,
+                  const int* __restrict__ unsorted, int* __restrict__ src) {
+  extern __shared__ unsigned sort_bits[];
+  __shared__ int warp_sum[kSortThreads / 32];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int t0 = blockIdx.x * (kSortThreads / 32);
+  if (t0 + w < n_nodes) {
+    const int n = count[t0 + w];
+    const long b = off[t0 + w];
+    if (n > 0 && b + n <= cap) {
+      if (n <= 32)
+        warp_sort_group<1>(unsorted + b, src + b, n, lane);
+      else if (n <= 64)
+        warp_sort_group<2>(unsorted + b, src + b, n, lane);
+      else if (n <= 128)
+        warp_sort_group<4>(unsorted + b, src + b, n, lane);
+      else if (n <= 256)
+        warp_sort_group<8>(unsorted + b, src + b, n, lane);
+      else if (n <= kSortWarpMax)
+        warp_sort_group<16>(unsorted + b, src + b, n, lane);
+    }
   }
-  const unsigned same = __match_any_sync(0xffffffffu, target);
-  if (target >= 0 && lane == __ffs(same) - 1) atomicAdd(&count[target], __popc(same));
+  for (int k = 0; k < kSortThreads / 32 && t0 + k < n_nodes; ++k) {
+    const int n = count[t0 + k];
+    const long b = off[t0 + k];
+    if (n <= kSortWarpMax || b + n > cap) continue;
+    int first = 0;  // sources written so far
+    for (int r0 = 0; r0 < n_nodes; r0 += kSortBits) {
+      const int bits = min(kSortBits, n_nodes - r0), words = (bits + 31) / 32;
+      const int per = ((words + kSortThreads - 1) / kSortThreads) | 1;  // odd: the threads' runs in distinct banks
+      __syncthreads();
+      for (int i = tid; i < words; i += kSortThreads) sort_bits[i] = 0;
+      __syncthreads();
+      for (int i = tid; i < n; i += kSortThreads) {
+        const unsigned v = static_cast<unsigned>(unsorted[b + i] - r0);
+        if (v < static_cast<unsigned>(bits)) atomicOr(&sort_bits[v >> 5], 1u << (v & 31));
+      }
+      __syncthreads();
+      const int w0 = min(tid * per, words), w1 = min(w0 + per, words);
+      int mine = 0;
+      for (int i = w0; i < w1; ++i) mine += __popc(sort_bits[i]);
+      int incl = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      if (lane == 31) warp_sum[w] = incl;
+      __syncthreads();
+      int at = first + incl - mine, all = 0;
+      for (int x = 0; x < kSortThreads / 32; ++x) {
+        if (x < w) at += warp_sum[x];
+        all += warp_sum[x];
+      }
+      for (int i = w0; i < w1; ++i)
+        for (unsigned m = sort_bits[i]; m; m &= m - 1) src[b + at++] = r0 + 32 * i + __ffs(m) - 1;
+      first += all;
+    }
+  }
 }
 
 struct Grouped {
@@ -2731,38 +2899,27 @@ __global__ void zero_forces_kernel(View v) {
   v.fz[i] = 0.0;
 }
 
-int group_pairs(amk_ctx* c, const int2* pairs, long n_pairs, long n_nodes, int slot_off, int slot_cnt, int slot_src,
-                int slot_cursor, Grouped* g) {
-  (void)slot_cursor;
+// Groups the pairs of one list by target (g->count holds the counts); nothing
+// is read back: the list's length stays on the device, `cap` bounds it.
+int group_pairs(amk_ctx* c, const int2* pairs, const int* rank, const int* n_pairs, long cap, long n_nodes,
+                int slot_off, int slot_src, int slot_tmp, Grouped* g) {
   int rc = AMK_OK;
   g->off = slot<int>(c, slot_off, n_nodes + 1, &rc);
   AMK_TRY(rc);
-  g->count = slot<int>(c, slot_cnt, n_nodes + 1, &rc);
+  g->src = slot<int>(c, slot_src, cap, &rc);
   AMK_TRY(rc);
-  g->src = slot<int>(c, slot_src, std::max<long>(n_pairs, 1), &rc);
+  int* unsorted = slot<int>(c, slot_tmp, cap, &rc);
   AMK_TRY(rc);
-  int* total = slot<int>(c, kSlotStatus, 8, &rc) + 6;
-  AMK_TRY(rc);
-  AMK_CUDA_TRY(cudaMemsetAsync(g->count, 0, (n_nodes + 1) * sizeof(int), c->stream));
-  if (n_pairs > 0) {
-    int bits = 1;
-    while ((1L << bits) < n_nodes) ++bits;
-    uint64_t* keys = slot<uint64_t>(c, kSlotKeysA, n_pairs, &rc);
-    AMK_TRY(rc);
-    uint32_t* vals = slot<uint32_t>(c, kSlotValsA, n_pairs, &rc);
-    AMK_TRY(rc);
-    uint64_t* skeys = slot<uint64_t>(c, kSlotTreeKeys, n_pairs, &rc);
-    AMK_TRY(rc);
-    uint32_t* svals = slot<uint32_t>(c, kSlotSorted0, n_pairs, &rc);
-    AMK_TRY(rc);
-    const unsigned gp = static_cast<unsigned>((n_pairs + 255) / 256);
-    pair_pack_kernel<<<gp, 256, 0, c->stream>>>(pairs, static_cast<int>(n_pairs), bits, keys, vals);
-    AMK_TRY(check_launch(c, "pair_pack_kernel"));
-    AMK_TRY(radix_sort_pairs(c, keys, vals, skeys, svals, n_pairs, 2 * bits));
-    pair_unpack_kernel<<<gp, 256, 0, c->stream>>>(skeys, static_cast<int>(n_pairs), bits, g->src, g->count);
-    AMK_TRY(check_launch(c, "pair_unpack_kernel"));
-  }
-  return exclusive_scan_int(c, g->count, n_nodes, g->off, total);
+  AMK_TRY(exclusive_scan_int(c, g->count, n_nodes, g->off, g->off + n_nodes));
+  pair_scatter_kernel<<<static_cast<unsigned>(std::min<long>((cap + 255) / 256, 148L * 16)), 256, 0, c->stream>>>(
+      pairs, rank, n_pairs, cap, g->off, unsorted);
+  AMK_TRY(check_launch(c, "pair_scatter_kernel"));
+  const size_t smem = static_cast<size_t>((std::min<long>(n_nodes, kSortBits) + 31) / 32) * sizeof(unsigned);
+  AMK_CUDA_TRY(cudaFuncSetAttribute(group_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    kSortBits / 8));
+  group_sort_kernel<<<static_cast<unsigned>((n_nodes + 7) / 8), kSortThreads, smem, c->stream>>>(
+      static_cast<int>(n_nodes), g->off, g->count, cap, unsorted, g->src);
+  return check_launch(c, "group_sort_kernel");
 }
 
 }  // namespace
@@ -2840,7 +2997,7 @@ int fmm_run(amk_ctx* c, const View& v, int order, double theta, long leaf_capaci
   AMK_TRY(phase_begin(c, AMK_PHASE_FMM_LISTS));
   FmmLists& lists = c->fmm->lists;
   const int n_levels = 2 * t.max_depth + 1;
-  const int n_tv = 8 + n_levels + 1;  // m2l, p2p, overflow, -, -, -, -, -, pairs per level
+  const int n_tv = 8 + n_levels + 1;  // m2l, p2p, overflow, not a pair, work items, partials, -, -, pairs per level
   int* tv = slot<int>(c, kSlotFmmAux0, n_tv, &rc);
   AMK_TRY(rc);
   unsigned long long* cnt64 = slot<unsigned long long>(c, kSlotFmmAux1, 4, &rc);
@@ -2854,6 +3011,22 @@ int fmm_run(amk_ctx* c, const View& v, int order, double theta, long leaf_capaci
   std::vector<int> hv(n_tv);
   unsigned long long h64[2] = {0, 0};
   TreeFrame hf;
+  const bool f32 = c->fmm_precision == AMK_FMM_TENSOR;
+  Grouped gm, gp;
+  int* counts = slot<int>(c, kSlotFmmLists1, 2 * static_cast<size_t>(nn), &rc);  // pairs per target: M2L, P2P
+  AMK_TRY(rc);
+  gm.count = counts;
+  gp.count = counts + nn;
+  // near-field work items and the layout of their partial sums
+  int* items = slot<int>(c, kSlotFmmAux2, nn + 1, &rc);
+  AMK_TRY(rc);
+  int* psize = slot<int>(c, kSlotTreeCount, nn + 1, &rc);  // tree build scratch, free again
+  AMK_TRY(rc);
+  int* ibase = slot<int>(c, kSlotTreeBase, nn + 1, &rc);
+  AMK_TRY(rc);
+  int* pbase = slot<int>(c, kSlotTreeL, nn + 1, &rc);
+  AMK_TRY(rc);
+  int ht[2] = {0, 0};  // work items, partial sums
   long want_front = std::max({lists.need_front, 8 * nn, 1024L});
   long want_m2l = std::max({lists.need_m2l, 64 * nn, 1024L}), want_p2p = std::max({lists.need_p2p, 16 * nn, 1024L});
   if (const char* env = getenv("AMK_FMM_LIST_CAP")) {  // small first capacities (tests of the overflow retry)
@@ -2863,6 +3036,8 @@ int fmm_run(amk_ctx* c, const View& v, int order, double theta, long leaf_capaci
       lists.next.release();
       lists.m2l.release();
       lists.p2p.release();
+      lists.m2l_rank.release();
+      lists.p2p_rank.release();
       want_front = want_m2l = want_p2p = v;
     }
   }
@@ -2872,20 +3047,28 @@ int fmm_run(amk_ctx* c, const View& v, int order, double theta, long leaf_capaci
     AMK_TRY(lists.next.reserve(static_cast<size_t>(want_front) * sizeof(int2)));
     AMK_TRY(lists.m2l.reserve(static_cast<size_t>(want_m2l) * sizeof(int2)));
     AMK_TRY(lists.p2p.reserve(static_cast<size_t>(want_p2p) * sizeof(int2)));
+    AMK_TRY(lists.m2l_rank.reserve(static_cast<size_t>(want_m2l) * sizeof(int)));
+    AMK_TRY(lists.p2p_rank.reserve(static_cast<size_t>(want_p2p) * sizeof(int)));
     TraverseLists tl;
     tl.m2l = lists.m2l.as<int2>();
     tl.p2p = lists.p2p.as<int2>();
+    tl.m2l_rank = lists.m2l_rank.as<int>();
+    tl.p2p_rank = lists.p2p_rank.as<int>();
+    tl.m2l_count = gm.count;
+    tl.p2p_count = gp.count;
     tl.cap_front = static_cast<long>(std::min(lists.cur.bytes, lists.next.bytes) / sizeof(int2));
-    tl.cap_m2l = static_cast<long>(lists.m2l.bytes / sizeof(int2));
-    tl.cap_p2p = static_cast<long>(lists.p2p.bytes / sizeof(int2));
+    tl.cap_m2l = static_cast<long>(std::min(lists.m2l.bytes / sizeof(int2), lists.m2l_rank.bytes / sizeof(int)));
+    tl.cap_p2p = static_cast<long>(std::min(lists.p2p.bytes / sizeof(int2), lists.p2p_rank.bytes / sizeof(int)));
+    AMK_CUDA_TRY(cudaMemsetAsync(counts, 0, 2 * static_cast<size_t>(nn) * sizeof(int), c->stream));
     AMK_CUDA_TRY(cudaMemsetAsync(tv, 0, n_tv * sizeof(int), c->stream));
     fmm_traverse_root_kernel<<<1, 32, 0, c->stream>>>(lists.cur.as<int2>(), tv + 8);
     AMK_TRY(check_launch(c, "fmm_traverse_root_kernel"));
-    const unsigned grid = static_cast<unsigned>(std::min<long>((tl.cap_front + 255) / 256, 148L * 8));
+    const unsigned grid = static_cast<unsigned>(
+        std::min<long>((tl.cap_front + kTravThreads * kTravPer - 1) / (kTravThreads * kTravPer), 148L * 6));
     for (int level = 0; level < n_levels; ++level) {
       int2* a = (level & 1) ? lists.next.as<int2>() : lists.cur.as<int2>();
       int2* b = (level & 1) ? lists.cur.as<int2>() : lists.next.as<int2>();
-      fmm_traverse_kernel<<<grid, 256, 0, c->stream>>>(t, rec, theta2, a, b, tl, tv + 8 + level, tv);
+      fmm_traverse_kernel<<<grid, kTravThreads, 0, c->stream>>>(t, rec, theta2, a, b, tl, tv + 8 + level, tv);
       AMK_TRY(check_launch(c, "fmm_traverse_kernel"));
     }
     // statistics: leaves and P2P particle pairs (before self / min_sq skips)
@@ -2894,6 +3077,16 @@ int fmm_run(amk_ctx* c, const View& v, int order, double theta, long leaf_capaci
     AMK_TRY(check_launch(c, "p2p_pair_count_kernel"));
     leaf_count_kernel<<<148, 256, 0, c->stream>>>(t, cnt64 + 1);
     AMK_TRY(check_launch(c, "leaf_count_kernel"));
+    AMK_TRY(group_pairs(c, tl.m2l, tl.m2l_rank, tv, tl.cap_m2l, nn, kSlotFmmLists0, kSlotFmmWork0, kSlotFmmWork1,
+                        &gm));
+    AMK_TRY(group_pairs(c, tl.p2p, tl.p2p_rank, tv + 1, tl.cap_p2p, nn, kSlotFmmLists2, kSlotFmmWork2,
+                        kSlotFmmWork3, &gp));
+    // near-field work items: a target leaf and up to kP2PChunk source leaves
+    // of its list (kP2P32Chunk in the FP32 near field)
+    p2p_items_count_kernel<<<gn, 256, 0, c->stream>>>(t, gp.count, f32 ? kP2P32Chunk : kP2PChunk, items, psize);
+    AMK_TRY(check_launch(c, "p2p_items_count_kernel"));
+    AMK_TRY(exclusive_scan_int(c, items, nn, ibase, tv + 4));
+    AMK_TRY(exclusive_scan_int(c, psize, nn, pbase, tv + 5));
     AMK_CUDA_TRY(cudaMemcpyAsync(hv.data(), tv, n_tv * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     AMK_CUDA_TRY(cudaMemcpyAsync(h64, cnt64, sizeof(h64), cudaMemcpyDeviceToHost, c->stream));
     AMK_CUDA_TRY(cudaMemcpyAsync(&hf, t.frame, sizeof(hf), cudaMemcpyDeviceToHost, c->stream));
@@ -2905,6 +3098,8 @@ int fmm_run(amk_ctx* c, const View& v, int order, double theta, long leaf_capaci
       if (hv[8 + n_levels] != 0) return fail(AMK_ERR_STATE, "FMM traversal: pairs left after the deepest level");
       n_m2l = hv[0];
       n_p2p = hv[1];
+      ht[0] = hv[4];
+      ht[1] = hv[5];
       lists.need_front = max_front;
       lists.need_m2l = n_m2l;
       lists.need_p2p = n_p2p;
@@ -2927,38 +3122,13 @@ int fmm_run(amk_ctx* c, const View& v, int order, double theta, long leaf_capaci
     st[6] = t.m;
     st[7] = order;
   }
-  Grouped gm, gp;
-  AMK_TRY(group_pairs(c, lists.m2l.as<int2>(), n_m2l, nn, kSlotFmmLists0, kSlotFmmLists1, kSlotFmmWork0,
-                      kSlotFmmWork1, &gm));
-  AMK_TRY(group_pairs(c, lists.p2p.as<int2>(), n_p2p, nn, kSlotFmmLists2, kSlotFmmLists3, kSlotFmmWork2,
-                      kSlotFmmWork3, &gp));
   AMK_TRY(phase_end(c, AMK_PHASE_FMM_LISTS));
 
-  // ---- near-field set-up: work items (a target leaf and up to kP2PChunk
-  // source leaves of its list, kP2P32Chunk in the FP32 near field) and the
-  // per-item partial sums' layout
+  // ---- near-field set-up
   double4* ef = slot<double4>(c, kSlotFmmWork4, t.m, &rc);
   AMK_TRY(rc);
   const double min_sq = kMinSquaredDistance / (hf.length * hf.length);
-  const bool f32 = c->fmm_precision == AMK_FMM_TENSOR;
   AMK_TRY(phase_begin(c, AMK_PHASE_FMM_P2P));
-  int* items = slot<int>(c, kSlotFmmAux2, nn + 1, &rc);
-  AMK_TRY(rc);
-  int* psize = slot<int>(c, kSlotTreeCount, nn + 1, &rc);  // tree build scratch, free again
-  AMK_TRY(rc);
-  int* ibase = slot<int>(c, kSlotTreeBase, nn + 1, &rc);
-  AMK_TRY(rc);
-  int* pbase = slot<int>(c, kSlotTreeL, nn + 1, &rc);
-  AMK_TRY(rc);
-  int* totals = slot<int>(c, kSlotFmmAux1, 8, &rc);
-  AMK_TRY(rc);
-  p2p_items_count_kernel<<<gn, 256, 0, c->stream>>>(t, gp.count, f32 ? kP2P32Chunk : kP2PChunk, items, psize);
-  AMK_TRY(check_launch(c, "p2p_items_count_kernel"));
-  AMK_TRY(exclusive_scan_int(c, items, nn, ibase, totals));
-  AMK_TRY(exclusive_scan_int(c, psize, nn, pbase, totals + 1));
-  int ht[2] = {0, 0};
-  AMK_CUDA_TRY(cudaMemcpyAsync(ht, totals, sizeof(ht), cudaMemcpyDeviceToHost, c->stream));
-  AMK_CUDA_TRY(cudaStreamSynchronize(c->stream));
   int2* work = slot<int2>(c, kSlotP2PWork, ht[0] + 1, &rc);
   AMK_TRY(rc);
   int* leaf_of = slot<int>(c, kSlotTreeLeafDepth, t.m + 1, &rc);
