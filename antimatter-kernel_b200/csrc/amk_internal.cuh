@@ -184,17 +184,9 @@ enum ScratchSlot {
   kSlotM2lTarget,
   kSlotM2lHist,
   kSlotM2lStart,
-  kSlotM2lUsed,
-  kSlotM2lClassIndex,
-  kSlotM2lTiles,
-  kSlotM2lTileStart,
   kSlotM2lCounters,
   kSlotM2lPerm,
   kSlotM2lFallback,
-  kSlotM2lClassCode,
-  kSlotM2lClassEnd,
-  kSlotM2lTileClass,
-  kSlotM2lTilePos,
   kSlotM2lTable,
   kSlotM2lHash,
   kSlotM2lSplit,
@@ -203,6 +195,9 @@ enum ScratchSlot {
   kSlotM2lTable3,
   kSlotM2lRefl,
   kSlotFmmNodeRec,
+  kSlotFmmCell,
+  kSlotM2lRank,
+  kSlotM2lClassKey,
   kNumSlots
 };
 static_assert(kNumSlots <= 128, "scratch slots");

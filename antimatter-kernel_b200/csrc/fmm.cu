@@ -541,13 +541,20 @@ fmm_m2m_kernel(const Octree t, FmmDevTables T, int depth, double* __restrict__ M
 // Per node, what the traversal reads of it in one 32-byte record: the
 // centre and the radius, negated for a leaf (a leaf of radius 0 stores -0.0;
 // the sign bit is the leaf flag, the magnitude the radius).
+// The M2L classes read the cell's place among the cells of its depth.
 __global__ void fmm_node_record_kernel(const Octree t, const double* __restrict__ radius,
-                                       double4* __restrict__ rec) {
+                                       double4* __restrict__ rec, int4* __restrict__ cell) {
   const int id = blockIdx.x * blockDim.x + threadIdx.x;
   if (id >= t.n_nodes) return;
   const double4 c = t.center[id];
   const double r = radius[id];
   rec[id] = make_double4(c.x, c.y, c.z, t.meta[id].y ? -r : r);
+  // c = root centre - root half edge + (2 i + 1) h
+  const TreeFrame f = *t.frame;
+  const double w = 0.5 / c.w;
+  cell[id] = make_int4(static_cast<int>(floor((c.x - f.root_c[0] + f.root_h) * w)),
+                       static_cast<int>(floor((c.y - f.root_c[1] + f.root_h) * w)),
+                       static_cast<int>(floor((c.z - f.root_c[2] + f.root_h) * w)), t.meta[id].x);
 }
 
 __global__ void fmm_traverse_root_kernel(int2* __restrict__ cur, int* __restrict__ lv) {
@@ -753,14 +760,18 @@ __device__ __forceinline__ void warp_sort(unsigned (&v)[K], int lane) {
 }
 
 template <int K>
-__device__ __forceinline__ void warp_sort_group(const int* __restrict__ in, int* __restrict__ src, int n, int lane) {
+__device__ __forceinline__ void warp_sort_group(const int* __restrict__ in, int* __restrict__ src, int n, int lane,
+                                                int* __restrict__ tgt, int ti) {
   unsigned v[K];
 #pragma unroll
   for (int r = 0; r < K; ++r) v[r] = r * 32 + lane < n ? static_cast<unsigned>(in[r * 32 + lane]) : 0xffffffffu;
   warp_sort<K>(v, lane);
 #pragma unroll
   for (int r = 0; r < K; ++r)
-    if (r * 32 + lane < n) src[r * 32 + lane] = static_cast<int>(v[r]);
+    if (r * 32 + lane < n) {
+      src[r * 32 + lane] = static_cast<int>(v[r]);
+      if (tgt) tgt[r * 32 + lane] = ti;
+    }
 }
 
 constexpr int kSortWarpMax = 512;      // sources a warp sorts in registers
@@ -772,10 +783,10 @@ constexpr int kSortBits = 1 << 19;     // sources per bitmap pass (64 KB of shar
 // bitmap over the nodes (a target's sources are distinct) and writes the set
 // bits out in order, so the work is n + n_nodes / 32 whatever the group's
 // size (groups of several thousand sources are common: a large leaf next to a
-// dense region).
+// dense region). tgt (may be null) receives the target of every pair.
 __global__ void __launch_bounds__(kSortThreads)
 group_sort_kernel(int n_nodes, const int* __restrict__ off, const int* __restrict__ count, long cap,
-                  const int* __restrict__ unsorted, int* __restrict__ src) {
+                  const int* __restrict__ unsorted, int* __restrict__ src, int* __restrict__ tgt) {
   extern __shared__ unsigned sort_bits[];
   __shared__ int warp_sum[kSortThreads / 32];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -785,21 +796,23 @@ group_sort_kernel(int n_nodes, const int* __restrict__ off, const int* __restric
     const long b = off[t0 + w];
     if (n > 0 && b + n <= cap) {
       if (n <= 32)
-        warp_sort_group<1>(unsorted + b, src + b, n, lane);
+        warp_sort_group<1>(unsorted + b, src + b, n, lane, tgt ? tgt + b : nullptr, t0 + w);
       else if (n <= 64)
-        warp_sort_group<2>(unsorted + b, src + b, n, lane);
+        warp_sort_group<2>(unsorted + b, src + b, n, lane, tgt ? tgt + b : nullptr, t0 + w);
       else if (n <= 128)
-        warp_sort_group<4>(unsorted + b, src + b, n, lane);
+        warp_sort_group<4>(unsorted + b, src + b, n, lane, tgt ? tgt + b : nullptr, t0 + w);
       else if (n <= 256)
-        warp_sort_group<8>(unsorted + b, src + b, n, lane);
+        warp_sort_group<8>(unsorted + b, src + b, n, lane, tgt ? tgt + b : nullptr, t0 + w);
       else if (n <= kSortWarpMax)
-        warp_sort_group<16>(unsorted + b, src + b, n, lane);
+        warp_sort_group<16>(unsorted + b, src + b, n, lane, tgt ? tgt + b : nullptr, t0 + w);
     }
   }
   for (int k = 0; k < kSortThreads / 32 && t0 + k < n_nodes; ++k) {
     const int n = count[t0 + k];
     const long b = off[t0 + k];
     if (n <= kSortWarpMax || b + n > cap) continue;
+    if (tgt)
+      for (int i = tid; i < n; i += kSortThreads) tgt[b + i] = t0 + k;
     int first = 0;  // sources written so far
     for (int r0 = 0; r0 < n_nodes; r0 += kSortBits) {
       const int bits = min(kSortBits, n_nodes - r0), words = (bits + 31) / 32;
@@ -839,6 +852,7 @@ struct Grouped {
   int* off = nullptr;
   int* count = nullptr;
   int* src = nullptr;
+  int* tgt = nullptr;  // target of every grouped pair (M2L)
 };
 
 // ------------------------------------------------------------ M2L
@@ -860,12 +874,12 @@ struct Grouped {
 // pairs, up to 8 tiles of one class per block. The products are written per pair and summed per target in the
 // pairs' (target, source) order, so the result is run-to-run deterministic.
 // A class is found through an open-addressing hash of (d_t - d_s, v) with
-// bounded probing; pairs off the lattice, beyond the class reach or left
-// without a hash slot take a per-pair path with the derivative recurrence.
+// bounded probing; pairs beyond the class reach or left without a hash slot
+// take a per-pair path with the derivative recurrence.
 // The pairs are processed in chunks that bound the per-pair scratch.
 constexpr int kM2lTileP = 64;      // pairs per product tile
-constexpr int kM2lUnitTiles = 8;   // tiles of one class per block
-constexpr int kM2lUnitPairs = kM2lUnitTiles * kM2lTileP;
+constexpr int kM2lUnitPairs = 4 * kM2lTileP;    // pairs of one class taken at a time (FP64 products)
+constexpr int kM2lTcUnitPairs = 8 * kM2lTileP;  // the same for the tensor-core products
 // classes below this size take the per-pair path in both precision modes (in
 // tensor-core mode a class-matrix build per tiny class costs more than the
 // per-pair path: measured at 1,048,576 particles, leaf 128)
@@ -891,25 +905,18 @@ __device__ __forceinline__ int m2l_key_v(unsigned long long k, int axis) {
   return static_cast<int>((k >> (38 - 19 * axis)) & ((1u << 19) - 1)) - kM2lVBias;
 }
 
-// Class key of a pair, kM2lEmpty = off the lattice or out of reach. The
-// centres are sums of power-of-two fractions of the root half edge, rounded
-// to FP64 at every level, so a lattice offset v carries a rounding error of
-// a few dozen ulp of max|c| / u; the acceptance tolerance tracks that bound
-// (256 ulp), and a pair further off the lattice takes the per-pair path,
-// where D is built from the actual centres as in the reference.
-__device__ __forceinline__ unsigned long long m2l_class_key(const Octree& t, int ti, int si, int reach, bool fold,
+// Class key of a pair of cells given by their place among the cells of their
+// depth {ix, iy, iz, depth}: in units of the smaller half edge the centres are
+// odd integers times a power of two, so the lattice offset is integer
+// arithmetic. kM2lEmpty = out of reach.
+__device__ __forceinline__ unsigned long long m2l_class_key(const int4& tc, const int4& sc, int reach, bool fold,
                                                             int* refl) {
-  const double4 tc = t.center[ti], sc = t.center[si];
-  const int dd = static_cast<int>(t.meta[ti].x) - static_cast<int>(t.meta[si].x);
-  const double u = fmin(tc.w, sc.w);
-  const double vx = (tc.x - sc.x) / u, vy = (tc.y - sc.y) / u, vz = (tc.z - sc.z) / u;
-  const double rx = rint(vx), ry = rint(vy), rz = rint(vz);
-  const double cmax = fmax(fmax(fmax(fabs(tc.x), fabs(tc.y)), fmax(fabs(tc.z), fabs(sc.x))),
-                           fmax(fabs(sc.y), fabs(sc.z)));
-  const double tol = 256.0 * 2.220446049250313e-16 * (cmax / u + fabs(rx) + fabs(ry) + fabs(rz) + 1.0);
-  if (fabs(vx - rx) > tol || fabs(vy - ry) > tol || fabs(vz - rz) > tol) return kM2lEmpty;
-  if (fabs(rx) > reach || fabs(ry) > reach || fabs(rz) > reach) return kM2lEmpty;
-  int ix = static_cast<int>(rx), iy = static_cast<int>(ry), iz = static_cast<int>(rz), r = 0;
+  const int dd = tc.w - sc.w, st = max(-dd, 0), ss = max(dd, 0);
+  int ix = ((2 * tc.x + 1) << st) - ((2 * sc.x + 1) << ss);
+  int iy = ((2 * tc.y + 1) << st) - ((2 * sc.y + 1) << ss);
+  int iz = ((2 * tc.z + 1) << st) - ((2 * sc.z + 1) << ss);
+  if (abs(ix) > reach || abs(iy) > reach || abs(iz) > reach) return kM2lEmpty;
+  int r = 0;
   if (fold) {  // the class of |v|; the reflection that maps |v| to v in bits x, y, z
     if (ix < 0) ix = -ix, r |= 1;
     if (iy < 0) iy = -iy, r |= 2;
@@ -971,25 +978,26 @@ __global__ void m2l_rescale_red_kernel(const Octree t, FmmDevTables T, const dou
   Mr[e] = v;
 }
 
-// Class slot (-1: per-pair path) and target of every pair (a warp per target);
-// refl (tensor-core mode) is cleared: every pair starts unreflected.
-__global__ void m2l_classify_kernel(const Octree t, const int* __restrict__ off, const int* __restrict__ count,
+// Class slot (-1: per-pair path) of every pair, the pairs per class in hist
+// and (one chunk) each pair's place among them; refl (tensor-core mode) is
+// cleared: every pair starts unreflected. A thread per pair: the chain of
+// dependent loads (source, cell, hash slot, count) is hidden by occupancy (a
+// warp walking one target's pairs took 870 us at 11.6 M pairs).
+__global__ void m2l_classify_kernel(long n, const int4* __restrict__ cell, const int* __restrict__ tgt,
                                     const int* __restrict__ src, int reach, unsigned long long* __restrict__ keys,
-                                    int* __restrict__ codes, int* __restrict__ tgt,
+                                    int* __restrict__ codes, int* __restrict__ hist, int* __restrict__ rank,
                                     unsigned char* __restrict__ refl) {
-  const int lane = threadIdx.x & 31;
-  const long w0 = (blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x) >> 5;
-  const long nw = (static_cast<long>(gridDim.x) * blockDim.x) >> 5;
-  for (long ti = w0; ti < t.n_nodes; ti += nw) {
-    const int b = off[ti], n = count[ti];
-    for (int e = b + lane; e < b + n; e += 32) {
-      int r = 0;
-      const unsigned long long key = m2l_class_key(t, static_cast<int>(ti), src[e], reach, false, &r);
-      codes[e] = key == kM2lEmpty ? -1 : m2l_hash_slot(keys, key);
-      tgt[e] = static_cast<int>(ti);
-      if (refl) refl[e] = 0;
-    }
+  const long e = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
+  if (e >= n) return;
+  int r = 0;
+  const unsigned long long key = m2l_class_key(cell[tgt[e]], cell[src[e]], reach, false, &r);
+  const int code = key == kM2lEmpty ? -1 : m2l_hash_slot(keys, key);
+  codes[e] = code;
+  if (hist && code >= 0) {
+    const int at = atomicAdd(hist + code, 1);
+    if (rank) rank[e] = at;
   }
+  if (refl) refl[e] = 0;
 }
 
 // Tensor-core mode: a pair of a class smaller than min_class (over all
@@ -1001,89 +1009,98 @@ __global__ void m2l_classify_kernel(const Octree t, const int* __restrict__ off,
 // Folding the 8 reflections merges most of the small classes into classes
 // large enough for a class product (or into the class of |v| itself when
 // that one exists), while the pairs of large classes keep their own.
-__global__ void m2l_refold_kernel(const Octree t, const int* __restrict__ hist, int min_class,
+// hist and rank follow the move (one chunk): a class of fewer than min_class
+// pairs with v != |v| moves whole -- its pairs share v -- so its count becomes
+// zero, and no class loses pairs that another is counted into.
+__global__ void m2l_refold_kernel(const int4* __restrict__ cell, int* __restrict__ hist, int min_class,
                                   const int* __restrict__ tgt, const int* __restrict__ src, int reach, long n,
                                   unsigned long long* __restrict__ keys, int* __restrict__ codes,
-                                  unsigned char* __restrict__ refl) {
+                                  int* __restrict__ rank, unsigned char* __restrict__ refl) {
   const long e = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
   if (e >= n) return;
   const int code = codes[e];
   if (code < 0 || hist[code] >= min_class) return;
   int r = 0;
-  const unsigned long long key = m2l_class_key(t, tgt[e], src[e], reach, true, &r);
+  const unsigned long long key = m2l_class_key(cell[tgt[e]], cell[src[e]], reach, true, &r);
   if (key == kM2lEmpty || r == 0) return;
   const int folded = m2l_hash_slot(keys, key);
   if (folded < 0) return;  // no slot: the pair stays in its own (small) class
   codes[e] = folded;
   refl[e] = static_cast<unsigned char>(r);
-}
-
-// Pairs per class code over all pairs (tensor-core mode, before folding).
-__global__ void m2l_code_count_kernel(const int* __restrict__ codes, long n, int* __restrict__ hist) {
-  const long e = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
-  if (e < n && codes[e] >= 0) atomicAdd(hist + codes[e], 1);
-}
-
-// Pairs per class code in [e0, e1); off-lattice pairs listed for the per-pair path.
-__global__ void m2l_histogram_kernel(const int* __restrict__ codes, long e0, long e1, int* __restrict__ hist,
-                                     int* __restrict__ fallback, int* __restrict__ n_fallback) {
-  const long e = e0 + blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
-  if (e >= e1) return;
-  const int code = codes[e];
-  if (code >= 0)
-    atomicAdd(hist + code, 1);
-  else
-    fallback[atomicAdd(n_fallback, 1)] = static_cast<int>(e);
-}
-
-// Classes of fewer than min_class pairs go the per-pair path; their counts
-// are cleared, so the scan of hist places the pairs of the classes taken
-// contiguously at the start of the chunk's permutation.
-__global__ void m2l_code_flags_kernel(int* __restrict__ hist, long n_codes, int min_class,
-                                      int* __restrict__ used, int* __restrict__ units) {
-  const long code = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
-  if (code >= n_codes) return;
-  const int n = hist[code];
-  const bool take = n > 0 && n >= min_class;
-  used[code] = take;
-  units[code] = take ? (n + kM2lUnitPairs - 1) / kM2lUnitPairs : 0;
-  if (!take) hist[code] = 0;
-}
-
-// Class list and product units (<= 8 tiles of one class) from the scanned
-// per-code counts.
-__global__ void m2l_class_fill_kernel(const int* __restrict__ hist, const int* __restrict__ start,
-                                      const int* __restrict__ cls_index, const int* __restrict__ unit_start,
-                                      long n_codes, const int* __restrict__ used, int* __restrict__ cls_code,
-                                      int* __restrict__ cls_end, int* __restrict__ unit_cls,
-                                      int* __restrict__ unit_pos) {
-  const long code = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
-  if (code >= n_codes) return;
-  const int n = hist[code];
-  if (!used[code]) return;
-  const int cls = cls_index[code];
-  cls_code[cls] = static_cast<int>(code);
-  cls_end[cls] = start[code] + n;
-  const int nu = (n + kM2lUnitPairs - 1) / kM2lUnitPairs;
-  for (int k = 0; k < nu; ++k) {
-    unit_cls[unit_start[code] + k] = cls;
-    unit_pos[unit_start[code] + k] = start[code] + k * kM2lUnitPairs;
+  if (rank) {
+    rank[e] = atomicAdd(hist + folded, 1);
+    hist[code] = 0;
   }
 }
 
+// Pairs per class code in [e0, e1) and each pair's place among them (chunks).
+__global__ void m2l_histogram_kernel(const int* __restrict__ codes, long e0, long e1, int* __restrict__ hist,
+                                     int* __restrict__ rank) {
+  const long e = e0 + blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
+  if (e < e1 && codes[e] >= 0) rank[e] = atomicAdd(hist + codes[e], 1);
+}
+
+// The classes of at least min_class pairs: a class number, the first place of
+// the class in the chunk's permutation and its product units {class, first
+// pair, pairs, depth difference}; start[code] = -1 for the others (per-pair
+// path). A warp reserves for its 32 codes with one atomic per counter:
+// counters = {pairs, classes, units}. (Flags, three scans over the 2^21 codes
+// and a fill took eleven launches.)
+__global__ void m2l_class_build_kernel(const int* __restrict__ hist, long n_codes, int min_class, int unit_pairs,
+                                       const unsigned long long* __restrict__ keys, int* __restrict__ counters,
+                                       int* __restrict__ start, unsigned long long* __restrict__ cls_key,
+                                       int4* __restrict__ ud) {
+  const long code = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const int n = code < n_codes ? hist[code] : 0;
+  const bool take = n > 0 && n >= min_class;
+  if (n > 0 && !take) start[code] = -1;
+  const unsigned m = __ballot_sync(0xffffffffu, take);
+  if (m == 0) return;
+  const int nu = take ? (n + unit_pairs - 1) / unit_pairs : 0;
+  int pairs = take ? n : 0, units = nu;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int a = __shfl_up_sync(0xffffffffu, pairs, o), b = __shfl_up_sync(0xffffffffu, units, o);
+    if (lane >= o) {
+      pairs += a;
+      units += b;
+    }
+  }
+  int base[3] = {0, 0, 0};
+  if (lane == 31) {
+    base[0] = atomicAdd(counters, pairs);
+    base[1] = atomicAdd(counters + 1, __popc(m));
+    base[2] = atomicAdd(counters + 2, units);
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) base[k] = __shfl_sync(0xffffffffu, base[k], 31);
+  if (!take) return;
+  const int first = base[0] + pairs - n, cls = base[1] + __popc(m & ((1u << lane) - 1u));
+  const unsigned long long key = keys[code];
+  start[code] = first;
+  cls_key[cls] = key;
+  for (int k = 0; k < nu; ++k)
+    ud[base[2] + units - nu + k] =
+        make_int4(cls, first + k * unit_pairs, min(unit_pairs, n - k * unit_pairs), m2l_key_dd(key));
+}
+
 // Pair positions grouped by class (order inside a class is irrelevant: every
-// pair's product is computed on its own); pairs of small classes join the
-// per-pair list. Consumes hist.
-__global__ void m2l_scatter_kernel(const int* __restrict__ codes, long e0, long e1, const int* __restrict__ start,
-                                   const int* __restrict__ used, int* __restrict__ hist, int* __restrict__ perm,
-                                   int* __restrict__ fallback, int* __restrict__ n_fallback,
-                                   unsigned char* __restrict__ refl) {
+// pair's product is computed on its own) and the source rows in that order
+// (with refl a folded pair reads the reflected copy of the split expansions);
+// pairs without a class join the per-pair list.
+__global__ void m2l_scatter_kernel(const int* __restrict__ codes, const int* __restrict__ rank, long e0, long e1,
+                                   const int* __restrict__ start, const int* __restrict__ src, int n_cells,
+                                   int* __restrict__ perm, int* __restrict__ psrc, int* __restrict__ fallback,
+                                   int* __restrict__ n_fallback, unsigned char* __restrict__ refl) {
   const long e = e0 + blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
   if (e >= e1) return;
   const int code = codes[e];
-  if (code < 0) return;
-  if (used[code]) {
-    perm[start[code] + atomicSub(hist + code, 1) - 1] = static_cast<int>(e);
+  const int first = code >= 0 ? start[code] : -1;
+  if (first >= 0) {
+    const int at = first + rank[e];
+    perm[at] = static_cast<int>(e);
+    psrc[at] = (refl ? static_cast<int>(refl[e]) * n_cells : 0) + src[e];
   } else {
     fallback[atomicAdd(n_fallback, 1)] = static_cast<int>(e);
     if (refl) refl[e] = 0;  // the per-pair path works from the actual centres
@@ -1119,15 +1136,14 @@ __device__ __forceinline__ void split3_bf16(double v, __nv_bfloat16* t);
 // (tensor-core mode, table3 given) split into three BF16 terms packed as
 // {t0 | t1 << 16, t2} into table3[class * nd3 + k], zero for k >= n.
 __global__ void __launch_bounds__(32 * kFmmWarps)
-m2l_table_kernel(DerivTables T, const int* __restrict__ cls_code, int n_classes,
-                 const unsigned long long* __restrict__ keys, double* __restrict__ table,
-                 uint2* __restrict__ table3, int nd3) {
+m2l_table_kernel(DerivTables T, const unsigned long long* __restrict__ cls_key, int n_classes,
+                 double* __restrict__ table, uint2* __restrict__ table3, int nd3) {
   extern __shared__ __align__(16) unsigned char tab_smem[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   double* D = reinterpret_cast<double*>(tab_smem) + static_cast<size_t>(w) * T.n;
   const int cls = blockIdx.x * kFmmWarps + w;
   if (cls >= n_classes) return;
-  const unsigned long long key = keys[cls_code[cls]];
+  const unsigned long long key = cls_key[cls];
   const double xs[3] = {static_cast<double>(m2l_key_v(key, 0)), static_cast<double>(m2l_key_v(key, 1)),
                         static_cast<double>(m2l_key_v(key, 2))};
   m2l_derivatives(T, lane, xs, D);
@@ -1344,10 +1360,10 @@ m2l_class_mma_kernel(FmmDevTables T, int n_units, int* __restrict__ unit_counter
 //
 // Before the kernel, per evaluation chunk: the cells' rescaled expansions
 // are split into BF16 rows of kKp elements (m2l_split_kernel), each class's
-// D(v) into packed BF16 terms (m2l_table_kernel), and every unit gets a
+// D(v) into packed BF16 terms (m2l_table_kernel), and every unit has a
 // descriptor {class, first pair, pairs, depth difference} and every pair its
-// source cell (m2l_unit_prep_kernel), so each role reads one value where it
-// would otherwise follow a chain of dependent loads.
+// source row, so each role reads one value where it would otherwise follow a
+// chain of dependent loads.
 //
 // Roles (one CTA per SM, units of one class taken in a fixed stride; every
 // role prefetches the next unit's descriptor and the next tile's indices):
@@ -1440,25 +1456,6 @@ __global__ void m2l_split_kernel(long n_cells, int nm, int kp, const int4* __res
     const size_t row = (static_cast<size_t>(R) * n_cells + cell) * 3;
 #pragma unroll
     for (int q = 0; q < 3; ++q) Mh3[(row + q) * kp + a] = (odd & 1) ? __hneg(t[q]) : t[q];
-  }
-}
-
-// Unit descriptors {class, first pair, pairs, depth difference} and the
-// source row of every class pair.
-__global__ void m2l_unit_prep_kernel(int n_units, const int* __restrict__ unit_cls, const int* __restrict__ unit_pos,
-                                   const int* __restrict__ cls_code, const int* __restrict__ cls_end,
-                                   const unsigned long long* __restrict__ keys, int n_pairs,
-                                   const int* __restrict__ perm, const int* __restrict__ src,
-                                   const unsigned char* __restrict__ refl, int n_cells, int4* __restrict__ ud,
-                                   int* __restrict__ psrc) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x < n_units) {
-    const int cls = unit_cls[x], pos0 = unit_pos[x];
-    ud[x] = make_int4(cls, pos0, min(kM2lUnitPairs, cls_end[cls] - pos0), m2l_key_dd(keys[cls_code[cls]]));
-  }
-  if (x < n_pairs) {  // the source's row in the split expansions (its reflected copy when folded)
-    const int e = perm[x];
-    psrc[x] = (refl ? static_cast<int>(refl[e]) * n_cells : 0) + src[e];
   }
 }
 
@@ -1865,14 +1862,13 @@ m2l_pair_red_kernel(const Octree t, FmmDevTables T, const int* __restrict__ list
 template <int V>
 __global__ void __launch_bounds__(256)
 m2l_reduce_red_kernel(const Octree t, FmmDevTables T, const int* __restrict__ off, const int* __restrict__ count,
-                      int t_first, int n_targets, long e0, long e1, const double* __restrict__ out,
-                      double* __restrict__ L) {
+                      int n_targets, long e0, long e1, const double* __restrict__ out, double* __restrict__ L) {
   constexpr int kU = V == 1 ? 8 : 4;
   __shared__ double2 qs[8][32 * V];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int k = blockIdx.x * 8 + w;
   if (k >= n_targets) return;
-  const int ti = t_first + k, nv = T.n_rp >> 1;
+  const int ti = k, nv = T.n_rp >> 1;
   const long b = max(static_cast<long>(off[ti]), e0), end = min(static_cast<long>(off[ti]) + count[ti], e1);
   if (b >= end) return;
   double2 s[V];
@@ -1958,13 +1954,12 @@ m2l_refl_sign_kernel(FmmDevTables T, long e0, long e1, const unsigned char* __re
 // coefficient is the FP64 sum in pair order.
 __global__ void __launch_bounds__(256)
 m2l_reduce_f4_kernel(const Octree t, FmmDevTables T, const int* __restrict__ off, const int* __restrict__ count,
-                     int t_first, int n_targets, long e0, long e1, const float* __restrict__ out,
-                     double* __restrict__ L) {
+                     int n_targets, long e0, long e1, const float* __restrict__ out, double* __restrict__ L) {
   constexpr int kU = 8;
   const int lane = threadIdx.x & 31;
   const int k = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (k >= n_targets) return;
-  const int ti = t_first + k, nm = T.n_m, nv = nm >> 2;
+  const int ti = k, nm = T.n_m, nv = nm >> 2;
   const long b = max(static_cast<long>(off[ti]), e0), end = min(static_cast<long>(off[ti]) + count[ti], e1);
   if (b >= end || lane >= nv) return;
   double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
@@ -2082,8 +2077,8 @@ int m2l_reach() {
 // All M2L pairs (grouped by target in gm) into L. after_products (may be
 // empty) runs once the last chunk's products are enqueued on the context
 // stream, before their per-target sums and the final status read.
-int m2l_products(amk_ctx* c, int order, const Octree& t, const FmmDevTables& T, const Grouped& gm, long n_m2l,
-                 const double* M, double* L, const std::function<int()>& after_products) {
+int m2l_products(amk_ctx* c, int order, const Octree& t, const FmmDevTables& T, const Grouped& gm, const int4* cell,
+                 long n_m2l, const double* M, double* L, const std::function<int()>& after_products) {
   int rc = AMK_OK;
   const long nn = t.n_nodes;
   const int reach = m2l_reach();
@@ -2099,19 +2094,12 @@ int m2l_products(amk_ctx* c, int order, const Octree& t, const FmmDevTables& T, 
   AMK_TRY(rc);
   int* codes = slot<int>(c, kSlotM2lCodes, n_m2l, &rc);
   AMK_TRY(rc);
-  int* tgt = slot<int>(c, kSlotM2lTarget, n_m2l, &rc);
-  AMK_TRY(rc);
+  const int* tgt = gm.tgt;
   int* hist = slot<int>(c, kSlotM2lHist, n_codes + 1, &rc);
   AMK_TRY(rc);
   int* start = slot<int>(c, kSlotM2lStart, n_codes + 1, &rc);
   AMK_TRY(rc);
-  int* used = slot<int>(c, kSlotM2lUsed, n_codes + 1, &rc);
-  AMK_TRY(rc);
-  int* cls_index = slot<int>(c, kSlotM2lClassIndex, n_codes + 1, &rc);
-  AMK_TRY(rc);
-  int* nunit = slot<int>(c, kSlotM2lTiles, n_codes + 1, &rc);
-  AMK_TRY(rc);
-  int* unit_start = slot<int>(c, kSlotM2lTileStart, n_codes + 1, &rc);
+  int* rank = slot<int>(c, kSlotM2lRank, n_m2l, &rc);
   AMK_TRY(rc);
   int* counters = slot<int>(c, kSlotM2lCounters, 8, &rc);  // pairs, classes, units, fallback pairs
   AMK_TRY(rc);
@@ -2127,22 +2115,24 @@ int m2l_products(amk_ctx* c, int order, const Octree& t, const FmmDevTables& T, 
     AMK_TRY(rc);
   }
   AMK_CUDA_TRY(cudaMemsetAsync(keys, 0xff, kM2lHashSlots * sizeof(unsigned long long), c->stream));
-  m2l_classify_kernel<<<4 * 148, 256, 0, c->stream>>>(t, gm.off, gm.count, gm.src, reach, keys, codes, tgt, refl);
-  AMK_TRY(check_launch(c, "m2l_classify_kernel"));
-  if (tc) {  // class sizes over all pairs, then the small classes folded by reflection
-    AMK_CUDA_TRY(cudaMemsetAsync(hist, 0, n_codes * sizeof(int), c->stream));
-    const unsigned ga = static_cast<unsigned>((n_m2l + 255) / 256);
-    m2l_code_count_kernel<<<ga, 256, 0, c->stream>>>(codes, n_m2l, hist);
-    AMK_TRY(check_launch(c, "m2l_code_count_kernel"));
-    m2l_refold_kernel<<<ga, 256, 0, c->stream>>>(t, hist, kM2lMinClass, tgt, gm.src, reach, n_m2l, keys, codes,
-                                                  refl);
-    AMK_TRY(check_launch(c, "m2l_refold_kernel"));
-  }
   const size_t esz = tc ? sizeof(float) : sizeof(double);
   long cap = std::max<long>(1L << 20, static_cast<long>((tc ? kM2lTcChunkBytes : kM2lChunkBytes) / (esz * row)));
   if (const char* env = getenv("AMK_FMM_M2L_CHUNK_PAIRS")) {  // smaller chunks (tests of the chunk seams)
     const long v = atol(env);
     if (v > 0) cap = std::min(cap, v);
+  }
+  const bool one_chunk = n_m2l <= cap;  // the counts of the classification are the chunk's
+  const int unit_pairs = tc ? kM2lTcUnitPairs : kM2lUnitPairs;
+  int* class_hist = tc || one_chunk ? hist : nullptr;
+  int* class_rank = one_chunk ? rank : nullptr;
+  if (class_hist) AMK_CUDA_TRY(cudaMemsetAsync(hist, 0, n_codes * sizeof(int), c->stream));
+  m2l_classify_kernel<<<static_cast<unsigned>((n_m2l + 255) / 256), 256, 0, c->stream>>>(
+      n_m2l, cell, gm.tgt, gm.src, reach, keys, codes, class_hist, class_rank, refl);
+  AMK_TRY(check_launch(c, "m2l_classify_kernel"));
+  if (tc) {  // the small classes (over all pairs) folded by reflection
+    m2l_refold_kernel<<<static_cast<unsigned>((n_m2l + 255) / 256), 256, 0, c->stream>>>(
+        cell, hist, kM2lMinClass, tgt, gm.src, reach, n_m2l, keys, codes, class_rank, refl);
+    AMK_TRY(check_launch(c, "m2l_refold_kernel"));
   }
   Fmm* f = c->fmm;
   if (!f->side) {
@@ -2152,18 +2142,16 @@ int m2l_products(amk_ctx* c, int order, const Octree& t, const FmmDevTables& T, 
       AMK_CUDA_TRY(cudaEventCreateWithFlags(&f->sums_done[i], cudaEventDisableTiming));
     }
   }
-  const long max_cls = std::min<long>(cap, n_codes) + 1, max_units = cap / kM2lUnitPairs + max_cls + 1;
+  const long max_cls = std::min({cap, n_m2l, n_codes}) / kM2lMinClass + 1, max_units = std::min(cap, n_m2l) / unit_pairs + max_cls + 1;
   int* perm = slot<int>(c, kSlotM2lPerm, std::min(cap, n_m2l), &rc);
   AMK_TRY(rc);
   int* fallback = slot<int>(c, kSlotM2lFallback, std::min(cap, n_m2l), &rc);
   AMK_TRY(rc);
-  int* cls_code = slot<int>(c, kSlotM2lClassCode, max_cls, &rc);
+  int* psrc = slot<int>(c, kSlotM2lPairSrc, std::min(cap, n_m2l), &rc);
   AMK_TRY(rc);
-  int* cls_end = slot<int>(c, kSlotM2lClassEnd, max_cls, &rc);
+  unsigned long long* cls_key = slot<unsigned long long>(c, kSlotM2lClassKey, max_cls, &rc);
   AMK_TRY(rc);
-  int* unit_cls = slot<int>(c, kSlotM2lTileClass, max_units, &rc);
-  AMK_TRY(rc);
-  int* unit_pos = slot<int>(c, kSlotM2lTilePos, max_units, &rc);
+  int4* ud = slot<int4>(c, kSlotM2lUnitDesc, max_units, &rc);
   AMK_TRY(rc);
   int* tc_status = counters + 6;
   __nv_bfloat16* Mh3 = nullptr;
@@ -2184,26 +2172,21 @@ int m2l_products(amk_ctx* c, int order, const Octree& t, const FmmDevTables& T, 
     const long e1 = std::min(n_m2l, e0 + cap), ne = e1 - e0;
     const int buf = chunk & 1;
     void* out = f->m2l_out[buf].ptr;
-    AMK_CUDA_TRY(cudaMemsetAsync(hist, 0, n_codes * sizeof(int), c->stream));
     AMK_CUDA_TRY(cudaMemsetAsync(counters, 0, 6 * sizeof(int), c->stream));  // [6]: the tensor-core status
     const unsigned ge = static_cast<unsigned>((ne + 255) / 256), gc = static_cast<unsigned>((n_codes + 255) / 256);
-    m2l_histogram_kernel<<<ge, 256, 0, c->stream>>>(codes, e0, e1, hist, fallback, counters + 3);
-    AMK_TRY(check_launch(c, "m2l_histogram_kernel"));
-    m2l_code_flags_kernel<<<gc, 256, 0, c->stream>>>(hist, n_codes, kM2lMinClass, used, nunit);
-    AMK_TRY(check_launch(c, "m2l_code_flags_kernel"));
-    AMK_TRY(exclusive_scan_int(c, hist, n_codes, start, counters));
-    AMK_TRY(exclusive_scan_int(c, used, n_codes, cls_index, counters + 1));
-    AMK_TRY(exclusive_scan_int(c, nunit, n_codes, unit_start, counters + 2));
-    m2l_class_fill_kernel<<<gc, 256, 0, c->stream>>>(hist, start, cls_index, unit_start, n_codes, used, cls_code,
-                                                     cls_end, unit_cls, unit_pos);
-    AMK_TRY(check_launch(c, "m2l_class_fill_kernel"));
-    m2l_scatter_kernel<<<ge, 256, 0, c->stream>>>(codes, e0, e1, start, used, hist, perm, fallback, counters + 3,
-                                                  refl);
+    if (!one_chunk) {
+      AMK_CUDA_TRY(cudaMemsetAsync(hist, 0, n_codes * sizeof(int), c->stream));
+      m2l_histogram_kernel<<<ge, 256, 0, c->stream>>>(codes, e0, e1, hist, rank);
+      AMK_TRY(check_launch(c, "m2l_histogram_kernel"));
+    }
+    m2l_class_build_kernel<<<gc, 256, 0, c->stream>>>(hist, n_codes, kM2lMinClass, unit_pairs, keys, counters, start,
+                                                      cls_key, ud);
+    AMK_TRY(check_launch(c, "m2l_class_build_kernel"));
+    m2l_scatter_kernel<<<ge, 256, 0, c->stream>>>(codes, rank, e0, e1, start, gm.src, static_cast<int>(nn), perm, psrc,
+                                                  fallback, counters + 3, refl);
     AMK_TRY(check_launch(c, "m2l_scatter_kernel"));
-    int h[4] = {0, 0, 0, 0}, tr[2] = {0, 0};
+    int h[4] = {0, 0, 0, 0};
     AMK_CUDA_TRY(cudaMemcpyAsync(h, counters, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
-    AMK_CUDA_TRY(cudaMemcpyAsync(tr, tgt + e0, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    AMK_CUDA_TRY(cudaMemcpyAsync(tr + 1, tgt + e1 - 1, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     AMK_CUDA_TRY(cudaStreamSynchronize(c->stream));
     const int n_cls = h[1], n_units = h[2], n_fb = h[3];
     // the classes' pairs fill perm[0, h[0]) and every other pair is on the per-pair list
@@ -2230,19 +2213,8 @@ int m2l_products(amk_ctx* c, int order, const Octree& t, const FmmDevTables& T, 
       AMK_CUDA_TRY(cudaFuncSetAttribute(m2l_table_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         static_cast<int>(tsm)));
       m2l_table_kernel<<<(n_cls + kFmmWarps - 1) / kFmmWarps, 32 * kFmmWarps, tsm, c->stream>>>(
-          dt, cls_code, n_cls, keys, table, table3, nd3);
+          dt, cls_key, n_cls, table, table3, nd3);
       AMK_TRY(check_launch(c, "m2l_table_kernel"));
-      // unit descriptors, pair sources
-      const long n_cp = ne - n_fb;  // pairs in classes: perm[0, n_cp)
-      int4* ud = slot<int4>(c, kSlotM2lUnitDesc, static_cast<size_t>(n_units), &rc);
-      AMK_TRY(rc);
-      int* psrc = slot<int>(c, kSlotM2lPairSrc, static_cast<size_t>(std::max<long>(1, n_cp)), &rc);
-      AMK_TRY(rc);
-      const long np_ = std::max<long>(n_units, n_cp);
-      m2l_unit_prep_kernel<<<static_cast<unsigned>((np_ + 255) / 256), 256, 0, c->stream>>>(
-          n_units, unit_cls, unit_pos, cls_code, cls_end, keys, static_cast<int>(n_cp), perm, gm.src, refl,
-          static_cast<int>(nn), ud, psrc);
-      AMK_TRY(check_launch(c, "m2l_unit_prep_kernel"));
       AMK_TRY(phase_begin(c, AMK_PHASE_FMM_M2L_PRODUCTS));
       if (tc)
         AMK_TRY(class_tc(c, order, T, n_units, ud, perm, psrc, Mh3, table3, e0, static_cast<float*>(out),
@@ -2281,16 +2253,16 @@ int m2l_products(amk_ctx* c, int order, const Octree& t, const FmmDevTables& T, 
     // per-target sums on the side stream, in chunk order
     AMK_CUDA_TRY(cudaEventRecord(f->products_done[buf], c->stream));
     AMK_CUDA_TRY(cudaStreamWaitEvent(f->side, f->products_done[buf], 0));
-    const int n_tgt = tr[1] - tr[0] + 1;
+    const int n_tgt = static_cast<int>(nn);  // (targets without pairs in the chunk return at once)
     const unsigned gt = static_cast<unsigned>((n_tgt + 7) / 8);
     if (tc)
-      m2l_reduce_f4_kernel<<<gt, 256, 0, f->side>>>(t, T, gm.off, gm.count, tr[0], n_tgt, e0, e1,
+      m2l_reduce_f4_kernel<<<gt, 256, 0, f->side>>>(t, T, gm.off, gm.count, n_tgt, e0, e1,
                                                     static_cast<const float*>(out), L);
     else if (T.n_rp <= 64)
-      m2l_reduce_red_kernel<1><<<gt, 256, 0, f->side>>>(t, T, gm.off, gm.count, tr[0], n_tgt, e0, e1,
+      m2l_reduce_red_kernel<1><<<gt, 256, 0, f->side>>>(t, T, gm.off, gm.count, n_tgt, e0, e1,
                                                         static_cast<const double*>(out), L);
     else
-      m2l_reduce_red_kernel<2><<<gt, 256, 0, f->side>>>(t, T, gm.off, gm.count, tr[0], n_tgt, e0, e1,
+      m2l_reduce_red_kernel<2><<<gt, 256, 0, f->side>>>(t, T, gm.off, gm.count, n_tgt, e0, e1,
                                                         static_cast<const double*>(out), L);
     AMK_TRY(check_launch(c, "m2l_reduce_kernel"));
     AMK_CUDA_TRY(cudaEventRecord(f->sums_done[buf], f->side));
@@ -2902,8 +2874,12 @@ __global__ void zero_forces_kernel(View v) {
 // Groups the pairs of one list by target (g->count holds the counts); nothing
 // is read back: the list's length stays on the device, `cap` bounds it.
 int group_pairs(amk_ctx* c, const int2* pairs, const int* rank, const int* n_pairs, long cap, long n_nodes,
-                int slot_off, int slot_src, int slot_tmp, Grouped* g) {
+                int slot_off, int slot_src, int slot_tmp, int slot_tgt, Grouped* g) {
   int rc = AMK_OK;
+  if (slot_tgt >= 0) {
+    g->tgt = slot<int>(c, slot_tgt, cap, &rc);
+    AMK_TRY(rc);
+  }
   g->off = slot<int>(c, slot_off, n_nodes + 1, &rc);
   AMK_TRY(rc);
   g->src = slot<int>(c, slot_src, cap, &rc);
@@ -2918,7 +2894,7 @@ int group_pairs(amk_ctx* c, const int2* pairs, const int* rank, const int* n_pai
   AMK_CUDA_TRY(cudaFuncSetAttribute(group_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     kSortBits / 8));
   group_sort_kernel<<<static_cast<unsigned>((n_nodes + 7) / 8), kSortThreads, smem, c->stream>>>(
-      static_cast<int>(n_nodes), g->off, g->count, cap, unsorted, g->src);
+      static_cast<int>(n_nodes), g->off, g->count, cap, unsorted, g->src, g->tgt);
   return check_launch(c, "group_sort_kernel");
 }
 
@@ -3005,7 +2981,9 @@ int fmm_run(amk_ctx* c, const View& v, int order, double theta, long leaf_capaci
   const double theta2 = theta * theta;
   double4* rec = slot<double4>(c, kSlotFmmNodeRec, nn, &rc);
   AMK_TRY(rc);
-  fmm_node_record_kernel<<<gn, 256, 0, c->stream>>>(t, radius, rec);
+  int4* cell = slot<int4>(c, kSlotFmmCell, nn, &rc);
+  AMK_TRY(rc);
+  fmm_node_record_kernel<<<gn, 256, 0, c->stream>>>(t, radius, rec, cell);
   AMK_TRY(check_launch(c, "fmm_node_record_kernel"));
   long n_m2l = 0, n_p2p = 0;
   std::vector<int> hv(n_tv);
@@ -3078,9 +3056,9 @@ int fmm_run(amk_ctx* c, const View& v, int order, double theta, long leaf_capaci
     leaf_count_kernel<<<148, 256, 0, c->stream>>>(t, cnt64 + 1);
     AMK_TRY(check_launch(c, "leaf_count_kernel"));
     AMK_TRY(group_pairs(c, tl.m2l, tl.m2l_rank, tv, tl.cap_m2l, nn, kSlotFmmLists0, kSlotFmmWork0, kSlotFmmWork1,
-                        &gm));
+                        kSlotM2lTarget, &gm));
     AMK_TRY(group_pairs(c, tl.p2p, tl.p2p_rank, tv + 1, tl.cap_p2p, nn, kSlotFmmLists2, kSlotFmmWork2,
-                        kSlotFmmWork3, &gp));
+                        kSlotFmmWork3, -1, &gp));
     // near-field work items: a target leaf and up to kP2PChunk source leaves
     // of its list (kP2P32Chunk in the FP32 near field)
     p2p_items_count_kernel<<<gn, 256, 0, c->stream>>>(t, gp.count, f32 ? kP2P32Chunk : kP2PChunk, items, psize);
@@ -3177,7 +3155,7 @@ int fmm_run(amk_ctx* c, const View& v, int order, double theta, long leaf_capaci
   AMK_TRY(phase_begin(c, AMK_PHASE_FMM_M2L));
   if (n_m2l > 0) {
     const std::function<int()> hook(launch_near);
-    AMK_TRY(m2l_products(c, order, t, T, gm, n_m2l, M, Lx, f32 ? hook : no_hook));
+    AMK_TRY(m2l_products(c, order, t, T, gm, cell, n_m2l, M, Lx, f32 ? hook : no_hook));
   } else if (f32) {
     AMK_TRY(launch_near());
   }
