@@ -878,8 +878,7 @@ struct Grouped {
 // take a per-pair path with the derivative recurrence.
 // The pairs are processed in chunks that bound the per-pair scratch.
 constexpr int kM2lTileP = 64;      // pairs per product tile
-constexpr int kM2lUnitPairs = 4 * kM2lTileP;    // pairs of one class taken at a time (FP64 products)
-constexpr int kM2lTcUnitPairs = 8 * kM2lTileP;  // the same for the tensor-core products
+constexpr int kM2lUnitPairs = 8 * kM2lTileP;  // pairs of one class taken at a time
 // classes below this size take the per-pair path in both precision modes (in
 // tensor-core mode a class-matrix build per tiny class costs more than the
 // per-pair path: measured at 1,048,576 particles, leaf 128)
@@ -1161,8 +1160,6 @@ m2l_table_kernel(DerivTables T, const unsigned long long* __restrict__ cls_key, 
   }
 }
 
-constexpr int kM2lStages = 2;  // B tiles in flight
-
 __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool valid);
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
@@ -1177,48 +1174,51 @@ __device__ __forceinline__ void cp_async_wait() {
 // D is harmonic, d_z^2 = -(d_x^2 + d_y^2), so of the n_m = (p+1)(p+2)(p+3)/6
 // rows and columns of A[g][a] = D_{g+a} only the n_r = (p+1)^2 with z exponent
 // 0 or 1 are independent: m2l_rescale_red_kernel collects the source
-// coefficients onto them, m2l_reduce_red_kernel builds the other target
+// coefficients onto them, m2l_reduce_kernel builds the other target
 // coefficients from the summed rows, both exactly the linear relation above.
 // n_r^2 against n_m^2 products per pair: 625 against 1,225 at p = 4, 2,401
 // against 7,056 at p = 6, 6,561 against 27,225 at p = 8; and n_r instead of
 // n_m doubles per pair written and read back.
 //
-// A block covers 8 * kGb >= n_r rows and 64 pairs; warp (wr, wc) owns
-// kWr x kWc 8 x 8 output tiles. A fragments are gathered from the class's
-// D(v) through the transposed index map (both in shared memory) and scaled by
-// the source factor where the source is the larger cell; B is a tile of 64
-// source rows [pair][k], copied whole by cp.async (16-byte copies, two tiles
-// in flight) with a row pitch that is 4 or 12 doubles past a multiple of 16,
-// so that the fragments' eight rows fall into distinct banks. Rows are
-// zero-padded to kNk, so padded A entries only need to be finite.
+// A block covers 8 * kGb >= n_r rows and a tile of 64 pairs; each of its
+// warps owns all the rows of 8 * kWc pairs. Per unit (up to 256 pairs of one
+// class) the block gathers A once, from the class's D(v) through the index
+// map and with the source factor, into shared memory in fragment order (one
+// conflict-free 8-byte read per lane and fragment; gathered anew by every
+// warp and tile, the two dependent reads and their conflicts held the kernel
+// at half the FP64 rate). B is a tile of 64 source rows [pair][k], copied
+// whole by cp.async in 16-byte pieces with a row pitch that is 4 or 12 doubles
+// past a multiple of 16, so that the fragments' eight rows fall into distinct
+// banks. One tile per block is in flight: the blocks of an SM (2 at p = 8, 4
+// at p = 6, 6 at p = 4) cover each other's copies. Rows are zero-padded to kNk.
 template <int P>
 struct M2lMma;
-#define AMK_M2L_MMA(P, WR, WC)                                                                    \
+#define AMK_M2L_MMA(P, WC, CTAS)                                                                  \
   template <>                                                                                     \
   struct M2lMma<P> {                                                                              \
     static constexpr int kNr = (P + 1) * (P + 1);                                                 \
     static constexpr int kNd = (2 * P + 1) * (P + 1) + (2 * P) * (2 * P + 1) / 2 + (2 * P - 1) * P; \
-    static constexpr int kGb = (kNr + 7) / 8, kNg = 8 * kGb, kNk = 4 * ((kNr + 3) / 4);           \
+    static constexpr int kGb = (kNr + 7) / 8, kNk = 4 * ((kNr + 3) / 4);                          \
     static constexpr int kPitch = kNk + ((kNk & 7) == 0 ? 4 : 0);                                 \
-    static constexpr int kWr = WR, kWc = WC;                                                      \
-    static constexpr int kWarpsR = kGb / WR, kWarps = kWarpsR * (8 / WC), kThreads = 32 * kWarps;  \
-    static_assert(kGb % WR == 0 && 8 % WC == 0, "M2L mma shape");                                 \
+    static constexpr int kFrags = kGb * (kNk / 4);  /* 8 x 4 fragments of A */                    \
+    static constexpr int kWc = WC, kWarps = 8 / WC, kThreads = 32 * kWarps, kCtas = CTAS;         \
+    static constexpr int kStages = P <= 5 ? 2 : 1;  /* B tiles in shared memory */                \
+    static_assert(8 % WC == 0, "M2L mma shape");                                                  \
   };
-AMK_M2L_MMA(1, 1, 4)
-AMK_M2L_MMA(2, 2, 4)
-AMK_M2L_MMA(3, 2, 4)
-AMK_M2L_MMA(4, 4, 4)
-AMK_M2L_MMA(5, 5, 4)
-AMK_M2L_MMA(6, 7, 4)
-AMK_M2L_MMA(7, 8, 2)
-AMK_M2L_MMA(8, 11, 2)
+AMK_M2L_MMA(1, 2, 8)
+AMK_M2L_MMA(2, 2, 8)
+AMK_M2L_MMA(3, 2, 8)
+AMK_M2L_MMA(4, 2, 6)
+AMK_M2L_MMA(5, 2, 5)
+AMK_M2L_MMA(6, 2, 4)
+AMK_M2L_MMA(7, 2, 3)
+AMK_M2L_MMA(8, 2, 2)
 #undef AMK_M2L_MMA
 
 template <int P>
 size_t m2l_mma_smem() {
   using S = M2lMma<P>;
-  return sizeof(double) * (static_cast<size_t>(kM2lStages) * kM2lTileP * S::kPitch + S::kNd + S::kNg + S::kNk) +
-         sizeof(short) * static_cast<size_t>(S::kNk) * S::kNg + 2 * kM2lUnitPairs * sizeof(int) + 16;
+  return sizeof(double) * (static_cast<size_t>(S::kStages) * kM2lTileP * S::kPitch + 32 * S::kFrags);
 }
 
 __device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
@@ -1227,123 +1227,126 @@ __device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
                : "d"(a), "d"(b));
 }
 
-// Persistent blocks: the index map is built once per block, then units are
-// taken from a counter; within a tile, warps skip the 8-pair column blocks
-// past the tile's last pair, so a class of a few pairs costs a fraction of a
-// tile.
+__device__ __forceinline__ double exp2i(int e) { return __longlong_as_double(static_cast<long long>(1023 + e) << 52); }
+
+// Persistent blocks take units from a counter; within a tile, warps skip the
+// 8-pair column blocks past the tile's last pair, so a class of a few pairs
+// costs a fraction of a tile.
 template <int P>
-__global__ void __launch_bounds__(M2lMma<P>::kThreads)
+__global__ void __launch_bounds__(M2lMma<P>::kThreads, M2lMma<P>::kCtas)
 m2l_class_mma_kernel(FmmDevTables T, int n_units, int* __restrict__ unit_counter, const int4* __restrict__ ud,
                      const int* __restrict__ perm, const int* __restrict__ psrc, const double* __restrict__ Mr,
                      const double* __restrict__ table, long e0, double* __restrict__ out) {
   using S = M2lMma<P>;
-  constexpr int kNr = S::kNr, kNg = S::kNg, kNk = S::kNk, kTh = S::kThreads, kPitch = S::kPitch;
+  constexpr int kNr = S::kNr, kNk = S::kNk, kTh = S::kThreads, kPitch = S::kPitch, kKs = kNk / 4;
   extern __shared__ __align__(16) unsigned char mma_smem[];
-  double* Bs = reinterpret_cast<double*>(mma_smem);   // [kM2lStages][kM2lTileP][kPitch]
-  double* Ds = Bs + kM2lStages * kM2lTileP * kPitch;  // [kNd]
-  double* rowf = Ds + S::kNd;                         // [kNg]
-  double* colf = rowf + kNg;                          // [kNk]
-  int* pe = reinterpret_cast<int*>(colf + kNk);       // [kM2lUnitPairs]
-  int* ps = pe + kM2lUnitPairs;                       // [kM2lUnitPairs]
-  short* idx = reinterpret_cast<short*>(ps + kM2lUnitPairs);  // [kNk][kNg]
-  __shared__ int s_unit;
+  constexpr int kStage = kM2lTileP * kPitch;
+  double* Bs = reinterpret_cast<double*>(mma_smem);  // [kStages][kM2lTileP][kPitch]
+  double* Af = Bs + S::kStages * kStage;             // [kKs][kGb][32]
+  __shared__ int4 s_u;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wr = warp % S::kWarpsR, wc = warp / S::kWarpsR;
   const int lr = lane >> 2, lc = lane & 3;  // fragment row / column within a tile
-  const int g_base = 8 * S::kWr * wr + lr, p_base = 8 * S::kWc * wc + lr;
-  for (int x = tid; x < kNk * kNg; x += kTh) {
-    const int a = x / kNg, g = x - a * kNg;
-    idx[x] = (a < kNr && g < kNr) ? T.red_index_t[a * kNr + g] : 0;
+  if (tid == 0) {
+    const int first = atomicAdd(unit_counter, 1);
+    s_u = first < n_units ? ud[first] : make_int4(0, 0, 0, 0);
   }
-  int next = 0;  // thread 0: the unit after the current one
-  if (tid == 0) next = atomicAdd(unit_counter, 1);
   for (;;) {
-    if (tid == 0) s_unit = next;
-    __syncthreads();  // also: the previous unit is done with the shared arrays
-    const int unit = s_unit;
-    if (unit >= n_units) break;
-    if (tid == 0) next = atomicAdd(unit_counter, 1);
-    const int4 u = ud[unit];
-    const int cls = u.x, pos0 = u.y, np = u.z;
-    const int n_tiles = (np + kM2lTileP - 1) / kM2lTileP;
+    __syncthreads();  // s_u is set, the previous unit is done with A and B
+    const int4 u = s_u;
+    if (u.z == 0) break;
+    const int pos0 = u.y, np = u.z;
     const int et = u.w < 0 ? -u.w : 0, es = u.w > 0 ? u.w : 0;  // log2(h_t / u), log2(h_s / u)
-    for (int k = tid; k < S::kNd; k += kTh) Ds[k] = table[static_cast<size_t>(cls) * S::kNd + k];
-    for (int g = tid; g < kNg; g += kTh) rowf[g] = g < kNr ? ldexp(1.0, (T.red_deg[g] + 1) * et) : 0.0;
-    for (int a = tid; a < kNk; a += kTh) colf[a] = a < kNr ? ldexp(1.0, T.red_deg[a] * es) : 0.0;
-    for (int p = tid; p < n_tiles * kM2lTileP; p += kTh) {
-      pe[p] = p < np ? perm[pos0 + p] : -1;
-      ps[p] = p < np ? psrc[pos0 + p] : -1;
-    }
-    __syncthreads();
-    auto issue = [&](int tile) {
-      if (tile < n_tiles) {
-        const int rows = (min(kM2lTileP, np - tile * kM2lTileP) + 7) & ~7;  // column blocks past them are not read
-        double* B = Bs + (tile % kM2lStages) * kM2lTileP * kPitch;
-        for (int x = tid; x < rows * (kNk / 2); x += kTh) {
-          const int p = x / (kNk / 2), v = x - p * (kNk / 2);
-          const int sp = ps[tile * kM2lTileP + p];
-          cp_async16(B + p * kPitch + 2 * v, Mr + static_cast<size_t>(max(sp, 0)) * kNk + 2 * v, sp >= 0);
-        }
+    auto fetch = [&](int tile) {
+      const int live = min(kM2lTileP, np - tile * kM2lTileP);
+      const int rows = (live + 7) & ~7;  // column blocks past them are not read
+      const int* ps = psrc + pos0 + tile * kM2lTileP;
+      for (int x = tid; x < rows * (kNk / 2); x += kTh) {
+        const int p = x / (kNk / 2), v = x - p * (kNk / 2);
+        const bool ok = p < live;
+        cp_async16(Bs + (tile % S::kStages) * kStage + p * kPitch + 2 * v, Mr + (ok ? static_cast<size_t>(ps[p]) * kNk + 2 * v : 0), ok);
       }
       cp_async_commit();
     };
-    issue(0);
-#pragma unroll 1
-    for (int tile = 0; tile < n_tiles; ++tile) {
-      cp_async_wait<0>();
-      __syncthreads();  // the tile is complete, and the one before it has been read
-      issue(tile + 1);
-      const int live = min(kM2lTileP, np - tile * kM2lTileP);  // pairs in this tile
-      const int jn = min(S::kWc, max(0, (live - 8 * S::kWc * wc + 7) / 8));  // this warp's live column blocks
-      if (jn == 0) continue;
-      const double* B = Bs + (tile % kM2lStages) * kM2lTileP * kPitch + p_base * kPitch + lc;
-      double acc[S::kWr][S::kWc][2];
-#pragma unroll
-      for (int i = 0; i < S::kWr; ++i)
-#pragma unroll
-        for (int j = 0; j < S::kWc; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-      auto products = [&](auto scaled) {
-#pragma unroll 2
-        for (int ks = 0; ks < kNk / 4; ++ks) {
-          const int a = 4 * ks + lc;
-          const short* irow = idx + a * kNg + g_base;
-          double af[S::kWr], bf[S::kWc];
-#pragma unroll
-          for (int i = 0; i < S::kWr; ++i) af[i] = Ds[irow[8 * i]];
-          if (decltype(scaled)::value) {
-            const double cf = colf[a];
-#pragma unroll
-            for (int i = 0; i < S::kWr; ++i) af[i] *= cf;
-          }
-#pragma unroll
-          for (int j = 0; j < S::kWc; ++j)
-            if (j < jn) bf[j] = B[8 * j * kPitch + 4 * ks];
-#pragma unroll
-          for (int j = 0; j < S::kWc; ++j)
-            if (j < jn)
-#pragma unroll
-              for (int i = 0; i < S::kWr; ++i) mma_f64(acc[i][j], af[i], bf[j]);
-        }
-      };
-      if (es > 0)
-        products(std::true_type());
-      else
-        products(std::false_type());
+    fetch(0);
+    const double* D = table + static_cast<size_t>(u.x) * S::kNd;
+#pragma unroll 4
+    for (int x = tid; x < 32 * S::kFrags; x += kTh) {
+      const int f = x >> 5, ks = f / S::kGb, g = 8 * (f - ks * S::kGb) + lr, a = 4 * ks + lc;  // x & 31 is this lane
+      double v = 0.0;
+      if (a < kNr && g < kNr) {
+        v = D[T.red_index_t[a * kNr + g]];
+        if (es > 0) v *= exp2i(T.red_deg[a] * es);
+      }
+      Af[x] = v;
+    }
+    int4 un = make_int4(0, 0, 0, 0);
+    if (tid == 0) {
+      const int next = atomicAdd(unit_counter, 1);
+      if (next < n_units) un = ud[next];
+    }
+    for (int tile = 0, left = np; left > 0; ++tile, left -= kM2lTileP) {
+      const int live = min(kM2lTileP, left);  // pairs in this tile
+      const int* perm_t = perm + pos0 + tile * kM2lTileP;
+      int pe[S::kWc][2];  // this lane's pairs, in flight during the products
 #pragma unroll
       for (int j = 0; j < S::kWc; ++j)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          const int e = pe[tile * kM2lTileP + 8 * S::kWc * wc + 8 * j + 2 * lc + h];
-          if (e < 0) continue;
-          double* o = out + static_cast<size_t>(e - e0) * kNk;
+          const int p = 8 * (S::kWc * warp + j) + 2 * lc + h;
+          pe[j][h] = p < live ? perm_t[p] : -1;
+        }
+      if (S::kStages == 1 && tile > 0) {
+        __syncthreads();  // the tile before this one has been read
+        fetch(tile);
+      }
+      cp_async_wait<0>();
+      __syncthreads();  // this tile has landed (two stages: the one before it has been read)
+      if (S::kStages == 2 && left > kM2lTileP) fetch(tile + 1);
+      const int jn = min(S::kWc, max(0, (live - 8 * S::kWc * warp + 7) / 8));  // this warp's live column blocks
+      if (jn == 0) continue;
+      const double* B = Bs + (tile % S::kStages) * kStage + (8 * S::kWc * warp + lr) * kPitch + lc;
+      double acc[S::kGb][S::kWc][2];
 #pragma unroll
-          for (int i = 0; i < S::kWr; ++i) {
-            const int g = 8 * S::kWr * wr + 8 * i + lr;
-            if (g < kNr) o[g] = acc[i][j][h] * rowf[g];
+      for (int i = 0; i < S::kGb; ++i)
+#pragma unroll
+        for (int j = 0; j < S::kWc; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+#pragma unroll 2
+      for (int ks = 0; ks < kKs; ++ks) {
+        double af[S::kGb], bf[S::kWc];
+#pragma unroll
+        for (int i = 0; i < S::kGb; ++i) af[i] = Af[(ks * S::kGb + i) * 32 + lane];
+#pragma unroll
+        for (int j = 0; j < S::kWc; ++j)
+          if (j < jn) bf[j] = B[8 * j * kPitch + 4 * ks];
+#pragma unroll
+        for (int j = 0; j < S::kWc; ++j)
+          if (j < jn)
+#pragma unroll
+            for (int i = 0; i < S::kGb; ++i) mma_f64(acc[i][j], af[i], bf[j]);
+      }
+      if (et > 0)
+#pragma unroll
+        for (int i = 0; i < S::kGb; ++i) {
+          const double rf = exp2i(8 * i + lr < kNr ? (T.red_deg[8 * i + lr] + 1) * et : 0);
+#pragma unroll
+          for (int j = 0; j < S::kWc; ++j) {
+            acc[i][j][0] *= rf;
+            acc[i][j][1] *= rf;
           }
         }
+#pragma unroll
+      for (int j = 0; j < S::kWc; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if (pe[j][h] < 0) continue;
+          double* o = out + static_cast<size_t>(pe[j][h] - e0) * kNk;
+#pragma unroll
+          for (int i = 0; i < S::kGb; ++i)  // whole 32-byte sectors: the padding rows are written too (zero)
+            if (8 * i + lr < kNk) o[8 * i + lr] = acc[i][j][h];
+        }
     }
-    cp_async_wait<0>();
+    __syncthreads();  // every thread has read s_u
+    if (tid == 0) s_u = un;
   }
 }
 
@@ -1855,62 +1858,6 @@ m2l_pair_red_kernel(const Octree t, FmmDevTables T, const int* __restrict__ list
   }
 }
 
-// L_g(t) += 1/g! h_t^{-|g|-1} Q_g, Q the sum of the target's rows in [e0, e1)
-// in pair order on the harmonic basis, its other coefficients built from it.
-// A warp per target; a lane holds V 16-byte vectors of a row (n_rp a multiple
-// of 4), eight (V = 1) or four rows in flight.
-template <int V>
-__global__ void __launch_bounds__(256)
-m2l_reduce_red_kernel(const Octree t, FmmDevTables T, const int* __restrict__ off, const int* __restrict__ count,
-                      int n_targets, long e0, long e1, const double* __restrict__ out, double* __restrict__ L) {
-  constexpr int kU = V == 1 ? 8 : 4;
-  __shared__ double2 qs[8][32 * V];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int k = blockIdx.x * 8 + w;
-  if (k >= n_targets) return;
-  const int ti = k, nv = T.n_rp >> 1;
-  const long b = max(static_cast<long>(off[ti]), e0), end = min(static_cast<long>(off[ti]) + count[ti], e1);
-  if (b >= end) return;
-  double2 s[V];
-#pragma unroll
-  for (int r = 0; r < V; ++r) s[r] = make_double2(0.0, 0.0);
-  const double2* o = reinterpret_cast<const double2*>(out + static_cast<size_t>(b - e0) * T.n_rp) + lane;
-  long e = b;
-  for (; e + kU <= end; e += kU, o += kU * nv) {
-    double2 v[kU][V];
-#pragma unroll
-    for (int u = 0; u < kU; ++u)
-#pragma unroll
-      for (int r = 0; r < V; ++r) v[u][r] = lane + 32 * r < nv ? o[u * nv + 32 * r] : make_double2(0.0, 0.0);
-#pragma unroll
-    for (int u = 0; u < kU; ++u)
-#pragma unroll
-      for (int r = 0; r < V; ++r) {
-        s[r].x += v[u][r].x;
-        s[r].y += v[u][r].y;
-      }
-  }
-  for (; e < end; ++e, o += nv)
-#pragma unroll
-    for (int r = 0; r < V; ++r)
-      if (lane + 32 * r < nv) {
-        s[r].x += o[32 * r].x;
-        s[r].y += o[32 * r].y;
-      }
-#pragma unroll
-  for (int r = 0; r < V; ++r) qs[w][lane + 32 * r] = s[r];
-  __syncwarp();
-  const double* q = reinterpret_cast<const double*>(qs[w]);
-  const double ih = 1.0 / t.center[ti].w;
-  for (int g = lane; g < T.n_m; g += 32) {
-    double f = 0.0;
-    for (int x = T.ex_off[g]; x < T.ex_off[g + 1]; ++x) f += T.ex_c[x] * q[T.ex_r[x]];
-    f *= T.inv_fact[g];
-    for (int d = 0; d <= T.multi[g].w; ++d) f *= ih;
-    L[static_cast<size_t>(ti) * T.n_m + g] += f;
-  }
-}
-
 // Reflection-folded class pairs (tensor-core mode): the product row of a
 // pair with reflection R gets s^g on coefficient g, in place (refl = 0 for
 // every other pair, the per-pair path's included). A warp takes 32 pairs and
@@ -1948,51 +1895,92 @@ m2l_refl_sign_kernel(FmmDevTables T, long e0, long e1, const unsigned char* __re
   }
 }
 
-// The sum over FP32 per-pair products (tensor-core mode, n_m a multiple of
-// 4, at most 128): lane l holds coefficients 4l..4l+3 and reads them as one
-// 16-byte vector, eight pairs' rows in flight per warp. The sum per
-// coefficient is the FP64 sum in pair order.
+// Sum of a target's product rows in [e0, e1), a block per target (targets of
+// several thousand pairs exist: with a warp per target they were the tail
+// that held the kernel at a third of the HBM rate). A row is nv 16-byte
+// vectors; a warp's lanes form 32 / nv groups (V = 1) that take every
+// (8 * groups)-th row with eight rows in flight, or lane l holds vectors l and
+// l + 32 (V = 2). The sums are FP64; the groups are added in order, so the
+// result does not depend on scheduling.
+//   FP64 mode: rows Q on the harmonic basis, L_g += 1/g! h_t^{-|g|-1} Q_g with
+//   the other coefficients built from the basis; tensor-core mode: FP32 rows
+//   of all n_m coefficients (1/g! applied), L_g += h_t^{-|g|-1} row_g.
+__device__ __forceinline__ void row_add(double (&s)[2], const double2& v) {
+  s[0] += v.x;
+  s[1] += v.y;
+}
+__device__ __forceinline__ void row_add(double (&s)[4], const float4& v) {
+  s[0] += v.x;
+  s[1] += v.y;
+  s[2] += v.z;
+  s[3] += v.w;
+}
+
+template <typename Vec, int V>
 __global__ void __launch_bounds__(256)
-m2l_reduce_f4_kernel(const Octree t, FmmDevTables T, const int* __restrict__ off, const int* __restrict__ count,
-                     int n_targets, long e0, long e1, const float* __restrict__ out, double* __restrict__ L) {
-  constexpr int kU = 8;
-  const int lane = threadIdx.x & 31;
-  const int k = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (k >= n_targets) return;
-  const int ti = k, nm = T.n_m, nv = nm >> 2;
+m2l_reduce_kernel(const Octree t, FmmDevTables T, const int* __restrict__ off, const int* __restrict__ count,
+                  int t_first, int nv, long e0, long e1, const Vec* __restrict__ out, double* __restrict__ L) {
+  constexpr int kE = sizeof(Vec) == sizeof(float4) && std::is_same<Vec, float4>::value ? 4 : 2;  // values per vector
+  constexpr int kU = V == 1 ? 8 : 4;
+  __shared__ double part[8 * 32 * V * kE];
+  __shared__ double q[32 * V * kE];
+  const int ti = t_first + blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const long b = max(static_cast<long>(off[ti]), e0), end = min(static_cast<long>(off[ti]) + count[ti], e1);
-  if (b >= end || lane >= nv) return;
-  double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-  const float4* o = reinterpret_cast<const float4*>(out + static_cast<size_t>(b - e0) * nm) + lane;
-  long e = b;
-  for (; e + kU <= end; e += kU, o += kU * nv) {
-    float4 v[kU];
+  if (b >= end) return;
+  const int per = V == 1 ? 32 / nv : 1, groups = 8 * per;
+  const int g = V == 1 ? lane / nv : 0, v0 = V == 1 ? lane - g * nv : lane;
+  double s[V][kE];
 #pragma unroll
-    for (int u = 0; u < kU; ++u) v[u] = o[u * nv];
+  for (int r = 0; r < V; ++r)
 #pragma unroll
-    for (int u = 0; u < kU; ++u) {
-      s0 += v[u].x;
-      s1 += v[u].y;
-      s2 += v[u].z;
-      s3 += v[u].w;
+    for (int c = 0; c < kE; ++c) s[r][c] = 0.0;
+  if (g < per) {
+    const Vec* o = out + v0;
+    long e = b + w * per + g;
+    const long step = groups;
+    for (; e + (kU - 1) * step < end; e += kU * step) {
+      Vec v[kU][V];
+#pragma unroll
+      for (int u = 0; u < kU; ++u)
+#pragma unroll
+        for (int r = 0; r < V; ++r)
+          if (V == 1 || v0 + 32 * r < nv) v[u][r] = o[(e + u * step - e0) * nv + 32 * r];
+#pragma unroll
+      for (int u = 0; u < kU; ++u)
+#pragma unroll
+        for (int r = 0; r < V; ++r)
+          if (V == 1 || v0 + 32 * r < nv) row_add(s[r], v[u][r]);
     }
+    for (; e < end; e += step)
+#pragma unroll
+      for (int r = 0; r < V; ++r)
+        if (V == 1 || v0 + 32 * r < nv) row_add(s[r], o[(e - e0) * nv + 32 * r]);
+#pragma unroll
+    for (int r = 0; r < V; ++r)
+      if (V == 1 || v0 + 32 * r < nv)
+#pragma unroll
+        for (int c = 0; c < kE; ++c) part[(w * per + g) * nv * kE + (v0 + 32 * r) * kE + c] = s[r][c];
   }
-  for (; e < end; ++e, o += nv) {
-    const float4 v = *o;
-    s0 += v.x;
-    s1 += v.y;
-    s2 += v.z;
-    s3 += v.w;
+  __syncthreads();
+  const int row = nv * kE;
+  if (threadIdx.x < row) {
+    double a = 0.0;
+    for (int k = 0; k < groups; ++k) a += part[k * row + threadIdx.x];
+    q[threadIdx.x] = a;
+  }
+  __syncthreads();
+  if (threadIdx.x >= T.n_m) return;
+  const int gg = threadIdx.x;
+  double f = 0.0;
+  if (kE == 2) {
+    for (int x = T.ex_off[gg]; x < T.ex_off[gg + 1]; ++x) f += T.ex_c[x] * q[T.ex_r[x]];
+    f *= T.inv_fact[gg];
+  } else {
+    f = q[gg];
   }
   const double ih = 1.0 / t.center[ti].w;
-  const double sv[4] = {s0, s1, s2, s3};
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    const int g = 4 * lane + c;
-    double f = sv[c];
-    for (int d = 0; d <= T.multi[g].w; ++d) f *= ih;
-    L[static_cast<size_t>(ti) * nm + g] += f;
-  }
+  for (int d = 0; d <= T.multi[gg].w; ++d) f *= ih;
+  L[static_cast<size_t>(ti) * T.n_m + gg] += f;
 }
 
 template <int P>
@@ -2122,7 +2110,6 @@ int m2l_products(amk_ctx* c, int order, const Octree& t, const FmmDevTables& T, 
     if (v > 0) cap = std::min(cap, v);
   }
   const bool one_chunk = n_m2l <= cap;  // the counts of the classification are the chunk's
-  const int unit_pairs = tc ? kM2lTcUnitPairs : kM2lUnitPairs;
   int* class_hist = tc || one_chunk ? hist : nullptr;
   int* class_rank = one_chunk ? rank : nullptr;
   if (class_hist) AMK_CUDA_TRY(cudaMemsetAsync(hist, 0, n_codes * sizeof(int), c->stream));
@@ -2142,7 +2129,7 @@ int m2l_products(amk_ctx* c, int order, const Octree& t, const FmmDevTables& T, 
       AMK_CUDA_TRY(cudaEventCreateWithFlags(&f->sums_done[i], cudaEventDisableTiming));
     }
   }
-  const long max_cls = std::min({cap, n_m2l, n_codes}) / kM2lMinClass + 1, max_units = std::min(cap, n_m2l) / unit_pairs + max_cls + 1;
+  const long max_cls = std::min({cap, n_m2l, n_codes}) / kM2lMinClass + 1, max_units = std::min(cap, n_m2l) / kM2lUnitPairs + max_cls + 1;
   int* perm = slot<int>(c, kSlotM2lPerm, std::min(cap, n_m2l), &rc);
   AMK_TRY(rc);
   int* fallback = slot<int>(c, kSlotM2lFallback, std::min(cap, n_m2l), &rc);
@@ -2179,14 +2166,16 @@ int m2l_products(amk_ctx* c, int order, const Octree& t, const FmmDevTables& T, 
       m2l_histogram_kernel<<<ge, 256, 0, c->stream>>>(codes, e0, e1, hist, rank);
       AMK_TRY(check_launch(c, "m2l_histogram_kernel"));
     }
-    m2l_class_build_kernel<<<gc, 256, 0, c->stream>>>(hist, n_codes, kM2lMinClass, unit_pairs, keys, counters, start,
+    m2l_class_build_kernel<<<gc, 256, 0, c->stream>>>(hist, n_codes, kM2lMinClass, kM2lUnitPairs, keys, counters, start,
                                                       cls_key, ud);
     AMK_TRY(check_launch(c, "m2l_class_build_kernel"));
     m2l_scatter_kernel<<<ge, 256, 0, c->stream>>>(codes, rank, e0, e1, start, gm.src, static_cast<int>(nn), perm, psrc,
                                                   fallback, counters + 3, refl);
     AMK_TRY(check_launch(c, "m2l_scatter_kernel"));
-    int h[4] = {0, 0, 0, 0};
+    int h[4] = {0, 0, 0, 0}, tr[2] = {0, 0};  // counters, the chunk's first and last target
     AMK_CUDA_TRY(cudaMemcpyAsync(h, counters, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
+    AMK_CUDA_TRY(cudaMemcpyAsync(tr, tgt + e0, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    AMK_CUDA_TRY(cudaMemcpyAsync(tr + 1, tgt + e1 - 1, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     AMK_CUDA_TRY(cudaStreamSynchronize(c->stream));
     const int n_cls = h[1], n_units = h[2], n_fb = h[3];
     // the classes' pairs fill perm[0, h[0]) and every other pair is on the per-pair list
@@ -2253,17 +2242,16 @@ int m2l_products(amk_ctx* c, int order, const Octree& t, const FmmDevTables& T, 
     // per-target sums on the side stream, in chunk order
     AMK_CUDA_TRY(cudaEventRecord(f->products_done[buf], c->stream));
     AMK_CUDA_TRY(cudaStreamWaitEvent(f->side, f->products_done[buf], 0));
-    const int n_tgt = static_cast<int>(nn);  // (targets without pairs in the chunk return at once)
-    const unsigned gt = static_cast<unsigned>((n_tgt + 7) / 8);
+    const unsigned gt = static_cast<unsigned>(tr[1] - tr[0] + 1);
     if (tc)
-      m2l_reduce_f4_kernel<<<gt, 256, 0, f->side>>>(t, T, gm.off, gm.count, n_tgt, e0, e1,
-                                                    static_cast<const float*>(out), L);
+      m2l_reduce_kernel<float4, 1><<<gt, 256, 0, f->side>>>(t, T, gm.off, gm.count, tr[0], T.n_m / 4, e0, e1,
+                                                            static_cast<const float4*>(out), L);
     else if (T.n_rp <= 64)
-      m2l_reduce_red_kernel<1><<<gt, 256, 0, f->side>>>(t, T, gm.off, gm.count, n_tgt, e0, e1,
-                                                        static_cast<const double*>(out), L);
+      m2l_reduce_kernel<double2, 1><<<gt, 256, 0, f->side>>>(t, T, gm.off, gm.count, tr[0], T.n_rp / 2, e0, e1,
+                                                             static_cast<const double2*>(out), L);
     else
-      m2l_reduce_red_kernel<2><<<gt, 256, 0, f->side>>>(t, T, gm.off, gm.count, n_tgt, e0, e1,
-                                                        static_cast<const double*>(out), L);
+      m2l_reduce_kernel<double2, 2><<<gt, 256, 0, f->side>>>(t, T, gm.off, gm.count, tr[0], T.n_rp / 2, e0, e1,
+                                                             static_cast<const double2*>(out), L);
     AMK_TRY(check_launch(c, "m2l_reduce_kernel"));
     AMK_CUDA_TRY(cudaEventRecord(f->sums_done[buf], f->side));
   }
