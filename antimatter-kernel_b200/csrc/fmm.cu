@@ -18,9 +18,10 @@
 //                   is built degree by degree in shared memory (lanes over the
 //                   multi-indices of one degree) and contracted with the
 //                   source's multipole, lanes over local coefficients
-//   L2P + P2P       work items of (target leaf, <= 8 source leaves); a warp
-//                   per item with lanes split into groups over the sources;
-//                   partials added in a fixed order
+//   P2P, L2P        work items of (target leaf, a chunk of its source
+//                   leaves); a warp per item with lanes split into groups over
+//                   the sources; partials added in a fixed order, L2P a thread
+//                   per particle
 // Arithmetic is FP64 throughout, as in the reference; inverse distances use
 // rsqrt (the reference divides by sqrt), a difference of an ulp.
 #include <algorithm>
@@ -2302,13 +2303,14 @@ fmm_l2l_kernel(const Octree t, FmmDevTables T, int depth, double* __restrict__ L
 
 // ------------------------------------------------------------ L2P + P2P
 // Work items = (target leaf, chunk of <= kP2PChunk source leaves of its P2P
-// list; kP2P32Chunk in the FP32 near field); every leaf has at least one item (its L2P). A warp takes one item;
-// its lanes are split into G = 32 / n_targets groups, group g summing every
-// G-th source particle for all the leaf's targets, so small leaves still
-// fill the warp. Group sums are added in group order and item partials in
-// chunk order (fast-multipole.cc:580-661), so results do not depend on
-// scheduling.
-constexpr int kP2PChunk = 8;
+// list; kP2P32Chunk in the FP32 near field); every leaf has at least one item.
+// A warp takes one item; its lanes are split into G = 32 / n_targets groups,
+// group g summing every G-th source particle for all the leaf's targets, so
+// small leaves still fill the warp. Group sums are added in group order and
+// item partials in chunk order (fast-multipole.cc:580-661), so results do not
+// depend on scheduling.
+constexpr int kP2PChunk = 64;
+constexpr int kP2PWindow = 256;  // sources staged per warp at a time (FP64)
 
 __global__ void p2p_items_count_kernel(const Octree t, const int* __restrict__ count, int chunk,
                                        int* __restrict__ items, int* __restrict__ psize) {
@@ -2331,18 +2333,27 @@ __global__ void p2p_items_fill_kernel(const Octree t, const int* __restrict__ it
   for (int k = r.x; k < r.y; ++k) leaf_of[k] = id;
 }
 
+// FP64 pair sums of one item. The item's sources are staged in shared memory
+// as one run, leaf boundaries gone: the particles of 32 leaves at a time are
+// numbered by a warp scan of the leaf sizes and copied in windows of 256 (read
+// leaf by leaf from global memory, 9 particles on average at leaf capacity 32,
+// the kernel waited on those loads: 1.47 ms at 262,144 particles, 35 % of the
+// FP64 pipe). About 20 FP64 operations per pair; the target itself and pairs
+// below the minimum distance get 1/r := 0.
+template <bool kPhi>
 __global__ void __launch_bounds__(32 * kFmmWarps)
-fmm_p2p_kernel(const Octree t, FmmDevTables T, const int2* __restrict__ work, int n_work,
-               const int* __restrict__ off, const int* __restrict__ count, const int* __restrict__ src,
-               const int* __restrict__ pbase, const double* __restrict__ L, double min_sq, bool want_phi,
-               double4* __restrict__ part) {
-  __shared__ double4 red[kFmmWarps][32];
+fmm_p2p_kernel(const Octree t, const int2* __restrict__ work, int n_work, const int* __restrict__ off,
+               const int* __restrict__ count, const int* __restrict__ src, const int* __restrict__ pbase,
+               double min_sq, double4* __restrict__ part) {
+  __shared__ double4 stg_s[kFmmWarps][kP2PWindow];
+  __shared__ int end_s[kFmmWarps][32], beg_s[kFmmWarps][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int wi = blockIdx.x * kFmmWarps + w;
   if (wi >= n_work) return;
+  double4* stg = stg_s[w];
+  int *leaf_end = end_s[w], *leaf_beg = beg_s[w];
   const int2 item = work[wi];
   const int ti = item.x, chunk = item.y;
-  const double4 tc = t.center[ti];
   const int2 tr = t.range[ti];
   const int nt_all = tr.y - tr.x;
   const int sb = off[ti] + chunk * kP2PChunk;
@@ -2353,70 +2364,62 @@ fmm_p2p_kernel(const Octree t, FmmDevTables T, const int2* __restrict__ work, in
     const int groups = 32 / nt;
     const int g = lane / nt, tl = lane - g * nt;
     const bool active = g < groups;
-    const int i = base + tl;
-    double4 me = make_double4(0.0, 0.0, 0.0, 0.0);
-    if (active) me = t.src[i];
+    const double4 me = t.src[base + (active ? tl : 0)];
     double pot = 0.0, fx = 0.0, fy = 0.0, fz = 0.0;
-    if (active && g == 0 && chunk == 0) {  // L2P, once per target
-      const double* l = L + static_cast<size_t>(ti) * T.n_m;
-      double px[kMaxOrder + 1], py[kMaxOrder + 1], pz[kMaxOrder + 1];
-      powers(T.p, me.x - tc.x, me.y - tc.y, me.z - tc.z, px, py, pz);
-      if (want_phi)
-        for (int gg = 0; gg < T.n_m; ++gg) {
-          const int4 m = T.multi[gg];
-          pot += l[gg] * (px[m.x] * py[m.y] * pz[m.z]);
-        }
-      double gx = 0.0, gy = 0.0, gz = 0.0;
-      for (int gg = 1; gg < T.n_m; ++gg) {
-        const int4 m = T.multi[gg];
-        const int g0 = T.grad[3 * gg], g1 = T.grad[3 * gg + 1], g2 = T.grad[3 * gg + 2];
-        if (g0 >= 0) {
-          const int4 q = T.multi[g0];
-          gx += m.x * l[gg] * (px[q.x] * py[q.y] * pz[q.z]);
-        }
-        if (g1 >= 0) {
-          const int4 q = T.multi[g1];
-          gy += m.y * l[gg] * (px[q.x] * py[q.y] * pz[q.z]);
-        }
-        if (g2 >= 0) {
-          const int4 q = T.multi[g2];
-          gz += m.z * l[gg] * (px[q.x] * py[q.y] * pz[q.z]);
-        }
+    for (int e = sb; e < se; e += 32) {
+      // number the particles of up to 32 source leaves
+      int2 r = make_int2(0, 0);
+      if (e + lane < se) r = t.range[src[e + lane]];
+      int incl = r.y - r.x;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
       }
-      fx = -gx;
-      fy = -gy;
-      fz = -gz;
-    }
-    if (active) {
-      for (int e = sb; e < se; ++e) {
-        const int2 sr = t.range[src[e]];
-        for (int j = sr.x + g; j < sr.y; j += groups) {
-          const double4 s = t.src[j];
-          if (j == i || s.w == 0.0) continue;
-          const double rx = me.x - s.x, ry = me.y - s.y, rz = me.z - s.z;
-          const double r2 = rx * rx + ry * ry + rz * rz;
-          if (r2 < min_sq) continue;
-          const double inv_r = rsqrt(r2);
-          const double f = s.w * (inv_r * inv_r * inv_r);
-          fx += rx * f;
-          fy += ry * f;
-          fz += rz * f;
-          pot += s.w * inv_r;
+      const int total = __shfl_sync(0xffffffffu, incl, 31);
+      __syncwarp();
+      leaf_end[lane] = incl;
+      leaf_beg[lane] = r.y - incl;  // particle k of leaf j is at leaf_beg[j] + k
+      for (int w0 = 0; w0 < total; w0 += kP2PWindow) {
+        const int wn = min(kP2PWindow, total - w0);
+        __syncwarp();
+        for (int k = lane; k < wn; k += 32) {
+          int j = 0;  // leaves that end at or before particle w0 + k
+#pragma unroll
+          for (int st = 16; st > 0; st >>= 1)
+            if (leaf_end[j + st - 1] <= w0 + k) j += st;
+          stg[k] = t.src[leaf_beg[j] + w0 + k];
         }
+        __syncwarp();
+        if (active)
+#pragma unroll 2
+          for (int k = g; k < wn; k += groups) {
+            const double4 s = stg[k];
+            const double rx = me.x - s.x, ry = me.y - s.y, rz = me.z - s.z;
+            const double r2 = rx * rx + ry * ry + rz * rz;
+            const double inv = r2 < min_sq ? 0.0 : rsqrt(r2);
+            const double qi = s.w * inv;
+            const double f = qi * (inv * inv);
+            fx += rx * f;
+            fy += ry * f;
+            fz += rz * f;
+            if (kPhi) pot += qi;
+          }
       }
     }
-    red[w][lane] = make_double4(fx, fy, fz, pot);
+    __syncwarp();
+    stg[lane] = make_double4(fx, fy, fz, pot);
     __syncwarp();
     if (active && g == 0) {
-      double4 a = red[w][tl];
+      double4 a = stg[tl];
       for (int gg = 1; gg < groups; ++gg) {
-        const double4 b = red[w][gg * nt + tl];
+        const double4 b = stg[gg * nt + tl];
         a.x += b.x;
         a.y += b.y;
         a.z += b.z;
         a.w += b.w;
       }
-      out[i - tr.x] = a;
+      out[base + tl - tr.x] = a;
     }
     __syncwarp();
   }
@@ -2777,7 +2780,7 @@ fmm_p2p32_kernel(const Octree t, const int2* __restrict__ work, int n_work, cons
   }
 }
 
-// Per particle: item partials in chunk order.
+// Per particle: item partials in chunk order, four in flight.
 __global__ void fmm_p2p_reduce_kernel(const Octree t, const int* __restrict__ leaf_of, const int* __restrict__ items,
                                       const int* __restrict__ pbase, const double4* __restrict__ part,
                                       double4* __restrict__ ef) {
@@ -2785,10 +2788,23 @@ __global__ void fmm_p2p_reduce_kernel(const Octree t, const int* __restrict__ le
   if (k >= t.m) return;
   const int leaf = leaf_of[k];
   const int2 r = t.range[leaf];
-  const int nt = r.y - r.x;
+  const int nt = r.y - r.x, n = items[leaf];
   const double4* p = part + pbase[leaf] + (k - r.x);
   double4 a = p[0];
-  for (int c = 1; c < items[leaf]; ++c) {
+  int c = 1;
+  for (; c + 4 <= n; c += 4) {
+    double4 b[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) b[u] = p[static_cast<size_t>(c + u) * nt];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      a.x += b[u].x;
+      a.y += b[u].y;
+      a.z += b[u].z;
+      a.w += b[u].w;
+    }
+  }
+  for (; c < n; ++c) {
     const double4 b = p[static_cast<size_t>(c) * nt];
     a.x += b.x;
     a.y += b.y;
@@ -2798,7 +2814,7 @@ __global__ void fmm_p2p_reduce_kernel(const Octree t, const int* __restrict__ le
   ef[k] = a;
 }
 
-// FP32 near-field path: the FP64 L2P of every particle added to its summed
+// The FP64 L2P of every particle added to its summed
 // near field (a thread per particle; the table indices are the same on every
 // lane and a leaf's coefficients are shared by its particles' lanes).
 __global__ void fmm_l2p_add_kernel(const Octree t, FmmDevTables T, const int* __restrict__ leaf_of,
@@ -3093,7 +3109,8 @@ int fmm_run(amk_ctx* c, const View& v, int order, double theta, long leaf_capaci
   // ---- near-field set-up
   double4* ef = slot<double4>(c, kSlotFmmWork4, t.m, &rc);
   AMK_TRY(rc);
-  const double min_sq = kMinSquaredDistance / (hf.length * hf.length);
+  // (positive, so that a particle never pairs with itself)
+  const double min_sq = std::max(kMinSquaredDistance / (hf.length * hf.length), 2.2250738585072014e-308);
   AMK_TRY(phase_begin(c, AMK_PHASE_FMM_P2P));
   int2* work = slot<int2>(c, kSlotP2PWork, ht[0] + 1, &rc);
   AMK_TRY(rc);
@@ -3110,10 +3127,11 @@ int fmm_run(amk_ctx* c, const View& v, int order, double theta, long leaf_capaci
   AMK_TRY(check_launch(c, "p2p_items_fill_kernel"));
   AMK_TRY(phase_end(c, AMK_PHASE_FMM_P2P));
   const unsigned gwork = static_cast<unsigned>((ht[0] + kFmmWarps - 1) / kFmmWarps);
-  // FP32 near field: its pair sums need no expansion, so they run on their
-  // own stream once the last M2L products are enqueued (the product kernel
-  // holds every SM's shared memory), concurrently with the per-target M2L
-  // sums and L2L; the FP64 L2P is added after L2L on the context stream
+  // The near field's pair sums need no expansion, so they run on their own
+  // stream: the FP32 ones once the last M2L products are enqueued (the
+  // tensor-core product kernel holds every SM's shared memory), concurrently
+  // with the per-target M2L sums and L2L; the FP64 L2P is added after L2L on
+  // the context stream
   auto launch_near = [&]() -> int {
     if (!f->near) {
       AMK_CUDA_TRY(cudaStreamCreateWithFlags(&f->near, cudaStreamNonBlocking));
@@ -3122,12 +3140,21 @@ int fmm_run(amk_ctx* c, const View& v, int order, double theta, long leaf_capaci
     }
     AMK_CUDA_TRY(cudaEventRecord(f->near_start, c->stream));
     AMK_CUDA_TRY(cudaStreamWaitEvent(f->near, f->near_start, 0));
-    p2p_stage_kernel<<<static_cast<unsigned>((t.m + 255) / 256), 256, 0, f->near>>>(t, stage, stage + t.m);
-    AMK_TRY(check_launch(c, "p2p_stage_kernel"));
+    if (f32) {
+      p2p_stage_kernel<<<static_cast<unsigned>((t.m + 255) / 256), 256, 0, f->near>>>(t, stage, stage + t.m);
+      AMK_TRY(check_launch(c, "p2p_stage_kernel"));
+    }
     AMK_TRY(phase_begin_on(c, AMK_PHASE_FMM_NEAR, f->near));
-    fmm_p2p32_kernel<<<gwork, 32 * kFmmWarps, 0, f->near>>>(t, work, ht[0], gp.off, gp.count, gp.src, pbase, min_sq,
-                                                            stage, stage + t.m, radius, part);
-    AMK_TRY(check_launch(c, "fmm_p2p32_kernel"));
+    if (f32)
+      fmm_p2p32_kernel<<<gwork, 32 * kFmmWarps, 0, f->near>>>(t, work, ht[0], gp.off, gp.count, gp.src, pbase, min_sq,
+                                                              stage, stage + t.m, radius, part);
+    else if (want_phi)
+      fmm_p2p_kernel<true><<<gwork, 32 * kFmmWarps, 0, f->near>>>(t, work, ht[0], gp.off, gp.count, gp.src, pbase,
+                                                                  min_sq, part);
+    else
+      fmm_p2p_kernel<false><<<gwork, 32 * kFmmWarps, 0, f->near>>>(t, work, ht[0], gp.off, gp.count, gp.src, pbase,
+                                                                   min_sq, part);
+    AMK_TRY(check_launch(c, "fmm_p2p_kernel"));
     AMK_TRY(phase_end_on(c, AMK_PHASE_FMM_NEAR, f->near));
     fmm_p2p_reduce_kernel<<<static_cast<unsigned>((t.m + 255) / 256), 256, 0, f->near>>>(t, leaf_of, items, pbase,
                                                                                        part, ef);
@@ -3135,7 +3162,6 @@ int fmm_run(amk_ctx* c, const View& v, int order, double theta, long leaf_capaci
     AMK_CUDA_TRY(cudaEventRecord(f->near_done, f->near));
     return AMK_OK;
   };
-  const std::function<int()> no_hook;
 
   // ---- M2L (the multipoles: join the upward pass)
   AMK_CUDA_TRY(cudaStreamWaitEvent(c->stream, f->up_done, 0));
@@ -3143,8 +3169,8 @@ int fmm_run(amk_ctx* c, const View& v, int order, double theta, long leaf_capaci
   AMK_TRY(phase_begin(c, AMK_PHASE_FMM_M2L));
   if (n_m2l > 0) {
     const std::function<int()> hook(launch_near);
-    AMK_TRY(m2l_products(c, order, t, T, gm, cell, n_m2l, M, Lx, f32 ? hook : no_hook));
-  } else if (f32) {
+    AMK_TRY(m2l_products(c, order, t, T, gm, cell, n_m2l, M, Lx, hook));
+  } else {
     AMK_TRY(launch_near());
   }
   AMK_TRY(phase_end(c, AMK_PHASE_FMM_M2L));
@@ -3159,19 +3185,10 @@ int fmm_run(amk_ctx* c, const View& v, int order, double theta, long leaf_capaci
 
   // ---- L2P + P2P
   AMK_TRY(phase_begin(c, AMK_PHASE_FMM_P2P));
-  if (f32) {  // join the near-field stream, then the FP64 L2P
-    AMK_CUDA_TRY(cudaStreamWaitEvent(c->stream, f->near_done, 0));
-    fmm_l2p_add_kernel<<<static_cast<unsigned>((t.m + 127) / 128), 128, 0, c->stream>>>(t, T, leaf_of, Lx, want_phi,
-                                                                                        ef);
-    AMK_TRY(check_launch(c, "fmm_l2p_add_kernel"));
-  } else {
-    fmm_p2p_kernel<<<gwork, 32 * kFmmWarps, 0, c->stream>>>(t, T, work, ht[0], gp.off, gp.count, gp.src, pbase, Lx,
-                                                            min_sq, want_phi, part);
-    AMK_TRY(check_launch(c, "fmm_p2p_kernel"));
-    fmm_p2p_reduce_kernel<<<static_cast<unsigned>((t.m + 255) / 256), 256, 0, c->stream>>>(t, leaf_of, items, pbase,
-                                                                                          part, ef);
-    AMK_TRY(check_launch(c, "fmm_p2p_reduce_kernel"));
-  }
+  // join the near-field stream, then the FP64 L2P
+  AMK_CUDA_TRY(cudaStreamWaitEvent(c->stream, f->near_done, 0));
+  fmm_l2p_add_kernel<<<static_cast<unsigned>((t.m + 127) / 128), 128, 0, c->stream>>>(t, T, leaf_of, Lx, want_phi, ef);
+  AMK_TRY(check_launch(c, "fmm_l2p_add_kernel"));
   run->leaf_of = leaf_of;
   AMK_TRY(phase_end(c, AMK_PHASE_FMM_P2P));
   run->t = t;
