@@ -2333,7 +2333,9 @@ __global__ void p2p_items_fill_kernel(const Octree t, const int* __restrict__ it
   for (int k = r.x; k < r.y; ++k) leaf_of[k] = id;
 }
 
-// FP64 pair sums of one item. The item's sources are staged in shared memory
+// FP64 pair sums of one item, one warp per block (items differ by more than
+// ten times: with four to a block their slots stayed empty until the longest
+// had ended). The item's sources are staged in shared memory
 // as one run, leaf boundaries gone: the particles of 32 leaves at a time are
 // numbered by a warp scan of the leaf sizes and copied in windows of 256 (read
 // leaf by leaf from global memory, 9 particles on average at leaf capacity 32,
@@ -2341,18 +2343,14 @@ __global__ void p2p_items_fill_kernel(const Octree t, const int* __restrict__ it
 // FP64 pipe). About 20 FP64 operations per pair; the target itself and pairs
 // below the minimum distance get 1/r := 0.
 template <bool kPhi>
-__global__ void __launch_bounds__(32 * kFmmWarps)
-fmm_p2p_kernel(const Octree t, const int2* __restrict__ work, int n_work, const int* __restrict__ off,
+__global__ void __launch_bounds__(32)
+fmm_p2p_kernel(const Octree t, const int2* __restrict__ work, const int* __restrict__ off,
                const int* __restrict__ count, const int* __restrict__ src, const int* __restrict__ pbase,
                double min_sq, double4* __restrict__ part) {
-  __shared__ double4 stg_s[kFmmWarps][kP2PWindow];
-  __shared__ int end_s[kFmmWarps][32], beg_s[kFmmWarps][32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int wi = blockIdx.x * kFmmWarps + w;
-  if (wi >= n_work) return;
-  double4* stg = stg_s[w];
-  int *leaf_end = end_s[w], *leaf_beg = beg_s[w];
-  const int2 item = work[wi];
+  __shared__ double4 stg[kP2PWindow];
+  __shared__ int leaf_end[32], leaf_beg[32];
+  const int lane = threadIdx.x;
+  const int2 item = work[blockIdx.x];
   const int ti = item.x, chunk = item.y;
   const int2 tr = t.range[ti];
   const int nt_all = tr.y - tr.x;
@@ -2397,7 +2395,7 @@ fmm_p2p_kernel(const Octree t, const int2* __restrict__ work, int n_work, const 
             const double4 s = stg[k];
             const double rx = me.x - s.x, ry = me.y - s.y, rz = me.z - s.z;
             const double r2 = rx * rx + ry * ry + rz * rz;
-            const double inv = r2 < min_sq ? 0.0 : rsqrt(r2);
+            const double inv = r2 < min_sq ? 0.0 : rsqrt_f64(r2);
             const double qi = s.w * inv;
             const double f = qi * (inv * inv);
             fx += rx * f;
@@ -3149,11 +3147,11 @@ int fmm_run(amk_ctx* c, const View& v, int order, double theta, long leaf_capaci
       fmm_p2p32_kernel<<<gwork, 32 * kFmmWarps, 0, f->near>>>(t, work, ht[0], gp.off, gp.count, gp.src, pbase, min_sq,
                                                               stage, stage + t.m, radius, part);
     else if (want_phi)
-      fmm_p2p_kernel<true><<<gwork, 32 * kFmmWarps, 0, f->near>>>(t, work, ht[0], gp.off, gp.count, gp.src, pbase,
-                                                                  min_sq, part);
+      fmm_p2p_kernel<true><<<static_cast<unsigned>(ht[0]), 32, 0, f->near>>>(t, work, gp.off, gp.count, gp.src, pbase, min_sq,
+                                                                              part);
     else
-      fmm_p2p_kernel<false><<<gwork, 32 * kFmmWarps, 0, f->near>>>(t, work, ht[0], gp.off, gp.count, gp.src, pbase,
-                                                                   min_sq, part);
+      fmm_p2p_kernel<false><<<static_cast<unsigned>(ht[0]), 32, 0, f->near>>>(t, work, gp.off, gp.count, gp.src, pbase,
+                                                                               min_sq, part);
     AMK_TRY(check_launch(c, "fmm_p2p_kernel"));
     AMK_TRY(phase_end_on(c, AMK_PHASE_FMM_NEAR, f->near));
     fmm_p2p_reduce_kernel<<<static_cast<unsigned>((t.m + 255) / 256), 256, 0, f->near>>>(t, leaf_of, items, pbase,
