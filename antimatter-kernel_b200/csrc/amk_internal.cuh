@@ -183,6 +183,7 @@ enum ScratchSlot {
   kSlotTreeSortedKeys,
   kSlotBhPos,
   kSlotBhNeg,
+  kSlotBhInfo,
   kSlotWalkOut,
   kSlotFmmRadius,
   kSlotFmmWork0,

@@ -14,8 +14,13 @@
 // children for themselves. Leaves are summed directly, skipping the target
 // itself and q = 0 sources. Pairs closer than 1e-30 m^2 are skipped
 // (barnes-hut.cc:33-41). All arithmetic is FP64 (leaf sums FP32 in the
-// tensor precision mode, below); inverse distances use rsqrt where the
-// reference divides by sqrt (an ulp-level difference).
+// tensor precision mode, below); inverse distances are reciprocal square
+// roots where the reference divides by sqrt (an ulp-level difference).
+//
+// The walk is bound by the latency of a node's loads, not by its arithmetic
+// (FP64 pipe 36 % with pos, meta, centre and children read one after the
+// other): everything a visit may need of a node is loaded at once when it is
+// popped, and a block is two warps, since walks differ in length.
 #include <algorithm>
 #include <vector>
 
@@ -24,7 +29,7 @@
 namespace amk {
 namespace {
 
-constexpr int kWalkWarps = 4;
+constexpr int kWalkWarps = 2;
 constexpr int kStack = 176;  // >= 1 + 7 * 21 + 8
 
 __device__ __forceinline__ double dot_rn(double a, double b, double c) {
@@ -90,25 +95,28 @@ __global__ void bh_merge_kernel(const Octree t, int depth, double4* __restrict__
                      : make_double4(c.x, c.y, c.z, 0.0);
 }
 
-// AddPointCharge, barnes-hut.cc:20-28: force += r * (k qt qs / r^2 / r).
-__device__ __forceinline__ void add_point(double tx, double ty, double tz, double tq, double sx, double sy,
-                                          double sz, double sq, double* f) {
-  const double rx = tx - sx, ry = ty - sy, rz = tz - sz;
-  const double d2 = dot_rn(rx, ry, rz);
-  if (d2 < kMinSquaredDistance) return;
-  const double inv = rsqrt(d2);
-  const double w = kCoulombConstant * tq * sq * (inv * inv * inv);
+// What a visit reads of a node besides its centre and monopoles: particle
+// range, leaf flag.
+__global__ void bh_info_kernel(const Octree t, int4* __restrict__ info) {
+  const int id = blockIdx.x * blockDim.x + threadIdx.x;
+  if (id >= t.n_nodes) return;
+  const int2 r = t.range[id];
+  info[id] = make_int4(r.x, r.y, t.meta[id].y, 0);
+}
+
+// AddPointCharge, barnes-hut.cc:20-28, without the factor k q_t:
+// f += r q_s / r^3; pairs closer than the minimum distance (and `skip`) add 0.
+__device__ __forceinline__ void add_point(double rx, double ry, double rz, double d2, double sq, bool skip,
+                                          double* f) {
+  const double inv = skip || d2 < kMinSquaredDistance ? 0.0 : rsqrt_f64(d2);
+  const double w = sq * (inv * inv * inv);
   f[0] += rx * w;
   f[1] += ry * w;
   f[2] += rz * w;
 }
 
-__device__ __forceinline__ void add_phi(double tx, double ty, double tz, double sx, double sy, double sz,
-                                        double sq, double* phi) {
-  const double rx = tx - sx, ry = ty - sy, rz = tz - sz;
-  const double d2 = dot_rn(rx, ry, rz);
-  if (d2 < kMinSquaredDistance) return;
-  *phi += sq * rsqrt(d2);
+__device__ __forceinline__ void add_phi(double d2, double sq, bool skip, double* phi) {
+  *phi += sq * (skip || d2 < kMinSquaredDistance ? 0.0 : rsqrt_f64(d2));
 }
 
 // Leaf sums in FP32 (the tensor precision mode): sources as double-float
@@ -135,8 +143,9 @@ __global__ void bh_stage_kernel(const Octree t, double qs, float4* __restrict__ 
 
 template <bool kPhi, bool kF32>
 __global__ void __launch_bounds__(32 * kWalkWarps)
-bh_walk_kernel(const Octree t, const double4* __restrict__ pos, const double4* __restrict__ neg, double theta2,
-               BhF32 f32, double* __restrict__ out, int* __restrict__ status) {
+bh_walk_kernel(const Octree t, const int4* __restrict__ info, const double4* __restrict__ pos,
+               const double4* __restrict__ neg, double theta2, BhF32 f32, double* __restrict__ out,
+               int* __restrict__ status) {
   __shared__ int s_node[kWalkWarps][kStack];
   __shared__ unsigned s_mask[kWalkWarps][kStack];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -164,17 +173,20 @@ bh_walk_kernel(const Octree t, const double4* __restrict__ pos, const double4* _
     const unsigned mask = s_mask[w][sp];
     __syncwarp();
     const bool act = (mask >> lane) & 1u;
+    const int4 in = info[nd];
+    const double4 c = t.center[nd];
     const double4 pq = pos[nd], nq = neg[nd];
+    // children 7..0 (lane 0 holds child 7) so that octant 0 pops first
+    const int ch = lane < 8 ? t.child[8 * nd + (7 - lane)] : -1;
     if (pq.w == 0.0 && nq.w == 0.0) continue;  // barnes-hut.cc:186
-    if (t.meta[nd].y) {
-      const int2 r = t.range[nd];
-      if (act) {
-        if (kF32) {
+    if (in.z) {
+      if (kF32) {
+        if (act) {
           // sum over the leaf of (q_j / qs) r / r^3 (or / r) in FP32
           const float4 mh = f32.hi[k], ml = f32.lo[k];
           const float min_sq = 1e-30f;  // kMinSquaredDistance (m^2), a normal float
           float ax = 0.f, ay = 0.f, az = 0.f, ap = 0.f;
-          for (int j = r.x; j < r.y; ++j) {
+          for (int j = in.x; j < in.y; ++j) {
             const float4 s = f32.hi[j], q = f32.lo[j];
             const float rx = fmaf(s.x, -1.f, mh.x) + fmaf(q.x, -1.f, ml.x);
             const float ry = fmaf(s.y, -1.f, mh.y) + fmaf(q.y, -1.f, ml.y);
@@ -186,53 +198,59 @@ bh_walk_kernel(const Octree t, const double4* __restrict__ pos, const double4* _
             if (kPhi) {
               ap += qr;
             } else {
-              const float w = qr * (inv * inv);
-              ax = fmaf(rx, w, ax);
-              ay = fmaf(ry, w, ay);
-              az = fmaf(rz, w, az);
+              const float wt = qr * (inv * inv);
+              ax = fmaf(rx, wt, ax);
+              ay = fmaf(ry, wt, ay);
+              az = fmaf(rz, wt, az);
             }
           }
           if (kPhi) {
             phi += f32.qs * static_cast<double>(ap);
           } else {
-            const double sc = kCoulombConstant * me.w * f32.qs;
-            f[0] += sc * static_cast<double>(ax);
-            f[1] += sc * static_cast<double>(ay);
-            f[2] += sc * static_cast<double>(az);
+            f[0] += f32.qs * static_cast<double>(ax);
+            f[1] += f32.qs * static_cast<double>(ay);
+            f[2] += f32.qs * static_cast<double>(az);
           }
-        } else {
-          for (int j = r.x; j < r.y; ++j) {
-            if (j == k) continue;
-            const double4 s = t.src[j];
-            if (s.w == 0.0) continue;
-            if (kPhi)
-              add_phi(me.x, me.y, me.z, s.x, s.y, s.z, s.w, &phi);
-            else
-              add_point(me.x, me.y, me.z, me.w, s.x, s.y, s.z, s.w, f);
-          }
+        }
+      } else if (act) {
+#pragma unroll 4
+        for (int j = in.x; j < in.y; ++j) {
+          const double4 s = t.src[j];
+          const double rx = me.x - s.x, ry = me.y - s.y, rz = me.z - s.z;
+          const double d2 = dot_rn(rx, ry, rz);
+          if (kPhi)
+            add_phi(d2, s.w, j == k, &phi);
+          else
+            add_point(rx, ry, rz, d2, s.w, j == k, f);
         }
       }
       continue;
     }
-    const double4 c = t.center[nd];
     const double dx = me.x - c.x, dy = me.y - c.y, dz = me.z - c.z;
     const double d2 = dot_rn(dx, dy, dz);
     const double width = 2.0 * c.w;
     const bool accept = act && (__dmul_rn(width, width) < __dmul_rn(theta2, d2));
     const unsigned acc = __ballot_sync(0xffffffffu, accept);
     if (accept) {
-      if (kPhi) {
-        if (pq.w > 0.0) add_phi(me.x, me.y, me.z, pq.x, pq.y, pq.z, pq.w, &phi);
-        if (nq.w > 0.0) add_phi(me.x, me.y, me.z, nq.x, nq.y, nq.z, -nq.w, &phi);
-      } else {
-        if (pq.w > 0.0) add_point(me.x, me.y, me.z, me.w, pq.x, pq.y, pq.z, pq.w, f);
-        if (nq.w > 0.0) add_point(me.x, me.y, me.z, me.w, nq.x, nq.y, nq.z, -nq.w, f);
+      if (pq.w > 0.0) {
+        const double rx = me.x - pq.x, ry = me.y - pq.y, rz = me.z - pq.z;
+        const double r2 = dot_rn(rx, ry, rz);
+        if (kPhi)
+          add_phi(r2, pq.w, false, &phi);
+        else
+          add_point(rx, ry, rz, r2, pq.w, false, f);
+      }
+      if (nq.w > 0.0) {
+        const double rx = me.x - nq.x, ry = me.y - nq.y, rz = me.z - nq.z;
+        const double r2 = dot_rn(rx, ry, rz);
+        if (kPhi)
+          add_phi(r2, -nq.w, false, &phi);
+        else
+          add_point(rx, ry, rz, r2, -nq.w, false, f);
       }
     }
     const unsigned open = mask & ~acc;
     if (open) {
-      // push children 7..0 (lane 0 holds child 7) so that octant 0 pops first
-      const int ch = lane < 8 ? t.child[8 * nd + (7 - lane)] : -1;
       const unsigned has = __ballot_sync(0xffffffffu, ch >= 0);
       const int pushed = __popc(has);
       if (sp + pushed > kStack) {  // cannot happen for depth <= 21; guarded anyway
@@ -252,9 +270,10 @@ bh_walk_kernel(const Octree t, const double4* __restrict__ pos, const double4* _
     if (kPhi) {
       out[k] = phi;
     } else {
-      out[3 * k + 0] = f[0];
-      out[3 * k + 1] = f[1];
-      out[3 * k + 2] = f[2];
+      const double sc = kCoulombConstant * me.w;
+      out[3 * k + 0] = sc * f[0];
+      out[3 * k + 1] = sc * f[1];
+      out[3 * k + 2] = sc * f[2];
     }
   }
 }
@@ -323,6 +342,10 @@ int barnes_hut_forces(amk_ctx* c, const View& v, double theta, long leaf_capacit
   int* status = slot<int>(c, kSlotStatus, 8, &rc) + 4;
   AMK_TRY(rc);
   AMK_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int), c->stream));
+  int4* info = slot<int4>(c, kSlotBhInfo, t.n_nodes, &rc);
+  AMK_TRY(rc);
+  bh_info_kernel<<<static_cast<unsigned>((t.n_nodes + 255) / 256), 256, 0, c->stream>>>(t, info);
+  AMK_TRY(check_launch(c, "bh_info_kernel"));
   const unsigned blocks = static_cast<unsigned>((t.m + 32 * kWalkWarps - 1) / (32 * kWalkWarps));
   const double theta2 = theta * theta;  // squared_theta_, barnes-hut.cc:36
   const bool f32 = c->fmm_precision == AMK_FMM_TENSOR;
@@ -337,15 +360,15 @@ int barnes_hut_forces(amk_ctx* c, const View& v, double theta, long leaf_capacit
   }
   AMK_TRY(phase_begin(c, AMK_PHASE_BH_WALK));
   if (f32)
-    bh_walk_kernel<false, true><<<blocks, 32 * kWalkWarps, 0, c->stream>>>(t, pos, neg, theta2, fs, fo, status);
+    bh_walk_kernel<false, true><<<blocks, 32 * kWalkWarps, 0, c->stream>>>(t, info, pos, neg, theta2, fs, fo, status);
   else
-    bh_walk_kernel<false, false><<<blocks, 32 * kWalkWarps, 0, c->stream>>>(t, pos, neg, theta2, fs, fo, status);
+    bh_walk_kernel<false, false><<<blocks, 32 * kWalkWarps, 0, c->stream>>>(t, info, pos, neg, theta2, fs, fo, status);
   AMK_TRY(check_launch(c, "bh_walk_kernel"));
   if (po) {
     if (f32)
-      bh_walk_kernel<true, true><<<blocks, 32 * kWalkWarps, 0, c->stream>>>(t, pos, neg, theta2, fs, po, status);
+      bh_walk_kernel<true, true><<<blocks, 32 * kWalkWarps, 0, c->stream>>>(t, info, pos, neg, theta2, fs, po, status);
     else
-      bh_walk_kernel<true, false><<<blocks, 32 * kWalkWarps, 0, c->stream>>>(t, pos, neg, theta2, fs, po, status);
+      bh_walk_kernel<true, false><<<blocks, 32 * kWalkWarps, 0, c->stream>>>(t, info, pos, neg, theta2, fs, po, status);
     AMK_TRY(check_launch(c, "bh_walk_kernel"));
   }
   AMK_TRY(phase_end(c, AMK_PHASE_BH_WALK));
