@@ -183,7 +183,7 @@ enum ScratchSlot {
   kSlotTreeSortedKeys,
   kSlotBhPos,
   kSlotBhNeg,
-  kSlotBhInfo,
+  kSlotBhRec,
   kSlotWalkOut,
   kSlotFmmRadius,
   kSlotFmmWork0,

@@ -6,21 +6,24 @@
 // level from the deepest.
 //
 // Walk (barnes-hut.cc:183-269): a warp takes 32 consecutive targets in tree
-// order and walks one shared depth-first stack. Each entry carries the mask
-// of lanes that still need that node. A lane accepts an internal node when
-// (2h)^2 < theta^2 |x - c|^2 (the reference's test, evaluated in FP64
-// without contraction, so the accepted-node set of every target is the
-// reference's); accepting lanes add the two monopoles, the others push the
-// children for themselves. Leaves are summed directly, skipping the target
-// itself and q = 0 sources. Pairs closer than 1e-30 m^2 are skipped
+// order and walks one shared stack of nodes to open. Each entry carries the
+// mask of lanes that open that node; the node's children are tested there and
+// then. A lane accepts an internal node when (2h)^2 < theta^2 |x - c|^2 (the
+// reference's test, evaluated in FP64 without contraction, so the
+// accepted-node set of every target is the reference's); accepting lanes add
+// the two monopoles, for the others the child goes on the stack. Leaves are
+// summed directly, skipping the target itself and q = 0 sources. Pairs closer than 1e-30 m^2 are skipped
 // (barnes-hut.cc:33-41). All arithmetic is FP64 (leaf sums FP32 in the
 // tensor precision mode, below); inverse distances are reciprocal square
 // roots where the reference divides by sqrt (an ulp-level difference).
 //
-// The walk is bound by the latency of a node's loads, not by its arithmetic
-// (FP64 pipe 36 % with pos, meta, centre and children read one after the
-// other): everything a visit may need of a node is loaded at once when it is
-// popped, and a block is two warps, since walks differ in length.
+// The walk is bound by the latency of the node loads, not by its arithmetic,
+// so the records of a node's children (128 bytes each) lie side by side and
+// the warp copies them into shared memory with two loads per opened node: one
+// memory latency per up to eight tests. (A node popped and read at a time:
+// 3.75 ms at 524,309 particles, theta = 0.7, with its loads one after the
+// other, 3.0 ms with them together, FP64 pipe at 36 and 42 %.) A block is two
+// warps, since walks differ in length.
 #include <algorithm>
 #include <vector>
 
@@ -30,7 +33,7 @@ namespace amk {
 namespace {
 
 constexpr int kWalkWarps = 2;
-constexpr int kStack = 176;  // >= 1 + 7 * 21 + 8
+constexpr int kStack = 176;  // >= 1 + 7 * 21 + 8 nodes to open
 
 __device__ __forceinline__ double dot_rn(double a, double b, double c) {
   // ((0 + a*a) + b*b) + c*c without contraction (the reference's Real3 dot)
@@ -95,13 +98,50 @@ __global__ void bh_merge_kernel(const Octree t, int depth, double4* __restrict__
                      : make_double4(c.x, c.y, c.z, 0.0);
 }
 
-// What a visit reads of a node besides its centre and monopoles: particle
-// range, leaf flag.
-__global__ void bh_info_kernel(const Octree t, int4* __restrict__ info) {
+// What the walk reads of a node.
+struct __align__(128) BhRec {
+  double4 c;    // centre, half edge
+  double4 pos;  // positive charge centre and sum
+  double4 neg;  // |negative| charge centre and sum
+  int4 info;    // internal: first child's record, children, 0; leaf: particles [x, y), 1
+  int4 pad;
+};
+static_assert(sizeof(BhRec) == 128, "eight 16-byte pieces");
+
+__global__ void bh_child_count_kernel(const Octree t, int* __restrict__ n_child) {
   const int id = blockIdx.x * blockDim.x + threadIdx.x;
   if (id >= t.n_nodes) return;
-  const int2 r = t.range[id];
-  info[id] = make_int4(r.x, r.y, t.meta[id].y, 0);
+  const int4* c = reinterpret_cast<const int4*>(t.child + 8 * static_cast<size_t>(id));
+  const int4 a = c[0], b = c[1];
+  n_child[id] = (a.x >= 0) + (a.y >= 0) + (a.z >= 0) + (a.w >= 0) + (b.x >= 0) + (b.y >= 0) + (b.z >= 0) + (b.w >= 0);
+}
+
+// Records grouped by parent: the children of node p (octant order) at
+// first[p], first[p] + 1, ...; the root's record is the last one. Eight
+// threads per parent.
+__global__ void bh_record_kernel(const Octree t, const int* __restrict__ n_child, const int* __restrict__ first,
+                                 const double4* __restrict__ pos, const double4* __restrict__ neg,
+                                 BhRec* __restrict__ rec) {
+  const long x = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
+  const long p = x >> 3;
+  const int o = static_cast<int>(x & 7), lane = threadIdx.x & 31;
+  const int id = p < t.n_nodes ? t.child[x] : -1;
+  const unsigned has = __ballot_sync(0xffffffffu, id >= 0);
+  long at = 0;
+  if (id >= 0) {
+    const unsigned mine = (has >> (lane & 24)) & 0xffu;
+    at = first[p] + __popc(mine & ((1u << o) - 1u));
+  }
+  auto put = [&](int node, long slot) {
+    const int2 r = t.range[node];
+    BhRec* d = rec + slot;
+    d->c = t.center[node];
+    d->pos = pos[node];
+    d->neg = neg[node];
+    d->info = t.meta[node].y ? make_int4(r.x, r.y, 1, 0) : make_int4(first[node], n_child[node], 0, 0);
+  };
+  if (id >= 0) put(id, at);
+  if (x == 0) put(0, t.n_nodes - 1);
 }
 
 // AddPointCharge, barnes-hut.cc:20-28, without the factor k q_t:
@@ -143,10 +183,11 @@ __global__ void bh_stage_kernel(const Octree t, double qs, float4* __restrict__ 
 
 template <bool kPhi, bool kF32>
 __global__ void __launch_bounds__(32 * kWalkWarps)
-bh_walk_kernel(const Octree t, const int4* __restrict__ info, const double4* __restrict__ pos,
-               const double4* __restrict__ neg, double theta2, BhF32 f32, double* __restrict__ out,
+bh_walk_kernel(const Octree t, const BhRec* __restrict__ rec, double theta2, BhF32 f32, double* __restrict__ out,
                int* __restrict__ status) {
-  __shared__ int s_node[kWalkWarps][kStack];
+  __shared__ BhRec s_rec[kWalkWarps][8];
+  __shared__ int s_first[kWalkWarps][kStack];
+  __shared__ int s_count[kWalkWarps][kStack];
   __shared__ unsigned s_mask[kWalkWarps][kStack];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const long k = (static_cast<long>(blockIdx.x) * kWalkWarps + w) * 32 + lane;
@@ -161,109 +202,115 @@ bh_walk_kernel(const Octree t, const int4* __restrict__ info, const double4* __r
   int sp = 0;
   if (lanes) {
     if (lane == 0) {
-      s_node[w][0] = 0;
+      s_first[w][0] = static_cast<int>(t.n_nodes) - 1;  // the root's record
+      s_count[w][0] = 1;
       s_mask[w][0] = lanes;
     }
     sp = 1;
   }
-  __syncwarp();
+  const BhRec* child = s_rec[w];
   while (sp > 0) {
+    __syncwarp();  // the last node's records have been read, its pushes are complete
     --sp;
-    const int nd = s_node[w][sp];
+    const int first = s_first[w][sp], n = s_count[w][sp];
     const unsigned mask = s_mask[w][sp];
-    __syncwarp();
     const bool act = (mask >> lane) & 1u;
-    const int4 in = info[nd];
-    const double4 c = t.center[nd];
-    const double4 pq = pos[nd], nq = neg[nd];
-    // children 7..0 (lane 0 holds child 7) so that octant 0 pops first
-    const int ch = lane < 8 ? t.child[8 * nd + (7 - lane)] : -1;
-    if (pq.w == 0.0 && nq.w == 0.0) continue;  // barnes-hut.cc:186
-    if (in.z) {
-      if (kF32) {
-        if (act) {
-          // sum over the leaf of (q_j / qs) r / r^3 (or / r) in FP32
-          const float4 mh = f32.hi[k], ml = f32.lo[k];
-          const float min_sq = 1e-30f;  // kMinSquaredDistance (m^2), a normal float
-          float ax = 0.f, ay = 0.f, az = 0.f, ap = 0.f;
-          for (int j = in.x; j < in.y; ++j) {
-            const float4 s = f32.hi[j], q = f32.lo[j];
-            const float rx = fmaf(s.x, -1.f, mh.x) + fmaf(q.x, -1.f, ml.x);
-            const float ry = fmaf(s.y, -1.f, mh.y) + fmaf(q.y, -1.f, ml.y);
-            const float rz = fmaf(s.z, -1.f, mh.z) + fmaf(q.z, -1.f, ml.z);
-            const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
-            // the target itself (r = 0), closer pairs and neutral sources add zero
-            const float inv = (j != k && r2 >= min_sq) ? rsqrtf(r2) : 0.f;
-            const float qr = s.w * inv;
+    const float4* from = reinterpret_cast<const float4*>(rec + first);
+    float4* to = reinterpret_cast<float4*>(s_rec[w]);
+    if (lane < 8 * n) to[lane] = from[lane];
+    if (lane + 32 < 8 * n) to[lane + 32] = from[lane + 32];
+    __syncwarp();
+    for (int o = 0; o < n; ++o) {
+      const int4 in = child[o].info;
+      const double pw = child[o].pos.w, nw = child[o].neg.w;
+      if (pw == 0.0 && nw == 0.0) continue;  // barnes-hut.cc:186
+      if (in.z) {
+        if (kF32) {
+          if (act) {
+            // sum over the leaf of (q_j / qs) r / r^3 (or / r) in FP32
+            const float4 mh = f32.hi[k], ml = f32.lo[k];
+            const float min_sq = 1e-30f;  // kMinSquaredDistance (m^2), a normal float
+            float ax = 0.f, ay = 0.f, az = 0.f, ap = 0.f;
+            for (int j = in.x; j < in.y; ++j) {
+              const float4 s = f32.hi[j], q = f32.lo[j];
+              const float rx = fmaf(s.x, -1.f, mh.x) + fmaf(q.x, -1.f, ml.x);
+              const float ry = fmaf(s.y, -1.f, mh.y) + fmaf(q.y, -1.f, ml.y);
+              const float rz = fmaf(s.z, -1.f, mh.z) + fmaf(q.z, -1.f, ml.z);
+              const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
+              // the target itself (r = 0), closer pairs and neutral sources add zero
+              const float inv = (j != k && r2 >= min_sq) ? rsqrtf(r2) : 0.f;
+              const float qr = s.w * inv;
+              if (kPhi) {
+                ap += qr;
+              } else {
+                const float wt = qr * (inv * inv);
+                ax = fmaf(rx, wt, ax);
+                ay = fmaf(ry, wt, ay);
+                az = fmaf(rz, wt, az);
+              }
+            }
             if (kPhi) {
-              ap += qr;
+              phi += f32.qs * static_cast<double>(ap);
             } else {
-              const float wt = qr * (inv * inv);
-              ax = fmaf(rx, wt, ax);
-              ay = fmaf(ry, wt, ay);
-              az = fmaf(rz, wt, az);
+              f[0] += f32.qs * static_cast<double>(ax);
+              f[1] += f32.qs * static_cast<double>(ay);
+              f[2] += f32.qs * static_cast<double>(az);
             }
           }
-          if (kPhi) {
-            phi += f32.qs * static_cast<double>(ap);
-          } else {
-            f[0] += f32.qs * static_cast<double>(ax);
-            f[1] += f32.qs * static_cast<double>(ay);
-            f[2] += f32.qs * static_cast<double>(az);
+        } else if (act) {
+#pragma unroll 4
+          for (int j = in.x; j < in.y; ++j) {
+            const double4 s = t.src[j];
+            const double rx = me.x - s.x, ry = me.y - s.y, rz = me.z - s.z;
+            const double d2 = dot_rn(rx, ry, rz);
+            if (kPhi)
+              add_phi(d2, s.w, j == k, &phi);
+            else
+              add_point(rx, ry, rz, d2, s.w, j == k, f);
           }
         }
-      } else if (act) {
-#pragma unroll 4
-        for (int j = in.x; j < in.y; ++j) {
-          const double4 s = t.src[j];
-          const double rx = me.x - s.x, ry = me.y - s.y, rz = me.z - s.z;
-          const double d2 = dot_rn(rx, ry, rz);
+        continue;
+      }
+      const double4 c = child[o].c;
+      const double dx = me.x - c.x, dy = me.y - c.y, dz = me.z - c.z;
+      const double d2 = dot_rn(dx, dy, dz);
+      const double width = 2.0 * c.w;
+      const bool accept = act && (__dmul_rn(width, width) < __dmul_rn(theta2, d2));
+      const unsigned acc = __ballot_sync(0xffffffffu, accept);
+      if (accept) {
+        if (pw > 0.0) {
+          const double4 pq = child[o].pos;
+          const double rx = me.x - pq.x, ry = me.y - pq.y, rz = me.z - pq.z;
+          const double r2 = dot_rn(rx, ry, rz);
           if (kPhi)
-            add_phi(d2, s.w, j == k, &phi);
+            add_phi(r2, pw, false, &phi);
           else
-            add_point(rx, ry, rz, d2, s.w, j == k, f);
+            add_point(rx, ry, rz, r2, pw, false, f);
+        }
+        if (nw > 0.0) {
+          const double4 nq = child[o].neg;
+          const double rx = me.x - nq.x, ry = me.y - nq.y, rz = me.z - nq.z;
+          const double r2 = dot_rn(rx, ry, rz);
+          if (kPhi)
+            add_phi(r2, -nw, false, &phi);
+          else
+            add_point(rx, ry, rz, r2, -nw, false, f);
         }
       }
-      continue;
-    }
-    const double dx = me.x - c.x, dy = me.y - c.y, dz = me.z - c.z;
-    const double d2 = dot_rn(dx, dy, dz);
-    const double width = 2.0 * c.w;
-    const bool accept = act && (__dmul_rn(width, width) < __dmul_rn(theta2, d2));
-    const unsigned acc = __ballot_sync(0xffffffffu, accept);
-    if (accept) {
-      if (pq.w > 0.0) {
-        const double rx = me.x - pq.x, ry = me.y - pq.y, rz = me.z - pq.z;
-        const double r2 = dot_rn(rx, ry, rz);
-        if (kPhi)
-          add_phi(r2, pq.w, false, &phi);
-        else
-          add_point(rx, ry, rz, r2, pq.w, false, f);
+      const unsigned open = mask & ~acc;
+      if (open) {
+        if (sp >= kStack) {  // cannot happen for depth <= 21; guarded anyway
+          if (lane == 0) atomicExch(status, 1);
+          sp = 0;
+          break;
+        }
+        if (lane == 0) {
+          s_first[w][sp] = in.x;
+          s_count[w][sp] = in.y;
+          s_mask[w][sp] = open;
+        }
+        ++sp;
       }
-      if (nq.w > 0.0) {
-        const double rx = me.x - nq.x, ry = me.y - nq.y, rz = me.z - nq.z;
-        const double r2 = dot_rn(rx, ry, rz);
-        if (kPhi)
-          add_phi(r2, -nq.w, false, &phi);
-        else
-          add_point(rx, ry, rz, r2, -nq.w, false, f);
-      }
-    }
-    const unsigned open = mask & ~acc;
-    if (open) {
-      const unsigned has = __ballot_sync(0xffffffffu, ch >= 0);
-      const int pushed = __popc(has);
-      if (sp + pushed > kStack) {  // cannot happen for depth <= 21; guarded anyway
-        if (lane == 0) atomicExch(status, 1);
-        break;
-      }
-      if (ch >= 0) {
-        const int slot_i = sp + __popc(has & ((1u << lane) - 1u));
-        s_node[w][slot_i] = ch;
-        s_mask[w][slot_i] = open;
-      }
-      sp += pushed;
-      __syncwarp();
     }
   }
   if (valid) {
@@ -342,10 +389,18 @@ int barnes_hut_forces(amk_ctx* c, const View& v, double theta, long leaf_capacit
   int* status = slot<int>(c, kSlotStatus, 8, &rc) + 4;
   AMK_TRY(rc);
   AMK_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int), c->stream));
-  int4* info = slot<int4>(c, kSlotBhInfo, t.n_nodes, &rc);
+  BhRec* rec = slot<BhRec>(c, kSlotBhRec, t.n_nodes, &rc);
   AMK_TRY(rc);
-  bh_info_kernel<<<static_cast<unsigned>((t.n_nodes + 255) / 256), 256, 0, c->stream>>>(t, info);
-  AMK_TRY(check_launch(c, "bh_info_kernel"));
+  int* n_child = slot<int>(c, kSlotTreeCount, t.n_nodes, &rc);  // tree build scratch, free again
+  AMK_TRY(rc);
+  int* first = slot<int>(c, kSlotTreeBase, t.n_nodes + 1, &rc);
+  AMK_TRY(rc);
+  bh_child_count_kernel<<<static_cast<unsigned>((t.n_nodes + 255) / 256), 256, 0, c->stream>>>(t, n_child);
+  AMK_TRY(check_launch(c, "bh_child_count_kernel"));
+  AMK_TRY(exclusive_scan_int(c, n_child, t.n_nodes, first, first + t.n_nodes));
+  bh_record_kernel<<<static_cast<unsigned>((8 * t.n_nodes + 255) / 256), 256, 0, c->stream>>>(t, n_child, first, pos,
+                                                                                             neg, rec);
+  AMK_TRY(check_launch(c, "bh_record_kernel"));
   const unsigned blocks = static_cast<unsigned>((t.m + 32 * kWalkWarps - 1) / (32 * kWalkWarps));
   const double theta2 = theta * theta;  // squared_theta_, barnes-hut.cc:36
   const bool f32 = c->fmm_precision == AMK_FMM_TENSOR;
@@ -360,15 +415,15 @@ int barnes_hut_forces(amk_ctx* c, const View& v, double theta, long leaf_capacit
   }
   AMK_TRY(phase_begin(c, AMK_PHASE_BH_WALK));
   if (f32)
-    bh_walk_kernel<false, true><<<blocks, 32 * kWalkWarps, 0, c->stream>>>(t, info, pos, neg, theta2, fs, fo, status);
+    bh_walk_kernel<false, true><<<blocks, 32 * kWalkWarps, 0, c->stream>>>(t, rec, theta2, fs, fo, status);
   else
-    bh_walk_kernel<false, false><<<blocks, 32 * kWalkWarps, 0, c->stream>>>(t, info, pos, neg, theta2, fs, fo, status);
+    bh_walk_kernel<false, false><<<blocks, 32 * kWalkWarps, 0, c->stream>>>(t, rec, theta2, fs, fo, status);
   AMK_TRY(check_launch(c, "bh_walk_kernel"));
   if (po) {
     if (f32)
-      bh_walk_kernel<true, true><<<blocks, 32 * kWalkWarps, 0, c->stream>>>(t, info, pos, neg, theta2, fs, po, status);
+      bh_walk_kernel<true, true><<<blocks, 32 * kWalkWarps, 0, c->stream>>>(t, rec, theta2, fs, po, status);
     else
-      bh_walk_kernel<true, false><<<blocks, 32 * kWalkWarps, 0, c->stream>>>(t, info, pos, neg, theta2, fs, po, status);
+      bh_walk_kernel<true, false><<<blocks, 32 * kWalkWarps, 0, c->stream>>>(t, rec, theta2, fs, po, status);
     AMK_TRY(check_launch(c, "bh_walk_kernel"));
   }
   AMK_TRY(phase_end(c, AMK_PHASE_BH_WALK));
