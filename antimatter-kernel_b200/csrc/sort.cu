@@ -1,10 +1,16 @@
-// Stable LSD radix sort of (uint64 key, uint32 value) pairs, 8 bits per
-// pass: per-tile digit histograms -> one exclusive scan (digit-major, so the
-// result is stable across tiles) -> scatter with in-tile stable ranks from
-// warp match masks (the context's sort stages each tile in digit order in
-// shared memory first, so that a digit's writes are contiguous). HBM-bound:
-// each pass reads 12 B and writes 12 B per element plus the key read of the
-// histogram pass.
+// Stable sort of (uint64 key, uint32 value) pairs.
+//
+// Small sets (kRankMax): every key's rank by comparison with all keys, two
+// launches. Larger ones: LSD radix, 8 bits per pass, two launches per pass: a
+// histogram of each tile's digits, and a scatter whose blocks add up the
+// histograms before theirs (rows of tiles inside a group of 16, sums of whole
+// groups), rank their tile's elements by warp match masks and stage it in
+// digit order in shared memory, so that a digit's writes are contiguous. Each
+// pass reads 20 B and writes 12 B per element; up to a million keys all of it
+// stays in L2 and the launches and the dependent loads of a tile are what it
+// takes, so tiles shrink with n until they fill the chip. Past kMaxTiles tiles
+// (and in the allocation-free sort) the digit counters are scanned by kernels
+// of their own.
 #include <algorithm>
 
 #include "amk_internal.cuh"
@@ -19,10 +25,6 @@ constexpr int kWarps = kSortThreads / 32;
 // counters the one-CTA scan_kernel handles (64 per thread; the bound of the
 // allocation-free sort, which has no scratch for the multi-CTA scan)
 constexpr long kSingleScanCounters = 65536;
-// the context's sort scans more than this many counters (n > 32,768 keys)
-// with the multi-CTA scan: the one-CTA scan of 65,536 counters takes about
-// 100 us per pass, the multi-CTA one about 15 us
-constexpr long kCtxSingleScanCounters = 2048;
 
 __global__ void __launch_bounds__(kSortThreads)
 hist_kernel(const uint64_t* __restrict__ keys, long n, int shift, int nb, uint32_t* __restrict__ hist) {
@@ -110,48 +112,112 @@ scatter_kernel(const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vi
   }
 }
 
-// The same scatter with the tile staged in shared memory in digit order, so
-// that the global writes of one digit are contiguous. Warp w ranks the
-// contiguous chunk [w * kWarpChunk, (w + 1) * kWarpChunk) of the tile with
-// counters of its own (match masks per round, no block barrier), which keeps
-// the ranks stable; one block pass then turns the per-warp digit counts into
-// tile positions, the elements are placed in shared memory in sorted order
-// and written out in that order. Element j of the staged tile goes to
-// offs[d][tile] + j - (tile start of digit d).
-constexpr int kWarpChunk = kTile / kWarps;  // 512 consecutive elements per warp
-constexpr size_t kStagedSmem = static_cast<size_t>(kTile) * (sizeof(uint64_t) + sizeof(uint32_t)) +
-                               sizeof(uint32_t) * (kWarps * 256 + 256 + kWarps);
+// ---------------------------------------------------------------- radix, two launches per pass
+constexpr int kGroup = 16;         // tiles per group of the second level
+constexpr long kMaxTiles = 4096;   // 256 groups of 1 KB to add per block at most
 
+template <int kI>
+__global__ void __launch_bounds__(kSortThreads)
+tile_hist_kernel(const uint64_t* __restrict__ keys, long n, int shift, uint32_t* __restrict__ rows,
+                 uint32_t* __restrict__ groups) {
+  __shared__ uint32_t h[256];
+  h[threadIdx.x] = 0;
+  __syncthreads();
+  const long base = static_cast<long>(blockIdx.x) * (kSortThreads * kI);
+#pragma unroll
+  for (int k = 0; k < kI; ++k) {
+    const long i = base + k * kSortThreads + threadIdx.x;
+    if (i < n) atomicAdd(&h[(keys[i] >> shift) & 0xFF], 1u);
+  }
+  __syncthreads();
+  const uint32_t c = h[threadIdx.x];
+  rows[static_cast<size_t>(blockIdx.x) * 256 + threadIdx.x] = c;
+  if (c) atomicAdd(&groups[static_cast<size_t>(blockIdx.x / kGroup) * 256 + threadIdx.x], c);
+}
+
+// Sum over the block's warps before this one of a per-thread value's warp
+// total, plus the exclusive scan inside the warp: exclusive block scan.
+__device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t* wsum) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint32_t incl = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  __syncthreads();  // wsum is free
+  if (lane == 31) wsum[warp] = incl;
+  __syncthreads();
+  uint32_t before = 0;
+  for (int w = 0; w < warp; ++w) before += wsum[w];
+  return before + incl - v;
+}
+
+template <int kI>
+constexpr size_t staged_smem() {
+  return static_cast<size_t>(kSortThreads) * kI * (sizeof(uint64_t) + sizeof(uint32_t)) +
+         sizeof(uint32_t) * (kWarps * 256 + 256 + kWarps);
+}
+
+// offs (digit-major, scanned) gives digit d of this tile its first place, or
+// (offs null) the rows and groups of tile_hist_kernel do. Warp w ranks the
+// contiguous chunk w of the tile with counters of its own (match masks per
+// round, no block barrier), which keeps the ranks stable; one block pass then
+// turns the per-warp digit counts into tile positions, the elements are placed
+// in shared memory in sorted order and written out in that order. Element j of
+// the staged tile goes to first[d] + j - (tile start of digit d).
+template <int kI>
 __global__ void __launch_bounds__(kSortThreads)
 scatter_staged_kernel(const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin, long n, int shift,
-                      int nb, const uint32_t* __restrict__ offs, uint64_t* __restrict__ kout,
+                      int nb, const uint32_t* __restrict__ offs, const uint32_t* __restrict__ rows,
+                      const uint32_t* __restrict__ groups, uint64_t* __restrict__ kout,
                       uint32_t* __restrict__ vout) {
+  constexpr int kT = kSortThreads * kI, kChunk = kT / kWarps;
   extern __shared__ __align__(16) unsigned char sort_smem[];
   uint64_t* sk = reinterpret_cast<uint64_t*>(sort_smem);
-  uint32_t* sv = reinterpret_cast<uint32_t*>(sk + kTile);
-  uint32_t* wc = sv + kTile;                 // [kWarps][256]: counts, then tile positions
-  uint32_t* dstart = wc + kWarps * 256;      // [256]
-  uint32_t* wsum = dstart + 256;             // [kWarps]
+  uint32_t* sv = reinterpret_cast<uint32_t*>(sk + kT);
+  uint32_t* wc = sv + kT;                    // [kWarps][256]: counts, then tile positions
+  uint32_t* first = wc + kWarps * 256;       // [256]: place of digit d minus its tile start
+  uint32_t* wsum = first + 256;              // [kWarps]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long base = static_cast<long>(blockIdx.x) * kTile;
-  const long wbase = base + static_cast<long>(warp) * kWarpChunk;
+  const long base = static_cast<long>(blockIdx.x) * kT;
+  const long wbase = base + static_cast<long>(warp) * kChunk;
   const uint32_t lt_mask = (1u << lane) - 1u;
   uint32_t* mine = wc + warp * 256;
-  for (int d = lane; d < 256; d += 32) mine[d] = 0;
-  __syncwarp();
-  uint64_t key[kItems];
-  uint32_t val[kItems], dr[kItems];  // dr: digit | rank in the warp's chunk << 8
+  uint64_t key[kI];
+  uint32_t val[kI], dr[kI];  // dr: digit | rank in the warp's chunk << 8
 #pragma unroll
-  for (int k = 0; k < kItems; ++k) {
+  for (int k = 0; k < kI; ++k) {
     const long i = wbase + k * 32 + lane;
-    const bool valid = i < n;
-    key[k] = 0;
-    val[k] = 0;
+    key[k] = i < n ? kin[i] : 0;
+    val[k] = i < n ? vin[i] : 0;
+  }
+  for (int d = lane; d < 256; d += 32) mine[d] = 0;
+  // digit d = thread d: its place in the output before this tile
+  uint32_t place;
+  if (offs) {
+    place = offs[static_cast<size_t>(threadIdx.x) * nb + blockIdx.x];
+  } else {
+    const int my = blockIdx.x / kGroup, n_groups = (nb + kGroup - 1) / kGroup;
+    uint32_t before = 0, total = 0;
+#pragma unroll 8
+    for (int g = 0; g < n_groups; ++g) {
+      const uint32_t c = groups[static_cast<size_t>(g) * 256 + threadIdx.x];
+      total += c;
+      if (g < my) before += c;
+    }
+#pragma unroll 8
+    for (int r = my * kGroup; r < static_cast<int>(blockIdx.x); ++r)
+      before += rows[static_cast<size_t>(r) * 256 + threadIdx.x];
+    place = block_exclusive(total, wsum) + before;
+  }
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < kI; ++k) {
+    const bool valid = wbase + k * 32 + lane < n;
     dr[k] = 0;
     const uint32_t active = __ballot_sync(0xffffffffu, valid);
     if (valid) {
-      key[k] = kin[i];
-      val[k] = vin[i];
       const int d = static_cast<int>((key[k] >> shift) & 0xFF);
       const uint32_t peers = __match_any_sync(active, d);
       const int leader = __ffs(peers) - 1;
@@ -173,85 +239,149 @@ scatter_staged_kernel(const uint64_t* __restrict__ kin, const uint32_t* __restri
       wc[w * 256 + d] = run;
       run += c;
     }
-    uint32_t incl = run;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += t;
-    }
-    if (lane == 31) wsum[warp] = incl;
-    __syncthreads();
-    uint32_t before = 0;
-    for (int w = 0; w < warp; ++w) before += wsum[w];
-    const uint32_t start = before + incl - run;
-    dstart[d] = start;
+    const uint32_t start = block_exclusive(run, wsum);
+    first[d] = place - start;
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) wc[w * 256 + d] += start;
   }
   __syncthreads();
 #pragma unroll
-  for (int k = 0; k < kItems; ++k) {
-    const long i = wbase + k * 32 + lane;
-    if (i < n) {
+  for (int k = 0; k < kI; ++k) {
+    if (wbase + k * 32 + lane < n) {
       const uint32_t pos = mine[dr[k] & 0xFF] + (dr[k] >> 8);
       sk[pos] = key[k];
       sv[pos] = val[k];
     }
   }
   __syncthreads();
-  const int tile_n = static_cast<int>(min(static_cast<long>(kTile), n - base));
+  const int tile_n = static_cast<int>(min(static_cast<long>(kT), n - base));
+#pragma unroll 4
   for (int j = threadIdx.x; j < tile_n; j += kSortThreads) {
     const uint64_t kk = sk[j];
-    const int d = static_cast<int>((kk >> shift) & 0xFF);
-    const long pos = static_cast<long>(offs[static_cast<long>(d) * nb + blockIdx.x]) + (j - dstart[d]);
+    const uint32_t pos = first[(kk >> shift) & 0xFF] + static_cast<uint32_t>(j);
     kout[pos] = kk;
     vout[pos] = sv[j];
   }
 }
 
+// ---------------------------------------------------------------- ranks
+// Up to this many keys the comparisons are cheaper than the passes: us per
+// 63-bit sort, ranks / 8 passes: 500 keys 19 / 93, 5,000 29 / 88, 12,000
+// 51 / 100, 16,384 73 / 104, 20,000 98 / 102, 32,768 205 / 102. (With five
+// launches per pass 210 us at 30,000 and 288 us at 524,309 keys, where the
+// two-launch passes take 103 and 165.)
+constexpr long kRankMax = 16384;
+constexpr int kRankSeg = 1024;  // keys a block compares its 256 elements with
+
+// rank[i] += keys of segment blockIdx.y before key i (ties by index)
+__global__ void __launch_bounds__(kSortThreads)
+rank_kernel(const uint64_t* __restrict__ keys, int n, uint64_t mask, int* __restrict__ rank) {
+  __shared__ uint64_t s[kRankSeg];
+  const int j0 = blockIdx.y * kRankSeg, cnt = min(kRankSeg, n - j0);
+  for (int j = threadIdx.x; j < cnt; j += kSortThreads) s[j] = keys[j0 + j] & mask;
+  __syncthreads();
+  const int i = blockIdx.x * kSortThreads + threadIdx.x;
+  if (i >= n) return;
+  const uint64_t k = keys[i] & mask;
+  int r = 0;
+  if (j0 + cnt <= static_cast<int>(blockIdx.x) * kSortThreads) {  // all before: ties count
+#pragma unroll 8
+    for (int j = 0; j < cnt; ++j) r += s[j] <= k ? 1 : 0;
+  } else if (j0 > i) {  // all after
+#pragma unroll 8
+    for (int j = 0; j < cnt; ++j) r += s[j] < k ? 1 : 0;
+  } else {
+#pragma unroll 8
+    for (int j = 0; j < cnt; ++j) r += s[j] < k || (s[j] == k && j0 + j < i) ? 1 : 0;
+  }
+  if (r) atomicAdd(rank + i, r);
+}
+
+__global__ void rank_scatter_kernel(const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin, int n,
+                                    const int* __restrict__ rank, uint64_t* __restrict__ kout,
+                                    uint32_t* __restrict__ vout) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  kout[rank[i]] = kin[i];
+  vout[rank[i]] = vin[i];
+}
+
 }  // namespace
 
-int radix_sort_pairs(amk_ctx* c, const uint64_t* keys_in, const uint32_t* vals_in, uint64_t* keys_out,
-                     uint32_t* vals_out, long n, int key_bits) {
-  if (n <= 0) return AMK_OK;
-  if (n > 0xFFFFFFF0L) return fail(AMK_ERR_LIMIT, "radix sort of %ld elements exceeds 32-bit ranks", n);
-  const int passes = std::max(1, (key_bits + 7) / 8);
-  const int nb = static_cast<int>((n + kTile - 1) / kTile);
+namespace {
+
+template <int kI>
+int radix_passes(amk_ctx* c, const uint64_t* ksrc, const uint32_t* vsrc, uint64_t* keys_out, uint32_t* vals_out,
+                 uint64_t* kt, uint32_t* vt, long n, int passes) {
+  const int nb = static_cast<int>((n + kSortThreads * kI - 1) / (kSortThreads * kI));
+  const bool own = nb <= kMaxTiles;
+  const size_t n_groups = static_cast<size_t>((nb + kGroup - 1) / kGroup);
   int rc = AMK_OK;
-  uint64_t* kt = slot<uint64_t>(c, kSlotKeysB, static_cast<size_t>(n), &rc);
+  // rows (or digit-major counters), then the groups of every pass
+  uint32_t* rows = slot<uint32_t>(c, kSlotSortHist, 256 * (static_cast<size_t>(nb) + (own ? passes * n_groups : 0)), &rc);
   AMK_TRY(rc);
-  uint32_t* vt = slot<uint32_t>(c, kSlotValsB, static_cast<size_t>(n), &rc);
-  AMK_TRY(rc);
-  uint32_t* hist = slot<uint32_t>(c, kSlotSortHist, static_cast<size_t>(256) * nb, &rc);
-  AMK_TRY(rc);
+  uint32_t* groups = rows + 256 * static_cast<size_t>(nb);
   int* total = slot<int>(c, kSlotSortFlags, 8, &rc);
   AMK_TRY(rc);
-  // the staged scatter's shared memory is above the 48 KB default (set per call: per device)
-  AMK_CUDA_TRY(cudaFuncSetAttribute(scatter_staged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(kStagedSmem)));
-  const uint64_t* ksrc = keys_in;
-  const uint32_t* vsrc = vals_in;
+  // the staged scatter's shared memory may be above the 48 KB default (set per call: per device)
+  AMK_CUDA_TRY(cudaFuncSetAttribute(scatter_staged_kernel<kI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    static_cast<int>(staged_smem<kI>())));
+  if (own) AMK_CUDA_TRY(cudaMemsetAsync(groups, 0, 256 * sizeof(uint32_t) * passes * n_groups, c->stream));
   for (int p = 0; p < passes; ++p) {
     const bool to_out = ((passes - 1 - p) % 2) == 0;
     uint64_t* kdst = to_out ? keys_out : kt;
     uint32_t* vdst = to_out ? vals_out : vt;
     const int shift = 8 * p;
-    hist_kernel<<<nb, kSortThreads, 0, c->stream>>>(ksrc, n, shift, nb, hist);
-    AMK_TRY(check_launch(c, "hist_kernel"));
-    if (static_cast<long>(256) * nb > kCtxSingleScanCounters) {
-      // many tiles: the multi-CTA scan (in place; counts stay below 2^31)
-      AMK_TRY(exclusive_scan_int(c, reinterpret_cast<const int*>(hist), static_cast<long>(256) * nb,
-                                 reinterpret_cast<int*>(hist), total));
+    uint32_t* gp = groups + 256 * n_groups * p;
+    if (own) {
+      tile_hist_kernel<kI><<<nb, kSortThreads, 0, c->stream>>>(ksrc, n, shift, rows, gp);
+      AMK_TRY(check_launch(c, "tile_hist_kernel"));
     } else {
-      scan_kernel<<<1, 1024, 0, c->stream>>>(hist, static_cast<long>(256) * nb);
-      AMK_TRY(check_launch(c, "scan_kernel"));
+      hist_kernel<<<nb, kSortThreads, 0, c->stream>>>(ksrc, n, shift, nb, rows);  // kItems = the largest kI
+      AMK_TRY(check_launch(c, "hist_kernel"));
+      // in place; counts stay below 2^31
+      AMK_TRY(exclusive_scan_int(c, reinterpret_cast<const int*>(rows), static_cast<long>(256) * nb,
+                                 reinterpret_cast<int*>(rows), total));
     }
-    scatter_staged_kernel<<<nb, kSortThreads, kStagedSmem, c->stream>>>(ksrc, vsrc, n, shift, nb, hist, kdst, vdst);
+    scatter_staged_kernel<kI><<<nb, kSortThreads, staged_smem<kI>(), c->stream>>>(
+        ksrc, vsrc, n, shift, nb, own ? nullptr : rows, rows, gp, kdst, vdst);
     AMK_TRY(check_launch(c, "scatter_staged_kernel"));
     ksrc = kdst;
     vsrc = vdst;
   }
   return AMK_OK;
+}
+
+}  // namespace
+
+// Tiles of 1,024 keys up to 150,000 (147 of them: one per SM), 2,048 up to
+// 600,000, 4,096 above.
+int radix_sort_pairs(amk_ctx* c, const uint64_t* keys_in, const uint32_t* vals_in, uint64_t* keys_out,
+                     uint32_t* vals_out, long n, int key_bits) {
+  if (n <= 0) return AMK_OK;
+  if (n > 0xFFFFFFF0L) return fail(AMK_ERR_LIMIT, "radix sort of %ld elements exceeds 32-bit ranks", n);
+  const int passes = std::max(1, (key_bits + 7) / 8);
+  int rc = AMK_OK;
+  if (n <= kRankMax) {
+    int* rank = slot<int>(c, kSlotValsB, static_cast<size_t>(n), &rc);
+    AMK_TRY(rc);
+    const uint64_t mask = passes >= 8 ? ~0ull : (1ull << (8 * passes)) - 1ull;
+    const unsigned gb = static_cast<unsigned>((n + kSortThreads - 1) / kSortThreads);
+    AMK_CUDA_TRY(cudaMemsetAsync(rank, 0, static_cast<size_t>(n) * sizeof(int), c->stream));
+    rank_kernel<<<dim3(gb, static_cast<unsigned>((n + kRankSeg - 1) / kRankSeg)), kSortThreads, 0, c->stream>>>(
+        keys_in, static_cast<int>(n), mask, rank);
+    AMK_TRY(check_launch(c, "rank_kernel"));
+    rank_scatter_kernel<<<gb, kSortThreads, 0, c->stream>>>(keys_in, vals_in, static_cast<int>(n), rank, keys_out,
+                                                            vals_out);
+    return check_launch(c, "rank_scatter_kernel");
+  }
+  uint64_t* kt = slot<uint64_t>(c, kSlotKeysB, static_cast<size_t>(n), &rc);
+  AMK_TRY(rc);
+  uint32_t* vt = slot<uint32_t>(c, kSlotValsB, static_cast<size_t>(n), &rc);
+  AMK_TRY(rc);
+  if (n <= 150000) return radix_passes<4>(c, keys_in, vals_in, keys_out, vals_out, kt, vt, n, passes);
+  if (n <= 600000) return radix_passes<8>(c, keys_in, vals_in, keys_out, vals_out, kt, vt, n, passes);
+  return radix_passes<16>(c, keys_in, vals_in, keys_out, vals_out, kt, vt, n, passes);
 }
 
 }  // namespace amk
