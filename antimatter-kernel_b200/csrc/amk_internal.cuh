@@ -213,6 +213,8 @@ enum ScratchSlot {
   kSlotFmmCell,
   kSlotM2lRank,
   kSlotM2lClassKey,
+  kSlotFmmArrived,
+  kSlotFmmFamily,
   kNumSlots
 };
 static_assert(kNumSlots <= 128, "scratch slots");

@@ -66,8 +66,7 @@ struct FmmHostTables {
   std::vector<int> rec_axis;                 // per k
   std::vector<int> rec_delta, rec_m1, rec_m2;  // 3 per k
   std::vector<short> m2l_index_t;            // [a * n_m + g]
-  std::vector<int> m2m_off, m2m_b, m2m_c;    // CSR by a
-  std::vector<int> l2l_off, l2l_b, l2l_c;    // CSR by a
+  std::vector<short> prev, next;             // [axis * n_m + a]: a - e_axis, a + e_axis (-1: none)
   std::vector<int> grad;                     // 3 per g, -1 none
   // Harmonic basis of the FP64 M2L products (see m2l_class_mma_kernel): the
   // n_r = (p+1)^2 coefficients with z exponent 0 or 1, the derivatives with
@@ -129,28 +128,15 @@ struct FmmHostTables {
         const int s3[3] = {multi[g].x + multi[a].x, multi[g].y + multi[a].y, multi[g].z + multi[a].z};
         m2l_index_t[static_cast<size_t>(a) * n_m + g] = static_cast<short>(pos(s3));
       }
-    // M2M (child -> parent): M_a += M_b * d^(a-b) / (a-b)! over b <= a;
-    // L2L (parent -> child): L_a += L_b * (b!/a!) d^(b-a) / (b-a)! over b >= a
-    // with |b| <= p. Both enumerated componentwise.
-    m2m_off.push_back(0);
-    l2l_off.push_back(0);
-    for (int a = 0; a < n_m; ++a) {
-      const int4 ma = multi[a];
-      for (int b0 = 0; b0 <= ma.x; ++b0)
-        for (int b1 = 0; b1 <= ma.y; ++b1)
-          for (int b2 = 0; b2 <= ma.z; ++b2) {
-            m2m_b.push_back(graded_index(b0, b1, b2));
-            m2m_c.push_back(graded_index(ma.x - b0, ma.y - b1, ma.z - b2));
-          }
-      m2m_off.push_back(static_cast<int>(m2m_b.size()));
-      for (int c = 0; c < n_m; ++c) {
-        const int4 mc = multi[c];
-        if (ma.w + mc.w > p) break;  // graded order: every later c has a higher degree
-        l2l_b.push_back(graded_index(ma.x + mc.x, ma.y + mc.y, ma.z + mc.z));
-        l2l_c.push_back(c);
+    // neighbours along the axes: the one-axis shifts of M2M and L2L walk them
+    for (int k = 0; k < 3; ++k)
+      for (int a = 0; a < n_m; ++a) {
+        int t[3] = {multi[a].x, multi[a].y, multi[a].z};
+        t[k] -= 1;
+        prev.push_back(static_cast<short>(pos(t)));
+        t[k] += 2;
+        next.push_back(static_cast<short>(multi[a].w < p ? pos(t) : -1));
       }
-      l2l_off.push_back(static_cast<int>(l2l_b.size()));
-    }
     // gradient of the local expansion: d/dx_k of x^g is g_k x^(g - e_k)
     grad.assign(3 * n_m, -1);
     for (int g = 0; g < n_m; ++g) {
@@ -254,12 +240,8 @@ struct FmmDevTables {
   const int* ex_off;
   const int* ex_r;
   const double* ex_c;
-  const int* m2m_off;
-  const int* m2m_b;
-  const int* m2m_c;
-  const int* l2l_off;
-  const int* l2l_b;
-  const int* l2l_c;
+  const short* prev;
+  const short* next;
   const int* grad;
 };
 
@@ -307,7 +289,6 @@ struct Fmm {
 namespace {
 
 constexpr int kMaxOrder = 8;
-constexpr int kMaxNm = 165;  // n_m(8)
 constexpr int kFmmWarps = 4;
 
 template <typename T>
@@ -331,9 +312,8 @@ int get_tables(amk_ctx* c, int order, FmmDevTables* out) {
   const size_t o_multi = append(blob, h.multi), o_fact = append(blob, h.fact), o_if = append(blob, h.inv_fact),
                o_sign = append(blob, h.sign), o_ds = append(blob, h.deg_start), o_ax = append(blob, h.rec_axis),
                o_de = append(blob, h.rec_delta), o_m1 = append(blob, h.rec_m1), o_m2 = append(blob, h.rec_m2),
-               o_idt = append(blob, h.m2l_index_t), o_mo = append(blob, h.m2m_off), o_mb = append(blob, h.m2m_b),
-               o_mc = append(blob, h.m2m_c), o_lo = append(blob, h.l2l_off), o_lb = append(blob, h.l2l_b),
-               o_lc = append(blob, h.l2l_c), o_g = append(blob, h.grad), o_ds2 = append(blob, h.deg_start2),
+               o_idt = append(blob, h.m2l_index_t), o_pv = append(blob, h.prev), o_nx = append(blob, h.next),
+               o_g = append(blob, h.grad), o_ds2 = append(blob, h.deg_start2),
                o_ax2 = append(blob, h.rec_axis2), o_de2 = append(blob, h.rec_delta2), o_m12 = append(blob, h.rec_m12),
                o_m22 = append(blob, h.rec_m22), o_rit = append(blob, h.red_index_t), o_rdeg = append(blob, h.red_deg),
                o_rdo = append(blob, h.rd_off), o_rda = append(blob, h.rd_a), o_rdc = append(blob, h.rd_c),
@@ -368,12 +348,8 @@ int get_tables(amk_ctx* c, int order, FmmDevTables* out) {
   t.ex_r = ints(o_exr);
   t.ex_c = reinterpret_cast<const double*>(b + o_exc);
   t.m2l_index_t = reinterpret_cast<const short*>(b + o_idt);
-  t.m2m_off = reinterpret_cast<const int*>(b + o_mo);
-  t.m2m_b = reinterpret_cast<const int*>(b + o_mb);
-  t.m2m_c = reinterpret_cast<const int*>(b + o_mc);
-  t.l2l_off = reinterpret_cast<const int*>(b + o_lo);
-  t.l2l_b = reinterpret_cast<const int*>(b + o_lb);
-  t.l2l_c = reinterpret_cast<const int*>(b + o_lc);
+  t.prev = reinterpret_cast<const short*>(b + o_pv);
+  t.next = reinterpret_cast<const short*>(b + o_nx);
   t.grad = reinterpret_cast<const int*>(b + o_g);
   c->fmm->tables[order] = {buf, t};
   *out = t;
@@ -392,137 +368,264 @@ __device__ __forceinline__ void powers(int p, double x, double y, double z, doub
 }
 
 // ------------------------------------------------------------ radii
-__global__ void fmm_leaf_radius_kernel(const Octree t, double* __restrict__ radius) {
-  const int id = blockIdx.x * blockDim.x + threadIdx.x;
-  if (id >= t.n_nodes || !t.meta[id].y) return;
+// One launch from the leaves to the root: eight lanes per leaf take its
+// particles, then the group whose child arrives last at a parent takes the
+// parent, a lane per child; no group waits for another. A launch per level
+// over all nodes spent its time on launches and empty threads (262k
+// particles, 9 levels, leaves included: 98 -> 27 us). Also counts the internal nodes of every depth.
+__global__ void __launch_bounds__(256)
+fmm_radius_kernel(const Octree t, double* __restrict__ radius, int* __restrict__ arrived,
+                  int* __restrict__ level_count) {
+  __shared__ int hist[32];
+  if (threadIdx.x < 32) hist[threadIdx.x] = 0;
+  __syncthreads();
+  const int id = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+  const int sub = threadIdx.x & 7;
+  const unsigned group = 0xffu << (threadIdx.x & 24);
+  bool leaf = false;
+  if (id < t.n_nodes) {
+    const uchar2 mt = t.meta[id];
+    leaf = mt.y;
+    if (!leaf && sub == 0) atomicAdd(&hist[mt.x], 1);
+  }
+  __syncthreads();
+  if (threadIdx.x < 32 && hist[threadIdx.x] > 0) atomicAdd(&level_count[threadIdx.x], hist[threadIdx.x]);
+  if (!leaf) return;
+  auto dist2 = [](const double4& a, const double4& b) {
+    const double dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
+    return __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+  };
+  auto group_max = [&](double v) {
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(group, v, o));
+    return v;
+  };
   const double4 c = t.center[id];
   const int2 r = t.range[id];
   double r2 = 0.0;
-  for (int k = r.x; k < r.y; ++k) {
-    const double4 s = t.src[k];
-    const double dx = s.x - c.x, dy = s.y - c.y, dz = s.z - c.z;
-    r2 = fmax(r2, __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)));
+  for (int k = r.x + sub; k < r.y; k += 8) r2 = fmax(r2, dist2(t.src[k], c));
+  double rad = sqrt(group_max(r2));
+  for (int node = id;;) {
+    if (sub == 0) radius[node] = rad;
+    const int par = t.parent[node];
+    if (par < 0) return;
+    const int ch = t.child[8 * par + sub];
+    const int children = __popc(__ballot_sync(group, ch >= 0) & group);
+    int last = 0;
+    if (sub == 0) {
+      __threadfence();
+      last = atomicAdd(&arrived[par], 1) == children - 1;
+      __threadfence();
+    }
+    __syncwarp(group);
+    if (!__shfl_sync(group, last, 0, 8)) return;
+    double v = 0.0;
+    if (ch >= 0) v = sqrt(dist2(t.center[ch], t.center[par])) + __ldcg(&radius[ch]);
+    rad = group_max(v);
+    node = par;
   }
-  radius[id] = sqrt(r2);
-}
-
-__global__ void fmm_parent_radius_kernel(const Octree t, int depth, double* __restrict__ radius) {
-  const int id = blockIdx.x * blockDim.x + threadIdx.x;
-  if (id >= t.n_nodes) return;
-  const uchar2 mt = t.meta[id];
-  if (mt.y || mt.x != depth) return;
-  const double4 c = t.center[id];
-  double r = 0.0;
-  for (int o = 0; o < 8; ++o) {
-    const int ch = t.child[8 * id + o];
-    if (ch < 0) continue;
-    const double4 cc = t.center[ch];
-    const double dx = cc.x - c.x, dy = cc.y - c.y, dz = cc.z - c.z;
-    r = fmax(r, sqrt(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz))) + radius[ch]);
-  }
-  radius[id] = r;
 }
 
 // ------------------------------------------------------------ P2M, M2M
+// One launch from the leaves to the root: a warp per leaf forms its
+// multipole, then the warp whose child arrives last at a parent shifts the
+// children's multipoles there (in octant order, so the sum does not depend on
+// which warp it is); no warp waits for another.
+//
 // P2M (fast-multipole.cc:443-461): M_a = sum_j q_j d_j^a / a!, d_j = x_j - c.
-// A warp per leaf; lanes over particles (up to kP2mPer per lane per round).
-// The multi-indices a are visited in the lexicographic order of three
-// nested loops with running powers, so each monomial of each particle costs
-// one multiply; the lanes' partial sums of a coefficient are added by a
-// shuffle tree (fixed order: run-to-run deterministic) and lane 0 keeps the
-// leaf's sums in shared memory across rounds.
-constexpr int kP2mPer = 4;
+// Lanes over particles (U per lane and round). The multi-indices a are
+// visited in the lexicographic order of three nested loops with running
+// powers, so each monomial of each particle costs one multiply; the lanes'
+// terms of 32 coefficients go through a transposed block of shared memory and
+// each lane sums one row (a shuffle tree per coefficient took ten shuffles
+// for each).
+//
+// M2M (fast-multipole.cc:463-482): M_a += M_b d^(a-b) / (a-b)!. The shift is
+// a product of one-axis shifts and siblings share their offsets per axis, so
+// the eight children are shifted along x and added in pairs, the four sums
+// along y, the two along z: 14 one-axis shifts of C(p+4,4) terms instead of 8
+// shifts of C(p+6,6) (order 7: 4,620 terms for 13,728), from shared memory.
+// Measured, P2M + M2M (serialised): order 4, 262k: 402 -> 185 us; order 6,
+// 1M: 1756 -> 745 us; order 7, 1M, 128 per leaf: 1178 -> 451 us.
+constexpr int kPow = kMaxOrder + 1;
 
-__global__ void __launch_bounds__(32 * kFmmWarps)
-fmm_p2m_kernel(const Octree t, FmmDevTables T, double* __restrict__ M) {
-  __shared__ double acc_s[kFmmWarps][kMaxNm];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int id = blockIdx.x * kFmmWarps + w;
-  if (id >= t.n_nodes || !t.meta[id].y) return;
-  const double4 c = t.center[id];
-  const int2 r = t.range[id];
-  const int P = T.p;
-  double* acc = acc_s[w];
-  for (int a = lane; a < T.n_m; a += 32) acc[a] = 0.0;
-  __syncwarp();
-  for (int r0 = r.x; r0 < r.y; r0 += 32 * kP2mPer) {
-    double dx[kP2mPer], dy[kP2mPer], dz[kP2mPer], qx[kP2mPer];
-#pragma unroll
-    for (int u = 0; u < kP2mPer; ++u) {
-      const int k = r0 + lane + 32 * u;
-      const double4 s = k < r.y ? t.src[k] : make_double4(c.x, c.y, c.z, 0.0);
-      dx[u] = s.x - c.x;
-      dy[u] = s.y - c.y;
-      dz[u] = s.z - c.z;
-      qx[u] = s.w;  // q x^i, running
-    }
-    for (int i = 0; i <= P; ++i) {
-      double qy[kP2mPer];
-#pragma unroll
-      for (int u = 0; u < kP2mPer; ++u) qy[u] = qx[u];  // q x^i y^j, running
-      for (int j = 0; i + j <= P; ++j) {
-        double m[kP2mPer];
-#pragma unroll
-        for (int u = 0; u < kP2mPer; ++u) m[u] = qy[u];  // q x^i y^j z^k, running
-        for (int k = 0; i + j + k <= P; ++k) {
-          double v = 0.0;
-#pragma unroll
-          for (int u = 0; u < kP2mPer; ++u) {
-            v += m[u];
-            m[u] *= dz[u];
-          }
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-          if (lane == 0) acc[graded_index(i, j, k)] += v;
-        }
-#pragma unroll
-        for (int u = 0; u < kP2mPer; ++u) qy[u] *= dy[u];
-      }
-#pragma unroll
-      for (int u = 0; u < kP2mPer; ++u) qx[u] *= dx[u];
-    }
-  }
-  __syncwarp();
-  for (int a = lane; a < T.n_m; a += 32) M[static_cast<size_t>(id) * T.n_m + a] = acc[a] * T.inv_fact[a];
+// doubles of shared memory per warp
+__host__ __device__ constexpr int up_smem(int n_m) {
+  const int p2m = 32 * 33 + n_m, m2m = 12 * n_m + 6 * kPow;
+  return p2m > m2m ? p2m : m2m;
 }
+__host__ __device__ constexpr int down_smem(int n_m) { return 7 * n_m + 6 * kPow; }
 
-// M2M for parents at `depth` (fast-multipole.cc:463-482). A warp per
-// parent, lanes over the parent's coefficients; per child the lanes first
-// write the offset's monomials d^c / c! (c over all multi-indices) into
-// shared memory, then each term of coefficient a is one product
-// M_child[b] * mono[a - b] with b and a - b from the table.
-__global__ void __launch_bounds__(32 * kFmmWarps)
-fmm_m2m_kernel(const Octree t, FmmDevTables T, int depth, double* __restrict__ M) {
-  __shared__ double mono_s[kFmmWarps][kMaxNm];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int id = blockIdx.x * kFmmWarps + w;
-  if (id >= t.n_nodes) return;
-  const uchar2 mt = t.meta[id];
-  if (mt.y || mt.x != depth) return;
-  const double4 c = t.center[id];
-  double* mono = mono_s[w];
-  double acc[(kMaxNm + 31) / 32];
-  for (int u = 0; u < (kMaxNm + 31) / 32; ++u) acc[u] = 0.0;
-  double px[kMaxOrder + 1], py[kMaxOrder + 1], pz[kMaxOrder + 1];
-  for (int o = 0; o < 8; ++o) {
-    const int ch = t.child[8 * id + o];
-    if (ch < 0) continue;
-    const double4 cc = t.center[ch];
-    powers(T.p, cc.x - c.x, cc.y - c.y, cc.z - c.z, px, py, pz);
-    __syncwarp();  // the previous child's monomials are no longer read
-    for (int a = lane; a < T.n_m; a += 32) {
-      const int4 m = T.multi[a];
-      mono[a] = (px[m.x] * py[m.y] * pz[m.z]) * T.inv_fact[a];
+template <int U>
+__device__ __forceinline__ void p2m_round(const Octree& t, const double4& c, int r0, int r1, int P, int lane,
+                                          double* __restrict__ rows, double* __restrict__ acc) {
+  double dx[U], dy[U], dz[U], qx[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int k = r0 + lane + 32 * u;
+    const double4 s = k < r1 ? t.src[k] : make_double4(c.x, c.y, c.z, 0.0);
+    dx[u] = s.x - c.x;
+    dy[u] = s.y - c.y;
+    dz[u] = s.z - c.z;
+    qx[u] = s.w;  // q x^i, running
+  }
+  const int n_lanes = min(32, r1 - r0);
+  int row = 0, mine = 0;
+  auto sum_rows = [&](int n_rows) {
+    __syncwarp();
+    if (lane < n_rows) {
+      double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+      for (int l = 0; l < n_lanes; l += 4) {  // lanes past the particles hold zeros
+        s0 += rows[lane * 33 + l];
+        s1 += rows[lane * 33 + l + 1];
+        s2 += rows[lane * 33 + l + 2];
+        s3 += rows[lane * 33 + l + 3];
+      }
+      acc[mine] += (s0 + s1) + (s2 + s3);
     }
     __syncwarp();
-    const double* mc = M + static_cast<size_t>(ch) * T.n_m;
-    for (int u = 0, a = lane; a < T.n_m; ++u, a += 32) {
-      double s = acc[u];
-      for (int e = T.m2m_off[a]; e < T.m2m_off[a + 1]; ++e) s += mc[T.m2m_b[e]] * mono[T.m2m_c[e]];
-      acc[u] = s;
+  };
+  for (int i = 0; i <= P; ++i) {
+    double qy[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) qy[u] = qx[u];  // q x^i y^j, running
+    for (int j = 0; i + j <= P; ++j) {
+      double m[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) m[u] = qy[u];  // q x^i y^j z^k, running
+      for (int k = 0; i + j + k <= P; ++k) {
+        double v = 0.0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          v += m[u];
+          m[u] *= dz[u];
+        }
+        rows[row * 33 + lane] = v;
+        if (lane == row) mine = graded_index(i, j, k);
+        if (++row == 32) {
+          sum_rows(32);
+          row = 0;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) qy[u] *= dy[u];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) qx[u] *= dx[u];
+  }
+  if (row > 0) sum_rows(row);
+}
+
+// pw[(2 axis + bit) * kPow + k] = d^k / k!, d the offset along the axis of
+// the children of `id` whose octant has that bit (siblings' centres agree).
+// ch: the child of octant `lane` (lanes 0-7), -1 none.
+__device__ __forceinline__ void child_powers(const Octree& t, const FmmDevTables& T, int id, int ch, int lane,
+                                             double* __restrict__ pw) {
+  const unsigned present = __ballot_sync(0xffffffffu, ch >= 0);
+  const double4 c = t.center[id], cc = ch >= 0 ? t.center[ch] : c;
+  const int axis = min(lane >> 1, 2);
+  const unsigned upper = axis == 0 ? 0xAAu : axis == 1 ? 0xCCu : 0xF0u;
+  const unsigned m = present & ((lane & 1) ? upper : ~upper);
+  const int from = m ? __ffs(m) - 1 : 8;  // lane 8 has no child: offset 0
+  const double dx = __shfl_sync(0xffffffffu, cc.x - c.x, from);
+  const double dy = __shfl_sync(0xffffffffu, cc.y - c.y, from);
+  const double dz = __shfl_sync(0xffffffffu, cc.z - c.z, from);
+  if (lane < 6) {
+    const double d = axis == 0 ? dx : axis == 1 ? dy : dz;
+    double v = 1.0;
+    for (int k = 0; k <= T.p; ++k) {
+      pw[lane * kPow + k] = v * T.inv_fact[graded_index(k, 0, 0)];
+      v *= d;
     }
   }
-  for (int u = 0, a = lane; a < T.n_m; ++u, a += 32) M[static_cast<size_t>(id) * T.n_m + a] = acc[u];
+}
+
+// out_q = the pair (in_2q, in_2q+1) shifted along one axis and added, N pairs
+// of n_m coefficients each, walking a - e, a - 2 e, ... by `prev`.
+template <int N, typename Out>
+__device__ __forceinline__ void m2m_axis(const short* __restrict__ prev, const double* __restrict__ pw, int n_m,
+                                         int lane, const double* __restrict__ in, Out out) {
+  for (int a = lane; a < n_m; a += 32) {
+    double s[N];
+#pragma unroll
+    for (int q = 0; q < N; ++q) s[q] = 0.0;
+    for (int i = a, k = 0; i >= 0; i = prev[i], ++k) {
+      const double p0 = pw[k], p1 = pw[kPow + k];
+#pragma unroll
+      for (int q = 0; q < N; ++q) s[q] += in[2 * q * n_m + i] * p0 + in[(2 * q + 1) * n_m + i] * p1;
+    }
+#pragma unroll
+    for (int q = 0; q < N; ++q) out(q, a, s[q]);
+  }
+}
+
+__global__ void __launch_bounds__(32 * kFmmWarps)
+fmm_up_kernel(const Octree t, FmmDevTables T, int* __restrict__ arrived, double* __restrict__ M) {
+  extern __shared__ __align__(16) unsigned char up_sm[];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int n_m = T.n_m;
+  double* sm = reinterpret_cast<double*>(up_sm) + w * up_smem(n_m);
+  short* prev = reinterpret_cast<short*>(reinterpret_cast<double*>(up_sm) + kFmmWarps * up_smem(n_m));
+  for (int i = threadIdx.x; i < 3 * n_m; i += blockDim.x) prev[i] = T.prev[i];
+  __syncthreads();
+  const int id = blockIdx.x * kFmmWarps + w;
+  if (id >= t.n_nodes || !t.meta[id].y) return;
+  {  // P2M
+    const double4 c = t.center[id];
+    const int2 r = t.range[id];
+    double* acc = sm + 32 * 33;
+    for (int a = lane; a < n_m; a += 32) acc[a] = 0.0;
+    __syncwarp();
+    for (int r0 = r.x; r0 < r.y;) {
+      const int rem = r.y - r0;
+      if (rem > 64) {
+        p2m_round<4>(t, c, r0, r.y, T.p, lane, sm, acc);
+        r0 += 128;
+      } else if (rem > 32) {
+        p2m_round<2>(t, c, r0, r.y, T.p, lane, sm, acc);
+        r0 += 64;
+      } else {
+        p2m_round<1>(t, c, r0, r.y, T.p, lane, sm, acc);
+        r0 += 32;
+      }
+    }
+    __syncwarp();
+    for (int a = lane; a < n_m; a += 32) M[static_cast<size_t>(id) * n_m + a] = acc[a] * T.inv_fact[a];
+  }
+  double* kids = sm;                 // 8 multipoles, then (2) the sums along y
+  double* sums = sm + 8 * n_m;       // 4 sums along x
+  double* pw = sm + 12 * n_m;
+  for (int node = id;;) {
+    const int par = t.parent[node];
+    if (par < 0) return;
+    const int ch = lane < 8 ? t.child[8 * par + lane] : -1;
+    const unsigned present = __ballot_sync(0xffffffffu, ch >= 0);
+    __threadfence();  // this warp's multipole, before its arrival
+    __syncwarp();
+    int last = 0;
+    if (lane == 0) {
+      last = atomicAdd(&arrived[par], 1) == __popc(present) - 1;
+      __threadfence();
+    }
+    __syncwarp();
+    if (!__shfl_sync(0xffffffffu, last, 0)) return;
+#pragma unroll
+    for (int o = 0; o < 8; ++o) {
+      const int co = __shfl_sync(0xffffffffu, ch, o);
+      const double* mc = M + static_cast<size_t>(max(co, 0)) * n_m;
+      for (int a = lane; a < n_m; a += 32) kids[o * n_m + a] = co >= 0 ? __ldcg(mc + a) : 0.0;
+    }
+    child_powers(t, T, par, ch, lane, pw);
+    __syncwarp();
+    m2m_axis<4>(prev, pw, n_m, lane, kids, [&](int q, int a, double s) { sums[q * n_m + a] = s; });
+    __syncwarp();
+    m2m_axis<2>(prev + n_m, pw + 2 * kPow, n_m, lane, sums, [&](int q, int a, double s) { kids[q * n_m + a] = s; });
+    __syncwarp();
+    double* mp = M + static_cast<size_t>(par) * n_m;
+    m2m_axis<1>(prev + 2 * n_m, pw + 4 * kPow, n_m, lane, kids, [&](int, int a, double s) { mp[a] = s; });
+    __syncwarp();
+    node = par;
+  }
 }
 
 // ------------------------------------------------------------ dual traversal
@@ -543,10 +646,28 @@ fmm_m2m_kernel(const Octree t, FmmDevTables T, int depth, double* __restrict__ M
 // centre and the radius, negated for a leaf (a leaf of radius 0 stores -0.0;
 // the sign bit is the leaf flag, the magnitude the radius).
 // The M2L classes read the cell's place among the cells of its depth.
+// The internal nodes are listed by depth for L2L (`next` counts a depth's
+// nodes listed so far).
 __global__ void fmm_node_record_kernel(const Octree t, const double* __restrict__ radius,
-                                       double4* __restrict__ rec, int4* __restrict__ cell) {
+                                       const int* __restrict__ level_count, int* __restrict__ next,
+                                       int* __restrict__ family, double4* __restrict__ rec,
+                                       int4* __restrict__ cell) {
+  __shared__ int count[32], first[32];
+  if (threadIdx.x < 32) count[threadIdx.x] = 0;
+  __syncthreads();
   const int id = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool internal = id < t.n_nodes && !t.meta[id].y;
+  const int depth = internal ? t.meta[id].x : 0;
+  const int rank = internal ? atomicAdd(&count[depth], 1) : 0;
+  __syncthreads();
+  if (threadIdx.x < 32 && count[threadIdx.x] > 0) {
+    int b = atomicAdd(&next[threadIdx.x], count[threadIdx.x]);
+    for (int d = 0; d < threadIdx.x; ++d) b += level_count[d];
+    first[threadIdx.x] = b;
+  }
+  __syncthreads();
   if (id >= t.n_nodes) return;
+  if (internal) family[first[depth] + rank] = id;
   const double4 c = t.center[id];
   const double r = radius[id];
   rec[id] = make_double4(c.x, c.y, c.z, t.meta[id].y ? -r : r);
@@ -2268,36 +2389,73 @@ int m2l_products(amk_ctx* c, int order, const Octree& t, const FmmDevTables& T, 
 }
 
 // ------------------------------------------------------------ L2L
-// Children at `depth` receive their parent's expansion (fast-multipole.cc:557-578).
-// A warp per child, lanes over its coefficients; the offset's monomials
-// d^c / c! and the parent's L_b b! are staged in shared memory first, so a
-// term is one product; 1/a! is applied once per coefficient.
-__global__ void __launch_bounds__(32 * kFmmWarps)
-fmm_l2l_kernel(const Octree t, FmmDevTables T, int depth, double* __restrict__ L) {
-  __shared__ double mono_s[kFmmWarps][kMaxNm], lps_s[kFmmWarps][kMaxNm];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int id = blockIdx.x * kFmmWarps + w;
-  if (id >= t.n_nodes) return;
-  if (t.meta[id].x != depth) return;
-  const int par = t.parent[id];
-  if (par < 0) return;
-  const double4 c = t.center[id], pc = t.center[par];
-  double px[kMaxOrder + 1], py[kMaxOrder + 1], pz[kMaxOrder + 1];
-  powers(T.p, c.x - pc.x, c.y - pc.y, c.z - pc.z, px, py, pz);
-  const double* lp = L + static_cast<size_t>(par) * T.n_m;
-  double* lc = L + static_cast<size_t>(id) * T.n_m;
-  double* mono = mono_s[w];
-  double* lps = lps_s[w];
-  for (int a = lane; a < T.n_m; a += 32) {
-    const int4 m = T.multi[a];
-    mono[a] = (px[m.x] * py[m.y] * pz[m.z]) * T.inv_fact[a];
-    lps[a] = lp[a] * T.fact[a];
+// The children of every node at `depth` receive its expansion
+// (fast-multipole.cc:557-578): L_a += L_b (b! / a!) d^(b-a) / (b-a)!. As in
+// M2M the shift is one axis at a time and siblings share their offsets: a
+// warp per parent shifts b! L_b to the two x offsets, those to the two y
+// offsets each, those along z to the children (14 one-axis shifts instead of
+// 8 full ones, and a parent's expansion read once). A depth's parents are listed,
+// so a launch covers only them. Measured: order 4, 262k, 8 levels 128 -> 103 us;
+// order 6, 1M 612 -> 241 us.
+template <int N, typename Out>
+__device__ __forceinline__ void l2l_axis(const short* __restrict__ next, const double* __restrict__ pw, int n_m,
+                                         int lane, const double* __restrict__ in, Out out) {
+  for (int a = lane; a < n_m; a += 32) {
+    double s[2 * N];
+#pragma unroll
+    for (int q = 0; q < 2 * N; ++q) s[q] = 0.0;
+    for (int i = a, k = 0; i >= 0; i = next[i], ++k) {
+      const double p0 = pw[k], p1 = pw[kPow + k];
+#pragma unroll
+      for (int q = 0; q < N; ++q) {
+        const double v = in[q * n_m + i];
+        s[2 * q] += v * p0;
+        s[2 * q + 1] += v * p1;
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 2 * N; ++q) out(q, a, s[q]);
   }
-  __syncwarp();
-  for (int a = lane; a < T.n_m; a += 32) {
-    double s = 0.0;
-    for (int e = T.l2l_off[a]; e < T.l2l_off[a + 1]; ++e) s += lps[T.l2l_b[e]] * mono[T.l2l_c[e]];
-    lc[a] += s * T.inv_fact[a];
+}
+
+__global__ void __launch_bounds__(32 * kFmmWarps)
+fmm_l2l_kernel(const Octree t, FmmDevTables T, int depth, const int* __restrict__ level_count,
+               const int* __restrict__ family, double* __restrict__ L) {
+  extern __shared__ __align__(16) unsigned char down_sm[];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int n_m = T.n_m;
+  const int here = level_count[lane];
+  const int n = __shfl_sync(0xffffffffu, here, depth);
+  if (static_cast<int>(blockIdx.x) * kFmmWarps >= n) return;
+  const int start = __reduce_add_sync(0xffffffffu, lane < depth ? here : 0);
+  double* sm = reinterpret_cast<double*>(down_sm) + w * down_smem(n_m);
+  short* next = reinterpret_cast<short*>(reinterpret_cast<double*>(down_sm) + kFmmWarps * down_smem(n_m));
+  for (int i = threadIdx.x; i < 3 * n_m; i += blockDim.x) next[i] = T.next[i];
+  __syncthreads();
+  double* lx = sm + n_m;        // 2
+  double* ly = lx + 2 * n_m;    // 4
+  double* pw = ly + 4 * n_m;
+  for (int f = blockIdx.x * kFmmWarps + w; f < n; f += gridDim.x * kFmmWarps) {
+    const int id = family[start + f];
+    const int ch = lane < 8 ? t.child[8 * id + lane] : -1;
+    const double* lp = L + static_cast<size_t>(id) * n_m;
+    for (int a = lane; a < n_m; a += 32) sm[a] = lp[a] * T.fact[a];
+    child_powers(t, T, id, ch, lane, pw);
+    __syncwarp();
+    l2l_axis<1>(next, pw, n_m, lane, sm, [&](int q, int a, double s) { lx[q * n_m + a] = s; });
+    __syncwarp();
+    // q = 2 x + y
+    l2l_axis<2>(next + n_m, pw + 2 * kPow, n_m, lane, lx, [&](int q, int a, double s) { ly[q * n_m + a] = s; });
+    __syncwarp();
+    int kid[8];
+#pragma unroll
+    for (int o = 0; o < 8; ++o) kid[o] = __shfl_sync(0xffffffffu, ch, o);
+    // q = 4 x + 2 y + z
+    l2l_axis<4>(next + 2 * n_m, pw + 4 * kPow, n_m, lane, ly, [&](int q, int a, double s) {
+      const int co = kid[(q >> 2) | (q & 2) | ((q & 1) << 2)];
+      if (co >= 0) L[static_cast<size_t>(co) * n_m + a] += s * T.inv_fact[a];
+    });
+    __syncwarp();
   }
 }
 
@@ -2950,20 +3108,25 @@ int fmm_run(amk_ctx* c, const View& v, int order, double theta, long leaf_capaci
     AMK_CUDA_TRY(cudaEventCreateWithFlags(&f->up_done, cudaEventDisableTiming));
   }
   AMK_TRY(phase_begin(c, AMK_PHASE_FMM_UP));
-  fmm_leaf_radius_kernel<<<gn, 256, 0, c->stream>>>(t, radius);
-  AMK_TRY(check_launch(c, "fmm_leaf_radius_kernel"));
-  for (int d = t.max_depth; d >= 0; --d) {
-    fmm_parent_radius_kernel<<<gn, 256, 0, c->stream>>>(t, d, radius);
-    AMK_TRY(check_launch(c, "fmm_parent_radius_kernel"));
-  }
+  // arrivals at the parents (radii, multipoles), internal nodes per depth, listed so far
+  int* arrived = slot<int>(c, kSlotFmmArrived, 2 * static_cast<size_t>(nn) + 64, &rc);
+  AMK_TRY(rc);
+  int* level_count = arrived + 2 * nn;
+  int* family = slot<int>(c, kSlotFmmFamily, nn, &rc);
+  AMK_TRY(rc);
+  AMK_CUDA_TRY(cudaMemsetAsync(arrived, 0, (2 * static_cast<size_t>(nn) + 64) * sizeof(int), c->stream));
+  fmm_radius_kernel<<<static_cast<unsigned>((8 * nn + 255) / 256), 256, 0, c->stream>>>(t, radius, arrived,
+                                                                                        level_count);
+  AMK_TRY(check_launch(c, "fmm_radius_kernel"));
   AMK_CUDA_TRY(cudaEventRecord(f->up_start, c->stream));
   AMK_CUDA_TRY(cudaStreamWaitEvent(f->up, f->up_start, 0));
-  fmm_p2m_kernel<<<gw, 32 * kFmmWarps, 0, f->up>>>(t, T, M);
-  AMK_TRY(check_launch(c, "fmm_p2m_kernel"));
-  for (int d = t.max_depth; d >= 0; --d) {
-    fmm_m2m_kernel<<<gw, 32 * kFmmWarps, 0, f->up>>>(t, T, d, M);
-    AMK_TRY(check_launch(c, "fmm_m2m_kernel"));
-  }
+  const int table_bytes = 3 * T.n_m * static_cast<int>(sizeof(short));
+  const int up_bytes = kFmmWarps * up_smem(T.n_m) * static_cast<int>(sizeof(double)) + table_bytes;
+  const int down_bytes = kFmmWarps * down_smem(T.n_m) * static_cast<int>(sizeof(double)) + table_bytes;
+  AMK_CUDA_TRY(cudaFuncSetAttribute(fmm_up_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, up_bytes));
+  AMK_CUDA_TRY(cudaFuncSetAttribute(fmm_l2l_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, down_bytes));
+  fmm_up_kernel<<<gw, 32 * kFmmWarps, up_bytes, f->up>>>(t, T, arrived + nn, M);
+  AMK_TRY(check_launch(c, "fmm_up_kernel"));
   AMK_CUDA_TRY(cudaEventRecord(f->up_done, f->up));
   AMK_TRY(phase_end(c, AMK_PHASE_FMM_UP));
 
@@ -2985,7 +3148,7 @@ int fmm_run(amk_ctx* c, const View& v, int order, double theta, long leaf_capaci
   AMK_TRY(rc);
   int4* cell = slot<int4>(c, kSlotFmmCell, nn, &rc);
   AMK_TRY(rc);
-  fmm_node_record_kernel<<<gn, 256, 0, c->stream>>>(t, radius, rec, cell);
+  fmm_node_record_kernel<<<gn, 256, 0, c->stream>>>(t, radius, level_count, level_count + 32, family, rec, cell);
   AMK_TRY(check_launch(c, "fmm_node_record_kernel"));
   long n_m2l = 0, n_p2p = 0;
   std::vector<int> hv(n_tv);
@@ -3175,8 +3338,9 @@ int fmm_run(amk_ctx* c, const View& v, int order, double theta, long leaf_capaci
 
   // ---- L2L
   AMK_TRY(phase_begin(c, AMK_PHASE_FMM_DOWN));
-  for (int d = 1; d <= t.max_depth; ++d) {
-    fmm_l2l_kernel<<<gw, 32 * kFmmWarps, 0, c->stream>>>(t, T, d, Lx);
+  for (int d = 0; d < t.max_depth; ++d) {
+    fmm_l2l_kernel<<<std::min(gw, 148u * 8), 32 * kFmmWarps, down_bytes, c->stream>>>(t, T, d, level_count, family,
+                                                                                      Lx);
     AMK_TRY(check_launch(c, "fmm_l2l_kernel"));
   }
   AMK_TRY(phase_end(c, AMK_PHASE_FMM_DOWN));
