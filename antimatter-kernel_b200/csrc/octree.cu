@@ -12,8 +12,8 @@
 //      the particles in the reference's tree order;
 //   2. with L_k = common leading digits of keys k-1 and k, the node of depth
 //      d holding k is [max{s<=k: L_s<d}, min{e>k: L_e<d}); the leaf depth of
-//      k is the smallest d whose node holds <= cap particles, found from a
-//      +-cap window of L values;
+//      k is the smallest d whose node holds <= cap particles, found from the
+//      digits that particles cap places apart share;
 //   3. particle k opens the nodes of depths L_k+1 .. leafdepth(k); an
 //      exclusive scan of those counts numbers all nodes in pre-order -- the
 //      reference's indices;
@@ -126,34 +126,78 @@ __device__ __forceinline__ int common_levels(uint64_t a, uint64_t b) {
   return (__clzll(static_cast<long long>(x)) - 1) / 3;
 }
 
-__global__ void tree_L_kernel(const uint64_t* __restrict__ keys, int m, int* __restrict__ L) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= m) return;
-  L[k] = (k == 0) ? -1 : common_levels(keys[k - 1], keys[k]);
+// Depth of every particle's leaf: the smallest depth whose cell around it
+// holds at most cap particles (the key depth at most). A cell of depth d
+// around k holds more than cap exactly if cap + 1 consecutive particles, k
+// among them, share d digits, so with W[s] = levels shared by s and s + cap
+//   leafdepth(k) = 1 + max of W[s] over s in [k - cap, k], both ends in the set
+// (0 without such an s). The maximum over a sliding window of up to 256 is
+// built in shared memory by doubling; a longer window is two of those, at its
+// ends, and the part that all the block's windows share. Scanning the 2 cap
+// neighbours in every thread took 269 us at 1M particles and a capacity of
+// 128, this 17 us.
+// Also L[k], the levels shared with the particle before, the nodes that start
+// at k (depths L[k] + 1 to its leaf's) and the deepest leaf.
+constexpr int kLeafThreads = 256;
+
+__device__ __forceinline__ int shared_levels(const uint64_t* __restrict__ keys, int m, int cap, int s) {
+  return s >= 0 && s < m - cap ? common_levels(keys[s], keys[s + cap]) : -1;
 }
 
-// leafdepth(k) = min over runs [s, e) containing k with e - s <= cap of
-// max(L_s, L_e) + 1 (L_0 = L_m = -1), capped at the key depth.
-__global__ void tree_leafdepth_kernel(const int* __restrict__ L, int m, int cap, int* __restrict__ ld,
-                                      int* __restrict__ count) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= m) return;
-  int best = kTreeLevels;
-  const int s0 = max(0, k - cap + 1);
-  int emin = 1 << 30;
-  int ehi = k;  // e range [k+1, ehi] scanned so far
-  for (int s = s0; s <= k; ++s) {
-    const int lim = min(m, s + cap);
-    while (ehi < lim) {
-      ++ehi;
-      const int le = (ehi == m) ? -1 : L[ehi];
-      emin = min(emin, le);
-    }
-    if (ehi >= k + 1) best = min(best, max(L[s], emin) + 1);
+// max of W over [first + threadIdx.x, + w), w <= 256; a and b: 512 entries
+__device__ __forceinline__ int window_max(const uint64_t* __restrict__ keys, int m, int cap, int first, int w, int* a,
+                                          int* b) {
+  const int n = kLeafThreads + w - 1;
+  for (int j = threadIdx.x; j < n; j += kLeafThreads) a[j] = shared_levels(keys, m, cap, first + j);
+  __syncthreads();
+  int len = 1;
+  for (; 2 * len <= w; len *= 2) {
+    for (int j = threadIdx.x; j < n; j += kLeafThreads) b[j] = max(a[j], a[min(j + len, n - 1)]);
+    __syncthreads();
+    int* x = a;
+    a = b;
+    b = x;
   }
-  ld[k] = best;
-  const int lk = L[k];
-  count[k] = (lk < best) ? best - lk : 0;
+  const int r = max(a[threadIdx.x], a[threadIdx.x + w - len]);
+  __syncthreads();
+  return r;
+}
+
+__global__ void __launch_bounds__(kLeafThreads)
+tree_leafdepth_kernel(const uint64_t* __restrict__ keys, int m, int cap, int* __restrict__ L, int* __restrict__ ld,
+                      int* __restrict__ count, int* __restrict__ deepest) {
+  __shared__ int a[2 * kLeafThreads], b[2 * kLeafThreads];
+  __shared__ int warp_max[kLeafThreads / 32];
+  const int first = blockIdx.x * kLeafThreads;
+  const int k = first + threadIdx.x;
+  const int w = min(cap, kLeafThreads - 1) + 1;
+  int best = window_max(keys, m, cap, first - w + 1, w, a, b);
+  if (cap >= kLeafThreads) {
+    best = max(best, window_max(keys, m, cap, first - cap, w, a, b));
+    int mid = -1;
+    for (int s = max(0, first + kLeafThreads - 1 - cap) + threadIdx.x; s <= min(first, m - cap - 1); s += kLeafThreads)
+      mid = max(mid, shared_levels(keys, m, cap, s));
+    mid = __reduce_max_sync(0xffffffffu, mid);
+    if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = mid;
+    __syncthreads();
+    for (int i = 0; i < kLeafThreads / 32; ++i) best = max(best, warp_max[i]);
+    __syncthreads();
+  }
+  best = min(best + 1, kTreeLevels);
+  if (k < m) {
+    const int lk = k == 0 ? -1 : common_levels(keys[k - 1], keys[k]);
+    L[k] = lk;
+    ld[k] = best;
+    count[k] = max(best - lk, 0);
+  }
+  const int d = __reduce_max_sync(0xffffffffu, k < m ? best : 0);
+  if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = d;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int e = 0;
+    for (int i = 0; i < kLeafThreads / 32; ++i) e = max(e, warp_max[i]);
+    if (e > 0) atomicMax(deepest, e);
+  }
 }
 
 __device__ __forceinline__ int digit(uint64_t key, int level) {
@@ -245,13 +289,6 @@ __global__ void tree_sources_kernel(View v, int mode, const TreeFrame* __restric
   src[k] = make_double4(p[0], p[1], p[2], v.q[i]);
 }
 
-__global__ void tree_max_depth_kernel(const int* __restrict__ ld, int m, int* out) {
-  int d = 0;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < m; k += gridDim.x * blockDim.x) d = max(d, ld[k]);
-  for (int o = 16; o > 0; o >>= 1) d = max(d, __shfl_xor_sync(0xffffffffu, d, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, d);
-}
-
 }  // namespace
 
 int build_octree(amk_ctx* c, const View& v, int leaf_cap, int mode, Octree* t) {
@@ -306,14 +343,10 @@ int build_octree(amk_ctx* c, const View& v, int leaf_cap, int mode, Octree* t) {
   int* base = slot<int>(c, kSlotTreeBase, m + 1, &rc);
   AMK_TRY(rc);
   const unsigned gm = static_cast<unsigned>((m + 255) / 256);
-  tree_L_kernel<<<gm, 256, 0, c->stream>>>(skeys, m, L);
-  AMK_TRY(check_launch(c, "tree_L_kernel"));
-  tree_leafdepth_kernel<<<gm, 256, 0, c->stream>>>(L, m, t->leaf_cap, ld, cnt);
+  AMK_CUDA_TRY(cudaMemsetAsync(small + 2, 0, sizeof(int), c->stream));
+  tree_leafdepth_kernel<<<gm, kLeafThreads, 0, c->stream>>>(skeys, m, std::min(t->leaf_cap, m), L, ld, cnt, small + 2);
   AMK_TRY(check_launch(c, "tree_leafdepth_kernel"));
   AMK_TRY(exclusive_scan_int(c, cnt, m, base, small + 1));
-  AMK_CUDA_TRY(cudaMemsetAsync(small + 2, 0, sizeof(int), c->stream));
-  tree_max_depth_kernel<<<std::min(gm, 148u), 256, 0, c->stream>>>(ld, m, small + 2);
-  AMK_TRY(check_launch(c, "tree_max_depth_kernel"));
   int hs[2] = {0, 0};
   AMK_CUDA_TRY(cudaMemcpyAsync(hs, small + 1, 2 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   AMK_CUDA_TRY(cudaStreamSynchronize(c->stream));
