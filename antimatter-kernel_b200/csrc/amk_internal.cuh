@@ -273,6 +273,7 @@ struct amk_ctx {
   amk::Fmm* fmm = nullptr;
   amk::Mlp* mlp = nullptr;
   amk::Batch* batch = nullptr;  // batched instances over segment offsets
+  amk::Batch* batch_spare = nullptr;  // its buffers, until the next batch or particle set
   // leaf capacities of the context's own solver calls (the reference's 32 and
   // 8 unless amk_autotune or amk_set_leaf_sizes changed them)
   int fmm_leaf = 32;
@@ -393,6 +394,7 @@ int annihilate_view(amk_ctx* c, const View& v, const uint8_t* species, const uin
                     double probability, uint32_t seed, uint64_t step_index, long* marked);
 // Batched instances (batch.cu).
 void batch_destroy(amk_ctx* c);
+void batch_retire(amk_ctx* c);
 // Coulomb potential energy (J) of a view under an energy method (energy.cu).
 int coulomb_energy_view(amk_ctx* c, View v, const amk_params& p, int method, double* out_host);
 // RMS / max relative error of a view's forces against the FP64 exact sum

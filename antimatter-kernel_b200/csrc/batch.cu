@@ -68,6 +68,32 @@ __device__ __forceinline__ void fold(float& hi, float& lo, float p) {
   hi = s;
 }
 
+// Set-up, a block per instance: the particles' instance ids and the largest
+// finite coordinate magnitude (a particle with an infinite or NaN largest
+// coordinate is left out), which sets the instance's scale and grids. Setting
+// a batch of 482k particles: 3.9 ms with the positions copied to the host for it
+// and new buffers (of which 3.6 ms more were freed at the next load), now 0.23 ms.
+__device__ __forceinline__ double larger(double a, double b) { return a < b ? b : a; }
+
+__global__ void __launch_bounds__(512)
+batch_extent_kernel(const long* __restrict__ offsets, const double* __restrict__ x, const double* __restrict__ y,
+                    const double* __restrict__ z, uint16_t* __restrict__ inst_of, double* __restrict__ extent) {
+  __shared__ double warp_max[16];
+  double mx = 0.0;
+  for (long k = offsets[blockIdx.x] + threadIdx.x; k < offsets[blockIdx.x + 1]; k += 512) {
+    inst_of[k] = static_cast<uint16_t>(blockIdx.x);
+    const double a = larger(fabs(x[k]), larger(fabs(y[k]), fabs(z[k])));
+    if (isfinite(a)) mx = fmax(mx, a);
+  }
+  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 16; ++w) mx = fmax(mx, warp_max[w]);
+    extent[blockIdx.x] = mx;
+  }
+}
+
 __global__ void batch_local_ids_kernel(long n, const uint16_t* __restrict__ inst_of,
                                        const InstanceDev* __restrict__ inst, uint32_t* __restrict__ ids) {
   const long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
@@ -589,6 +615,18 @@ struct Batch {
   std::vector<double> prev_trap, prev_coulomb;
   bool energy_has_previous = false;
   long graph_launches = 0;
+  DevBuf extent;  // set-up: offsets, then the instances' largest coordinates
+  // The device buffers of the batch that this one replaces (the same context
+  // and stream, so their earlier users come first in stream order): a sweep
+  // that loads and sets batch after batch allocates once. Allocating and
+  // freeing some twenty buffers per batch took up to 7 ms at 482k particles, and
+  // now and then 30 to 90 ms, beside 12 steps of 2.4 ms.
+  void take_buffers(Batch& o) {
+    for (auto m : {&Batch::inst, &Batch::inst_of, &Batch::units, &Batch::counters, &Batch::contacts, &Batch::best,
+                   &Batch::flags, &Batch::keys, &Batch::vals, &Batch::skeys, &Batch::perm, &Batch::rel, &Batch::boxes,
+                   &Batch::cell_at, &Batch::cell_count, &Batch::cell_first, &Batch::cell_rec, &Batch::extent})
+      (this->*m).swap(o.*m);
+  }
   ~Batch() {
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
@@ -624,6 +662,17 @@ struct Batch {
 void batch_destroy(amk_ctx* c) {
   delete c->batch;
   c->batch = nullptr;
+  delete c->batch_spare;
+  c->batch_spare = nullptr;
+}
+
+// Ends the batch when its particles are replaced. Its buffers wait for the
+// next batch, and are freed if the particles are replaced again before one.
+void batch_retire(amk_ctx* c) {
+  delete c->batch_spare;
+  c->batch_spare = c->batch;
+  c->batch = nullptr;
+  if (c->batch_spare) c->batch_spare->drop_graph();
 }
 
 namespace {
@@ -799,35 +848,37 @@ extern "C" int amk_batch_set(amk_ctx* c, int n_inst, const amk_params* params, c
       return fail(AMK_ERR_UNSUPPORTED, "instance %d: the learned correction is not available in batches", i);
   }
   AMK_CUDA_TRY(cudaSetDevice(c->device));
-  batch_destroy(c);
   Batch* B = new Batch();
+  if (c->batch || c->batch_spare) B->take_buffers(c->batch ? *c->batch : *c->batch_spare);
+  batch_destroy(c);
   c->batch = B;
   B->n_inst = n_inst;
   B->params.assign(params, params + n_inst);
   B->offsets.assign(offsets, offsets + n_inst + 1);
   B->step = static_cast<uint64_t>(c->step);
   const long n = c->n;
-  // host copies of the positions for the per-instance scales and grids
-  std::vector<double> hx(n), hy(n), hz(n);
+  const size_t nn = static_cast<size_t>(std::max<long>(n, 1));
+  AMK_TRY(B->inst_of.reserve(nn * sizeof(uint16_t)));
+  std::vector<double> extent(n_inst, 0.0);
   if (n > 0) {
-    AMK_CUDA_TRY(cudaMemcpyAsync(hx.data(), c->x.ptr, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    AMK_CUDA_TRY(cudaMemcpyAsync(hy.data(), c->y.ptr, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    AMK_CUDA_TRY(cudaMemcpyAsync(hz.data(), c->z.ptr, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    const size_t at = (n_inst + 1) * sizeof(long);
+    AMK_TRY(B->extent.reserve(at + n_inst * sizeof(double)));
+    long* off = B->extent.as<long>();
+    double* ext = reinterpret_cast<double*>(B->extent.as<char>() + at);
+    AMK_CUDA_TRY(cudaMemcpyAsync(off, offsets, at, cudaMemcpyHostToDevice, c->stream));
+    batch_extent_kernel<<<n_inst, 512, 0, c->stream>>>(off, c->x.as<double>(), c->y.as<double>(), c->z.as<double>(),
+                                                       B->inst_of.as<uint16_t>(), ext);
+    AMK_TRY(check_launch(c, "batch_extent_kernel"));
+    AMK_CUDA_TRY(cudaMemcpyAsync(extent.data(), ext, n_inst * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     AMK_CUDA_TRY(cudaStreamSynchronize(c->stream));
   }
   std::vector<InstanceDev> inst(n_inst);
-  std::vector<uint16_t> inst_of(n);
   std::vector<std::pair<long, int2>> units;  // (instance size, unit)
   long n_tiles = 0;  // all-pairs sub-tile slots (kBSubPerUnit per unit)
   for (int i = 0; i < n_inst; ++i) {
     const amk_params& p = params[i];
     const long off = offsets[i], cnt = offsets[i + 1] - off;
-    double mx = 0.0;
-    for (long k = off; k < off + cnt; ++k) {
-      inst_of[k] = static_cast<uint16_t>(i);
-      const double a = std::max(std::fabs(hx[k]), std::max(std::fabs(hy[k]), std::fabs(hz[k])));
-      if (std::isfinite(a)) mx = std::max(mx, a);
-    }
+    const double mx = extent[i];
     InstanceDev& d = inst[i];
     d.push = push_params_for(p);
     B->push.push_back(d.push);
@@ -868,9 +919,7 @@ extern "C" int amk_batch_set(amk_ctx* c, int n_inst, const amk_params* params, c
   AMK_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
   AMK_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_allpairs_kernel, kBT, 0));
   B->grid = static_cast<int>(std::max<long>(1, std::min<long>(B->n_units, static_cast<long>(sms) * std::max(1, per_sm))));
-  const size_t nn = static_cast<size_t>(std::max<long>(n, 1));
   AMK_TRY(B->inst.reserve(n_inst * sizeof(InstanceDev)));
-  AMK_TRY(B->inst_of.reserve(nn * sizeof(uint16_t)));
   AMK_TRY(B->units.reserve(std::max<size_t>(1, hu.size()) * sizeof(int2)));
   AMK_TRY(B->counters.reserve(64));
   AMK_TRY(B->reserve_contacts(std::max<long>(65536, n / 8), n));
@@ -892,9 +941,6 @@ extern "C" int amk_batch_set(amk_ctx* c, int n_inst, const amk_params* params, c
   AMK_TRY(B->boxes.reserve(static_cast<size_t>(std::max<long>(n_tiles, 1)) * sizeof(TileBox)));
   AMK_CUDA_TRY(cudaMemcpyAsync(B->inst.ptr, inst.data(), n_inst * sizeof(InstanceDev), cudaMemcpyHostToDevice,
                                c->stream));
-  if (n > 0)
-    AMK_CUDA_TRY(cudaMemcpyAsync(B->inst_of.ptr, inst_of.data(), n * sizeof(uint16_t), cudaMemcpyHostToDevice,
-                                 c->stream));
   if (!hu.empty())
     AMK_CUDA_TRY(cudaMemcpyAsync(B->units.ptr, hu.data(), hu.size() * sizeof(int2), cudaMemcpyHostToDevice, c->stream));
   const unsigned long long init[8] = {0, B->step, 0, 0, 0, 0, 0, 0};

@@ -388,7 +388,7 @@ __global__ void max_abs_kernel(long n, const double* __restrict__ x, const doubl
 }
 
 static int finish_load(amk_ctx* c, long n) {
-  batch_destroy(c);  // instance offsets refer to the previous particle set
+  batch_retire(c);  // instance offsets refer to the previous particle set
   c->n = n;
   c->ap_perm_n = -1;
   c->staggered = false;
