@@ -2772,17 +2772,20 @@ __device__ __forceinline__ int p2p32_stage_far(P2PPairs& sp, const float4* __res
   return np;
 }
 
-__global__ void __launch_bounds__(32 * kFmmWarps, 6)  // 6 blocks per SM (80 registers): measured best of 4-6
-fmm_p2p32_kernel(const Octree t, const int2* __restrict__ work, int n_work, const int* __restrict__ off,
+// One warp per block, 32 blocks per SM (64 registers): a block of four warps
+// kept its slots until its longest item was done, and the packed chain of a
+// pair (a third of the stalls) wants warps in flight. 1M particles, order 7, 128
+// per leaf: four warps, 6 blocks per SM 6.09 ms; one warp, 20 / 24 / 28 / 32
+// blocks 6.00 / 5.69 / 5.59 / 5.49 ms.
+__global__ void __launch_bounds__(32, 32)
+fmm_p2p32_kernel(const Octree t, const int2* __restrict__ work, const int* __restrict__ off,
                  const int* __restrict__ count, const int* __restrict__ src, const int* __restrict__ pbase,
                  double min_sq, const float4* __restrict__ shi, const float4* __restrict__ slo,
                  const double* __restrict__ radius, double4* __restrict__ part) {
-  __shared__ double4 red[kFmmWarps][32];
-  __shared__ P2PPairs stg[kFmmWarps];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int wi = blockIdx.x * kFmmWarps + w;
-  if (wi >= n_work) return;
-  const int2 item = work[wi];
+  __shared__ double4 red[32];
+  __shared__ P2PPairs sp;
+  const int lane = threadIdx.x;
+  const int2 item = work[blockIdx.x];
   const int ti = item.x, chunk = item.y;
   const int2 tr = t.range[ti];
   const int nt_all = tr.y - tr.x;
@@ -2790,7 +2793,6 @@ fmm_p2p32_kernel(const Octree t, const int2* __restrict__ work, int n_work, cons
   const int se = min(off[ti] + count[ti], sb + kP2P32Chunk);
   double4* out = part + pbase[ti] + static_cast<size_t>(chunk) * nt_all;
   const float min_sq32 = fmaxf(static_cast<float>(min_sq), 1.17549435e-38f);
-  P2PPairs& sp = stg[w];
   const double4 ct = t.center[ti];
   const double rt = radius[ti];
   // whether source leaf sl is separated (warp-uniform), and its centre
@@ -2891,12 +2893,12 @@ fmm_p2p32_kernel(const Octree t, const int2* __restrict__ work, int n_work, cons
       }
       p2p32_leaf_end(t0);
     }
-    red[w][lane] = t0.acc;
+    red[lane] = t0.acc;
     __syncwarp();
     if (active && g == 0) {
-      double4 a = red[w][tl];
+      double4 a = red[tl];
       for (int gg = 1; gg < groups; ++gg) {
-        const double4 b = red[w][gg * nt + tl];
+        const double4 b = red[gg * nt + tl];
         a.x += b.x;
         a.y += b.y;
         a.z += b.z;
@@ -2909,7 +2911,7 @@ fmm_p2p32_kernel(const Octree t, const int2* __restrict__ work, int n_work, cons
   }
 }
 
-// Per particle: item partials in chunk order, four in flight.
+// Per particle: item partials in chunk order, eight in flight.
 __global__ void fmm_p2p_reduce_kernel(const Octree t, const int* __restrict__ leaf_of, const int* __restrict__ items,
                                       const int* __restrict__ pbase, const double4* __restrict__ part,
                                       double4* __restrict__ ef) {
@@ -2921,12 +2923,12 @@ __global__ void fmm_p2p_reduce_kernel(const Octree t, const int* __restrict__ le
   const double4* p = part + pbase[leaf] + (k - r.x);
   double4 a = p[0];
   int c = 1;
-  for (; c + 4 <= n; c += 4) {
-    double4 b[4];
+  for (; c + 8 <= n; c += 8) {
+    double4 b[8];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) b[u] = p[static_cast<size_t>(c + u) * nt];
+    for (int u = 0; u < 8; ++u) b[u] = p[static_cast<size_t>(c + u) * nt];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < 8; ++u) {
       a.x += b[u].x;
       a.y += b[u].y;
       a.z += b[u].z;
@@ -3264,7 +3266,6 @@ int fmm_run(amk_ctx* c, const View& v, int order, double theta, long leaf_capaci
   p2p_items_fill_kernel<<<gn, 256, 0, c->stream>>>(t, items, ibase, work, leaf_of);
   AMK_TRY(check_launch(c, "p2p_items_fill_kernel"));
   AMK_TRY(phase_end(c, AMK_PHASE_FMM_P2P));
-  const unsigned gwork = static_cast<unsigned>((ht[0] + kFmmWarps - 1) / kFmmWarps);
   // The near field's pair sums need no expansion, so they run on their own
   // stream: the FP32 ones once the last M2L products are enqueued (the
   // tensor-core product kernel holds every SM's shared memory), concurrently
@@ -3284,7 +3285,7 @@ int fmm_run(amk_ctx* c, const View& v, int order, double theta, long leaf_capaci
     }
     AMK_TRY(phase_begin_on(c, AMK_PHASE_FMM_NEAR, f->near));
     if (f32)
-      fmm_p2p32_kernel<<<gwork, 32 * kFmmWarps, 0, f->near>>>(t, work, ht[0], gp.off, gp.count, gp.src, pbase, min_sq,
+      fmm_p2p32_kernel<<<static_cast<unsigned>(ht[0]), 32, 0, f->near>>>(t, work, gp.off, gp.count, gp.src, pbase, min_sq,
                                                               stage, stage + t.m, radius, part);
     else if (want_phi)
       fmm_p2p_kernel<true><<<static_cast<unsigned>(ht[0]), 32, 0, f->near>>>(t, work, gp.off, gp.count, gp.src, pbase, min_sq,
