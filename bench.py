@@ -241,9 +241,6 @@ PLAIN_P6 = "fmm p=6 theta=0.5"
 LEARNED_TRAINING = dict(sample_leaves=8192, steps=8000, batch=4096, lr=5e-4)
 LEARNED = "learned p=2 + MLP theta=0.5"
 
-# DRAM traffic (read + write) per launch of the FMM's M2L class-product kernel,
-# by order, from ncu captures of one launch (launches at N = 1,048,576 process
-# chunks of the same bounded size).
 # DRAM traffic per class pair of the tensor-core product kernel (the FP32
 # per-pair products written, the split expansions read past L2), from one
 # ncu launch at 262,144 particles scaled by the pairs of a launch here.
@@ -256,14 +253,6 @@ NEAR_TRAFFIC_PER_PAIR = (
     0.0300, "ncu dram__bytes_read.sum + dram__bytes_write.sum of fmm_p2p32_kernel on 262,144 particles (leaf 128, "
             "1.374 G particle pairs: 12.9 MB read + 28.4 MB written = 0.030 B per pair), scaled by this launch's "
             "pairs; profiles/fmm_p2p32_kernel_tree262k_leaf128.md")
-FMM_PRODUCT_TRAFFIC = {
-    7: (5.18e9, "ncu dram__bytes_read.sum + dram__bytes_write.sum of m2l_class_mma_kernel<7>, mean of two launches "
-                "of 4.47 M pairs each (0.89 / 1.10 GB read + 4.18 GB written: the per-pair products), "
-                "profiles/m2l_class_mma_kernel_tree1m.md"),
-    8: (5.17e9, "ncu dram__bytes_read.sum + dram__bytes_write.sum of m2l_class_mma_kernel<8>, mean of two launches "
-                "of 3.25 M pairs each (0.92 GB read + 4.26 GB written: the per-pair products), "
-                "profiles/m2l_class_mma_kernel_tree1m.md"),
-}
 
 
 def tree_cloud(n=1 << 20, seed=42):
@@ -314,10 +303,11 @@ def cpu_tree_step(x, y, z, vx, vy, vz, order=6, theta=0.5):
     return time.perf_counter() - t0
 
 
+REF_MISSING = ("oracle/_ref/libamkref.so (the reference's own code, built by `make -C oracle ref` from its source "
+               "tree) is not here")
+
+
 def cpu_tree_baseline(pos, vel, n_sample, warm, steps):
-    O = _oracle()
-    if not O.ref_available():
-        raise SystemExit("oracle/_ref/libamkref.so is missing: build it with `make -C oracle ref`")
     x, y, z = (np.ascontiguousarray(pos[:n_sample, k]) for k in range(3))
     vx, vy, vz = (np.ascontiguousarray(vel[:n_sample, k]) for k in range(3))
     times = []
@@ -452,14 +442,15 @@ def tree_roofline(sim, over, n):
             dominant["other_kernel"] = other
             return dominant
         peak = sim.measure_fp64_peak()
-        traffic = FMM_PRODUCT_TRAFFIC.get(p_)
+        # the harmonic basis: (p + 1)^2 coefficients per expansion
+        nr = (p_ + 1) ** 2
+        achieved = 2.0 * nr * nr * st["m2l_class_pairs"] / (prod_ms * 1e-3) / 1e12
         return {"bound": "fp64 tensor", "kernel": f"m2l_class_mma_kernel<{p_}>", "achieved": achieved,
                 "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
-                "traffic": None if traffic is None else traffic[0],
-                "traffic_source": None if traffic is None else traffic[1],
+                "traffic": None, "traffic_source": None,
                 "peak_source": "measured in this run: mma.m8n8k4 FP64 probe kernel over all SMs "
                                "(512 flop per warp instruction); the driver's peak file has no FP64 figure",
-                "flop_convention": f"2 n_m^2 flop (n_m = {nm}) per M2L pair evaluated as a class product "
+                "flop_convention": f"2 n_r^2 flop (n_r = {nr}) per M2L pair evaluated as a class product "
                                    f"({st['m2l_class_pairs']:,} of {st['m2l_pairs']:,} pairs; the rest take "
                                    "the per-pair path)",
                 "avg_launch_ms": prod_ms / max(1, prod_n), "launches_per_step": prod_n,
@@ -1316,6 +1307,12 @@ def main(argv=None):
     args = ap.parse_args(argv)
     args.warmup = max(3, args.warmup)  # at least three untimed warm-up steps
     amk_fn, ref_fn = WORKLOADS[args.workload]
+    if not _oracle().ref_available():
+        if args.impl == "reference":
+            if int(os.environ.get("RANK", "0")) == 0:
+                print(json.dumps({"impl": "reference", "unavailable": REF_MISSING}), flush=True)
+            return 0
+        args.cpu_baseline = 0  # reported as null
     return (ref_fn if args.impl == "reference" else amk_fn)(args)
 
 
