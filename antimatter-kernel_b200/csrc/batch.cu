@@ -616,8 +616,13 @@ struct Batch {
   bool energy_has_previous = false;
   long graph_launches = 0;
   DevBuf extent;  // set-up: offsets, then the instances' largest coordinates
-  // The device buffers of the batch that this one replaces (the same context
-  // and stream, so their earlier users come first in stream order): a sweep
+  // the stream of the batch's work; more than one: `mixed`
+  cudaStream_t stream = nullptr;
+  bool mixed = false;
+  void on(cudaStream_t s) { mixed = mixed || s != stream; }
+  // The device buffers of the batch that this one replaces (on the same stream
+  // their earlier users come first in stream order; a batch that worked on
+  // another one is waited for, as freeing its buffers would do): a sweep
   // that loads and sets batch after batch allocates once. Allocating and
   // freeing some twenty buffers per batch took up to 7 ms at 482k particles, and
   // now and then 30 to 90 ms, beside 12 steps of 2.4 ms.
@@ -849,7 +854,11 @@ extern "C" int amk_batch_set(amk_ctx* c, int n_inst, const amk_params* params, c
   }
   AMK_CUDA_TRY(cudaSetDevice(c->device));
   Batch* B = new Batch();
-  if (c->batch || c->batch_spare) B->take_buffers(c->batch ? *c->batch : *c->batch_spare);
+  B->stream = c->stream;
+  if (Batch* old = c->batch ? c->batch : c->batch_spare) {
+    if (old->mixed || old->stream != c->stream) cudaDeviceSynchronize();
+    B->take_buffers(*old);
+  }
   batch_destroy(c);
   c->batch = B;
   B->n_inst = n_inst;
@@ -960,6 +969,7 @@ extern "C" int amk_batch_step(amk_ctx* c, int nsteps, int graph_chunk, int seria
   if (!c->batch) return fail(AMK_ERR_STATE, "no batch: call amk_batch_set first");
   if (nsteps < 0) return fail(AMK_ERR_INVALID, "nsteps < 0");
   Batch& B = *c->batch;
+  B.on(c->stream);
   AMK_CUDA_TRY(cudaSetDevice(c->device));
   const bool use_graph = graph_chunk > 0 && !serial && B.graphable && !c->profiling;
   int done = 0;
@@ -1025,6 +1035,7 @@ extern "C" int amk_batch_coulomb(amk_ctx* c) {
   if (!c->batch) return fail(AMK_ERR_STATE, "no batch: call amk_batch_set first");
   AMK_CUDA_TRY(cudaSetDevice(c->device));
   Batch& B = *c->batch;
+  B.on(c->stream);
   if (c->n == 0) return AMK_OK;
   // the all-pairs queue head is reset by the step prologue; reset it here
   AMK_CUDA_TRY(cudaMemsetAsync(B.queue(), 0, sizeof(int), c->stream));
@@ -1036,6 +1047,7 @@ extern "C" int amk_batch_status(amk_ctx* c, int* overflow, long* alive_counts) {
   if (!c) return fail(AMK_ERR_INVALID, "null context");
   if (!c->batch) return fail(AMK_ERR_STATE, "no batch: call amk_batch_set first");
   Batch& B = *c->batch;
+  B.on(c->stream);
   AMK_CUDA_TRY(cudaSetDevice(c->device));
   unsigned long long ov = 0;
   AMK_CUDA_TRY(cudaMemcpyAsync(&ov, B.overflow(), sizeof(ov), cudaMemcpyDeviceToHost, c->stream));
@@ -1180,6 +1192,7 @@ extern "C" int amk_batch_energy(amk_ctx* c, int time_centre, amk_energy_out* out
   if (!c->batch) return fail(AMK_ERR_STATE, "no batch: call amk_batch_set first");
   AMK_CUDA_TRY(cudaSetDevice(c->device));
   Batch& B = *c->batch;
+  B.on(c->stream);
   const int ni = B.n_inst;
   int rc = AMK_OK;
   double* part = slot<double>(c, kSlotAuxState3, 3 * static_cast<size_t>(ni) + 8, &rc);

@@ -3093,6 +3093,8 @@ int fmm_run(amk_ctx* c, const View& v, int order, double theta, long leaf_capaci
   int* level_count = arrived + 2 * nn;
   int* family = slot<int>(c, kSlotFmmFamily, nn, &rc);
   AMK_TRY(rc);
+  // an evaluation that failed after its launches may still count arrivals on `up`
+  AMK_CUDA_TRY(cudaStreamWaitEvent(c->stream, f->up_done, 0));
   AMK_CUDA_TRY(cudaMemsetAsync(arrived, 0, (2 * static_cast<size_t>(nn) + 64) * sizeof(int), c->stream));
   fmm_radius_kernel<<<static_cast<unsigned>((8 * nn + 255) / 256), 256, 0, c->stream>>>(t, radius, arrived,
                                                                                         level_count);
