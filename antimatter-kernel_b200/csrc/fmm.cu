@@ -247,8 +247,8 @@ struct Fmm {
   // of the next chunk run on the context stream
   cudaStream_t side = nullptr;
   cudaEvent_t products_done[2] = {nullptr, nullptr}, sums_done[2] = {nullptr, nullptr};
-  // FP32 near field (tensor mode): its pair kernel runs on `near` after the
-  // last M2L products, concurrently with the per-target sums and L2L
+  // near field (both modes): its pair kernel runs on `near` after the last M2L
+  // products, concurrently with the per-target sums and L2L
   cudaStream_t near = nullptr;
   cudaEvent_t near_start = nullptr, near_done = nullptr;
   // P2M / M2M run on `up` concurrently with the traversal, which needs only
