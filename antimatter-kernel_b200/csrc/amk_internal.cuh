@@ -215,6 +215,7 @@ enum ScratchSlot {
   kSlotM2lClassKey,
   kSlotFmmArrived,
   kSlotFmmFamily,
+  kSlotBhArrived,
   kNumSlots
 };
 static_assert(kNumSlots <= 128, "scratch slots");
