@@ -33,8 +33,9 @@ constexpr double kMinSquaredDistance = 1e-30;
 // 1 / sqrt(x) for normal positive x: the hardware's double-precision estimate
 // (rsqrt.approx.ftz.f64, 20 bits) and one step of Householder's third-order
 // iteration, y + y e (1/2 + 3/8 e) with e = 1 - x y^2, whose error is 5/16 e^3:
-// within 2 ulp, five operations and no branch (rsqrt() checks its argument's
-// range). x = 0 gives NaN: callers select such pairs away.
+// within 2 ulp over the normal range (tests/test_gpu_rsqrt.py), five operations
+// and no branch (rsqrt() checks its argument's range). Zero and infinity give
+// NaN: callers select such pairs away.
 __device__ __forceinline__ double rsqrt_f64(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));

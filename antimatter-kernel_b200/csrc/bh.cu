@@ -167,11 +167,19 @@ __global__ void bh_record_kernel(const Octree t, const int* __restrict__ n_child
   if (x == 0) put(0, t.n_nodes - 1);
 }
 
+// 1 / r of a pair, 0 below the minimum distance and where r^2 overflowed (a
+// finite particle some 1e154 m away: its pull rounds to nothing, and
+// rsqrt_f64 has no value for infinity). The test reads r^2's upper word, an
+// integer comparison beside the FP64 ones.
+__device__ __forceinline__ double inverse_distance(double d2, bool skip) {
+  return skip || d2 < kMinSquaredDistance || __double2hiint(d2) >= 0x7ff00000 ? 0.0 : rsqrt_f64(d2);
+}
+
 // AddPointCharge, barnes-hut.cc:20-28, without the factor k q_t:
-// f += r q_s / r^3; pairs closer than the minimum distance (and `skip`) add 0.
+// f += r q_s / r^3; pairs without an inverse distance (and `skip`) add 0.
 __device__ __forceinline__ void add_point(double rx, double ry, double rz, double d2, double sq, bool skip,
                                           double* f) {
-  const double inv = skip || d2 < kMinSquaredDistance ? 0.0 : rsqrt_f64(d2);
+  const double inv = inverse_distance(d2, skip);
   const double w = sq * (inv * inv * inv);
   f[0] += rx * w;
   f[1] += ry * w;
@@ -179,7 +187,7 @@ __device__ __forceinline__ void add_point(double rx, double ry, double rz, doubl
 }
 
 __device__ __forceinline__ void add_phi(double d2, double sq, bool skip, double* phi) {
-  *phi += sq * (skip || d2 < kMinSquaredDistance ? 0.0 : rsqrt_f64(d2));
+  *phi += sq * inverse_distance(d2, skip);
 }
 
 // Leaf sums in FP32 (the tensor precision mode): sources as double-float
