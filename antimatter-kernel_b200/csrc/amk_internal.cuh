@@ -258,6 +258,7 @@ struct amk_ctx {
   long aux_capacity = 0;
 
   amk::Scratch scratch;
+  long scratch_moves = 0;  // scratch slots moved so far: an address from before it changed is stale
   amk::DevBuf host_status;  // pinned host word for small readbacks (unused)
 
   // energy time-centring (EnergyHistory, energy_analysis.h:23-28)
@@ -306,7 +307,9 @@ inline int check_launch(amk_ctx* c, const char* what) {
 
 template <typename T>
 inline T* slot(amk_ctx* c, int s, size_t count, int* rc) {
+  const void* before = c->scratch.b[s].ptr;
   *rc = c->scratch.b[s].reserve(count * sizeof(T));
+  if (c->scratch.b[s].ptr != before) ++c->scratch_moves;
   return c->scratch.b[s].as<T>();
 }
 

@@ -607,7 +607,12 @@ struct Batch {
   unsigned long long max_contacts = 0;  // largest contact count seen by a synchronised step
   int grid = 0;
   uint64_t step = 0;  // host mirror of the device step counter
-  bool warm = false;  // one uncaptured step done (scratch reserved)
+  // The context's scratch_moves after the last uncaptured step (which reserves
+  // the scratch of a step: nothing is allocated inside a capture) and at the
+  // capture. The sorts and scans of a step and the cutoff solver work in scratch
+  // slots that any other call on the context may grow, so a capture made before
+  // the last move is not replayed: a plain step and a new capture come first.
+  long warm_moves = -1, graph_moves = -1;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   int graph_steps = 0;
@@ -976,16 +981,16 @@ extern "C" int amk_batch_step(amk_ctx* c, int nsteps, int graph_chunk, int seria
   bool graphed = false;
   while (done < nsteps) {
     const bool stagger = !c->staggered;
-    if (!use_graph || !B.warm || stagger || nsteps - done < graph_chunk) {
+    if (!use_graph || B.warm_moves != c->scratch_moves || stagger || nsteps - done < graph_chunk) {
       AMK_TRY(serial ? serial_step_once(c, B, stagger) : batch_step_once(c, B, stagger, true));
       c->staggered = true;
-      B.warm = true;
+      if (!serial) B.warm_moves = c->scratch_moves;
       B.step++;
       c->step++;
       ++done;
       continue;
     }
-    if (!B.exec || B.graph_steps != graph_chunk) {
+    if (!B.exec || B.graph_steps != graph_chunk || B.graph_moves != c->scratch_moves) {
       B.drop_graph();
       // head room over the largest contact count seen so far: inside the
       // graph an overflow can only be recorded
@@ -1006,6 +1011,7 @@ extern "C" int amk_batch_step(amk_ctx* c, int nsteps, int graph_chunk, int seria
       B.graph = g;
       AMK_CUDA_TRY(cudaGraphInstantiate(&B.exec, B.graph, 0));
       B.graph_steps = graph_chunk;
+      B.graph_moves = c->scratch_moves;
     }
     if (!graphed) AMK_CUDA_TRY(cudaMemsetAsync(B.call_overflow(), 0, sizeof(unsigned long long), c->stream));
     graphed = true;
