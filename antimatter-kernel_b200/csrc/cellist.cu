@@ -389,7 +389,10 @@ grid_setup_kernel(View v, const uint8_t* __restrict__ species, double radius, lo
     g.o[d] = isfinite(lo) ? lo : 0.0;
     fin = fin && ext[d] >= 0.0 && isfinite(ext[d]);
   }
-  double cs = radius * (1.0 + 1e-9);
+  // At most 2^21 cells along an axis: a cell coordinate is computed to 2^-52 of
+  // itself, so two of them err by less than the 1e-9 that a cell is wider than
+  // the radius, and partners are never two cells apart.
+  double cs = fmax(radius * (1.0 + 1e-9), fmax(ext[0], fmax(ext[1], ext[2])) / kCellMax);
   double cells = INFINITY, dim[3] = {1.0, 1.0, 1.0};
   for (int it = 0; fin && it < 256; ++it) {  // cells no smaller than the radius, at most cell_cap of them
     for (int d = 0; d < 3; ++d) dim[d] = floor(ext[d] / cs) + 1.0;
