@@ -13,11 +13,13 @@
 // decisions are bit-identical to a scalar FP64 evaluation.
 //
 // Up to kBruteMax particles every pair is tested (one launch, no list). Above
-// it the particles are binned into a dense grid over their bounding box:
-// cells no smaller than the radius and at most 4 per particle, x fastest, so
-// that the 27 neighbour cells of a particle are nine contiguous runs of the
-// sorted records. A counting sort builds it (count, scan, scatter; the
-// members of a cell ordered by particle index, so sums have a fixed order).
+// it the particles are binned into cells no smaller than the radius: a dense
+// grid over their bounding box, x fastest, so that the 27 neighbour cells of a
+// particle are nine contiguous runs of the sorted records, or, where the box is
+// too large for that (a sparse cloud, particles far from the others), hashed
+// cells. A counting sort with four counters per particle builds either (count,
+// scan, scatter; a counter's members ordered by particle index, so sums have a
+// fixed order).
 // The allocation-free solver keeps its Morton-sorted keys: its static scratch
 // has no room for the grid's counters.
 #include <algorithm>
@@ -347,18 +349,62 @@ contact_brute_kernel(View v, const uint8_t* __restrict__ species, const uint32_t
   }
 }
 
-// ---------------------------------------------------------------- dense grid
+// ---------------------------------------------------------------- cells
+// Dense: the cells of the box, x fastest. Hashed: cells of twice the radius,
+// blocks of 4 x 4 x 4 of them hashed onto the same counters (a block's cells
+// side by side), so that cells cost nothing where no particle is and their
+// width does not depend on the box.
 struct CellGrid {
   double o[3], inv_cs;
   int dim[3];
   int species;  // bit s: a live particle of species s
+  int hashed;
 };
 
 constexpr long kGridCellsPer = 4;          // cells per particle at most
 constexpr long kGridCellsMax = 1L << 25;
 inline long grid_cell_cap(long n) { return std::min(kGridCellsMax, std::max(4096L, kGridCellsPer * n)); }
 
-// Box of the particles that take part; the last block turns it into the grid.
+// Cutoff (species null): live charged particles. Contacts: live particles
+// whose partner species is alive.
+__device__ __forceinline__ bool takes_part(const View& v, const uint8_t* __restrict__ species, int alive_species,
+                                           long i) {
+  if (!usable(v, i)) return false;
+  if (!species) return v.q[i] != 0.0;
+  return has_partner(species[i]) && ((alive_species >> partner_of(species[i])) & 1);
+}
+
+__device__ __forceinline__ void grid_cell(const CellGrid& g, double x, double y, double z, int c[3]) {
+  const double p[3] = {x, y, z};
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+    c[d] = max(0, static_cast<int>(fmin(floor((p[d] - g.o[d]) * g.inv_cs), static_cast<double>(g.dim[d] - 1))));
+}
+
+__device__ __forceinline__ int cell_entry(const CellGrid& g, int n_cells, int x, int y, int z) {
+  if (!g.hashed) return (z * g.dim[1] + y) * g.dim[0] + x;
+  const uint64_t block = static_cast<uint64_t>(x >> 2) | (static_cast<uint64_t>(y >> 2) << 21) |
+                         (static_cast<uint64_t>(z >> 2) << 42);
+  const uint32_t h = static_cast<uint32_t>((block * 0x9E3779B97F4A7C15ull) >> 32);  // Fibonacci hashing
+  const uint32_t b = __umulhi(h, static_cast<uint32_t>(n_cells) >> 6);
+  return static_cast<int>((b << 6) | ((z & 3) << 4) | ((y & 3) << 2) | (x & 3));
+}
+
+// Tells the 27 cells around a particle apart (hashed cells share counters).
+__device__ __forceinline__ int cell_tag(int x, int y, int z) { return ((z & 3) << 4) | ((y & 3) << 2) | (x & 3); }
+
+// Hashed cells are this many radii wide, and taken where the dense ones would be
+// wider. us per cutoff evaluation of a ball, dense / hashed: 100,003 particles
+// with 0.02, 0.1, 0.25, 0.6 and 12 neighbours inside the radius 68/65, 68/67,
+// 68/69, 68/73, 90/156 (the dense cells are 2 radii wide at 0.25), 1,000,003
+// 251/227, 253/239, 255/254, 258/275, 385/822. Cells of 1, 1.5 and 3 radii: 83,
+// 77 and 65 at 0.02, 128, 169 and 323 at 12. With a dense grid alone one
+// particle 0.01 m away from 100,003 within 2e-4 m took a step from 223 to
+// 17,600 us, and one 1 m away from a million one of 735 us to 2.4 s; now 295
+// and 1,133 us.
+constexpr double kHashWidth = 2.0;
+
+// Box of the usable particles; the last block turns it into the grid.
 // bb: six box words, the species mask (~0 preset: complemented bits are
 // cleared) and the count of finished blocks (preset ~0).
 __global__ void __launch_bounds__(kBboxThreads)
@@ -392,7 +438,8 @@ grid_setup_kernel(View v, const uint8_t* __restrict__ species, double radius, lo
   // At most 2^21 cells along an axis: a cell coordinate is computed to 2^-52 of
   // itself, so two of them err by less than the 1e-9 that a cell is wider than
   // the radius, and partners are never two cells apart.
-  double cs = fmax(radius * (1.0 + 1e-9), fmax(ext[0], fmax(ext[1], ext[2])) / kCellMax);
+  const double finest = fmax(radius * (1.0 + 1e-9), fmax(ext[0], fmax(ext[1], ext[2])) / kCellMax);
+  double cs = finest;
   double cells = INFINITY, dim[3] = {1.0, 1.0, 1.0};
   for (int it = 0; fin && it < 256; ++it) {  // cells no smaller than the radius, at most cell_cap of them
     for (int d = 0; d < 3; ++d) dim[d] = floor(ext[d] / cs) + 1.0;
@@ -401,36 +448,25 @@ grid_setup_kernel(View v, const uint8_t* __restrict__ species, double radius, lo
     cs *= fmax(1.05, fmin(cbrt(cells / static_cast<double>(cell_cap)), 1e6));
   }
   const bool ok = fin && cells <= static_cast<double>(cell_cap);
-  g.inv_cs = ok ? 1.0 / cs : 0.0;
-  for (int d = 0; d < 3; ++d) g.dim[d] = ok ? static_cast<int>(dim[d]) : 1;
+  g.hashed = fin && !(cs <= kHashWidth * finest);
+  if (g.hashed) cs = kHashWidth * finest;
+  g.inv_cs = ok || g.hashed ? 1.0 / cs : 0.0;
+  for (int d = 0; d < 3; ++d) g.dim[d] = g.hashed ? 1 << kCellBits : ok ? static_cast<int>(dim[d]) : 1;
   g.species = static_cast<int>(~vb[6] & 0xffull);
   *grid = g;
 }
 
-__device__ __forceinline__ void grid_cell(const CellGrid& g, double x, double y, double z, int c[3]) {
-  const double p[3] = {x, y, z};
-#pragma unroll
-  for (int d = 0; d < 3; ++d)
-    c[d] = max(0, static_cast<int>(fmin(floor((p[d] - g.o[d]) * g.inv_cs), static_cast<double>(g.dim[d] - 1))));
-}
-
-// cell[i] = cell of particle i, -1 when it takes no part; rank[i] = a place
-// among the cell's members. Cutoff (species null): live charged particles;
-// the others get their zero force here. Contacts: live particles whose
-// partner species is alive.
+// cell[i] = counter of particle i's cell, -1 when it takes no part; rank[i] = a
+// place among the counter's members. Cutoff: the particles that take no part
+// get their zero force here.
 template <bool kEnergy>
 __global__ void grid_count_kernel(View v, const uint8_t* __restrict__ species, const CellGrid* __restrict__ grid,
-                                  int* __restrict__ cell, int* __restrict__ rank, int* __restrict__ count,
+                                  int n_cells, int* __restrict__ cell, int* __restrict__ rank, int* __restrict__ count,
                                   double* __restrict__ epart) {
   const long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
   if (i >= v.n) return;
   const CellGrid g = *grid;
-  bool part = usable(v, i);
-  if (species)
-    part = part && has_partner(species[i]) && ((g.species >> partner_of(species[i])) & 1);
-  else
-    part = part && v.q[i] != 0.0;
-  if (!part) {
+  if (!takes_part(v, species, g.species, i)) {
     cell[i] = -1;
     if (!species) {
       const double f[3] = {0.0, 0.0, 0.0};
@@ -440,7 +476,7 @@ __global__ void grid_count_kernel(View v, const uint8_t* __restrict__ species, c
   }
   int c[3];
   grid_cell(g, v.x[i], v.y[i], v.z[i], c);
-  const int id = (c[2] * g.dim[1] + c[1]) * g.dim[0] + c[0];
+  const int id = cell_entry(g, n_cells, c[0], c[1], c[2]);
   cell[i] = id;
   rank[i] = atomicAdd(&count[id], 1);
 }
@@ -451,11 +487,14 @@ __global__ void grid_scatter_kernel(long n, const int* __restrict__ cell, const 
   if (i < n && cell[i] >= 0) member[start[cell[i]] + rank[i]] = static_cast<int>(i);
 }
 
-// The records in cell order, a cell's members in ascending particle index:
-// position and charge (cutoff) or position and {id, species} (contacts).
+// The records in cell order, a counter's members in ascending particle index:
+// position and charge (cutoff) or position and {id, species} (contacts); the
+// tags of hashed cells.
 __global__ void grid_record_kernel(View v, const uint8_t* __restrict__ species, const uint32_t* __restrict__ ids,
-                                   const int* __restrict__ cell, const int* __restrict__ start, const int* __restrict__ m,
-                                   const int* __restrict__ member, double4* __restrict__ rec, int* __restrict__ index) {
+                                   const CellGrid* __restrict__ grid, const int* __restrict__ cell,
+                                   const int* __restrict__ start, const int* __restrict__ m,
+                                   const int* __restrict__ member, double4* __restrict__ rec, int* __restrict__ index,
+                                   int* __restrict__ tag) {
   const long p = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
   if (p >= *m) return;
   const int i = member[p], b = start[cell[i]], e = start[cell[i] + 1];
@@ -464,68 +503,92 @@ __global__ void grid_record_kernel(View v, const uint8_t* __restrict__ species, 
   const double w = species ? __longlong_as_double(static_cast<long long>(
                                  (static_cast<unsigned long long>(ids[i]) << 8) | species[i]))
                            : v.q[i];
-  rec[b + r] = make_double4(v.x[i], v.y[i], v.z[i], w);
+  const double x = v.x[i], y = v.y[i], z = v.z[i];
+  rec[b + r] = make_double4(x, y, z, w);
   index[b + r] = i;
+  if (grid->hashed) {
+    int c[3];
+    grid_cell(*grid, x, y, z, c);
+    tag[b + r] = cell_tag(c[0], c[1], c[2]);
+  }
 }
 
-// Calls f(first, last) for the nine runs of records of the neighbour cells.
+// Calls f(k) for the records k of the 27 cells around a position: nine runs of
+// the dense cells; of the hashed ones those that the sphere of the radius
+// touches.
 template <typename F>
-__device__ __forceinline__ void neighbour_runs(const CellGrid& g, const int* __restrict__ start, double x, double y,
-                                               double z, F f) {
-  int c[3];
+__device__ __forceinline__ void neighbours(const CellGrid& g, int n_cells, const int* __restrict__ start,
+                                           const int* __restrict__ tag, double radius, double x, double y, double z,
+                                           F f) {
+  int c[3], lo[3], hi[3];
   grid_cell(g, x, y, z, c);
-  const int x0 = max(c[0] - 1, 0), x1 = min(c[0] + 1, g.dim[0] - 1);
-  for (int cz = max(c[2] - 1, 0); cz <= min(c[2] + 1, g.dim[2] - 1); ++cz)
-    for (int cy = max(c[1] - 1, 0); cy <= min(c[1] + 1, g.dim[1] - 1); ++cy) {
-      const int row = (cz * g.dim[1] + cy) * g.dim[0];
-      f(start[row + x0], start[row + x1 + 1]);
-    }
+  if (!g.hashed) {
+    const int x0 = max(c[0] - 1, 0), x1 = min(c[0] + 1, g.dim[0] - 1);
+    for (int cz = max(c[2] - 1, 0); cz <= min(c[2] + 1, g.dim[2] - 1); ++cz)
+      for (int cy = max(c[1] - 1, 0); cy <= min(c[1] + 1, g.dim[1] - 1); ++cy) {
+        const int row = (cz * g.dim[1] + cy) * g.dim[0];
+        const int end = start[row + x1 + 1];
+        for (int k = start[row + x0]; k < end; ++k) f(k);
+      }
+    return;
+  }
+  // a partner's coordinates differ by less than this (rounding of the
+  // differences, of the squares and of the bounds included)
+  const double r = radius * (1.0 + 1e-9);
+  const double ex = r + 4.5e-16 * fabs(x), ey = r + 4.5e-16 * fabs(y), ez = r + 4.5e-16 * fabs(z);
+  grid_cell(g, x - ex, y - ey, z - ez, lo);
+  grid_cell(g, x + ex, y + ey, z + ez, hi);
+  for (int cz = max(lo[2], c[2] - 1); cz <= min(hi[2], c[2] + 1); ++cz)
+    for (int cy = max(lo[1], c[1] - 1); cy <= min(hi[1], c[1] + 1); ++cy)
+      for (int cx = max(lo[0], c[0] - 1); cx <= min(hi[0], c[0] + 1); ++cx) {
+        const int id = cell_entry(g, n_cells, cx, cy, cz), want = cell_tag(cx, cy, cz);
+        const int end = start[id + 1];
+        for (int k = start[id]; k < end; ++k)
+          if (tag[k] == want) f(k);
+      }
 }
 
 template <bool kEnergy>
 __global__ void __launch_bounds__(128)
-cutoff_grid_kernel(View v, const CellGrid* __restrict__ grid, double rc, const int* __restrict__ start,
-                   const int* __restrict__ m, const double4* __restrict__ rec, const int* __restrict__ index,
+cutoff_grid_kernel(View v, const CellGrid* __restrict__ grid, int n_cells, double rc, const int* __restrict__ start,
+                   const int* __restrict__ tag, const double4* __restrict__ rec, const int* __restrict__ index,
                    double* __restrict__ epart) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= *m) return;
+  if (p >= start[n_cells]) return;
   const double4 me = rec[p];
   const double rc2 = rc * rc, inv_rc = 1.0 / rc;
   double f[3] = {0.0, 0.0, 0.0}, e = 0.0;
-  neighbour_runs(*grid, start, me.x, me.y, me.z, [&](int b, int end) {
-    for (int k = b; k < end; ++k) {
-      const double4 s = rec[k];
-      if (k != p) cutoff_pair<kEnergy>(me.x - s.x, me.y - s.y, me.z - s.z, s.w, rc2, inv_rc, f, e);
-    }
+  neighbours(*grid, n_cells, start, tag, rc, me.x, me.y, me.z, [&](int k) {
+    const double4 s = rec[k];
+    if (k != p) cutoff_pair<kEnergy>(me.x - s.x, me.y - s.y, me.z - s.z, s.w, rc2, inv_rc, f, e);
   });
   cutoff_store<kEnergy>(v, index[p], me.w, f, e, epart);
 }
 
 __global__ void __launch_bounds__(128)
-contact_grid_kernel(const CellGrid* __restrict__ grid, ContactRule R, const int* __restrict__ start,
-                    const int* __restrict__ m, const double4* __restrict__ rec, const int* __restrict__ index,
-                    Contact* __restrict__ out, unsigned long long* count, long cap) {
+contact_grid_kernel(const CellGrid* __restrict__ grid, int n_cells, double radius, ContactRule R,
+                    const int* __restrict__ start, const int* __restrict__ tag, const double4* __restrict__ rec,
+                    const int* __restrict__ index, Contact* __restrict__ out, unsigned long long* count, long cap) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= *m) return;
+  if (p >= start[n_cells]) return;
   const double4 me = rec[p];
-  const unsigned long long tag = static_cast<unsigned long long>(__double_as_longlong(me.w));
-  const unsigned want = static_cast<unsigned>(partner_of(static_cast<int>(tag & 0xff)));
-  neighbour_runs(*grid, start, me.x, me.y, me.z, [&](int b, int end) {
-    for (int k = b; k < end; ++k) {
-      const double4 s = rec[k];
-      const unsigned long long st = static_cast<unsigned long long>(__double_as_longlong(s.w));
-      if ((st & 0xff) != want) continue;
-      contact_pair(R, dist2_exact(me.x - s.x, me.y - s.y, me.z - s.z), static_cast<uint32_t>(index[p]),
-                   static_cast<uint32_t>(index[k]), static_cast<uint32_t>(tag >> 8), static_cast<uint32_t>(st >> 8),
-                   out, count, cap);
-    }
+  const unsigned long long own = static_cast<unsigned long long>(__double_as_longlong(me.w));
+  const unsigned want = static_cast<unsigned>(partner_of(static_cast<int>(own & 0xff)));
+  neighbours(*grid, n_cells, start, tag, radius, me.x, me.y, me.z, [&](int k) {
+    const double4 s = rec[k];
+    const unsigned long long st = static_cast<unsigned long long>(__double_as_longlong(s.w));
+    if ((st & 0xff) != want) return;
+    contact_pair(R, dist2_exact(me.x - s.x, me.y - s.y, me.z - s.z), static_cast<uint32_t>(index[p]),
+                 static_cast<uint32_t>(index[k]), static_cast<uint32_t>(own >> 8), static_cast<uint32_t>(st >> 8),
+                 out, count, cap);
   });
 }
 
 struct CellList {
   CellGrid* grid;
+  int n_cells;
   int* start;      // per cell, and the member count after the last one
-  int* m;          // = start + cells
+  int* tag;
   double4* rec;
   int* index;
 };
@@ -540,7 +603,7 @@ int build_cell_list(amk_ctx* c, const View& v, double radius, const uint8_t* spe
   CellGrid* grid = reinterpret_cast<CellGrid*>(bb + 8);
   int* cell = slot<int>(c, kSlotKeysA, 2 * static_cast<size_t>(n), &rc);
   AMK_TRY(rc);
-  int* rank = cell + n;
+  int* rank = cell + n;  // once the members are placed: the records' tags
   int* start = slot<int>(c, kSlotKeysB, static_cast<size_t>(cells) + 1, &rc);
   AMK_TRY(rc);
   int* member = slot<int>(c, kSlotValsA, static_cast<size_t>(n), &rc);
@@ -549,6 +612,7 @@ int build_cell_list(amk_ctx* c, const View& v, double radius, const uint8_t* spe
   AMK_TRY(rc);
   double4* rec = slot<double4>(c, kSlotSorted1, static_cast<size_t>(n), &rc);
   AMK_TRY(rc);
+  const int n_cells = static_cast<int>(cells);
   const unsigned gn = static_cast<unsigned>((n + 255) / 256);
   AMK_TRY(phase_begin(c, AMK_PHASE_SORT));
   AMK_CUDA_TRY(cudaMemsetAsync(bb, 0xFF, 8 * sizeof(unsigned long long), c->stream));
@@ -556,19 +620,21 @@ int build_cell_list(amk_ctx* c, const View& v, double radius, const uint8_t* spe
   grid_setup_kernel<<<bbox_grid(n), kBboxThreads, 0, c->stream>>>(v, species, radius, cells, bb, grid);
   AMK_TRY(check_launch(c, "grid_setup_kernel"));
   if (epart)
-    grid_count_kernel<true><<<gn, 256, 0, c->stream>>>(v, species, grid, cell, rank, start, epart);
+    grid_count_kernel<true><<<gn, 256, 0, c->stream>>>(v, species, grid, n_cells, cell, rank, start, epart);
   else
-    grid_count_kernel<false><<<gn, 256, 0, c->stream>>>(v, species, grid, cell, rank, start, nullptr);
+    grid_count_kernel<false><<<gn, 256, 0, c->stream>>>(v, species, grid, n_cells, cell, rank, start, nullptr);
   AMK_TRY(check_launch(c, "grid_count_kernel"));
   AMK_TRY(exclusive_scan_int(c, start, cells, start, start + cells));
   grid_scatter_kernel<<<gn, 256, 0, c->stream>>>(n, cell, rank, start, member);
   AMK_TRY(check_launch(c, "grid_scatter_kernel"));
-  grid_record_kernel<<<gn, 256, 0, c->stream>>>(v, species, ids, cell, start, start + cells, member, rec, index);
+  grid_record_kernel<<<gn, 256, 0, c->stream>>>(v, species, ids, grid, cell, start, start + cells, member, rec, index,
+                                                rank);
   AMK_TRY(check_launch(c, "grid_record_kernel"));
   AMK_TRY(phase_end(c, AMK_PHASE_SORT));
   out->grid = grid;
+  out->n_cells = n_cells;
   out->start = start;
-  out->m = start + cells;
+  out->tag = rank;
   out->rec = rec;
   out->index = index;
   return AMK_OK;
@@ -605,11 +671,11 @@ int cutoff_forces(amk_ctx* c, const View& v, double cutoff, double* energy_out) 
     AMK_TRY(phase_begin(c, AMK_PHASE_CUTOFF));
     const unsigned grid = static_cast<unsigned>((n + 127) / 128);
     if (epart)
-      cutoff_grid_kernel<true><<<grid, 128, 0, c->stream>>>(v, cl.grid, cutoff, cl.start, cl.m, cl.rec, cl.index,
-                                                            epart);
+      cutoff_grid_kernel<true><<<grid, 128, 0, c->stream>>>(v, cl.grid, cl.n_cells, cutoff, cl.start, cl.tag, cl.rec,
+                                                            cl.index, epart);
     else
-      cutoff_grid_kernel<false><<<grid, 128, 0, c->stream>>>(v, cl.grid, cutoff, cl.start, cl.m, cl.rec, cl.index,
-                                                             nullptr);
+      cutoff_grid_kernel<false><<<grid, 128, 0, c->stream>>>(v, cl.grid, cl.n_cells, cutoff, cl.start, cl.tag, cl.rec,
+                                                             cl.index, nullptr);
     AMK_TRY(check_launch(c, "cutoff_grid_kernel"));
     AMK_TRY(phase_end(c, AMK_PHASE_CUTOFF));
   }
@@ -691,7 +757,7 @@ int annihilate_view(amk_ctx* c, const View& v, const uint8_t* species, const uin
           v, species, ids, R, edges, words, cap, nullptr, nullptr, nullptr);
     else
       contact_grid_kernel<<<static_cast<unsigned>((v.n + 127) / 128), 128, 0, c->stream>>>(
-          cl.grid, R, cl.start, cl.m, cl.rec, cl.index, edges, words, cap);
+          cl.grid, cl.n_cells, radius, R, cl.start, cl.tag, cl.rec, cl.index, edges, words, cap);
     AMK_TRY(check_launch(c, "contact kernel"));
     unsigned long long m = 0;
     AMK_CUDA_TRY(cudaMemcpyAsync(&m, words, sizeof(m), cudaMemcpyDeviceToHost, c->stream));

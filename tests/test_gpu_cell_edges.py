@@ -23,7 +23,7 @@ def test_pair_near_the_radius_in_a_thin_cloud(sim, low, a, b):
     assert 0.0 < b - a < RC and np.floor((b - low) * inv) - np.floor((a - low) * inv) >= 2.0
     n = 1 << 22
     x = np.linspace(low, 15.9, n)  # 3.8 radii apart
-    x[0] = low
+    x[0], x[1] = low, 16.0  # the pair is inside the cloud
     x[-2:] = a, b
     o = np.zeros(n)
     fx, fy, fz = sim.solve_cutoff(x, o, o, np.full(n, E), RC)
