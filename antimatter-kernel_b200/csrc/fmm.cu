@@ -3053,7 +3053,8 @@ struct FmmRun {
   int* p2p_count = nullptr;   // per node: P2P source leaves
 };
 
-int fmm_run(amk_ctx* c, const View& v, int order, double theta, long leaf_capacity, bool want_phi, FmmRun* run) {
+static int fmm_evaluate(amk_ctx* c, const View& v, int order, double theta, long leaf_capacity, bool want_phi,
+                        FmmRun* run) {
   run->t = Octree{};
   const long n = v.n;
   if (n == 0) return AMK_OK;
@@ -3093,8 +3094,6 @@ int fmm_run(amk_ctx* c, const View& v, int order, double theta, long leaf_capaci
   int* level_count = arrived + 2 * nn;
   int* family = slot<int>(c, kSlotFmmFamily, nn, &rc);
   AMK_TRY(rc);
-  // an evaluation that failed after its launches may still count arrivals on `up`
-  AMK_CUDA_TRY(cudaStreamWaitEvent(c->stream, f->up_done, 0));
   AMK_CUDA_TRY(cudaMemsetAsync(arrived, 0, (2 * static_cast<size_t>(nn) + 64) * sizeof(int), c->stream));
   fmm_radius_kernel<<<static_cast<unsigned>((8 * nn + 255) / 256), 256, 0, c->stream>>>(t, radius, arrived,
                                                                                         level_count);
@@ -3314,6 +3313,7 @@ int fmm_run(amk_ctx* c, const View& v, int order, double theta, long leaf_capaci
   } else {
     AMK_TRY(launch_near());
   }
+  if (getenv("AMK_FMM_FAIL")) return fail(AMK_ERR_STATE, "AMK_FMM_FAIL is set");  // tests of a failed evaluation
   AMK_TRY(phase_end(c, AMK_PHASE_FMM_M2L));
 
   // ---- L2L
@@ -3354,6 +3354,18 @@ int fmm_run(amk_ctx* c, const View& v, int order, double theta, long leaf_capaci
   run->ef = ef;
   run->p2p_count = gp.count;
   return AMK_OK;
+}
+
+// One evaluation. Its upward pass, per-target sums and near field run on
+// streams of their own, which the context stream joins only where all went
+// well; they read the tree, the lists and the staging of the context's scratch,
+// which the next call rewrites. So an evaluation that fails waits for them.
+int fmm_run(amk_ctx* c, const View& v, int order, double theta, long leaf_capacity, bool want_phi, FmmRun* run) {
+  const int rc = fmm_evaluate(c, v, order, theta, leaf_capacity, want_phi, run);
+  if (rc != AMK_OK && c->fmm)
+    for (cudaStream_t s : {c->fmm->up, c->fmm->side, c->fmm->near})
+      if (s) cudaStreamSynchronize(s);
+  return rc;
 }
 
 int fmm_apply_learned(amk_ctx* c, const FmmRun& r);  // below
