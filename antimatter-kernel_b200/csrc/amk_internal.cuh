@@ -245,7 +245,6 @@ struct amk_ctx {
   long capacity = 0;
   // particle state (device)
   amk::DevBuf x, y, z, vx, vy, vz, fx, fy, fz, q, m, species, alive, ids;
-  amk::DevBuf hq, lo;  // staged positions of the batched all-pairs kernel
   double length_scale = 1.0;
   bool staggered = false;     // first push done (lorentz.h:34)
   long step = 0;              // completed steps

@@ -599,7 +599,7 @@ struct Batch {
   bool any_annihilation = false;
   bool graphable = true;
   DevBuf inst, inst_of, units, counters, contacts, best, flags, keys, vals, skeys;
-  DevBuf perm, rel, boxes;  // all-pairs order, tile offsets, tile boxes
+  DevBuf perm, hq, lo, rel, boxes;  // all-pairs: order, staged positions, tile offsets, tile boxes
   DevBuf cell_at, cell_count, cell_first, cell_rec;  // annihilation: hashed cells
   int cell_bits = 0;
   long n_units = 0;
@@ -633,8 +633,9 @@ struct Batch {
   // now and then 30 to 90 ms, beside 12 steps of 2.4 ms.
   void take_buffers(Batch& o) {
     for (auto m : {&Batch::inst, &Batch::inst_of, &Batch::units, &Batch::counters, &Batch::contacts, &Batch::best,
-                   &Batch::flags, &Batch::keys, &Batch::vals, &Batch::skeys, &Batch::perm, &Batch::rel, &Batch::boxes,
-                   &Batch::cell_at, &Batch::cell_count, &Batch::cell_first, &Batch::cell_rec, &Batch::extent})
+                   &Batch::flags, &Batch::keys, &Batch::vals, &Batch::skeys, &Batch::perm, &Batch::hq, &Batch::lo,
+                   &Batch::rel, &Batch::boxes, &Batch::cell_at, &Batch::cell_count, &Batch::cell_first,
+                   &Batch::cell_rec, &Batch::extent})
       (this->*m).swap(o.*m);
   }
   ~Batch() {
@@ -777,14 +778,14 @@ int batch_coulomb(amk_ctx* c, Batch& B) {
                              B.perm.as<uint32_t>(), n, kInstBits + 30));
     batch_tile_stage_kernel<<<static_cast<unsigned>(B.n_units), kBUnit, 0, c->stream>>>(
         B.units.as<int2>(), B.inst.as<InstanceDev>(), B.perm.as<uint32_t>(), c->x.as<double>(), c->y.as<double>(),
-        c->z.as<double>(), c->q.as<double>(), c->alive.as<uint8_t>(), c->hq.as<float4>(), c->lo.as<float4>(),
+        c->z.as<double>(), c->q.as<double>(), c->alive.as<uint8_t>(), B.hq.as<float4>(), B.lo.as<float4>(),
         B.rel.as<float4>(), B.boxes.as<TileBox>());
     AMK_TRY(check_launch(c, "batch_tile_stage_kernel"));
     AMK_TRY(phase_end(c, AMK_PHASE_STAGE));
     AMK_TRY(phase_begin(c, AMK_PHASE_ALLPAIRS));
     batch_allpairs_kernel<<<B.grid, kBT, 0, c->stream>>>(
-        B.units.as<int2>(), static_cast<int>(B.n_units), B.inst.as<InstanceDev>(), c->hq.as<float4>(),
-        c->lo.as<float4>(), B.rel.as<float4>(), B.boxes.as<TileBox>(), B.perm.as<uint32_t>(), c->q.as<double>(),
+        B.units.as<int2>(), static_cast<int>(B.n_units), B.inst.as<InstanceDev>(), B.hq.as<float4>(),
+        B.lo.as<float4>(), B.rel.as<float4>(), B.boxes.as<TileBox>(), B.perm.as<uint32_t>(), c->q.as<double>(),
         c->fx.as<double>(), c->fy.as<double>(), c->fz.as<double>(), B.queue());
     AMK_TRY(check_launch(c, "batch_allpairs_kernel"));
     AMK_TRY(phase_end(c, AMK_PHASE_ALLPAIRS));
@@ -951,7 +952,8 @@ extern "C" int amk_batch_set(amk_ctx* c, int n_inst, const amk_params* params, c
     AMK_TRY(B->cell_count.reserve(entries * sizeof(int)));
     AMK_TRY(B->cell_first.reserve((entries + 1) * sizeof(int)));
   }
-  AMK_TRY(B->rel.reserve(nn * sizeof(float4)));
+  if (B->n_units > 0)
+    for (DevBuf* b : {&B->hq, &B->lo, &B->rel}) AMK_TRY(b->reserve(nn * sizeof(float4)));
   AMK_TRY(B->boxes.reserve(static_cast<size_t>(std::max<long>(n_tiles, 1)) * sizeof(TileBox)));
   AMK_CUDA_TRY(cudaMemcpyAsync(B->inst.ptr, inst.data(), n_inst * sizeof(InstanceDev), cudaMemcpyHostToDevice,
                                c->stream));

@@ -340,8 +340,6 @@ static int ensure_capacity(amk_ctx* c, long n) {
   const size_t nd = static_cast<size_t>(n) * sizeof(double);
   for (amk::DevBuf* b : {&c->x, &c->y, &c->z, &c->vx, &c->vy, &c->vz, &c->fx, &c->fy, &c->fz, &c->q, &c->m})
     AMK_TRY(b->reserve(nd));
-  AMK_TRY(c->hq.reserve(static_cast<size_t>(n) * sizeof(float4)));
-  AMK_TRY(c->lo.reserve(static_cast<size_t>(n) * sizeof(float4)));
   AMK_TRY(c->species.reserve(static_cast<size_t>(n)));
   AMK_TRY(c->alive.reserve(static_cast<size_t>(n)));
   AMK_TRY(c->ids.reserve(static_cast<size_t>(n) * sizeof(uint32_t)));
