@@ -190,13 +190,11 @@ enum ScratchSlot {
   kSlotFmmWork0,
   kSlotFmmWork1,
   kSlotFmmWork2,
-  kSlotFmmWork3,
   kSlotFmmWork4,
   kSlotFmmWork5,
   kSlotP2PWork,
   kSlotP2PPart,
   kSlotP2PStage,
-  kSlotM2lCodes,
   kSlotM2lTarget,
   kSlotM2lHist,
   kSlotM2lStart,
@@ -212,7 +210,6 @@ enum ScratchSlot {
   kSlotM2lRefl,
   kSlotFmmNodeRec,
   kSlotFmmCell,
-  kSlotM2lRank,
   kSlotM2lClassKey,
   kSlotFmmArrived,
   kSlotFmmFamily,

@@ -233,11 +233,15 @@ struct FmmDevTables {
 };
 
 struct FmmLists {
-  DevBuf cur, next, m2l, p2p;
-  DevBuf m2l_rank, p2p_rank;  // a pair's place among its target's pairs
+  DevBuf cur, next;
+  DevBuf m2l, p2p;  // pairs, then (list_ranks) each pair's place among its target's pairs
   // list lengths the last traversal needed (the next one reserves them)
   long need_front = 0, need_m2l = 0, need_p2p = 0;
 };
+
+constexpr size_t kListEntry = sizeof(int2) + sizeof(int);
+inline long list_cap(const DevBuf& b) { return static_cast<long>(b.bytes / kListEntry); }
+inline int* list_ranks(const DevBuf& b) { return reinterpret_cast<int*>(b.as<int2>() + list_cap(b)); }
 
 struct Fmm {
   std::map<int, std::pair<DevBuf*, FmmDevTables>> tables;
@@ -2177,14 +2181,14 @@ int m2l_products(amk_ctx* c, int order, const Octree& t, const FmmDevTables& T, 
   const int row = tc ? T.n_m : T.n_rp;  // coefficients of a cell's and of a pair's row
   double* Mh = slot<double>(c, kSlotFmmWork5, static_cast<size_t>(nn) * row, &rc);
   AMK_TRY(rc);
-  int* codes = slot<int>(c, kSlotM2lCodes, n_m2l, &rc);
+  // the lists are grouped: their scatter scratch and ranks are free again
+  int* codes = slot<int>(c, kSlotFmmWork1, n_m2l, &rc);
   AMK_TRY(rc);
+  int* rank = list_ranks(c->fmm->lists.m2l);
   const int* tgt = gm.tgt;
   int* hist = slot<int>(c, kSlotM2lHist, n_codes + 1, &rc);
   AMK_TRY(rc);
   int* start = slot<int>(c, kSlotM2lStart, n_codes + 1, &rc);
-  AMK_TRY(rc);
-  int* rank = slot<int>(c, kSlotM2lRank, n_m2l, &rc);
   AMK_TRY(rc);
   int* counters = slot<int>(c, kSlotM2lCounters, 8, &rc);  // pairs, classes, units, fallback pairs
   AMK_TRY(rc);
@@ -3159,8 +3163,6 @@ static int fmm_evaluate(amk_ctx* c, const View& v, int order, double theta, long
       lists.next.release();
       lists.m2l.release();
       lists.p2p.release();
-      lists.m2l_rank.release();
-      lists.p2p_rank.release();
       want_front = want_m2l = want_p2p = v;
     }
   }
@@ -3168,20 +3170,18 @@ static int fmm_evaluate(amk_ctx* c, const View& v, int order, double theta, long
     if (attempt > 12) return fail(AMK_ERR_LIMIT, "FMM traversal: interaction lists did not fit");
     AMK_TRY(lists.cur.reserve(static_cast<size_t>(want_front) * sizeof(int2)));
     AMK_TRY(lists.next.reserve(static_cast<size_t>(want_front) * sizeof(int2)));
-    AMK_TRY(lists.m2l.reserve(static_cast<size_t>(want_m2l) * sizeof(int2)));
-    AMK_TRY(lists.p2p.reserve(static_cast<size_t>(want_p2p) * sizeof(int2)));
-    AMK_TRY(lists.m2l_rank.reserve(static_cast<size_t>(want_m2l) * sizeof(int)));
-    AMK_TRY(lists.p2p_rank.reserve(static_cast<size_t>(want_p2p) * sizeof(int)));
+    AMK_TRY(lists.m2l.reserve(static_cast<size_t>(want_m2l) * kListEntry));
+    AMK_TRY(lists.p2p.reserve(static_cast<size_t>(want_p2p) * kListEntry));
     TraverseLists tl;
     tl.m2l = lists.m2l.as<int2>();
     tl.p2p = lists.p2p.as<int2>();
-    tl.m2l_rank = lists.m2l_rank.as<int>();
-    tl.p2p_rank = lists.p2p_rank.as<int>();
+    tl.m2l_rank = list_ranks(lists.m2l);
+    tl.p2p_rank = list_ranks(lists.p2p);
     tl.m2l_count = gm.count;
     tl.p2p_count = gp.count;
     tl.cap_front = static_cast<long>(std::min(lists.cur.bytes, lists.next.bytes) / sizeof(int2));
-    tl.cap_m2l = static_cast<long>(std::min(lists.m2l.bytes / sizeof(int2), lists.m2l_rank.bytes / sizeof(int)));
-    tl.cap_p2p = static_cast<long>(std::min(lists.p2p.bytes / sizeof(int2), lists.p2p_rank.bytes / sizeof(int)));
+    tl.cap_m2l = list_cap(lists.m2l);
+    tl.cap_p2p = list_cap(lists.p2p);
     AMK_CUDA_TRY(cudaMemsetAsync(counts, 0, 2 * static_cast<size_t>(nn) * sizeof(int), c->stream));
     AMK_CUDA_TRY(cudaMemsetAsync(tv, 0, n_tv * sizeof(int), c->stream));
     fmm_traverse_root_kernel<<<1, 32, 0, c->stream>>>(lists.cur.as<int2>(), tv + 8);
@@ -3203,7 +3203,7 @@ static int fmm_evaluate(amk_ctx* c, const View& v, int order, double theta, long
     AMK_TRY(group_pairs(c, tl.m2l, tl.m2l_rank, tv, tl.cap_m2l, nn, kSlotFmmLists0, kSlotFmmWork0, kSlotFmmWork1,
                         kSlotM2lTarget, &gm));
     AMK_TRY(group_pairs(c, tl.p2p, tl.p2p_rank, tv + 1, tl.cap_p2p, nn, kSlotFmmLists2, kSlotFmmWork2,
-                        kSlotFmmWork3, -1, &gp));
+                        kSlotFmmWork1, -1, &gp));
     // near-field work items: a target leaf and up to kP2PChunk source leaves
     // of its list (kP2P32Chunk in the FP32 near field)
     p2p_items_count_kernel<<<gn, 256, 0, c->stream>>>(t, gp.count, f32 ? kP2P32Chunk : kP2PChunk, items, psize);
