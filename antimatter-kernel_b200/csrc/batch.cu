@@ -417,12 +417,13 @@ __device__ __forceinline__ bool has_partner(int s) {
 // Annihilation cells: a cell's key is the instance id above 10 bits per axis.
 // Cells are clamped to the instance's grid, which is monotonic in the
 // position, so a particle outside the grid is still found. Particles are
-// counted into a table of hashed cells (at least two entries per particle),
-// the counts scanned, and each particle's position, index and key with its
-// species written to its cell's entries, so that a candidate that is not of the
-// partner species of the cell costs one 8-byte read. A 39-bit radix sort of the
-// keys and 27 binary searches per particle took 96 + 220 us per step (96
-// instances, 482k particles); the table 42 us and the search of it 73 us.
+// counted into a table of hashed cells (two to four entries per particle, at
+// most 2^24: fewer above 8.4 million particles), the counts scanned, and each
+// particle's position, index and key with its species written to its cell's
+// entries, so that a candidate that is not of the partner species of the cell
+// costs one 8-byte read. A 39-bit radix sort of the keys and 27 binary searches
+// per particle took 96 + 220 us per step (96 instances, 482k particles); the
+// table 42 us and the search of it 73 us.
 constexpr uint32_t kNoCell = ~0u;
 
 __device__ __forceinline__ uint64_t batch_cell_key(uint64_t prefix, uint32_t cx, uint32_t cy, uint32_t cz) {

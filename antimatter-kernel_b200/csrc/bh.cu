@@ -2,8 +2,8 @@
 //
 // Monopoles (barnes-hut.cc:76-159): every node keeps the positive charge sum
 // and the |negative| charge sum with their charge centres; leaves sum their
-// particles, internal nodes merge their children in octant order, level by
-// level from the deepest.
+// particles, internal nodes merge their children in octant order (one launch:
+// the thread whose child arrives last at a node merges it).
 //
 // Walk (barnes-hut.cc:183-269): a warp takes 32 consecutive targets in tree
 // order and walks one shared stack of nodes to open. Each entry carries the

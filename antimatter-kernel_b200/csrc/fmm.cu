@@ -8,22 +8,27 @@
 // leaf capacity 32, theta acceptance (r_T + r_S)^2 < theta^2 d^2.
 //
 // GPU mapping:
-//   radii, P2M      leaves in parallel (a thread per leaf / a warp per leaf)
-//   M2M, L2L        level-synchronous, a warp per node, lanes over coefficients
+//   radii           one launch from the leaves to the root: eight lanes per
+//                   leaf, the group whose child arrives last at a parent goes
+//                   on with the parent
+//   P2M, M2M        likewise in one launch, a warp per leaf and then per parent,
+//                   on a stream of its own beside the traversal
 //   lists           the reference's dual-tree recursion run breadth-first over
 //                   (target, source) pairs; each target's M2L and P2P sources
 //                   are sorted, so every sum has a fixed order (run-to-run
 //                   deterministic)
-//   M2L             a warp per target cell; per source the derivative tensor
-//                   is built degree by degree in shared memory (lanes over the
-//                   multi-indices of one degree) and contracted with the
-//                   source's multipole, lanes over local coefficients
+//   M2L             pairs grouped into displacement classes, one dense product
+//                   per class on the tensor cores (per-pair derivatives for the
+//                   few others), a block per target for the sums
+//   L2L             a launch per depth, a warp per parent
 //   P2P, L2P        work items of (target leaf, a chunk of its source
 //                   leaves); a warp per item with lanes split into groups over
-//                   the sources; partials added in a fixed order, L2P a thread
-//                   per particle
-// Arithmetic is FP64 throughout, as in the reference; inverse distances use
-// rsqrt (the reference divides by sqrt), a difference of an ulp.
+//                   the sources, on a stream of its own beside the M2L sums;
+//                   partials added in a fixed order, L2P a thread per particle
+// Arithmetic is FP64, as in the reference; inverse distances are reciprocal
+// square roots (the reference divides by sqrt), a difference of an ulp. In the
+// tensor precision mode the M2L products run in split BF16 with FP32
+// accumulation and the near field in FP32 on double-float differences.
 #include <algorithm>
 #include <array>
 #include <functional>
@@ -970,10 +975,11 @@ struct Grouped {
 // a pair contributes Lh(t) += A_{v,dd} Mh(s) with the n_m x n_m matrix
 //     A_{v,dd}[g][a] = 1/g! (h_t/u)^{|g|+1} (h_s/u)^{|a|} D_{g+a}(v),
 // which depends only on the class (v, dd = d_t - d_s): h_t/u and h_s/u are
-// powers of two. Pairs are sorted by class and each class is one FP64
+// powers of two. Pairs are grouped by class and each class is one FP64
 // product A (n_m x n_m) x [Mh of its sources] (n_m x k), in tiles of 64
-// pairs, up to 8 tiles of one class per block. The products are written per pair and summed per target in the
-// pairs' (target, source) order, so the result is run-to-run deterministic.
+// pairs, up to 8 tiles of one class per block. The products are written per
+// pair and summed per target in the pairs' (target, source) order, so the
+// result is run-to-run deterministic.
 // A class is found through an open-addressing hash of (d_t - d_s, v) with
 // bounded probing; pairs beyond the class reach or left without a hash slot
 // take a per-pair path with the derivative recurrence.
@@ -1282,7 +1288,7 @@ __device__ __forceinline__ void cp_async_wait() {
 // n_m doubles per pair written and read back.
 //
 // A block covers 8 * kGb >= n_r rows and a tile of 64 pairs; each of its
-// warps owns all the rows of 8 * kWc pairs. Per unit (up to 256 pairs of one
+// warps owns all the rows of 8 * kWc pairs. Per unit (up to 512 pairs of one
 // class) the block gathers A once, from the class's D(v) through the index
 // map and with the source factor, into shared memory in fragment order (one
 // conflict-free 8-byte read per lane and fragment; gathered anew by every
