@@ -366,6 +366,7 @@ struct Octree {
   long n_nodes = 0;
   int leaf_cap = 8;
   int max_depth = 0;           // deepest node
+  bool wide = false;           // squared distances may overflow
   TreeFrame* frame = nullptr;  // device
   uint32_t* order = nullptr;   // sorted position -> view index
   uint64_t* keys = nullptr;    // sorted keys

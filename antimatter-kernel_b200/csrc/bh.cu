@@ -167,27 +167,30 @@ __global__ void bh_record_kernel(const Octree t, const int* __restrict__ n_child
   if (x == 0) put(0, t.n_nodes - 1);
 }
 
-// 1 / r of a pair, 0 below the minimum distance and where r^2 overflowed (a
-// finite particle some 1e154 m away: its pull rounds to nothing, and
-// rsqrt_f64 has no value for infinity). The test reads r^2's upper word, an
-// integer comparison beside the FP64 ones.
+// 1 / r of a pair, 0 below the minimum distance and (kWide: a root cube of more
+// than 1e150 m) where r^2 overflowed: the pull of a finite particle that far
+// away rounds to nothing, and rsqrt_f64 has no value for infinity. The second
+// test costs the walk 0.8 %, so other trees go without it.
+template <bool kWide>
 __device__ __forceinline__ double inverse_distance(double d2, bool skip) {
-  return skip || d2 < kMinSquaredDistance || __double2hiint(d2) >= 0x7ff00000 ? 0.0 : rsqrt_f64(d2);
+  return skip || d2 < kMinSquaredDistance || (kWide && isinf(d2)) ? 0.0 : rsqrt_f64(d2);
 }
 
 // AddPointCharge, barnes-hut.cc:20-28, without the factor k q_t:
 // f += r q_s / r^3; pairs without an inverse distance (and `skip`) add 0.
+template <bool kWide>
 __device__ __forceinline__ void add_point(double rx, double ry, double rz, double d2, double sq, bool skip,
                                           double* f) {
-  const double inv = inverse_distance(d2, skip);
+  const double inv = inverse_distance<kWide>(d2, skip);
   const double w = sq * (inv * inv * inv);
   f[0] += rx * w;
   f[1] += ry * w;
   f[2] += rz * w;
 }
 
+template <bool kWide>
 __device__ __forceinline__ void add_phi(double d2, double sq, bool skip, double* phi) {
-  *phi += sq * inverse_distance(d2, skip);
+  *phi += sq * inverse_distance<kWide>(d2, skip);
 }
 
 // Leaf sums in FP32 (the tensor precision mode): sources as double-float
@@ -212,7 +215,7 @@ __global__ void bh_stage_kernel(const Octree t, double qs, float4* __restrict__ 
   lo[k] = make_float4(static_cast<float>(s.x - hx), static_cast<float>(s.y - hy), static_cast<float>(s.z - hz), 0.f);
 }
 
-template <bool kPhi, bool kF32>
+template <bool kPhi, bool kF32, bool kWide>
 __global__ void __launch_bounds__(32 * kWalkWarps)
 bh_walk_kernel(const Octree t, const BhRec* __restrict__ rec, double theta2, BhF32 f32, double* __restrict__ out,
                int* __restrict__ status) {
@@ -295,9 +298,9 @@ bh_walk_kernel(const Octree t, const BhRec* __restrict__ rec, double theta2, BhF
             const double rx = me.x - s.x, ry = me.y - s.y, rz = me.z - s.z;
             const double d2 = dot_rn(rx, ry, rz);
             if (kPhi)
-              add_phi(d2, s.w, j == k, &phi);
+              add_phi<kWide>(d2, s.w, j == k, &phi);
             else
-              add_point(rx, ry, rz, d2, s.w, j == k, f);
+              add_point<kWide>(rx, ry, rz, d2, s.w, j == k, f);
           }
         }
         continue;
@@ -314,18 +317,18 @@ bh_walk_kernel(const Octree t, const BhRec* __restrict__ rec, double theta2, BhF
           const double rx = me.x - pq.x, ry = me.y - pq.y, rz = me.z - pq.z;
           const double r2 = dot_rn(rx, ry, rz);
           if (kPhi)
-            add_phi(r2, pw, false, &phi);
+            add_phi<kWide>(r2, pw, false, &phi);
           else
-            add_point(rx, ry, rz, r2, pw, false, f);
+            add_point<kWide>(rx, ry, rz, r2, pw, false, f);
         }
         if (nw > 0.0) {
           const double4 nq = child[o].neg;
           const double rx = me.x - nq.x, ry = me.y - nq.y, rz = me.z - nq.z;
           const double r2 = dot_rn(rx, ry, rz);
           if (kPhi)
-            add_phi(r2, -nw, false, &phi);
+            add_phi<kWide>(r2, -nw, false, &phi);
           else
-            add_point(rx, ry, rz, r2, -nw, false, f);
+            add_point<kWide>(rx, ry, rz, r2, -nw, false, f);
         }
       }
       const unsigned open = mask & ~acc;
@@ -443,17 +446,19 @@ int barnes_hut_forces(amk_ctx* c, const View& v, double theta, long leaf_capacit
     fs.lo = stage + t.m;
   }
   AMK_TRY(phase_begin(c, AMK_PHASE_BH_WALK));
+  auto walk = [&](auto kernel, double* out) -> int {
+    kernel<<<blocks, 32 * kWalkWarps, 0, c->stream>>>(t, rec, theta2, fs, out, status);
+    return check_launch(c, "bh_walk_kernel");
+  };
   if (f32)
-    bh_walk_kernel<false, true><<<blocks, 32 * kWalkWarps, 0, c->stream>>>(t, rec, theta2, fs, fo, status);
+    AMK_TRY(walk(t.wide ? bh_walk_kernel<false, true, true> : bh_walk_kernel<false, true, false>, fo));
   else
-    bh_walk_kernel<false, false><<<blocks, 32 * kWalkWarps, 0, c->stream>>>(t, rec, theta2, fs, fo, status);
-  AMK_TRY(check_launch(c, "bh_walk_kernel"));
+    AMK_TRY(walk(t.wide ? bh_walk_kernel<false, false, true> : bh_walk_kernel<false, false, false>, fo));
   if (po) {
     if (f32)
-      bh_walk_kernel<true, true><<<blocks, 32 * kWalkWarps, 0, c->stream>>>(t, rec, theta2, fs, po, status);
+      AMK_TRY(walk(t.wide ? bh_walk_kernel<true, true, true> : bh_walk_kernel<true, true, false>, po));
     else
-      bh_walk_kernel<true, false><<<blocks, 32 * kWalkWarps, 0, c->stream>>>(t, rec, theta2, fs, po, status);
-    AMK_TRY(check_launch(c, "bh_walk_kernel"));
+      AMK_TRY(walk(t.wide ? bh_walk_kernel<true, false, true> : bh_walk_kernel<true, false, false>, po));
   }
   AMK_TRY(phase_end(c, AMK_PHASE_BH_WALK));
   bh_scatter_kernel<<<static_cast<unsigned>((t.m + 255) / 256), 256, 0, c->stream>>>(t, fo, po, v);

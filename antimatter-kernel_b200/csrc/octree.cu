@@ -44,7 +44,8 @@ __global__ void __launch_bounds__(kBboxThreads) tree_bbox_kernel(View v, int mod
 }
 
 // Root cube: barnes-hut.cc:46-61 (Barnes-Hut) / fast-multipole.cc:355-397.
-__global__ void tree_root_kernel(const unsigned long long* bb, int mode, TreeFrame* f) {
+// *wide: squared distances inside the cube may overflow.
+__global__ void tree_root_kernel(const unsigned long long* bb, int mode, TreeFrame* f, int* wide) {
   const double low[3] = {double_from_order_bits(bb[0]), double_from_order_bits(bb[1]),
                          double_from_order_bits(bb[2])};
   const double high[3] = {-double_from_order_bits(bb[3]), -double_from_order_bits(bb[4]),
@@ -69,6 +70,7 @@ __global__ void tree_root_kernel(const unsigned long long* bb, int mode, TreeFra
     t.root_h = 0.5 * (1.0 + 1e-9);
   }
   *f = t;
+  *wide = t.root_h > 1e150;
 }
 
 __device__ __forceinline__ void tree_coords(const TreeFrame& f, int mode, double x, double y, double z, double* p) {
@@ -315,7 +317,7 @@ int build_octree(amk_ctx* c, const View& v, int leaf_cap, int mode, Octree* t) {
   AMK_CUDA_TRY(cudaMemsetAsync(bb, 0xFF, 6 * sizeof(unsigned long long), c->stream));
   tree_bbox_kernel<<<bbox_grid(n), kBboxThreads, 0, c->stream>>>(v, mode, bb);
   AMK_TRY(check_launch(c, "tree_bbox_kernel"));
-  tree_root_kernel<<<1, 1, 0, c->stream>>>(bb, mode, frame);
+  tree_root_kernel<<<1, 1, 0, c->stream>>>(bb, mode, frame, small + 3);
   AMK_TRY(check_launch(c, "tree_root_kernel"));
   tree_key_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, c->stream>>>(v, mode, frame, keys, vals);
   AMK_TRY(check_launch(c, "tree_key_kernel"));
@@ -347,12 +349,13 @@ int build_octree(amk_ctx* c, const View& v, int leaf_cap, int mode, Octree* t) {
   tree_leafdepth_kernel<<<gm, kLeafThreads, 0, c->stream>>>(skeys, m, std::min(t->leaf_cap, m), L, ld, cnt, small + 2);
   AMK_TRY(check_launch(c, "tree_leafdepth_kernel"));
   AMK_TRY(exclusive_scan_int(c, cnt, m, base, small + 1));
-  int hs[2] = {0, 0};
-  AMK_CUDA_TRY(cudaMemcpyAsync(hs, small + 1, 2 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  int hs[3] = {0, 0, 0};
+  AMK_CUDA_TRY(cudaMemcpyAsync(hs, small + 1, 3 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   AMK_CUDA_TRY(cudaStreamSynchronize(c->stream));
   const int nn = hs[0];
   t->n_nodes = nn;
   t->max_depth = hs[1];
+  t->wide = hs[2] != 0;
 
   t->center = slot<double4>(c, kSlotTreeCenter, nn, &rc);
   AMK_TRY(rc);
