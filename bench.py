@@ -1216,12 +1216,13 @@ def run_kernels(args):
                               "unit": "165 B per particle-step: x, v read + written (96), F read + zeroed (48), "
                                       "q, m (16), id (4), alive (1)"}
         ms, per = phase_ms(sim, lambda: sim.annihilate(), "annihilation", args.steps)
-        bytes_ = (24.0 + 2 + 12 + 32 * 8 + 24 * 27 / 8) * n
-        out["annihilation (cell list, contact_kernel, matching)"] = {
+        bytes_ = (2 * 26.0 + 16 + 8 + 4 + 72 + 80) * n
+        out["annihilation (cell list, contact_grid_kernel, matching)"] = {
             "ms": ms, "algorithmic_bytes": bytes_, "achieved_gbs": bytes_ / (ms * 1e-3) / 1e9,
             "frac": bytes_ / (ms * 1e-3) / 1e9 / hbm,
-            "unit": "per particle: positions (24), species + alive (2), cell key + index written (12), 8 radix "
-                    "passes x 32 B, neighbour positions of the 27 cells read once per 8 particles (81)"}
+            "unit": "per particle: positions, species, alive read for the box and for the cells (52), cell and place "
+                    "written and read (16), member (8), id (4), record and index written and read (72), four "
+                    "counters cleared, counted and scanned (80)"}
     pos, vel, sp = tree_cloud(n)
     with amk.Simulation(tree_params(n, dict(coulomb_method="fast-multipole", fast_multipole_order=4,
                                             fast_multipole_theta=0.5)), device=local) as sim:
@@ -1240,7 +1241,7 @@ def run_kernels(args):
         tree_ms = ph["tree"][0] / max(ph["tree"][1], 1) - sort_ms  # the tree phase encloses the sort
         sb = 256.0 * n
         tb = 100.0 * n + 78.0 * nodes
-        out["radix sort (hist_kernel, scan, scatter_staged_kernel)"] = {
+        out["radix sort (tile_hist_kernel, scatter_staged_kernel)"] = {
             "ms": sort_ms, "algorithmic_bytes": sb, "achieved_gbs": sb / (sort_ms * 1e-3) / 1e9,
             "frac": sb / (sort_ms * 1e-3) / 1e9 / hbm,
             "unit": "256 B per key: 8 passes of 8 B key read (histogram) + 12 B read + 12 B written (scatter)"}
