@@ -351,7 +351,7 @@ contact_brute_kernel(View v, const uint8_t* __restrict__ species, const uint32_t
 
 // ---------------------------------------------------------------- cells
 // Dense: the cells of the box, x fastest. Hashed: cells of twice the radius,
-// blocks of 4 x 4 x 4 of them hashed onto the same counters (a block's cells
+// blocks of 16 x 16 x 16 of them hashed onto the same counters (a block's cells
 // side by side), so that cells cost nothing where no particle is and their
 // width does not depend on the box.
 struct CellGrid {
@@ -381,27 +381,29 @@ __device__ __forceinline__ void grid_cell(const CellGrid& g, double x, double y,
     c[d] = max(0, static_cast<int>(fmin(floor((p[d] - g.o[d]) * g.inv_cs), static_cast<double>(g.dim[d] - 1))));
 }
 
+constexpr int kBlockBits = 4, kBlockEdge = 1 << kBlockBits;
+
 __device__ __forceinline__ int cell_entry(const CellGrid& g, int n_cells, int x, int y, int z) {
   if (!g.hashed) return (z * g.dim[1] + y) * g.dim[0] + x;
-  const uint64_t block = static_cast<uint64_t>(x >> 2) | (static_cast<uint64_t>(y >> 2) << 21) |
-                         (static_cast<uint64_t>(z >> 2) << 42);
+  const uint64_t block = static_cast<uint64_t>(x >> kBlockBits) | (static_cast<uint64_t>(y >> kBlockBits) << 21) |
+                         (static_cast<uint64_t>(z >> kBlockBits) << 42);
   const uint32_t h = static_cast<uint32_t>((block * 0x9E3779B97F4A7C15ull) >> 32);  // Fibonacci hashing
-  const uint32_t b = __umulhi(h, static_cast<uint32_t>(n_cells) >> 6);
-  return static_cast<int>((b << 6) | ((z & 3) << 4) | ((y & 3) << 2) | (x & 3));
+  const uint32_t b = __umulhi(h, static_cast<uint32_t>(n_cells) >> (3 * kBlockBits));
+  constexpr int m = kBlockEdge - 1;
+  return static_cast<int>(((((b << kBlockBits) | (z & m)) << kBlockBits | (y & m)) << kBlockBits) | (x & m));
 }
-
-// Tells the 27 cells around a particle apart (hashed cells share counters).
-__device__ __forceinline__ int cell_tag(int x, int y, int z) { return ((z & 3) << 4) | ((y & 3) << 2) | (x & 3); }
 
 // Hashed cells are this many radii wide, and taken where the dense ones would be
 // wider. us per cutoff evaluation of a ball, dense / hashed: 100,003 particles
-// with 0.02, 0.1, 0.25, 0.6 and 12 neighbours inside the radius 68/65, 68/67,
-// 68/69, 68/73, 90/156 (the dense cells are 2 radii wide at 0.25), 1,000,003
-// 251/227, 253/239, 255/254, 258/275, 385/822. Cells of 1, 1.5 and 3 radii: 83,
-// 77 and 65 at 0.02, 128, 169 and 323 at 12. With a dense grid alone one
-// particle 0.01 m away from 100,003 within 2e-4 m took a step from 223 to
-// 17,600 us, and one 1 m away from a million one of 735 us to 2.4 s; now 295
-// and 1,133 us.
+// with 0.02, 0.1, 0.25, 0.5 and 12 neighbours inside the radius 67/60, 67/63,
+// 67/67, 67/73, 89/147 (the dense cells are 2 radii wide at 0.25), 1,000,003
+// 251/205, 252/212, 254/223, 256/238, 384/738. Cells of one radius: 259 at 0.02,
+// 461 at 12 (1,000,003). Blocks of 4^3 and 8^3 instead of 16^3: 216 and 210 at
+// 0.02, 782 and 766 at 12: a particle's neighbour cells lie closer together the
+// larger the blocks are.
+// With a dense grid alone one particle 0.01 m away from 100,003 within 2e-4 m took
+// a step from 223 to 17,600 us, and one 1 m away from a million one of 735 us to
+// 2.4 s; now 284 and 1,031.
 constexpr double kHashWidth = 2.0;
 
 // Box of the usable particles; the last block turns it into the grid.
@@ -488,13 +490,10 @@ __global__ void grid_scatter_kernel(long n, const int* __restrict__ cell, const 
 }
 
 // The records in cell order, a counter's members in ascending particle index:
-// position and charge (cutoff) or position and {id, species} (contacts); the
-// tags of hashed cells.
+// position and charge (cutoff) or position and {id, species} (contacts).
 __global__ void grid_record_kernel(View v, const uint8_t* __restrict__ species, const uint32_t* __restrict__ ids,
-                                   const CellGrid* __restrict__ grid, const int* __restrict__ cell,
-                                   const int* __restrict__ start, const int* __restrict__ m,
-                                   const int* __restrict__ member, double4* __restrict__ rec, int* __restrict__ index,
-                                   int* __restrict__ tag) {
+                                   const int* __restrict__ cell, const int* __restrict__ start, const int* __restrict__ m,
+                                   const int* __restrict__ member, double4* __restrict__ rec, int* __restrict__ index) {
   const long p = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
   if (p >= *m) return;
   const int i = member[p], b = start[cell[i]], e = start[cell[i] + 1];
@@ -503,24 +502,19 @@ __global__ void grid_record_kernel(View v, const uint8_t* __restrict__ species, 
   const double w = species ? __longlong_as_double(static_cast<long long>(
                                  (static_cast<unsigned long long>(ids[i]) << 8) | species[i]))
                            : v.q[i];
-  const double x = v.x[i], y = v.y[i], z = v.z[i];
-  rec[b + r] = make_double4(x, y, z, w);
+  rec[b + r] = make_double4(v.x[i], v.y[i], v.z[i], w);
   index[b + r] = i;
-  if (grid->hashed) {
-    int c[3];
-    grid_cell(*grid, x, y, z, c);
-    tag[b + r] = cell_tag(c[0], c[1], c[2]);
-  }
 }
 
 // Calls f(k) for the records k of the 27 cells around a position: nine runs of
 // the dense cells; of the hashed ones those that the sphere of the radius
-// touches.
+// touches, a block's cells of a row as one run. (Three cells in a row differ in
+// their place in a block, so no counter is read twice; the particles of other
+// blocks that share one are out of reach.)
 template <typename F>
-__device__ __forceinline__ void neighbours(const CellGrid& g, int n_cells, const int* __restrict__ start,
-                                           const int* __restrict__ tag, double radius, double x, double y, double z,
-                                           F f) {
-  int c[3], lo[3], hi[3];
+__device__ __forceinline__ void neighbours(const CellGrid& g, int n_cells, const int* __restrict__ start, double radius,
+                                           double x, double y, double z, F f) {
+  int c[3];
   grid_cell(g, x, y, z, c);
   if (!g.hashed) {
     const int x0 = max(c[0] - 1, 0), x1 = min(c[0] + 1, g.dim[0] - 1);
@@ -536,29 +530,34 @@ __device__ __forceinline__ void neighbours(const CellGrid& g, int n_cells, const
   // differences, of the squares and of the bounds included)
   const double r = radius * (1.0 + 1e-9);
   const double ex = r + 4.5e-16 * fabs(x), ey = r + 4.5e-16 * fabs(y), ez = r + 4.5e-16 * fabs(z);
+  int lo[3], hi[3];
   grid_cell(g, x - ex, y - ey, z - ez, lo);
   grid_cell(g, x + ex, y + ey, z + ez, hi);
-  for (int cz = max(lo[2], c[2] - 1); cz <= min(hi[2], c[2] + 1); ++cz)
-    for (int cy = max(lo[1], c[1] - 1); cy <= min(hi[1], c[1] + 1); ++cy)
-      for (int cx = max(lo[0], c[0] - 1); cx <= min(hi[0], c[0] + 1); ++cx) {
-        const int id = cell_entry(g, n_cells, cx, cy, cz), want = cell_tag(cx, cy, cz);
-        const int end = start[id + 1];
-        for (int k = start[id]; k < end; ++k)
-          if (tag[k] == want) f(k);
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    lo[d] = max(lo[d], c[d] - 1);
+    hi[d] = min(hi[d], c[d] + 1);
+  }
+  for (int cz = lo[2]; cz <= hi[2]; ++cz)
+    for (int cy = lo[1]; cy <= hi[1]; ++cy)
+      for (int cx = lo[0]; cx <= hi[0];) {
+        const int last = min(hi[0], cx | (kBlockEdge - 1));
+        const int id = cell_entry(g, n_cells, cx, cy, cz), end = start[id + last - cx + 1];
+        for (int k = start[id]; k < end; ++k) f(k);
+        cx = last + 1;
       }
 }
 
 template <bool kEnergy>
 __global__ void __launch_bounds__(128)
 cutoff_grid_kernel(View v, const CellGrid* __restrict__ grid, int n_cells, double rc, const int* __restrict__ start,
-                   const int* __restrict__ tag, const double4* __restrict__ rec, const int* __restrict__ index,
-                   double* __restrict__ epart) {
+                   const double4* __restrict__ rec, const int* __restrict__ index, double* __restrict__ epart) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= start[n_cells]) return;
   const double4 me = rec[p];
   const double rc2 = rc * rc, inv_rc = 1.0 / rc;
   double f[3] = {0.0, 0.0, 0.0}, e = 0.0;
-  neighbours(*grid, n_cells, start, tag, rc, me.x, me.y, me.z, [&](int k) {
+  neighbours(*grid, n_cells, start, rc, me.x, me.y, me.z, [&](int k) {
     const double4 s = rec[k];
     if (k != p) cutoff_pair<kEnergy>(me.x - s.x, me.y - s.y, me.z - s.z, s.w, rc2, inv_rc, f, e);
   });
@@ -567,14 +566,14 @@ cutoff_grid_kernel(View v, const CellGrid* __restrict__ grid, int n_cells, doubl
 
 __global__ void __launch_bounds__(128)
 contact_grid_kernel(const CellGrid* __restrict__ grid, int n_cells, double radius, ContactRule R,
-                    const int* __restrict__ start, const int* __restrict__ tag, const double4* __restrict__ rec,
-                    const int* __restrict__ index, Contact* __restrict__ out, unsigned long long* count, long cap) {
+                    const int* __restrict__ start, const double4* __restrict__ rec, const int* __restrict__ index,
+                    Contact* __restrict__ out, unsigned long long* count, long cap) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= start[n_cells]) return;
   const double4 me = rec[p];
   const unsigned long long own = static_cast<unsigned long long>(__double_as_longlong(me.w));
   const unsigned want = static_cast<unsigned>(partner_of(static_cast<int>(own & 0xff)));
-  neighbours(*grid, n_cells, start, tag, radius, me.x, me.y, me.z, [&](int k) {
+  neighbours(*grid, n_cells, start, radius, me.x, me.y, me.z, [&](int k) {
     const double4 s = rec[k];
     const unsigned long long st = static_cast<unsigned long long>(__double_as_longlong(s.w));
     if ((st & 0xff) != want) return;
@@ -588,7 +587,6 @@ struct CellList {
   CellGrid* grid;
   int n_cells;
   int* start;      // per cell, and the member count after the last one
-  int* tag;
   double4* rec;
   int* index;
 };
@@ -603,7 +601,7 @@ int build_cell_list(amk_ctx* c, const View& v, double radius, const uint8_t* spe
   CellGrid* grid = reinterpret_cast<CellGrid*>(bb + 8);
   int* cell = slot<int>(c, kSlotKeysA, 2 * static_cast<size_t>(n), &rc);
   AMK_TRY(rc);
-  int* rank = cell + n;  // once the members are placed: the records' tags
+  int* rank = cell + n;
   int* start = slot<int>(c, kSlotKeysB, static_cast<size_t>(cells) + 1, &rc);
   AMK_TRY(rc);
   int* member = slot<int>(c, kSlotValsA, static_cast<size_t>(n), &rc);
@@ -627,14 +625,12 @@ int build_cell_list(amk_ctx* c, const View& v, double radius, const uint8_t* spe
   AMK_TRY(exclusive_scan_int(c, start, cells, start, start + cells));
   grid_scatter_kernel<<<gn, 256, 0, c->stream>>>(n, cell, rank, start, member);
   AMK_TRY(check_launch(c, "grid_scatter_kernel"));
-  grid_record_kernel<<<gn, 256, 0, c->stream>>>(v, species, ids, grid, cell, start, start + cells, member, rec, index,
-                                                rank);
+  grid_record_kernel<<<gn, 256, 0, c->stream>>>(v, species, ids, cell, start, start + cells, member, rec, index);
   AMK_TRY(check_launch(c, "grid_record_kernel"));
   AMK_TRY(phase_end(c, AMK_PHASE_SORT));
   out->grid = grid;
   out->n_cells = n_cells;
   out->start = start;
-  out->tag = rank;
   out->rec = rec;
   out->index = index;
   return AMK_OK;
@@ -671,11 +667,11 @@ int cutoff_forces(amk_ctx* c, const View& v, double cutoff, double* energy_out) 
     AMK_TRY(phase_begin(c, AMK_PHASE_CUTOFF));
     const unsigned grid = static_cast<unsigned>((n + 127) / 128);
     if (epart)
-      cutoff_grid_kernel<true><<<grid, 128, 0, c->stream>>>(v, cl.grid, cl.n_cells, cutoff, cl.start, cl.tag, cl.rec,
-                                                            cl.index, epart);
+      cutoff_grid_kernel<true><<<grid, 128, 0, c->stream>>>(v, cl.grid, cl.n_cells, cutoff, cl.start, cl.rec, cl.index,
+                                                            epart);
     else
-      cutoff_grid_kernel<false><<<grid, 128, 0, c->stream>>>(v, cl.grid, cl.n_cells, cutoff, cl.start, cl.tag, cl.rec,
-                                                             cl.index, nullptr);
+      cutoff_grid_kernel<false><<<grid, 128, 0, c->stream>>>(v, cl.grid, cl.n_cells, cutoff, cl.start, cl.rec, cl.index,
+                                                             nullptr);
     AMK_TRY(check_launch(c, "cutoff_grid_kernel"));
     AMK_TRY(phase_end(c, AMK_PHASE_CUTOFF));
   }
@@ -757,7 +753,7 @@ int annihilate_view(amk_ctx* c, const View& v, const uint8_t* species, const uin
           v, species, ids, R, edges, words, cap, nullptr, nullptr, nullptr);
     else
       contact_grid_kernel<<<static_cast<unsigned>((v.n + 127) / 128), 128, 0, c->stream>>>(
-          cl.grid, cl.n_cells, radius, R, cl.start, cl.tag, cl.rec, cl.index, edges, words, cap);
+          cl.grid, cl.n_cells, radius, R, cl.start, cl.rec, cl.index, edges, words, cap);
     AMK_TRY(check_launch(c, "contact kernel"));
     unsigned long long m = 0;
     AMK_CUDA_TRY(cudaMemcpyAsync(&m, words, sizeof(m), cudaMemcpyDeviceToHost, c->stream));
