@@ -405,6 +405,7 @@ __device__ __forceinline__ int cell_entry(const CellGrid& g, int n_cells, int x,
 // a step from 223 to 17,600 us, and one 1 m away from a million one of 735 us to
 // 2.4 s; now 284 and 1,031.
 constexpr double kHashWidth = 2.0;
+static_assert(kBruteMax * kGridCellsPer >= 1L << (3 * kBlockBits), "a grid's counters hold a block");
 
 // Box of the usable particles; the last block turns it into the grid.
 // bb: six box words, the species mask (~0 preset: complemented bits are
